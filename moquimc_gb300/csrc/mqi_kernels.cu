@@ -333,7 +333,7 @@ score_step(Ctx& C, const Trk& t, uint32_t cnb, float rho, float vol) {
         float            vf = t.dE + t.ldE;
         if (s.type == MQI_SCORER_DOSE_W) {
             const float spr = t.spr0 >= 0.0f ? t.spr0 : spr_of(C.P->calib, rho, t.ke0, C.dbg);
-            vf              = (rho < 1.0e-7f) ? 0.0f : vf * 1.60218e-10f / (vol * rho * spr);
+            vf              = (rho < 1.0e-7f) ? 0.0f : div_guarded(vf * 1.60218e-10f, vol * rho * spr);
         }
         tally_add(s.tally, cnb, (double) vf, cnb > 0 && vf > 0.0f);
         return;
@@ -346,7 +346,7 @@ score_step(Ctx& C, const Trk& t, uint32_t cnb, float rho, float vol) {
         const ScorerDev& sd  = C.P->scorer[ch.scorer_begin];
         const ScorerDev& sp  = C.P->scorer[ch.scorer_begin + 1];
         const float      spr = t.spr0 >= 0.0f ? t.spr0 : spr_of(C.P->calib, rho, t.ke0, C.dbg);
-        const float dose_w = (rho < 1.0e-7f) ? 0.0f : (t.dE + t.ldE) * 1.60218e-10f / (vol * rho * spr);
+        const float dose_w = (rho < 1.0e-7f) ? 0.0f : div_guarded((t.dE + t.ldE) * 1.60218e-10f, vol * rho * spr);
         if (!(dose_w > 0.0f)) return;
         const double   v  = (double) dose_w;
         const uint64_t sc = (uint64_t) (C.spot >> kScenShift);
@@ -361,7 +361,7 @@ score_step(Ctx& C, const Trk& t, uint32_t cnb, float rho, float vol) {
     const float       spr = t.spr0 >= 0.0f ? t.spr0 : spr_of(P.calib, rho, t.ke0, C.dbg);
     // dose_to_water of the step, shared by the dose, dose^2 and Dij scorers (Dw_pointer,
     // mqi_scorer_energy_deposit.hpp:23-40): 0 in vacuum voxels
-    const float dose_w = (rho < 1.0e-7f) ? 0.0f : (t.dE + t.ldE) * 1.60218e-10f / (vol * rho * spr);
+    const float dose_w = (rho < 1.0e-7f) ? 0.0f : div_guarded((t.dE + t.ldE) * 1.60218e-10f, vol * rho * spr);
     for (int si = 0; si < ch.n_scorers; ++si) {
         const ScorerDev& s = P.scorer[ch.scorer_begin + si];
         bool     ok;
@@ -555,7 +555,7 @@ push_daughter(Ctx& C, Trk& t, float ke0, bool ke1_zero, float3 p, float3 d, floa
 /// range-table walk is guarded at index 0 (the reference's uint16 index wraps there).
 __device__ inline float
 energy_loss(const Tables& T, const Rel& rel, float rho, float len, float spr, float z) {
-    const float lw = len * spr * rho / kWaterDensity;
+    const float lw = div_by(len * spr * rho, kWaterDensity, kPerWaterDensity);
     int n = (int) ((rel.Ek - 0.1f) / 0.5f);
     if (n > MQI_TABLE_N - 2) n = MQI_TABLE_N - 2;
     if (n < 0) n = 0;
@@ -569,11 +569,12 @@ energy_loss(const Tables& T, const Rel& rel, float rho, float len, float spr, fl
     while (n > 0 && r < T.range[n]) --n;
     x0 = 0.1f + (float) n * 0.5f;
     x1 = x0 + 0.5f;
-    const float dE_mean = rel.Ek - intpl1d(r, T.range[n], T.range[n + 1], x0, x1);
+    // intpl1d: the range table increases strictly, so its x1 == x0 case cannot occur
+    const float dE_mean = rel.Ek - (x0 + div_rn((r - T.range[n]) * (x1 - x0), T.range[n + 1] - T.range[n]));
     const float Te      = (rel.Te_max >= kTeStragCap) ? kTeStragCap : rel.Te_max;
-    float       var     = dedx_term0() * rho / kWaterDensity * lw;
-    var *= Te / rel.beta_sq * (1.0f - 0.5f * rel.beta_sq);
-    float ret = z * sqrtf(var) + dE_mean;
+    float       var     = div_by(dedx_term0() * rho, kWaterDensity, kPerWaterDensity) * lw;
+    var *= div_rn(Te, rel.beta_sq) * (1.0f - 0.5f * rel.beta_sq);
+    float ret = z * sqrt_rn(var) + dE_mean;
     if (ret < 0.0f) ret = -ret;
     return ret;
 }
@@ -593,8 +594,10 @@ along_step(Ctx& C, Trk& t, const Rel& rel, float len, float rho, float spr, floa
     }
     const float P     = rel.momentum();
     const float X0    = x0_of(C.P->calib, rho, C.dbg);
-    const float th_sq = ((kEs / P) * (kEs / P) / rel.beta_sq) * len / X0;
-    float       th    = sqrtf(th_sq);
+    const float s     = div_rn(kEs, P);
+    const float th_n  = div_rn(s * s, rel.beta_sq) * len;
+    const float th_sq = C.P->calib.mode ? th_n / X0 : div_rn(th_n, X0);   // a user's X0 may lie anywhere
+    float       th    = sqrt_rn(th_sq);
     th                = z_mcs * (sqrtf(2.0f) * th);
     if (th < 0.0f) th = -th;
     const float phi = 2.0f * kPi * u_phi;
@@ -612,9 +615,8 @@ post_delta(Ctx& C, Trk& t, Rng& rng) {
     float     Te = 0.0f;
     for (int it = 0;; ++it) {
         const float n = rng.uniform();
-        Te            = C.tcut * rel.Te_max;
-        Te /= ((1.0f - n) * rel.Te_max + n * C.tcut);
-        if (rng.uniform() < 1.0f - rel.beta_sq * Te / rel.Te_max + Te * Te / (2.0f * rel.Et_sq)) break;
+        Te            = div_rn(C.tcut * rel.Te_max, (1.0f - n) * rel.Te_max + n * C.tcut);
+        if (rng.uniform() < 1.0f - div_rn(rel.beta_sq * Te, rel.Te_max) + div_rn(Te * Te, 2.0f * rel.Et_sq)) break;
         if (it >= 63) {   // acceptance >= 1 - beta^2 > 0: unreachable in practice, bounded anyway
             count_event(kCntErr);
             break;
@@ -778,7 +780,7 @@ stepping(Ctx& C, Trk& t, Rng& rng, float rho, float d2b) {
     const Rel   rel(t.ke0);
     const float spr      = spr_of(C.P->calib, rho, t.ke0, C.dbg);
     const float dedx     = dedx_lookup(T, rel.Ek);
-    const float cur_min  = kMaxStep * spr * rho / kWaterDensity;
+    const float cur_min  = div_by(kMaxStep * spr * rho, kWaterDensity, kPerWaterDensity);
     const float max_loss = -1.0f * cur_min * dedx;
     const CrossSections k1 = cross_sections(T, rel.Ek, rho);
     const CrossSections k2 = cross_sections(T, t.ke0 - max_loss, rho);
@@ -791,15 +793,16 @@ stepping(Ctx& C, Trk& t, Rng& rng, float rho, float d2b) {
     const float c2 = pick1 ? k1.poe : k2.poe;
     const float c3 = pick1 ? k1.poi : k2.poi;
     const float u_mfp      = rng.uniform();
-    const float mfp        = -1.0f * logf(u_mfp) / cs_sum;
-    const float step_limit = cur_min * kWaterDensity / (spr * rho);
+    // above the tables every cross section is 0 and the free path infinite
+    const float mfp        = cs_sum != 0.0f ? div_rn(-1.0f * logf(u_mfp), cs_sum) : __int_as_float(0x7f800000);
+    const float step_limit = div_guarded(cur_min * kWaterDensity, spr * rho);
     // Box-Muller pair and azimuth for along_step (words 1..3 of the step's first block)
     const float bm_u1 = rng.uniform();
     const float bm_u2 = rng.uniform();
     const float u_phi = rng.uniform();
     float       s_bm, c_bm;
     sincospif(2.0f * bm_u2, &s_bm, &c_bm);
-    const float bm_r  = sqrtf(-2.0f * logf(bm_u1));
+    const float bm_r  = sqrt_rn(-2.0f * logf(bm_u1));
     const float z1    = bm_r * c_bm;
     const float z2    = bm_r * s_bm;
     // The three branches of the reference (boundary, interaction, maximum step) differ only in the
