@@ -132,6 +132,7 @@ mqi_create(int device, mqi_ctx** out) {
         return cuda_fail(nullptr, e, "mqi_create: cudaStreamCreate");
     }
     c->own_stream = true;
+    static_assert(MQI_DENSITY_CORRECTION_N == kHuNodes, "one correction factor per HU value");
     const size_t tbytes = (6 * MQI_TABLE_N + MQI_DENSITY_CORRECTION_N) * sizeof(float);
     std::vector<float> host(6 * MQI_TABLE_N + MQI_DENSITY_CORRECTION_N);
     std::memcpy(&host[0 * MQI_TABLE_N], mqi_tab_cs_p_ion, sizeof(mqi_tab_cs_p_ion));
@@ -143,6 +144,7 @@ mqi_create(int device, mqi_ctx** out) {
     std::memcpy(&host[6 * MQI_TABLE_N], mqi_tab_density_correction, sizeof(mqi_tab_density_correction));
     if ((e = cudaMalloc(&c->tables, tbytes)) != cudaSuccess ||
         (e = cudaMemcpy(c->tables, host.data(), tbytes, cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = launch_hu_table(c->tables + 6 * MQI_TABLE_N, c->stream)) != cudaSuccess ||
         (e = cudaMalloc(&c->counters, 8 * sizeof(uint32_t))) != cudaSuccess ||
         (e = cudaMemset(c->counters, 0, 8 * sizeof(uint32_t))) != cudaSuccess ||
         (e = cudaMalloc(&c->stats, 8 * sizeof(unsigned long long))) != cudaSuccess ||
@@ -356,7 +358,7 @@ mqi_hu_to_density(mqi_ctx* c, const int16_t* hu, float* rho, uint64_t n, float s
     if (!valid_ctx(c) || (!hu && n) || (!rho && n)) return fail(c, MQI_ERR_INVALID, "mqi_hu_to_density: bad argument");
     DeviceGuard g(c->device);
     if (on_device) {
-        MQI_CUDA(c, launch_hu_to_density(c->tables + 6 * MQI_TABLE_N, hu, rho, n, scale, c->stream), "mqi_hu_to_density");
+        MQI_CUDA(c, launch_hu_to_density(c->tables + 6 * MQI_TABLE_N, hu, rho, n, scale, c->num_sms, c->stream), "mqi_hu_to_density");
         MQI_CUDA(c, cudaStreamSynchronize(c->stream), "mqi_hu_to_density");
         return MQI_OK;
     }
@@ -365,7 +367,7 @@ mqi_hu_to_density(mqi_ctx* c, const int16_t* hu, float* rho, uint64_t n, float s
     MQI_CUDA(c, cudaMalloc(&dh, n * sizeof(int16_t) + 16), "mqi_hu_to_density");
     cudaError_t e = cudaMalloc(&dr, n * sizeof(float) + 16);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dh, hu, n * sizeof(int16_t), cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = launch_hu_to_density(c->tables + 6 * MQI_TABLE_N, dh, dr, n, scale, c->stream);
+    if (e == cudaSuccess) e = launch_hu_to_density(c->tables + 6 * MQI_TABLE_N, dh, dr, n, scale, c->num_sms, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(rho, dr, n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     cudaFree(dh);
@@ -389,7 +391,7 @@ mqi_set_hu(mqi_ctx* c, int id, const int16_t* hu, float scale, int on_device) {
         if (e != cudaSuccess) { cudaFree(tmp); return cuda_fail(c, e, "mqi_set_hu"); }
         src = tmp;
     }
-    cudaError_t e = launch_hu_to_density(c->tables + 6 * MQI_TABLE_N, src, ch.rho, n, scale, c->stream);
+    cudaError_t e = launch_hu_to_density(c->tables + 6 * MQI_TABLE_N, src, ch.rho, n, scale, c->num_sms, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (tmp) cudaFree(tmp);
     if (e != cudaSuccess) return cuda_fail(c, e, "mqi_set_hu");

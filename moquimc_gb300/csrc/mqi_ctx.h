@@ -137,7 +137,7 @@ struct mqi_ctx {
     uint32_t*               counters = nullptr;     // [0,1] queue sizes, [2] head, [3] error flag, [4] deferred
     unsigned long long*     stats = nullptr;        // 8 x u64
     uint32_t*               host_counts = nullptr;  // pinned: 4 x u32
-    float*                  tables = nullptr;       // 6*600 physics + 3996 HU correction
+    float*                  tables = nullptr;       // 6*600 physics + 3996 HU densities
     mqi_gpu::CalibDev       calib{};                // SPR / X0 curves (mode 0: the defaults)
     float*                  calib_buf = nullptr;    // device: the tables of calib (SPR then X0)
     int                     num_sms = 0;

@@ -162,7 +162,7 @@ struct WaveParams {
     uint32_t*       n_def;      // device: entries in def (zeroed before each wave)
     int             smem_edge_floats; // shared-memory floats for staged child edges
     const float*    tables;     // device: the six physics tables, 6 x 600 floats in Tables order
-                                // (followed by the 3996 HU density-correction factors)
+                                // (a context's are followed by the density of each HU value)
     CalibDev        calib;      // SPR / X0 curves
 };
 
@@ -247,7 +247,11 @@ cudaError_t launch_sample_topup(const Queue& q, const TopUp* tu, const mqi_spot*
 cudaError_t launch_wave(const WaveParams& p, int grid, int block, int blocks_per_sm, cudaStream_t s);
 int         wave_smem_bytes(const WaveParams& p);
 int         wave_edge_floats(const ChildDev* c, int n);
-cudaError_t launch_hu_to_density(const float* corr, const int16_t* hu, float* rho, uint64_t n, float scale,
+constexpr int kHuNodes = 3996;   // HU -1000 .. 2995, what hu_to_density's clamp leaves
+constexpr int kHuBlock = 512;
+// The correction factors at `table` become densities (once per context); the conversion looks them up.
+cudaError_t launch_hu_table(float* table, cudaStream_t s);
+cudaError_t launch_hu_to_density(const float* table, const int16_t* hu, float* rho, uint64_t n, float scale, int sms,
                                  cudaStream_t s);
 cudaError_t launch_trace_rays(const ChildDev& c, const float* rays, uint64_t n_rays, uint32_t max_steps,
                               uint64_t* cnb, float* dist, int32_t* cells, uint32_t* counts, cudaStream_t s);
