@@ -1270,19 +1270,29 @@ namespace
 
 int
 ensure_stat_scratch(mqi_ctx* c) {
-    if (!c->stat_scratch) MQI_CUDA(c, cudaMalloc(&c->stat_scratch, 4 * sizeof(unsigned long long)), "statistics scratch");
+    if (!c->stat_scratch)
+        MQI_CUDA(c, cudaMalloc(&c->stat_scratch, 3 * kMaxScenarios * sizeof(unsigned long long)), "statistics scratch");
     return MQI_OK;
 }
 
+/// The estimates launch_stat left for `copies` scenarios: the worst one.
 int
-read_stat(mqi_ctx* c, double* mean_rel, uint64_t* n_vox) {
-    unsigned long long h[3] = { 0, 0, 0 };
-    MQI_CUDA(c, cudaMemcpyAsync(h, c->stat_scratch, sizeof(h), cudaMemcpyDeviceToHost, c->stream), "statistics");
+read_stat(mqi_ctx* c, uint32_t copies, double* mean_rel, uint64_t* n_vox) {
+    unsigned long long h[3 * kMaxScenarios];
+    MQI_CUDA(c, cudaMemcpyAsync(h, c->stat_scratch, 3 * copies * sizeof(h[0]), cudaMemcpyDeviceToHost, c->stream),
+             "statistics");
     MQI_CUDA(c, cudaStreamSynchronize(c->stream), "statistics");
-    double sum = 0.0;
-    std::memcpy(&sum, &h[2], sizeof(sum));
-    if (n_vox) *n_vox = h[1];
-    if (mean_rel) *mean_rel = h[1] ? sum / (double) h[1] : 0.0;
+    double   worst = -1.0;
+    uint64_t worst_n = 0;
+    for (uint32_t k = 0; k < copies; ++k) {
+        double sum = 0.0;
+        std::memcpy(&sum, &h[3 * k + 2], sizeof(sum));
+        const uint64_t nv = h[3 * k + 1];
+        const double   v  = nv ? sum / (double) nv : 0.0;
+        if (v > worst) { worst = v; worst_n = nv; }
+    }
+    if (n_vox) *n_vox = worst_n;
+    if (mean_rel) *mean_rel = worst;
     return MQI_OK;
 }
 
@@ -1371,21 +1381,9 @@ mqi_stat_uncertainty(mqi_ctx* c, int dose_id, int dose2_id, uint64_t n_histories
     DeviceGuard g(c->device);
     if (ensure_stat_scratch(c) != MQI_OK) return MQI_ERR_NOMEM;
     // robust scenarios: each scenario's estimate; the worst one is returned
-    double   worst = -1.0;
-    uint64_t worst_n = 0;
-    for (uint32_t k = 0; k < a.copies; ++k) {
-        MQI_CUDA(c, launch_stat(a.tally + k * a.tally_len * a.tstride, b.tally + k * b.tally_len * b.tstride, a.tally_len,
-                                a.tstride, (double) n_histories, 0, threshold, c->num_sms, c->stat_scratch, c->stream),
-                 "mqi_stat_uncertainty");
-        double   v = 0.0;
-        uint64_t nv = 0;
-        const int rc = read_stat(c, &v, &nv);
-        if (rc != MQI_OK) return rc;
-        if (v > worst) { worst = v; worst_n = nv; }
-    }
-    if (mean_rel_sigma) *mean_rel_sigma = worst;
-    if (n_voxels) *n_voxels = worst_n;
-    return MQI_OK;
+    MQI_CUDA(c, launch_stat(a.tally, b.tally, a.tally_len, a.tstride, a.copies, (double) n_histories, 0, threshold,
+                            c->num_sms, c->stat_scratch, c->stream), "mqi_stat_uncertainty");
+    return read_stat(c, a.copies, mean_rel_sigma, n_voxels);
 }
 
 int
@@ -1418,21 +1416,9 @@ mqi_batch_uncertainty(mqi_ctx* c, int scorer_id, float threshold, double* mean_r
     if (s.n_batches < 2) return fail(c, MQI_ERR_STATE, "mqi_batch_uncertainty: needs at least 2 accumulated batches");
     DeviceGuard g(c->device);
     if (ensure_stat_scratch(c) != MQI_OK) return MQI_ERR_NOMEM;
-    double   worst = -1.0;
-    uint64_t worst_n = 0;
-    for (uint32_t k = 0; k < s.copies; ++k) {
-        MQI_CUDA(c, launch_stat(s.batch_s1 + k * s.tally_len, s.batch_s2 + k * s.tally_len, s.tally_len, 1,
-                                (double) s.n_batches, 1, threshold, c->num_sms, c->stat_scratch, c->stream),
-                 "mqi_batch_uncertainty");
-        double   v = 0.0;
-        uint64_t nv = 0;
-        const int rc = read_stat(c, &v, &nv);
-        if (rc != MQI_OK) return rc;
-        if (v > worst) { worst = v; worst_n = nv; }
-    }
-    if (mean_rel_sigma) *mean_rel_sigma = worst;
-    if (n_voxels) *n_voxels = worst_n;
-    return MQI_OK;
+    MQI_CUDA(c, launch_stat(s.batch_s1, s.batch_s2, s.tally_len, 1, s.copies, (double) s.n_batches, 1, threshold, c->num_sms,
+                            c->stat_scratch, c->stream), "mqi_batch_uncertainty");
+    return read_stat(c, s.copies, mean_rel_sigma, n_voxels);
 }
 
 int
@@ -1460,6 +1446,7 @@ mqi_scale_tally(mqi_ctx* c, int scorer_id, double weight) {
     if (!valid_ctx(c)) return fail(c, MQI_ERR_INVALID, "mqi_scale_tally: ctx is NULL");
     if (scorer_id < 0 || scorer_id >= (int) c->scorers.size()) return fail(c, MQI_ERR_INVALID, "mqi_scale_tally: no such scorer");
     const ScorerHost& s = c->scorers[scorer_id];
+    if (weight == 1.0) return MQI_OK;   // a run that stopped after its first pass: every value stays
     DeviceGuard g(c->device);
     MQI_CUDA(c, launch_scale(s.tally, s.tstride, s.total(), weight, c->num_sms, c->stream), "mqi_scale_tally");
     MQI_CUDA(c, cudaStreamSynchronize(c->stream), "mqi_scale_tally");

@@ -255,9 +255,8 @@ cudaError_t launch_hu_to_density(const float* table, const int16_t* hu, float* r
                                  cudaStream_t s);
 cudaError_t launch_trace_rays(const ChildDev& c, const float* rays, uint64_t n_rays, uint32_t max_steps,
                               uint64_t* cnb, float* dist, int32_t* cells, uint32_t* counts, cudaStream_t s);
-cudaError_t launch_stat(const double* s1, const double* s2, uint64_t n, uint32_t stride, double nh, int mode,
-                        float threshold, int sms,
-                        unsigned long long* scratch, cudaStream_t s);
+cudaError_t launch_stat(const double* s1, const double* s2, uint64_t n, uint32_t stride, uint32_t copies, double nh,
+                        int mode, float threshold, int sms, unsigned long long* scratch, cudaStream_t s);
 cudaError_t launch_batch_fold(double* tally, uint32_t stride, double* s1, double* s2, uint64_t n, int sms, cudaStream_t s);
 cudaError_t launch_scale(double* a, uint32_t stride, uint64_t n, double w, int sms, cudaStream_t s);
 cudaError_t launch_copy_strided(const double* a, uint32_t stride, double* out, uint64_t n, int sms, cudaStream_t s);
