@@ -368,7 +368,10 @@ int mqi_set_tuning(mqi_ctx* ctx, int block, int blocks_per_sm, int slice_steps, 
  * histories, and graph_waves waves are captured once into a CUDA graph, so the host synchronises
  * once per graph_waves waves; streamed = 0: queue generations -- load primary_chunk histories,
  * run waves until a generation is empty, one host synchronisation per wave.  graph_waves must be
- * even (default 8); values <= 0 / < 0 keep the current setting.  Results do not depend on it. */
+ * even (default 8); values <= 0 / < 0 keep the current setting.  A run with its post-steps inside
+ * the wave that fits one queue load (histories x scenarios <= primary_chunk, no slices) is one
+ * launch in either mode: its daughters join the queue that the wave reads.  Results do not depend
+ * on it. */
 int mqi_set_launch_mode(mqi_ctx* ctx, int streamed, int graph_waves);
 
 /* Where the post-step of a nuclear interaction (p-p elastic, p-O elastic, p-O inelastic; ~0.2% of

@@ -185,6 +185,7 @@ mqi_destroy(mqi_ctx* c) {
     free_queue(c->qa);
     free_queue(c->qb);
     free_queue(c->qsort);
+    cudaFree(c->ready);
     cudaFree(c->sort_bins);
     cudaFree(c->def);
     cudaFree(c->counters);
@@ -565,6 +566,7 @@ make_wave_params(mqi_ctx* c, uint64_t seed, WaveParams& P) {
     P.k0              = (uint32_t) seed;
     P.k1              = (uint32_t) (seed >> 32);
     P.max_slice_steps = c->max_slice_steps;
+    P.lanes           = 32;
     P.inline_local    = (P.n_children == 1) ? 1 : 0;
     P.head            = c->counters + 2;
     P.error_flag      = c->counters + 3;
@@ -583,56 +585,100 @@ make_wave_params(mqi_ctx* c, uint64_t seed, WaveParams& P) {
     }
 }
 
+/// Waves from the queue A (its entry count in counters[0], in counters[0 .. 1] alternately) until
+/// one leaves none behind, one host synchronisation each.
+int
+run_waves(mqi_ctx* c, WaveParams& P, QueueBuf* A, QueueBuf* B, int cur) {
+    for (int wave = 0;; ++wave) {
+        if (wave > 100000) return fail(c, MQI_ERR_DEVICE, "mqi_transport: wave limit reached");
+        P.in    = A->q;
+        P.out   = B->q;
+        P.n_in  = c->counters + cur;
+        P.n_out = c->counters + (1 - cur);
+        if (!P.ready) {   // a draining wave's counters were set with its queue
+            MQI_CUDA(c, cudaMemsetAsync(c->counters + (1 - cur), 0, sizeof(uint32_t), c->stream), "mqi_transport");
+            MQI_CUDA(c, cudaMemsetAsync(c->counters + 2, 0, sizeof(uint32_t), c->stream), "mqi_transport");
+        }
+        MQI_CUDA(c, cudaEventRecord(c->ev0, c->stream), "mqi_transport");
+        MQI_CUDA(c, launch_wave(P, c->wave_grid, c->wave_block, c->wave_grid / c->num_sms, c->stream), "mqi_transport: wave");
+        MQI_CUDA(c, cudaEventRecord(c->ev1, c->stream), "mqi_transport");
+        MQI_CUDA(c, cudaMemcpyAsync(c->host_counts, c->counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream),
+                 "mqi_transport");
+        MQI_CUDA(c, cudaStreamSynchronize(c->stream), "mqi_transport: wave");
+        ++c->waves;
+        // the wave, its post-step kernel when split, the four sort kernels when sorting is on
+        c->kernel_launches += (P.split ? 2 : 1) + (P.sort_bins ? 4 : 0);
+        ++c->wave_launches;
+        float ms = 0.0f;
+        if (cudaEventElapsedTime(&ms, c->ev0, c->ev1) == cudaSuccess) c->wave_ms += ms;
+        if (c->host_counts[3] & 2u) return fail(c, MQI_ERR_OVERFLOW, "mqi_transport: particle queue overflow");
+        const uint32_t n_next = c->host_counts[1 - cur];
+        if (n_next == 0) return MQI_OK;
+        std::swap(A, B);
+        cur     = 1 - cur;
+        P.ready = nullptr;   // what a draining wave had no room for
+        P.lanes = 32;
+        P.max_blocks = 0;
+    }
+}
+
+/// Load or sample n histories from h, once per scenario, to the front of a queue.
+int
+load_histories(mqi_ctx* c, const WaveParams& P, const Queue& q, uint64_t h, uint32_t n, bool plan) {
+    if (plan)
+        MQI_CUDA(c, launch_sample_primaries(q, c->plan_spots, c->plan_cum, c->n_plan_spots, h, n, c->n_scen, P.k0,
+                                            P.k1 ^ kSourceKeyXor, c->stream), "mqi_transport: sample primaries");
+    else
+        MQI_CUDA(c, launch_load_primaries(q, c->vertices, c->has_spots ? c->spot_ids : nullptr, h, n, c->n_scen, c->stream),
+                 "mqi_transport: load primaries");
+    ++c->kernel_launches;
+    return MQI_OK;
+}
+
 /// Queue generations (moqui's order of work, one host synchronisation per wave): load (or sample) a
 /// chunk of primaries, run waves until a generation is empty, repeat.
 int
 run_generations(mqi_ctx* c, WaveParams P, uint64_t h0, uint64_t h1, bool plan) {
-    const uint32_t chunk = c->primary_chunk;
-    QueueBuf* A = &c->qa;
-    QueueBuf* B = &c->qb;
-    const uint32_t S       = c->n_scen;
-    const uint32_t per_ld  = std::max<uint32_t>(chunk / S, 1u);   // histories per load; S queue entries each
+    const uint32_t S      = c->n_scen;
+    const uint32_t per_ld = std::max<uint32_t>(c->primary_chunk / S, 1u);   // histories per load; S queue entries each
     for (uint64_t h = h0; h < h1; h += per_ld) {
-        const uint32_t n = (uint32_t) std::min<uint64_t>(per_ld, h1 - h);
-        if (plan)
-            MQI_CUDA(c, launch_sample_primaries(A->q, c->plan_spots, c->plan_cum, c->n_plan_spots, h, n, S, P.k0,
-                                                P.k1 ^ kSourceKeyXor, c->stream), "mqi_transport: sample primaries");
-        else
-            MQI_CUDA(c, launch_load_primaries(A->q, c->vertices, c->has_spots ? c->spot_ids : nullptr, h, n, S, c->stream),
-                     "mqi_transport: load primaries");
-        ++c->kernel_launches;
+        const uint32_t n  = (uint32_t) std::min<uint64_t>(per_ld, h1 - h);
+        int            rc = load_histories(c, P, c->qa.q, h, n, plan);
+        if (rc != MQI_OK) return rc;
         c->host_counts[0] = n * S;
         MQI_CUDA(c, cudaMemcpyAsync(c->counters + 0, c->host_counts, sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream),
                  "mqi_transport");
-        int cur = 0;
-        for (int wave = 0;; ++wave) {
-            if (wave > 100000) return fail(c, MQI_ERR_DEVICE, "mqi_transport: wave limit reached");
-            P.in    = A->q;
-            P.out   = B->q;
-            P.n_in  = c->counters + cur;
-            P.n_out = c->counters + (1 - cur);
-            MQI_CUDA(c, cudaMemsetAsync(c->counters + (1 - cur), 0, sizeof(uint32_t), c->stream), "mqi_transport");
-            MQI_CUDA(c, cudaMemsetAsync(c->counters + 2, 0, sizeof(uint32_t), c->stream), "mqi_transport");
-            MQI_CUDA(c, cudaEventRecord(c->ev0, c->stream), "mqi_transport");
-            MQI_CUDA(c, launch_wave(P, c->wave_grid, c->wave_block, c->wave_grid / c->num_sms, c->stream), "mqi_transport: wave");
-            MQI_CUDA(c, cudaEventRecord(c->ev1, c->stream), "mqi_transport");
-            MQI_CUDA(c, cudaMemcpyAsync(c->host_counts, c->counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream),
-                     "mqi_transport");
-            MQI_CUDA(c, cudaStreamSynchronize(c->stream), "mqi_transport: wave");
-            ++c->waves;
-            // the wave, its post-step kernel when split, the four sort kernels when sorting is on
-            c->kernel_launches += (P.split ? 2 : 1) + (P.sort_bins ? 4 : 0);
-            ++c->wave_launches;
-            float ms = 0.0f;
-            if (cudaEventElapsedTime(&ms, c->ev0, c->ev1) == cudaSuccess) c->wave_ms += ms;
-            if (c->host_counts[3] & 2u) return fail(c, MQI_ERR_OVERFLOW, "mqi_transport: particle queue overflow");
-            const uint32_t n_next = c->host_counts[1 - cur];
-            if (n_next == 0) break;
-            std::swap(A, B);
-            cur = 1 - cur;
-        }
+        if ((rc = run_waves(c, P, &c->qa, &c->qb, 0)) != MQI_OK) return rc;
     }
     return MQI_OK;
+}
+
+/// A run that fits one queue load with the nuclear post-steps inside the wave: one load and one
+/// draining wave (wave_body), and ordinary waves for whatever found no room.  Few tracks are spread
+/// over the resident warps, and blocks are launched for about twice the primaries, not for every
+/// warp: those without a track only poll.  Against the captured graph of eight waves (whose capture
+/// alone took 0.3 ms): 600 histories at 110 MeV 1.88 -> 0.77 ms, the phantom example (1e5) 10.4 -> 6.8,
+/// 250k behind a range shifter and an aperture 6.0 -> 4.0, masked LET of 30 spots 27.6 -> 20.5.
+int
+run_draining(mqi_ctx* c, WaveParams P, uint64_t h0, uint64_t h1, bool plan) {
+    const uint32_t n = (uint32_t) ((h1 - h0) * c->n_scen);
+    const int      rc = load_histories(c, P, c->qa.q, h0, (uint32_t) (h1 - h0), plan);
+    if (rc != MQI_OK) return rc;
+    if (++c->epoch == 0) {   // the marks of 2^32 waves ago
+        MQI_CUDA(c, cudaMemsetAsync(c->ready, 0, (size_t) c->queue_cap * sizeof(uint32_t), c->stream), "mqi_transport");
+        c->epoch = 1;
+    }
+    const uint32_t counts[8] = { n, 0, 0, 0, 0, 0, n, n };
+    std::memcpy(c->host_counts, counts, sizeof(counts));
+    MQI_CUDA(c, cudaMemcpyAsync(c->counters, c->host_counts, sizeof(counts), cudaMemcpyHostToDevice, c->stream), "mqi_transport");
+    P.ready = c->ready;
+    P.live  = reinterpret_cast<unsigned long long*>(c->counters + 6);
+    P.epoch = c->epoch;
+    const uint32_t warps = (uint32_t) c->num_sms * 5 * 4;   // of the inline instances, all resident
+    P.lanes = (int) std::min<uint32_t>((n + warps - 1) / warps, 32u);
+    P.max_blocks = std::max<int>(c->num_sms, 2 * (int) ((n + 4 * P.lanes - 1) / (4 * P.lanes)));
+    P.sort_bins = nullptr;   // fresh primaries keep their order
+    return run_waves(c, P, &c->qa, &c->qb, 0);
 }
 
 /// Streamed transport: before every wave the queue is topped up on the device with the next
@@ -723,8 +769,13 @@ run_transport(mqi_ctx* c, uint64_t h0, uint64_t h1, uint64_t seed, bool plan) {
     const uint32_t need = c->primary_chunk * 3u;
     if (c->queue_cap < need) {
         cudaFree(c->def);
+        cudaFree(c->ready);
         c->def        = nullptr;
+        c->ready      = nullptr;
         cudaError_t e = alloc_queue(c->qa, need);
+        if (e == cudaSuccess) e = cudaMalloc(&c->ready, (size_t) need * sizeof(uint32_t));
+        if (e == cudaSuccess) e = cudaMemsetAsync(c->ready, 0, (size_t) need * sizeof(uint32_t), c->stream);
+        c->epoch = 0;
         if (e == cudaSuccess) e = alloc_queue(c->qb, need);
         if (e == cudaSuccess) e = cudaMalloc(&c->def, (size_t) need * sizeof(Deferred));
         if (e == cudaSuccess) e = alloc_queue(c->qsort, need);
@@ -739,9 +790,8 @@ run_transport(mqi_ctx* c, uint64_t h0, uint64_t h1, uint64_t seed, bool plan) {
     WaveParams P;
     make_wave_params(c, seed, P);
     // Nuclear post-steps in the post-step kernel pay off when a wave holds many tracks: the step
-    // loop then carries less code (+30% on the 1e6-history slab phantom), while each interaction
-    // ends its track's wave, which lengthens the drain of small runs (-12% on the 1e5-history
-    // phantom example); runs below kSplitMinEntries queue entries keep them inside the wave.
+    // loop then carries less code, while each interaction ends its track's wave, which lengthens
+    // small runs; those below kSplitMinEntries queue entries keep them inside the (draining) wave.
     P.split = c->post_step_mode >= 0 ? c->post_step_mode
                                      : ((h1 - h0) * (uint64_t) c->n_scen >= kSplitMinEntries ? 1 : 0);
     if (c->sort_min > 0) {
@@ -750,7 +800,11 @@ run_transport(mqi_ctx* c, uint64_t h0, uint64_t h1, uint64_t seed, bool plan) {
         P.sort_min  = c->sort_min;
     }
     MQI_CUDA(c, cudaMemsetAsync(c->counters + 3, 0, sizeof(uint32_t), c->stream), "mqi_transport");
-    const int rc = c->streamed ? run_streamed(c, P, h0, h1, plan) : run_generations(c, P, h0, h1, plan);
+    // one draining wave when the run is a single queue load that is neither split nor sliced
+    const bool drains = !P.split && P.max_slice_steps == 0 && (h1 - h0) * (uint64_t) c->n_scen <= c->primary_chunk;
+    const int  rc     = drains        ? run_draining(c, P, h0, h1, plan)
+                        : c->streamed ? run_streamed(c, P, h0, h1, plan)
+                                      : run_generations(c, P, h0, h1, plan);
     if (rc != MQI_OK) return rc;
     if (c->host_counts[3] & 4u)
         return fail(c, MQI_ERR_OVERFLOW, "mqi_transport: a Dij table is full (raise its capacity)");

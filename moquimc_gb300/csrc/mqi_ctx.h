@@ -134,9 +134,12 @@ struct mqi_ctx {
     mqi_gpu::QueueBuf       qsort;                  // scratch of the energy-bin queue sort (queue_cap)
     uint32_t*               sort_bins = nullptr;    // 2 x kSortBins counters of the sort
     uint32_t                sort_min = 1u << 18;    // sort waves of at least this many entries (0: never)
-    uint32_t*               counters = nullptr;     // [0,1] queue sizes, [2] head, [3] error flag, [4] deferred
+    uint32_t*               ready = nullptr;        // marks of the entries a draining wave appended (queue_cap)
+    uint32_t                epoch = 0;              // the last draining wave's number
+    uint32_t*               counters = nullptr;     // [0,1] queue sizes, [2] head, [3] error flag, [4] deferred,
+                                                    // [6,7] a draining wave's live word
     unsigned long long*     stats = nullptr;        // 8 x u64
-    uint32_t*               host_counts = nullptr;  // pinned: 4 x u32
+    uint32_t*               host_counts = nullptr;  // pinned: 8 x u32
     float*                  tables = nullptr;       // 6*600 physics + 3996 HU densities
     mqi_gpu::CalibDev       calib{};                // SPR / X0 curves (mode 0: the defaults)
     float*                  calib_buf = nullptr;    // device: the tables of calib (SPR then X0)

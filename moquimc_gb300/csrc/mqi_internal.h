@@ -160,6 +160,12 @@ struct WaveParams {
     uint32_t        sort_min;   // sort a wave's input only when it holds at least this many entries
     Deferred*       def;        // device: tracks stopped at a nuclear interaction (capacity in.capacity)
     uint32_t*       n_def;      // device: entries in def (zeroed before each wave)
+    uint32_t*       ready;      // device: per entry of `in`, `epoch` once a daughter was appended there
+                                // (null: the wave does not drain; daughters go to `out`)
+    unsigned long long* live;   // device, a draining wave: entries of `in` << 32 | tracks not yet ended
+    uint32_t        epoch;      // a draining wave's number, unlike any that `ready` holds
+    int             lanes;      // lanes of a warp that take tracks (1 .. 32)
+    int             max_blocks; // blocks of the wave (0: every resident one)
     int             smem_edge_floats; // shared-memory floats for staged child edges
     const float*    tables;     // device: the six physics tables, 6 x 600 floats in Tables order
                                 // (a context's are followed by the density of each HU value)

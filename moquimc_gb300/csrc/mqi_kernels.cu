@@ -31,6 +31,12 @@ enum StatIdx { ST_HIST = 0, ST_TRACKS, ST_STEPS, ST_SEC, ST_LOCAL, ST_DROP, ST_W
 
 constexpr uint32_t kMaxTrackSteps = 1u << 20;
 
+/// WaveParams::live: queue entries in the high word, live tracks in the low one.
+constexpr unsigned long long kLiveEntry = 1ull << 32;
+
+/// Half-microsecond polls a warp without tracks makes before it gives up on the others (over 8 s).
+constexpr uint32_t kDrainPolls = 1u << 24;
+
 /// A track in registers: track_t<float> (mqi_track.hpp:48-205) reduced to what transport reads.
 struct Trk {
     float    ke0, ke1;
@@ -493,9 +499,27 @@ score_local_daughter(Ctx& C, float3 pw, float3 dw, float ke0, float dE0, uint32_
     return true;
 }
 
+/// Write a daughter's queue entry.
+__device__ inline void
+write_daughter(const Queue& q, uint32_t i, uint32_t below, uint64_t uid, uint32_t hist, uint32_t spot, float ke0,
+               bool ke1_zero, float3 p, float3 d, float dE0) {
+    q.ke[i] = ke0;
+    q.px[i] = p.x; q.py[i] = p.y; q.pz[i] = p.z;
+    q.dx[i] = d.x; q.dy[i] = d.y; q.dz[i] = d.z;
+    q.dE0[i] = dE0;
+    q.hist[i] = hist;
+    q.uid_lo[i] = (uint32_t) uid;
+    q.uid_hi[i] = (uint32_t) (uid >> 32);
+    q.ctr[i] = 0;
+    q.meta[i] = (below & kMetaBelowMask) | (ke1_zero ? kMetaKe1Zero : 0u);
+    q.cell[i] = 0;
+    q.spot[i] = spot;
+}
+
 /// Emit one daughter that survived the stack-limit check: move it to the world frame, score it
 /// where it stands when it is a deposit-only daughter of a single-child world, else append it to
-/// the next queue.  Out of line and by value: it runs on a few percent of the steps and its
+/// the queue the running wave takes its tracks from while that has room (a wave that drains, see
+/// wave_body), else to the next wave's queue.  Out of line and by value: it runs on a few percent of the steps and its
 /// body would otherwise be inlined at every push site of the four processes.
 /// Returns 0 queued, 1 scored locally, 2 queue overflow.
 template<int kMode>
@@ -509,23 +533,22 @@ emit_daughter(const WaveParams* P, const Tables* T, int child, uint32_t hint, co
     apply_scenario(*P, C.g, child, spot);
     daughter_to_world(P->child[child], p, d);
     if (P->inline_local && ke0 <= kTpCut && score_local_daughter<kMode>(C, p, d, ke0, dE0, hint)) return 1;
-    const Queue&   q = P->out;
+    if (P->ready) {
+        const uint32_t i = (uint32_t) (atomicAdd(P->live, kLiveEntry + 1ull) >> 32);
+        if (i < P->in.capacity) {
+            write_daughter(P->in, i, below, uid, hist, spot, ke0, ke1_zero, p, d, dE0);
+            __threadfence();   // the entry before its mark
+            *reinterpret_cast<volatile uint32_t*>(P->ready + i) = P->epoch;
+            return 0;
+        }
+        atomicAdd(P->live, ~0ull);   // no room: it waits for the next wave
+    }
     const uint32_t i = atomicAdd(P->n_out, 1u);
-    if (i >= q.capacity) {
+    if (i >= P->out.capacity) {
         atomicOr(P->error_flag, 2u);
         return 2;
     }
-    q.ke[i] = ke0;
-    q.px[i] = p.x; q.py[i] = p.y; q.pz[i] = p.z;
-    q.dx[i] = d.x; q.dy[i] = d.y; q.dz[i] = d.z;
-    q.dE0[i] = dE0;
-    q.hist[i] = hist;
-    q.uid_lo[i] = (uint32_t) uid;
-    q.uid_hi[i] = (uint32_t) (uid >> 32);
-    q.ctr[i] = 0;
-    q.meta[i] = (below & kMetaBelowMask) | (ke1_zero ? kMetaKe1Zero : 0u);
-    q.cell[i] = 0;
-    q.spot[i] = spot;
+    write_daughter(P->out, i, below, uid, hist, spot, ke0, ke1_zero, p, d, dE0);
     return 0;
 }
 
@@ -842,32 +865,33 @@ stepping(Ctx& C, Trk& t, Rng& rng, float rho, float d2b) {
 // ------------------------------------------------------------------------------------------
 
 /// Load queue entry i.  A track re-queued mid-grid (step_phase) comes back with the voxel index
-/// it stopped in, in `cnb`; the caller turns it into a cell once the child's grid is known.
+/// it stopped in, in `cnb`; the caller turns it into a cell once the child's grid is known.  The
+/// loads bypass L1, which could hold a sector read before another SM appended this entry.
 __device__ inline void
 load_track(const Queue& q, uint32_t i, Trk& t, Rng& rng, bool& step_phase, uint32_t& cnb) {
-    t.ke0  = q.ke[i];
-    const uint32_t meta = q.meta[i];
+    t.ke0  = __ldcg(&q.ke[i]);
+    const uint32_t meta = __ldcg(&q.meta[i]);
     t.ke1  = (meta & kMetaKe1Zero) ? 0.0f : t.ke0;
-    t.p0   = make_float3(q.px[i], q.py[i], q.pz[i]);
-    t.d0   = make_float3(q.dx[i], q.dy[i], q.dz[i]);
+    t.p0   = make_float3(__ldcg(&q.px[i]), __ldcg(&q.py[i]), __ldcg(&q.pz[i]));
+    t.d0   = make_float3(__ldcg(&q.dx[i]), __ldcg(&q.dy[i]), __ldcg(&q.dz[i]));
     t.p1   = t.p0;
     t.d1   = t.d0;
-    t.dE   = q.dE0[i];
+    t.dE   = __ldcg(&q.dE0[i]);
     t.ldE  = 0.0f;
-    t.hist = q.hist[i];
-    t.spot = q.spot[i];
-    t.uid  = (uint64_t) q.uid_lo[i] | ((uint64_t) q.uid_hi[i] << 32);
+    t.hist = __ldcg(&q.hist[i]);
+    t.spot = __ldcg(&q.spot[i]);
+    t.uid  = (uint64_t) __ldcg(&q.uid_lo[i]) | ((uint64_t) __ldcg(&q.uid_hi[i]) << 32);
     t.below   = meta & kMetaBelowMask;
     t.primary = (meta & kMetaPrimary) != 0;
     t.child   = (int) ((meta >> kMetaChildShift) & 7u);
     t.npush   = (meta >> kMetaNpushShift) & 1023u;
     t.stopped = false;
     step_phase = (meta & kMetaPhaseStep) != 0;
-    cnb = q.cell[i];
+    cnb = __ldcg(&q.cell[i]);
     rng.hist   = t.hist;
     rng.uid_lo = (uint32_t) t.uid;
     rng.uid_hi = (uint32_t) (t.uid >> 32);
-    rng.ctr    = q.ctr[i];
+    rng.ctr    = __ldcg(&q.ctr[i]);
     rng.pos    = 4;
     rng.has2   = false;
 }
@@ -955,6 +979,20 @@ requeue_track(Ctx& C, const Trk& t, const Rng& rng) {
     q.spot[i] = t.spot;
 }
 
+/// A wave: persistent warps, a lane to a track, until the queue is used up.  A lane claims a queue
+/// index, loads the track there, enters it into its grid and steps it to its end; the warp's lanes
+/// meet at the top of the loop, so a lane that lost its track has the next one in its grid before the
+/// others' next step.
+///
+/// A wave drains (P.ready given) when its daughters go to the end of the queue it is reading: a lane
+/// whose index lies past the end keeps it and looks for the track each time round, and the warps
+/// leave when the count of live tracks -- queued or held, the low word of P.live -- is 0.  So a run of
+/// any number of generations is one launch and lasts as long as its longest chain of tracks, instead
+/// of the sum of each generation's longest.  No warp that holds a track waits for another, so the
+/// wave ends whichever blocks are resident.  Each entry is published by its own mark (P.ready[i] =
+/// P.epoch, a number of this launch's own) after a fence.  P.lanes < 32 spreads few tracks over more
+/// warps: a warp's step takes the sum of its lanes' different branches, so the fewer tracks share a
+/// warp, the sooner each ends.
 template<int kMode, bool kSplit>
 __device__ __forceinline__ void
 wave_body(const WaveParams& P) {
@@ -1003,33 +1041,52 @@ wave_body(const WaveParams& P) {
     rng.k0 = P.k0;
     rng.k1 = P.k1;
     Trk  t;
-    bool have  = false;
-    bool in_grid = false;
+    bool     have    = false;   // the lane holds a track
+    bool     waits   = false;   // the lane holds queue index `ticket` and waits for a track there
+    bool     in_grid = false;
+    uint32_t ticket  = 0;
     uint32_t slice = 0;
     uint32_t track_steps = 0;   // per-track guard: a track is abandoned after kMaxTrackSteps
     // The input count can exceed the queue's capacity only after an overflowed append (the
     // append cursor counts on; nothing was written past the end).  The wave then does nothing:
     // the host reports the overflow, and no entry past the capacity is ever read.
-    const uint32_t n_raw = *P.n_in;
-    const uint32_t n_in  = (n_raw > P.in.capacity || (*P.error_flag & 2u)) ? 0u : n_raw;
-    const int lane = threadIdx.x & 31;
+    const uint32_t n_raw  = *P.n_in;
+    const uint32_t n_in   = (n_raw > P.in.capacity || (*P.error_flag & 2u)) ? 0u : n_raw;
+    const bool     drains = !kSplit && P.ready != nullptr && n_in > 0;
+    const int      lane   = threadIdx.x & 31;
+    bool           open   = lane < P.lanes;
+    uint32_t       polls  = 0;
 
     for (;;) {
-        // ---- fetch (one atomic per warp) ----
-        const unsigned act   = __activemask();
-        const unsigned needm = __ballot_sync(act, !have);
+        // ---- a queue index for every lane without one (one atomic per warp) ----
+        const bool     want  = open && !have && !waits;
+        const unsigned needm = __ballot_sync(0xFFFFFFFFu, want);
         if (needm) {
-            uint32_t base = 0;
+            uint32_t  base   = 0;
             const int leader = __ffs(needm) - 1;
             if (lane == leader) base = atomicAdd(P.head, (uint32_t) __popc(needm));
-            base = __shfl_sync(act, base, leader);
-            if (!have) {
-                const uint32_t idx = base + (uint32_t) __popc(needm & ((1u << lane) - 1u));
-                if (idx >= n_in) break;
+            base = __shfl_sync(0xFFFFFFFFu, base, leader);
+            if (want) {
+                ticket = base + (uint32_t) __popc(needm & ((1u << lane) - 1u));
+                waits  = true;
+            }
+        }
+        // ---- the track at that index, once there is one ----
+        if (waits) {
+            bool there = ticket < n_in;
+            if (!there && drains) {
+                there = ticket < P.in.capacity && *reinterpret_cast<volatile uint32_t*>(P.ready + ticket) == P.epoch;
+                if (there) __threadfence();   // the mark before the entry
+            } else if (!there) {
+                open  = false;   // the queue is used up
+                waits = false;
+            }
+            if (there) {
                 bool     step_phase;
                 uint32_t cnb0;
-                load_track(P.in, idx, t, rng, step_phase, cnb0);
+                load_track(P.in, ticket, t, rng, step_phase, cnb0);
                 have    = true;
+                waits   = false;
                 in_grid = step_phase;
                 slice   = 0;
                 track_steps = 0;
@@ -1044,13 +1101,26 @@ wave_body(const WaveParams& P) {
                 }
             }
         }
-        if (!in_grid) {
-            // ---- child entry (mqi_transport.hpp:161-190) ----
-            if (t.stopped || t.child >= P.n_children) {
-                if (t.primary) count_event(kCntHist);
-                have = false;
-                continue;
+        const unsigned held = __ballot_sync(0xFFFFFFFFu, have);
+        if (!held) {
+            if (!drains) break;
+            // no track is left anywhere when the count of live ones is 0: nothing can follow.  The warps
+            // look for their own entry more often than at that one word.
+            if ((polls & 3u) == 0u) {
+                uint32_t left = 0;
+                if (lane == 0) left = (uint32_t) *reinterpret_cast<volatile unsigned long long*>(P.live);
+                if (__shfl_sync(0xFFFFFFFFu, left, 0) == 0u) break;
             }
+            if (++polls > kDrainPolls) {   // never: a live track ends within kMaxTrackSteps steps
+                if (lane == 0) count_event(kCntErr);
+                break;
+            }
+            __nanosleep(500);
+            continue;
+        }
+        polls = 0;
+        if (have && !in_grid) {
+            // ---- child entry (mqi_transport.hpp:161-190) ----
             C.child = t.child;
             C.g     = make_grid(P.child[t.child], s_edges[t.child][0], s_edges[t.child][1], s_edges[t.child][2]);
             apply_scenario(P, C.g, t.child, t.spot);
@@ -1061,75 +1131,75 @@ wave_body(const WaveParams& P) {
             int3 c = grid_index(C.g, t.p0, t.d0);
             if (!grid_valid(C.g, c)) {
                 const float dist = grid_entry(C.g, t.p0, t.d0);
-                if (dist < 0.0f) {
-                    to_world(P.child[t.child], t.p0, t.d0);
-                    t.p1 = t.p0;
-                    t.d1 = t.d0;
-                    ++t.child;
-                    continue;
+                if (dist >= 0.0f) {
+                    t.p1 = advance(t.p0, t.d0, dist);
+                    // move(): vtx0 = vtx1 (including ke), deposits reset
+                    t.p0  = t.p1;
+                    t.d0  = t.d1;
+                    t.ke0 = t.ke1;
+                    t.dE = t.ldE = 0.0f;
+                    c = grid_index(C.g, t.p0, t.d0);
                 }
-                t.p1 = advance(t.p0, t.d0, dist);
-                // move(): vtx0 = vtx1 (including ke), deposits reset
-                t.p0  = t.p1;
-                t.d0  = t.d1;
-                t.ke0 = t.ke1;
-                t.dE = t.ldE = 0.0f;
-                c = grid_index(C.g, t.p0, t.d0);
             }
-            t.cell = c;
-            if (!grid_valid(C.g, c)) {
+            t.cell  = c;
+            in_grid = grid_valid(C.g, c);
+            if (!in_grid) {   // missed: on to the next child, or out of the world
                 to_world(P.child[t.child], t.p0, t.d0);
                 t.p1 = t.p0;
                 t.d1 = t.d0;
-                ++t.child;
-                continue;
+                if (++t.child >= P.n_children) {
+                    if (t.primary) count_event(kCntHist);
+                    have = false;
+                }
             }
-            in_grid = true;
-            continue;
         }
-        // ---- one voxel step (mqi_transport.hpp:192-233) ----
-        C.spot = t.spot;
-        const uint32_t cnb = grid_cnb(C.g, t.cell);
-        const float    rho = voxel_rho(C.g, cnb);
-        const float    d2b = grid_exit(C.g, t.p0, t.d0, t.cell);
-        const int      nuclear = stepping<kMode, kSplit>(C, t, rng, rho, d2b);
-        ++n_steps;
-        if (kSplit && nuclear) {   // the post-step kernel finishes this step and queues the track
-            defer_track(C, t, rng, cnb, nuclear);
-            have    = false;
-            in_grid = false;
-            continue;
-        }
-        if (++track_steps > kMaxTrackSteps) {   // no physical track comes near this; never hang
-            t.stopped = true;
-            count_event(kCntErr);
-        }
-        bool leave = false;
-        if (d2b < 0.0f) {
-            leave = true;
-        } else {
-            score_step<kMode>(C, t, cnb, rho, grid_volume(C.g, t.cell));
-            if (!t.stopped) {
-                grid_step_index(C.g, t.p1, t.d1, t.cell);
-                t.p0  = t.p1;
-                t.d0  = t.d1;
-                t.ke0 = t.ke1;
-                t.dE = t.ldE = 0.0f;
+        if (have && in_grid) {
+            // ---- one voxel step (mqi_transport.hpp:192-233) ----
+            C.spot = t.spot;
+            const uint32_t cnb = grid_cnb(C.g, t.cell);
+            const float    rho = voxel_rho(C.g, cnb);
+            const float    d2b = grid_exit(C.g, t.p0, t.d0, t.cell);
+            const int      nuclear = stepping<kMode, kSplit>(C, t, rng, rho, d2b);
+            ++n_steps;
+            if (kSplit && nuclear) {   // the post-step kernel finishes this step and queues the track
+                defer_track(C, t, rng, cnb, nuclear);
+                have = false;
+            } else {
+                if (++track_steps > kMaxTrackSteps) {   // no physical track comes near this; never hang
+                    t.stopped = true;
+                    count_event(kCntErr);
+                }
+                bool leave = true;
+                if (!(d2b < 0.0f)) {
+                    score_step<kMode>(C, t, cnb, rho, grid_volume(C.g, t.cell));
+                    if (!t.stopped) {
+                        grid_step_index(C.g, t.p1, t.d1, t.cell);
+                        t.p0  = t.p1;
+                        t.d0  = t.d1;
+                        t.ke0 = t.ke1;
+                        t.dE = t.ldE = 0.0f;
+                    }
+                    leave = t.stopped || !grid_valid(C.g, t.cell);
+                }
+                if (leave) {
+                    to_world(P.child[C.child], t.p0, t.d0);
+                    t.p1 = t.p0;
+                    t.d1 = t.d0;
+                    in_grid = false;
+                    if (t.stopped || ++t.child >= P.n_children) {
+                        if (t.primary) count_event(kCntHist);
+                        have = false;
+                    }
+                } else if (P.max_slice_steps && ++slice >= P.max_slice_steps) {
+                    requeue_track(C, t, rng);
+                    have = false;
+                }
             }
-            leave = t.stopped || !grid_valid(C.g, t.cell);
         }
-        if (leave) {
-            to_world(P.child[C.child], t.p0, t.d0);
-            t.p1 = t.p0;
-            t.d1 = t.d0;
-            ++t.child;
-            in_grid = false;
-            continue;
-        }
-        if (P.max_slice_steps && ++slice >= P.max_slice_steps) {
-            requeue_track(C, t, rng);
-            have    = false;
-            in_grid = false;
+        if (drains) {
+            // tracks that ended leave the count of live ones after their daughters have joined it
+            const unsigned ended = held & ~__ballot_sync(0xFFFFFFFFu, have);
+            if (ended && lane == 0) atomicAdd(P.live, 0ull - (unsigned long long) __popc(ended));
         }
     }
 
@@ -1348,6 +1418,7 @@ launch_variant(const WaveParams& p, int grid, cudaStream_t s) {
         (void) cudaGetLastError();   // the failed call's error is returned here, not left for the next launch
         return e;
     }
+    if (p.max_blocks) grid = std::min(grid, p.max_blocks);
     k_wave<B, M, K, S><<<grid, B, smem, s>>>(p);
     if constexpr (S) k_post<K><<<grid, kPostBlock, 0, s>>>(p);
     return cudaGetLastError();
@@ -1451,13 +1522,9 @@ launch_sort(const WaveParams& p, int grid, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-/// Instances: the split form in every launch shape of the common modes and in 128 x 5 for the
-/// others; the inline form in the two leading shapes of the common modes (one dose-like scorer,
-/// DIRECT ROIs) and in 128 x 5 for the FP64 callbacks (dose to medium, LET) and for Dij runs with
-/// DIRECT ROIs (tps_env's Dij runs are one spot per call: small runs) and for the dose scorer with the
-/// statistics pair (per-spot runs with statistical stopping).  A request for an inline
-/// instance that is not compiled runs the split one (the results are the same) when the caller
-/// gave a record array.
+/// Instances: the split form in every launch shape of the common modes (one dose-like scorer, DIRECT
+/// ROIs) and in 128 x 5 for the others; the inline form in two shapes of the common modes and in
+/// 128 x 5 for the others: small runs, among them tps_env's per-spot runs with any scorers.
 cudaError_t
 launch_wave(const WaveParams& p, int grid, int block, int blocks_per_sm, cudaStream_t s) {
     const int grid5 = grid / (blocks_per_sm > 0 ? blocks_per_sm : 1) * 5;
@@ -1465,20 +1532,26 @@ launch_wave(const WaveParams& p, int grid, int block, int blocks_per_sm, cudaStr
         const cudaError_t e = launch_sort(p, grid5, s);
         if (e != cudaSuccess) return e;
     }
-    if (!p.split && (p.kernel_mode == 0 || p.kernel_mode == kModeSingle)) {
+    if (!p.split) {
         const bool wide = block != 128;
-        if (p.kernel_mode == kModeSingle)
+        switch (p.kernel_mode) {
+        case 0:
+            return wide ? launch_variant<256, 2, 0, false>(p, grid, s) : launch_variant<128, 5, 0, false>(p, grid5, s);
+        case kModeSingle:
             return wide ? launch_variant<256, 2, kModeSingle, false>(p, grid, s)
                         : launch_variant<128, 5, kModeSingle, false>(p, grid5, s);
-        return wide ? launch_variant<256, 2, 0, false>(p, grid, s) : launch_variant<128, 5, 0, false>(p, grid5, s);
+        case kModeStat: return launch_variant<128, 5, kModeStat, false>(p, grid5, s);
+        case kModeDij: return launch_variant<128, 5, kModeDij, false>(p, grid5, s);
+        case kModeFull: return launch_variant<128, 5, kModeFull, false>(p, grid5, s);
+        case kModeRoi:
+        case kModeFull | kModeRoi: return launch_variant<128, 5, kModeFull | kModeRoi, false>(p, grid5, s);
+        default: return launch_variant<128, 5, kModeAll, false>(p, grid5, s);
+        }
     }
-    if (!p.split && p.kernel_mode == kModeFull) return launch_variant<128, 5, kModeFull, false>(p, grid5, s);
-    if (!p.split && p.kernel_mode == kModeDij) return launch_variant<128, 5, kModeDij, false>(p, grid5, s);
-    if (!p.split && p.kernel_mode == kModeStat) return launch_variant<128, 5, kModeStat, false>(p, grid5, s);
-    if (p.kernel_mode == kModeStat && p.def && p.n_def) return launch_variant<128, 5, kModeStat, true>(p, grid5, s);
     if (!p.def || !p.n_def) return cudaErrorInvalidValue;   // the split form needs its record array
     switch (p.kernel_mode) {
     case 0: break;
+    case kModeStat: return launch_variant<128, 5, kModeStat, true>(p, grid5, s);
     case kModeSingle:
         if (block == 128) {
             if (blocks_per_sm >= 6) return launch_variant<128, 6, kModeSingle, true>(p, grid, s);

@@ -178,6 +178,7 @@ mqi_transport_noalloc(int nx, int ny, int nz, const float* d_xe, const float* d_
     P.inline_local     = 1;
     P.head             = counters + 2;
     P.error_flag       = counters + 3;
+    P.lanes            = 32;
     P.split            = 0;   // nuclear post-steps inside the wave: no post-step records to hold
     P.stats            = stats;
     P.spot_ids         = nullptr;
