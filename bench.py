@@ -240,9 +240,8 @@ def plan_section(torch, capi, workloads, args) -> dict:
     est1, nv = c.stat_uncertainty(d1, d2, N, 0.5)
     st = c.stats()
     c.reset()
-    # the plain path: one mqi_transport_plan call per spot over the whole plan, in its best launch
-    # mode (queue generations: no graph is captured per call); the streamed mode, which captures
-    # and instantiates a graph on every call, is timed on a sample of spots beside it
+    # the plain path: one mqi_transport_plan call per spot over the whole plan in queue generations;
+    # the streamed mode is timed on a sample of spots beside it
     sub = list(range(0, len(wl.spots), args.plain_stride))
     h_sub = int(sum(int(cum[s + 1] - cum[s]) for s in sub))
 

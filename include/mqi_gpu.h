@@ -364,22 +364,20 @@ int mqi_run_until_stat(mqi_ctx* ctx, int dose_id, int dose2_id, uint64_t histori
 int mqi_set_tuning(mqi_ctx* ctx, int block, int blocks_per_sm, int slice_steps, int primary_chunk);
 
 /* How the queue is driven (no counterpart in moqui, which runs one kernel over all histories).
- * streamed = 1 (default): before every wave the queue is topped up on the device with the next
- * histories, and graph_waves waves are captured once into a CUDA graph, so the host synchronises
- * once per graph_waves waves; streamed = 0: queue generations -- load primary_chunk histories,
- * run waves until a generation is empty, one host synchronisation per wave.  graph_waves must be
- * even (default 8); values <= 0 / < 0 keep the current setting.  A run with its post-steps inside
- * the wave that fits one queue load (histories x scenarios <= primary_chunk, no slices) is one
- * launch in either mode: its daughters join the queue that the wave reads.  Results do not depend
- * on it. */
+ * streamed = 1 (default): before every wave the queue is topped up with the next histories;
+ * streamed = 0: queue generations -- load primary_chunk histories, run them to their end, repeat.
+ * graph_waves (even, at most 64; <= 0 keeps it) is checked and recorded but no longer used: waves
+ * are launched one by one, as a run takes few of them.  streamed < 0 keeps the current setting.
+ * Results do not depend on it. */
 int mqi_set_launch_mode(mqi_ctx* ctx, int streamed, int graph_waves);
 
 /* Where the post-step of a nuclear interaction (p-p elastic, p-O elastic, p-O inelastic; ~0.2% of
  * the steps) runs (no counterpart in moqui, which runs it inside the step, mqi_fippel_physics.hpp:
- * 178-196): 0 inside the wave kernel's step loop; 1 in a post-step kernel after each wave, which
- * takes that rarely used code out of the step loop (faster per step, one extra wave per
- * interaction); -1 (default) chooses 1 for runs of at least 2^19 queue entries (histories x
- * scenarios) and 0 below.  Results do not depend on it. */
+ * 178-196): 0 within the wave, by warps without tracks: each load's wave then drains -- daughters
+ * and resumed tracks join the queue it reads, and it ends with the last track; 1 in a post-step
+ * kernel after each wave, which ends its track's wave; -1 (default) drains with the last load's wave,
+ * after one ordinary wave if that load is of 2^19 fresh entries (histories x scenarios) or more.
+ * Results do not depend on it. */
 int mqi_set_post_step_mode(mqi_ctx* ctx, int mode);
 
 /* Sort the particle queue by energy before each wave that holds at least min_entries entries

@@ -248,7 +248,7 @@ class Context:
         return res[: n.value]
 
     def set_post_step_mode(self, mode: int) -> None:
-        """Nuclear post-steps: 0 inside the wave, 1 in the post-step kernel, -1 by run size."""
+        """Nuclear post-steps: 0 in draining waves, 1 in the post-step kernel, -1 automatic."""
         self._check(self.lib.mqi_set_post_step_mode(self.h, mode), self.h)
 
     def set_queue_sort(self, min_entries: int) -> None:

@@ -145,14 +145,11 @@ mqi_create(int device, mqi_ctx** out) {
     if ((e = cudaMalloc(&c->tables, tbytes)) != cudaSuccess ||
         (e = cudaMemcpy(c->tables, host.data(), tbytes, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = launch_hu_table(c->tables + 6 * MQI_TABLE_N, c->stream)) != cudaSuccess ||
-        (e = cudaMalloc(&c->counters, 8 * sizeof(uint32_t))) != cudaSuccess ||
-        (e = cudaMemset(c->counters, 0, 8 * sizeof(uint32_t))) != cudaSuccess ||
+        (e = cudaMalloc(&c->counters, 12 * sizeof(uint32_t))) != cudaSuccess ||
+        (e = cudaMemset(c->counters, 0, 12 * sizeof(uint32_t))) != cudaSuccess ||
         (e = cudaMalloc(&c->stats, 8 * sizeof(unsigned long long))) != cudaSuccess ||
         (e = cudaMemset(c->stats, 0, 8 * sizeof(unsigned long long))) != cudaSuccess ||
-        (e = cudaMallocHost(&c->host_counts, 8 * sizeof(uint32_t))) != cudaSuccess ||
-        (e = cudaMallocHost(&c->host_next, sizeof(unsigned long long))) != cudaSuccess ||
-        (e = cudaMalloc(&c->topup, sizeof(TopUp))) != cudaSuccess ||
-        (e = cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaMallocHost(&c->host_counts, 12 * sizeof(uint32_t))) != cudaSuccess ||
         (e = cudaEventCreate(&c->ev0)) != cudaSuccess || (e = cudaEventCreate(&c->ev1)) != cudaSuccess) {
         mqi_destroy(c);
         return cuda_fail(nullptr, e, "mqi_create: allocation");
@@ -193,9 +190,6 @@ mqi_destroy(mqi_ctx* c) {
     cudaFree(c->tables);
     cudaFree(c->calib_buf);
     if (c->host_counts) cudaFreeHost(c->host_counts);
-    if (c->host_next) cudaFreeHost(c->host_next);
-    cudaFree(c->topup);
-    if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
@@ -488,9 +482,10 @@ mqi_set_vertices(mqi_ctx* c, const mqi_vertex* v, const uint32_t* spot_ids, uint
 namespace
 {
 
-/// Runs with at least this many queue entries (histories x scenarios) hand nuclear post-steps to
-/// the post-step kernel when the post-step mode is automatic.
-constexpr uint64_t kSplitMinEntries = 1ull << 19;
+/// A load of at least this many fresh primaries goes through an ordinary wave before the draining one:
+/// its step loop is faster, and what it leaves is sorted by energy.  The slab phantom at 1e6: 19.7 ms
+/// so, 20.0 ms in one draining wave (20.4 ms in ordinary waves alone); at 5e5 the two are equal.
+constexpr uint32_t kDrainMaxFresh = 1u << 19;
 
 /// The source stream of a plan history is keyed apart from its transport streams.
 constexpr uint32_t kSourceKeyXor = 0xA5A5A5A5u;
@@ -570,8 +565,11 @@ make_wave_params(mqi_ctx* c, uint64_t seed, WaveParams& P) {
     P.inline_local    = (P.n_children == 1) ? 1 : 0;
     P.head            = c->counters + 2;
     P.error_flag      = c->counters + 3;
+    P.n_in            = c->counters + 0;
+    P.n_out           = c->counters + 1;
     P.def             = c->def;
-    P.n_def           = c->counters + 4;
+    P.def_cap         = c->queue_cap;
+    P.drain           = reinterpret_cast<DrainState*>(c->counters + 8);
     P.stats           = c->stats;
     P.spot_ids        = c->has_spots ? c->spot_ids : nullptr;
     P.tables          = c->tables;
@@ -585,181 +583,91 @@ make_wave_params(mqi_ctx* c, uint64_t seed, WaveParams& P) {
     }
 }
 
-/// Waves from the queue A (its entry count in counters[0], in counters[0 .. 1] alternately) until
-/// one leaves none behind, one host synchronisation each.
+/// Load or sample n histories from h, once per scenario, behind the `have` entries of a queue.
 int
-run_waves(mqi_ctx* c, WaveParams& P, QueueBuf* A, QueueBuf* B, int cur) {
-    for (int wave = 0;; ++wave) {
-        if (wave > 100000) return fail(c, MQI_ERR_DEVICE, "mqi_transport: wave limit reached");
-        P.in    = A->q;
-        P.out   = B->q;
-        P.n_in  = c->counters + cur;
-        P.n_out = c->counters + (1 - cur);
-        if (!P.ready) {   // a draining wave's counters were set with its queue
-            MQI_CUDA(c, cudaMemsetAsync(c->counters + (1 - cur), 0, sizeof(uint32_t), c->stream), "mqi_transport");
-            MQI_CUDA(c, cudaMemsetAsync(c->counters + 2, 0, sizeof(uint32_t), c->stream), "mqi_transport");
-        }
-        MQI_CUDA(c, cudaEventRecord(c->ev0, c->stream), "mqi_transport");
-        MQI_CUDA(c, launch_wave(P, c->wave_grid, c->wave_block, c->wave_grid / c->num_sms, c->stream), "mqi_transport: wave");
-        MQI_CUDA(c, cudaEventRecord(c->ev1, c->stream), "mqi_transport");
-        MQI_CUDA(c, cudaMemcpyAsync(c->host_counts, c->counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream),
-                 "mqi_transport");
-        MQI_CUDA(c, cudaStreamSynchronize(c->stream), "mqi_transport: wave");
-        ++c->waves;
-        // the wave, its post-step kernel when split, the four sort kernels when sorting is on
-        c->kernel_launches += (P.split ? 2 : 1) + (P.sort_bins ? 4 : 0);
-        ++c->wave_launches;
-        float ms = 0.0f;
-        if (cudaEventElapsedTime(&ms, c->ev0, c->ev1) == cudaSuccess) c->wave_ms += ms;
-        if (c->host_counts[3] & 2u) return fail(c, MQI_ERR_OVERFLOW, "mqi_transport: particle queue overflow");
-        const uint32_t n_next = c->host_counts[1 - cur];
-        if (n_next == 0) return MQI_OK;
-        std::swap(A, B);
-        cur     = 1 - cur;
-        P.ready = nullptr;   // what a draining wave had no room for
-        P.lanes = 32;
-        P.max_blocks = 0;
-    }
-}
-
-/// Load or sample n histories from h, once per scenario, to the front of a queue.
-int
-load_histories(mqi_ctx* c, const WaveParams& P, const Queue& q, uint64_t h, uint32_t n, bool plan) {
+load_histories(mqi_ctx* c, const WaveParams& P, const Queue& q, uint32_t have, uint64_t h, uint32_t n, bool plan) {
     if (plan)
-        MQI_CUDA(c, launch_sample_primaries(q, c->plan_spots, c->plan_cum, c->n_plan_spots, h, n, c->n_scen, P.k0,
+        MQI_CUDA(c, launch_sample_primaries(q, have, c->plan_spots, c->plan_cum, c->n_plan_spots, h, n, c->n_scen, P.k0,
                                             P.k1 ^ kSourceKeyXor, c->stream), "mqi_transport: sample primaries");
     else
-        MQI_CUDA(c, launch_load_primaries(q, c->vertices, c->has_spots ? c->spot_ids : nullptr, h, n, c->n_scen, c->stream),
-                 "mqi_transport: load primaries");
+        MQI_CUDA(c, launch_load_primaries(q, have, c->vertices, c->has_spots ? c->spot_ids : nullptr, h, n, c->n_scen,
+                                          c->stream), "mqi_transport: load primaries");
     ++c->kernel_launches;
     return MQI_OK;
 }
 
-/// Queue generations (moqui's order of work, one host synchronisation per wave): load (or sample) a
-/// chunk of primaries, run waves until a generation is empty, repeat.
+/// One wave over the n entries of queue A, of which the first `old` are no fresh primaries; what it
+/// leaves for the next is in B, and its count and the error flag in host_counts[1] and [3].
 int
-run_generations(mqi_ctx* c, WaveParams P, uint64_t h0, uint64_t h1, bool plan) {
-    const uint32_t S      = c->n_scen;
-    const uint32_t per_ld = std::max<uint32_t>(c->primary_chunk / S, 1u);   // histories per load; S queue entries each
-    for (uint64_t h = h0; h < h1; h += per_ld) {
-        const uint32_t n  = (uint32_t) std::min<uint64_t>(per_ld, h1 - h);
-        int            rc = load_histories(c, P, c->qa.q, h, n, plan);
-        if (rc != MQI_OK) return rc;
-        c->host_counts[0] = n * S;
-        MQI_CUDA(c, cudaMemcpyAsync(c->counters + 0, c->host_counts, sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream),
-                 "mqi_transport");
-        if ((rc = run_waves(c, P, &c->qa, &c->qb, 0)) != MQI_OK) return rc;
+run_wave(mqi_ctx* c, WaveParams& P, const QueueBuf& A, const QueueBuf& B, uint32_t n, uint32_t old, bool drains) {
+    P.in    = A.q;
+    P.out   = B.q;
+    P.ready = nullptr;
+    P.epoch = 0;
+    P.lanes = 32;
+    if (drains) {
+        if (++c->epoch >> 30) {   // the marks of 2^30 waves ago
+            MQI_CUDA(c, cudaMemsetAsync(c->ready, 0, (size_t) c->queue_cap * sizeof(uint32_t), c->stream), "mqi_transport");
+            MQI_CUDA(c, cudaMemsetAsync(c->def, 0, (size_t) c->queue_cap * sizeof(Deferred), c->stream), "mqi_transport");
+            c->epoch = 1;
+        }
+        P.ready = c->ready;
+        P.epoch = c->epoch;
+        plan_drain(P, n, c->num_sms);
     }
+    // fresh primaries keep their order: a queue that holds nothing else is not sorted
+    const bool sort = c->sort_min > 0 && old > 0 && n >= c->sort_min;
+    P.sort_bins     = sort ? c->sort_bins : nullptr;
+    const uint32_t counts[12] = { n, 0, 0, 0, 0, 0, 0, 0, n, n, 0, 0 };
+    std::memcpy(c->host_counts, counts, sizeof(counts));
+    MQI_CUDA(c, cudaMemcpyAsync(c->counters, c->host_counts, sizeof(counts), cudaMemcpyHostToDevice, c->stream),
+             "mqi_transport");
+    MQI_CUDA(c, cudaEventRecord(c->ev0, c->stream), "mqi_transport");
+    MQI_CUDA(c, launch_wave(P, c->wave_grid, c->wave_block, c->wave_grid / c->num_sms, c->stream), "mqi_transport: wave");
+    MQI_CUDA(c, cudaEventRecord(c->ev1, c->stream), "mqi_transport");
+    MQI_CUDA(c, cudaMemcpyAsync(c->host_counts, c->counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream),
+             "mqi_transport");
+    MQI_CUDA(c, cudaStreamSynchronize(c->stream), "mqi_transport: wave");
+    ++c->waves;
+    ++c->wave_launches;
+    c->kernel_launches += (drains ? 1 : 2) + (sort ? 4 : 0);   // the wave, its post-step kernel, the sort's four
+    float ms = 0.0f;
+    if (cudaEventElapsedTime(&ms, c->ev0, c->ev1) == cudaSuccess) c->wave_ms += ms;
     return MQI_OK;
 }
 
-/// A run that fits one queue load with the nuclear post-steps inside the wave: one load and one
-/// draining wave (wave_body), and ordinary waves for whatever found no room.  Few tracks are spread
-/// over the resident warps, and blocks are launched for about twice the primaries, not for every
-/// warp: those without a track only poll.  Against the captured graph of eight waves (whose capture
-/// alone took 0.3 ms): 600 histories at 110 MeV 1.88 -> 0.77 ms, the phantom example (1e5) 10.4 -> 6.8,
-/// 250k behind a range shifter and an aperture 6.0 -> 4.0, masked LET of 30 spots 27.6 -> 20.5.
+/// Waves over histories [h0, h1).  Streamed, the queue is topped up with the next histories before
+/// every wave, so the GPU stays full until the last ones are loaded; otherwise a load waits until the
+/// queue is empty (moqui's generations).  The last load's wave drains (wave_body), and in generations
+/// every load's, so that no generation of daughters waits for the longest track of the one before; a
+/// large load of fresh primaries takes an ordinary wave first (kDrainMaxFresh).  With post-step mode 1
+/// or slices all waves are ordinary.  The work done does not depend on how it is split into waves
+/// (every random number is keyed by history and track).
 int
-run_draining(mqi_ctx* c, WaveParams P, uint64_t h0, uint64_t h1, bool plan) {
-    const uint32_t n = (uint32_t) ((h1 - h0) * c->n_scen);
-    const int      rc = load_histories(c, P, c->qa.q, h0, (uint32_t) (h1 - h0), plan);
-    if (rc != MQI_OK) return rc;
-    if (++c->epoch == 0) {   // the marks of 2^32 waves ago
-        MQI_CUDA(c, cudaMemsetAsync(c->ready, 0, (size_t) c->queue_cap * sizeof(uint32_t), c->stream), "mqi_transport");
-        c->epoch = 1;
+run_waves(mqi_ctx* c, WaveParams& P, uint64_t h0, uint64_t h1, bool plan, uint32_t& flags) {
+    const uint32_t S      = c->n_scen;
+    const uint32_t target = std::max<uint32_t>(c->primary_chunk / S, 1u) * S;
+    const bool     may_drain = c->post_step_mode != 1 && P.max_slice_steps == 0;
+    const QueueBuf *A = &c->qa, *B = &c->qb;
+    uint64_t        h = h0;
+    uint32_t        old = 0;
+    for (int wave = 0; h < h1 || old > 0; ++wave) {
+        if (wave > 200000) return fail(c, MQI_ERR_DEVICE, "mqi_transport: wave limit reached");
+        uint32_t load = 0;
+        if (old == 0 || (c->streamed && old < target))
+            load = (uint32_t) std::min<uint64_t>((target - old) / S, h1 - h);
+        int rc = MQI_OK;
+        if (load > 0 && (rc = load_histories(c, P, A->q, old, h, load, plan)) != MQI_OK) return rc;
+        h += load;
+        const bool drains = may_drain && (h == h1 || !c->streamed) &&
+                            (c->post_step_mode == 0 || old > 0 || load * S < kDrainMaxFresh);
+        if ((rc = run_wave(c, P, *A, *B, old + load * S, old, drains)) != MQI_OK) return rc;
+        flags |= c->host_counts[3];
+        if (flags & 2u) return fail(c, MQI_ERR_OVERFLOW, "mqi_transport: particle queue overflow");
+        old = c->host_counts[1];
+        std::swap(A, B);
     }
-    const uint32_t counts[8] = { n, 0, 0, 0, 0, 0, n, n };
-    std::memcpy(c->host_counts, counts, sizeof(counts));
-    MQI_CUDA(c, cudaMemcpyAsync(c->counters, c->host_counts, sizeof(counts), cudaMemcpyHostToDevice, c->stream), "mqi_transport");
-    P.ready = c->ready;
-    P.live  = reinterpret_cast<unsigned long long*>(c->counters + 6);
-    P.epoch = c->epoch;
-    const uint32_t warps = (uint32_t) c->num_sms * 5 * 4;   // of the inline instances, all resident
-    P.lanes = (int) std::min<uint32_t>((n + warps - 1) / warps, 32u);
-    P.max_blocks = std::max<int>(c->num_sms, 2 * (int) ((n + 4 * P.lanes - 1) / (4 * P.lanes)));
-    P.sort_bins = nullptr;   // fresh primaries keep their order
-    return run_waves(c, P, &c->qa, &c->qb, 0);
-}
-
-/// Streamed transport: before every wave the queue is topped up on the device with the next
-/// histories, so waves never run with the GPU half empty while the long tracks of a generation
-/// finish; `graph_waves` waves (top-up, load, wave) are captured once into a CUDA graph, and the
-/// host synchronises once per graph launch.  The work done does not depend on how it is split
-/// into waves (every random number is keyed by history and track).
-int
-run_streamed(mqi_ctx* c, WaveParams P, uint64_t h0, uint64_t h1, bool plan) {
-    const int      K = c->graph_waves;
-    const uint32_t S = c->n_scen;
-    TopUp tu{};
-    tu.next   = h0;
-    tu.end    = h1;
-    tu.target = std::max<uint32_t>(c->primary_chunk / S, 1u) * S;
-    tu.n_scen = S;
-    MQI_CUDA(c, cudaMemcpyAsync(c->topup, &tu, sizeof(tu), cudaMemcpyHostToDevice, c->stream), "mqi_transport");
-    MQI_CUDA(c, cudaMemsetAsync(c->counters, 0, 2 * sizeof(uint32_t), c->stream), "mqi_transport");
-    MQI_CUDA(c, cudaStreamSynchronize(c->stream), "mqi_transport");
-
-    cudaStream_t cs = c->cap_stream;
-    cudaGraph_t  graph = nullptr;
-    cudaError_t  e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);
-    for (int i = 0; e == cudaSuccess && i < K; ++i) {
-        const int in  = i & 1;
-        QueueBuf& Qin = in ? c->qb : c->qa;
-        QueueBuf& Qo  = in ? c->qa : c->qb;
-        e = launch_topup(c->topup, c->counters + in, c->counters + 3, cs);
-        if (e == cudaSuccess)
-            e = plan ? launch_sample_topup(Qin.q, c->topup, c->plan_spots, c->plan_cum, c->n_plan_spots, P.k0,
-                                           P.k1 ^ kSourceKeyXor, c->num_sms, cs)
-                     : launch_load_topup(Qin.q, c->topup, c->vertices, c->has_spots ? c->spot_ids : nullptr, c->num_sms,
-                                         cs);
-        if (e == cudaSuccess) e = cudaMemsetAsync(c->counters + (1 - in), 0, sizeof(uint32_t), cs);
-        if (e == cudaSuccess) e = cudaMemsetAsync(c->counters + 2, 0, sizeof(uint32_t), cs);
-        P.in    = Qin.q;
-        P.out   = Qo.q;
-        P.n_in  = c->counters + in;
-        P.n_out = c->counters + (1 - in);
-        if (e == cudaSuccess) e = launch_wave(P, c->wave_grid, c->wave_block, c->wave_grid / c->num_sms, cs);
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(c->host_counts, c->counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, cs);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(c->host_next, &c->topup->next, sizeof(unsigned long long),
-                                              cudaMemcpyDeviceToHost, cs);
-    const cudaError_t e_end = cudaStreamEndCapture(cs, &graph);
-    if (e == cudaSuccess) e = e_end;
-    cudaGraphExec_t exec = nullptr;
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-    if (graph) cudaGraphDestroy(graph);
-    if (e != cudaSuccess) {
-        if (exec) cudaGraphExecDestroy(exec);
-        return cuda_fail(c, e, "mqi_transport: graph capture");
-    }
-    int rc = MQI_OK;
-    for (uint64_t launch = 0;; ++launch) {
-        if (launch * (uint64_t) K > 200000) {
-            rc = fail(c, MQI_ERR_DEVICE, "mqi_transport: wave limit reached");
-            break;
-        }
-        e = cudaEventRecord(c->ev0, c->stream);
-        if (e == cudaSuccess) e = cudaGraphLaunch(exec, c->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(c->ev1, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-        if (e != cudaSuccess) {
-            rc = cuda_fail(c, e, "mqi_transport: graph launch");
-            break;
-        }
-        c->waves += K;
-        c->wave_launches += K;
-        // per wave: top-up, load, wave (+ post-step when split, + 4 sort kernels when sorting is on)
-        c->kernel_launches += (3 + (P.split ? 1 : 0) + (P.sort_bins ? 4 : 0)) * (uint64_t) K;
-        float ms = 0.0f;
-        if (cudaEventElapsedTime(&ms, c->ev0, c->ev1) == cudaSuccess) c->wave_ms += ms;
-        if (c->host_counts[3] & 2u) {
-            rc = fail(c, MQI_ERR_OVERFLOW, "mqi_transport: particle queue overflow");
-            break;
-        }
-        if (*c->host_next >= h1 && c->host_counts[0] == 0) break;
-    }
-    cudaGraphExecDestroy(exec);
-    return rc;
+    return MQI_OK;
 }
 
 /// Transport histories [h0, h1) from the vertices or the spot plan.
@@ -778,6 +686,7 @@ run_transport(mqi_ctx* c, uint64_t h0, uint64_t h1, uint64_t seed, bool plan) {
         c->epoch = 0;
         if (e == cudaSuccess) e = alloc_queue(c->qb, need);
         if (e == cudaSuccess) e = cudaMalloc(&c->def, (size_t) need * sizeof(Deferred));
+        if (e == cudaSuccess) e = cudaMemsetAsync(c->def, 0, (size_t) need * sizeof(Deferred), c->stream);
         if (e == cudaSuccess) e = alloc_queue(c->qsort, need);
         if (e == cudaSuccess && !c->sort_bins) e = cudaMalloc(&c->sort_bins, 2 * kSortBins * sizeof(uint32_t));
         if (e == cudaSuccess) e = cudaMemsetAsync(c->sort_bins, 0, 2 * kSortBins * sizeof(uint32_t), c->stream);
@@ -789,26 +698,14 @@ run_transport(mqi_ctx* c, uint64_t h0, uint64_t h1, uint64_t seed, bool plan) {
     }
     WaveParams P;
     make_wave_params(c, seed, P);
-    // Nuclear post-steps in the post-step kernel pay off when a wave holds many tracks: the step
-    // loop then carries less code, while each interaction ends its track's wave, which lengthens
-    // small runs; those below kSplitMinEntries queue entries keep them inside the (draining) wave.
-    P.split = c->post_step_mode >= 0 ? c->post_step_mode
-                                     : ((h1 - h0) * (uint64_t) c->n_scen >= kSplitMinEntries ? 1 : 0);
-    if (c->sort_min > 0) {
-        P.sort_tmp  = c->qsort.q;
-        P.sort_bins = c->sort_bins;
-        P.sort_min  = c->sort_min;
-    }
-    MQI_CUDA(c, cudaMemsetAsync(c->counters + 3, 0, sizeof(uint32_t), c->stream), "mqi_transport");
-    // one draining wave when the run is a single queue load that is neither split nor sliced
-    const bool drains = !P.split && P.max_slice_steps == 0 && (h1 - h0) * (uint64_t) c->n_scen <= c->primary_chunk;
-    const int  rc     = drains        ? run_draining(c, P, h0, h1, plan)
-                        : c->streamed ? run_streamed(c, P, h0, h1, plan)
-                                      : run_generations(c, P, h0, h1, plan);
+    P.sort_tmp = c->qsort.q;
+    P.sort_min = c->sort_min;
+    uint32_t  flags = 0;
+    const int rc    = run_waves(c, P, h0, h1, plan, flags);
     if (rc != MQI_OK) return rc;
-    if (c->host_counts[3] & 4u)
+    if (flags & 4u)
         return fail(c, MQI_ERR_OVERFLOW, "mqi_transport: a Dij table is full (raise its capacity)");
-    if (c->host_counts[3] & 1u) return fail(c, MQI_ERR_DEVICE, "mqi_transport: a bounded device loop gave up");
+    if (flags & 1u) return fail(c, MQI_ERR_DEVICE, "mqi_transport: a bounded device loop gave up");
     return MQI_OK;
 }
 

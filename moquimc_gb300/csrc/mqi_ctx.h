@@ -7,6 +7,7 @@
 // receives what it reads by value.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -98,6 +99,19 @@ void dij_release(ScorerHost& s);
 /// Empty a Dij scorer's table and drop its matrix.
 cudaError_t dij_reset(ScorerHost& s, int sms, cudaStream_t st);
 
+/// The shape of a draining wave over n queue entries.  While every track has a lane of its own, the
+/// wave lasts as long as a chain of steps takes, and four blocks per SM (128 registers, no spills)
+/// take them sooner; beyond that throughput counts, and five blocks do.  Few tracks are spread over
+/// the resident warps, and blocks are launched for about twice the tracks, not for every warp: those
+/// without a track only poll.
+inline void
+plan_drain(WaveParams& P, uint32_t n, int sms) {
+    P.drain_shape = n <= (uint32_t) (sms * 4 * kDrainBlock) ? 4 : 5;
+    const uint32_t warps = (uint32_t) (sms * P.drain_shape * (kDrainBlock / 32));
+    P.lanes      = (int) std::min<uint32_t>((n + warps - 1) / warps, 32u);
+    P.max_blocks = std::max<int>(sms, 2 * (int) ((n + 4 * P.lanes - 1) / (4 * P.lanes)));
+}
+
 struct DeviceGuard {
     int prev = -1;
     explicit DeviceGuard(int dev) {
@@ -136,10 +150,10 @@ struct mqi_ctx {
     uint32_t                sort_min = 1u << 18;    // sort waves of at least this many entries (0: never)
     uint32_t*               ready = nullptr;        // marks of the entries a draining wave appended (queue_cap)
     uint32_t                epoch = 0;              // the last draining wave's number
-    uint32_t*               counters = nullptr;     // [0,1] queue sizes, [2] head, [3] error flag, [4] deferred,
-                                                    // [6,7] a draining wave's live word
+    uint32_t*               counters = nullptr;     // 12 words: [0] entries of the queue read, [1] of the next,
+                                                    // [2] head, [3] error flag, [8 ..] DrainState
     unsigned long long*     stats = nullptr;        // 8 x u64
-    uint32_t*               host_counts = nullptr;  // pinned: 8 x u32
+    uint32_t*               host_counts = nullptr;  // pinned: 12 x u32
     float*                  tables = nullptr;       // 6*600 physics + 3996 HU densities
     mqi_gpu::CalibDev       calib{};                // SPR / X0 curves (mode 0: the defaults)
     float*                  calib_buf = nullptr;    // device: the tables of calib (SPR then X0)
@@ -159,12 +173,9 @@ struct mqi_ctx {
     uint32_t                n_plan_spots = 0;
     uint64_t                plan_histories = 0;
     std::vector<uint64_t>   plan_cum_host;
-    int                     streamed = 1;             // 1: device top-up + graph-captured waves; 0: generations
-    int                     post_step_mode = -1;      // nuclear post-steps: -1 by run size, 0 in the wave, 1 post-step kernel
-    int                     graph_waves = 8;          // waves per captured graph (even)
-    mqi_gpu::TopUp*         topup = nullptr;          // device: streamed-transport state
-    unsigned long long*     host_next = nullptr;      // pinned: TopUp::next after a graph launch
-    cudaStream_t            cap_stream = nullptr;     // stream the graphs are captured on
+    int                     streamed = 1;             // 1: the queue is topped up before every wave; 0: generations
+    int                     post_step_mode = -1;      // nuclear post-steps: -1 automatic, 0 in draining waves, 1 post-step kernel
+    int                     graph_waves = 8;          // kept for the tuner's records
     uint32_t                n_scen = 1;               // robust scenarios (1: none)
     int                     scen_child = -1;
     int                     scen_stride = 0;

@@ -103,9 +103,9 @@ struct Queue {
 };
 
 /// A track stopped by the wave kernel at a nuclear interaction (p-p elastic, p-O elastic or p-O
-/// inelastic), after its along-step and the draw that chose the process: the post-step kernel runs
-/// the process, scores the step, moves the track and queues it (and its daughters) for the next
-/// wave.  These processes end ~0.2% of the steps, but their code is most of the step loop's
+/// inelastic), after its along-step and the draw that chose the process: the post-step kernel, or
+/// another warp of a draining wave, runs the process, scores the step, moves the track and queues it
+/// (and its daughters).  These processes end ~0.2% of the steps, but their code is most of the step loop's
 /// instructions and registers; taking it out of the loop shrinks what every step carries.
 struct Deferred {
     float    ke0, ke1;
@@ -116,7 +116,14 @@ struct Deferred {
     uint32_t uid_lo, uid_hi, hist, spot;
     uint32_t meta;     // below | primary | child | npush, as the queue's meta word
     uint32_t ctr;      // Philox counter after the step's process draw
-    uint32_t proc;     // 1 p-p elastic, 2 p-O elastic, 3 p-O inelastic
+    uint32_t mark;     // process (1 p-p elastic, 2 p-O elastic, 3 p-O inelastic) | wave's epoch << 2
+};
+
+/// What the warps of a draining wave share, read as one 16-byte word.
+struct alignas(16) DrainState {
+    unsigned long long live;   // entries of the queue being read << 32 | tracks not yet ended
+    uint32_t           tail;   // post-step records made (an ordinary wave counts them here too)
+    uint32_t           head;   // post-step records taken
 };
 
 /// A tabulated calibration (mqi_set_calibration); mode 0 = the default curves.
@@ -154,37 +161,27 @@ struct WaveParams {
     unsigned long long* stats;  // device: mqi_stats fields (8 x u64)
     const uint32_t* spot_ids;   // per history (may be null)
     uint32_t*       error_flag; // device: 1 a bounded loop gave up, 2 queue overflow, 4 Dij table full
-    int             split;      // 1: nuclear post-steps in the post-step kernel; 0: inside the wave
     Queue           sort_tmp;   // queue-sized scratch of the energy-bin sort (sort_bins null: no sort)
     uint32_t*       sort_bins;  // device: kSortBins counts (zero between sorts) then kSortBins cursors
     uint32_t        sort_min;   // sort a wave's input only when it holds at least this many entries
-    Deferred*       def;        // device: tracks stopped at a nuclear interaction (capacity in.capacity)
-    uint32_t*       n_def;      // device: entries in def (zeroed before each wave)
-    uint32_t*       ready;      // device: per entry of `in`, `epoch` once a daughter was appended there
-                                // (null: the wave does not drain; daughters go to `out`)
-    unsigned long long* live;   // device, a draining wave: entries of `in` << 32 | tracks not yet ended
-    uint32_t        epoch;      // a draining wave's number, unlike any that `ready` holds
+    Deferred*       def;        // device: def_cap records of tracks stopped at a nuclear interaction
+    uint32_t        def_cap;
+    DrainState*     drain;      // device; tail and head are 0 before a wave
+    uint32_t*       ready;      // device: per entry of `in`, `epoch` once a track was appended there
+                                // (null: the wave does not drain; its daughters go to `out`)
+    uint32_t        epoch;      // a draining wave's number, unlike any that `ready` or `def` hold (30 bits)
     int             lanes;      // lanes of a warp that take tracks (1 .. 32)
-    int             max_blocks; // blocks of the wave (0: every resident one)
+    int             max_blocks;  // a draining wave's blocks, at most
+    int             drain_shape; // a draining wave's blocks per SM, 4 or 5 (its register budget)
     int             smem_edge_floats; // shared-memory floats for staged child edges
     const float*    tables;     // device: the six physics tables, 6 x 600 floats in Tables order
                                 // (a context's are followed by the density of each HU value)
     CalibDev        calib;      // SPR / X0 curves
 };
 
-std::string& thread_error_slot();
+constexpr int kDrainBlock = 128;   // threads of a draining wave's block
 
-/// Device state of a streamed transport: before every wave the queue is topped up to `target`
-/// entries with the next histories, so the GPU stays full until the last histories drain.
-struct TopUp {
-    unsigned long long next;   // next history to load
-    unsigned long long end;    // one past the last history
-    unsigned long long base;   // first history of the current top-up
-    uint32_t target;           // queue entries a wave should start with
-    uint32_t n_scen;           // queue entries per history (robust scenarios)
-    uint32_t count;            // entries appended by the current top-up
-    uint32_t dst;              // first appended entry
-};
+std::string& thread_error_slot();
 
 /// Classes of the queue sort: 1 MeV energy bins, the last one open (tracks above 319 MeV), and
 /// one more class for primaries that have not taken a step yet.
@@ -235,21 +232,15 @@ cudaError_t dij_backward(const uint32_t* order, const uint64_t* seg_start, uint3
                          const void* g, void* grad, int fp64, int sms, cudaStream_t s);
 
 // ---- launchers (mqi_kernels.cu) ----
-// Loaders: n histories from h0, each once per scenario (n_scen >= 1), scenario-interleaved:
-// queue entry i holds history h0 + i / n_scen in scenario i % n_scen.
-cudaError_t launch_load_primaries(const Queue& q, const mqi_vertex* v, const uint32_t* spot_ids, uint64_t h0, uint32_t n,
-                                  uint32_t n_scen, cudaStream_t s);
-cudaError_t launch_sample_primaries(const Queue& q, const mqi_spot* spots, const uint64_t* cum, uint32_t n_spots,
-                                    uint64_t h0, uint32_t n, uint32_t n_scen, uint32_t k0, uint32_t k1, cudaStream_t s);
+// Loaders: n histories from h0 to queue entries dst .., each once per scenario (n_scen >= 1),
+// scenario-interleaved: entry dst + i holds history h0 + i / n_scen in scenario i % n_scen.
+cudaError_t launch_load_primaries(const Queue& q, uint32_t dst, const mqi_vertex* v, const uint32_t* spot_ids, uint64_t h0,
+                                  uint32_t n, uint32_t n_scen, cudaStream_t s);
+cudaError_t launch_sample_primaries(const Queue& q, uint32_t dst, const mqi_spot* spots, const uint64_t* cum,
+                                    uint32_t n_spots, uint64_t h0, uint32_t n, uint32_t n_scen, uint32_t k0, uint32_t k1,
+                                    cudaStream_t s);
 cudaError_t launch_sample_vertices(mqi_vertex* out, uint32_t* spot_out, const mqi_spot* spots, const uint64_t* cum,
                                    uint32_t n_spots, uint64_t h0, uint32_t n, uint32_t k0, uint32_t k1, cudaStream_t s);
-// Streamed loaders: k_topup sizes the top-up of the queue whose count is *n_in (one thread), the
-// loaders then append tu->count entries at tu->dst.
-cudaError_t launch_topup(TopUp* tu, uint32_t* n_in, const uint32_t* error_flag, cudaStream_t s);
-cudaError_t launch_load_topup(const Queue& q, const TopUp* tu, const mqi_vertex* v, const uint32_t* spot_ids, int sms,
-                              cudaStream_t s);
-cudaError_t launch_sample_topup(const Queue& q, const TopUp* tu, const mqi_spot* spots, const uint64_t* cum,
-                                uint32_t n_spots, uint32_t k0, uint32_t k1, int sms, cudaStream_t s);
 cudaError_t launch_wave(const WaveParams& p, int grid, int block, int blocks_per_sm, cudaStream_t s);
 int         wave_smem_bytes(const WaveParams& p);
 int         wave_edge_floats(const ChildDev* c, int n);

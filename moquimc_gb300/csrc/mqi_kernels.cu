@@ -4,9 +4,9 @@
 // (moqui/kernel_functions/mqi_transport.hpp:113-250, moqui/base/mqi_track_stack.hpp:11-67).
 // Here every track lives in a structure-of-arrays queue.  A wave kernel drains the queue: each
 // lane fetches a track (warp-aggregated cursor), steps it voxel by voxel in registers, scores
-// each step with warp-aggregated FP64 atomics, and appends its daughters -- and itself, when its
-// step budget for the wave runs out -- to the next queue.  The host (or a captured graph) swaps
-// queues until none is left.  Because each track's random stream is keyed by (seed, history,
+// each step with FP64 atomics, and appends its daughters -- and itself, when its step budget for the
+// wave runs out -- to the next queue, or in a draining wave to the end of the one it reads.  The
+// host swaps queues until none is left.  Because each track's random stream is keyed by (seed, history,
 // track uid) and the 200/10-deep stack limit is emulated from each track's recorded stack depth,
 // the result does not depend on the order the queue is drained in.
 #include <algorithm>
@@ -34,8 +34,11 @@ constexpr uint32_t kMaxTrackSteps = 1u << 20;
 /// WaveParams::live: queue entries in the high word, live tracks in the low one.
 constexpr unsigned long long kLiveEntry = 1ull << 32;
 
-/// Half-microsecond polls a warp without tracks makes before it gives up on the others (over 8 s).
+/// Polls a warp without tracks makes before it gives up on the others: seconds.
 constexpr uint32_t kDrainPolls = 1u << 24;
+
+/// A draining wave's blocks to one warp that only runs post-steps.
+constexpr uint32_t kPostEvery = 20;
 
 /// A track in registers: track_t<float> (mqi_track.hpp:48-205) reduced to what transport reads.
 struct Trk {
@@ -499,21 +502,35 @@ score_local_daughter(Ctx& C, float3 pw, float3 dw, float ke0, float dE0, uint32_
     return true;
 }
 
-/// Write a daughter's queue entry.
-__device__ inline void
-write_daughter(const Queue& q, uint32_t i, uint32_t below, uint64_t uid, uint32_t hist, uint32_t spot, float ke0,
-               bool ke1_zero, float3 p, float3 d, float dE0) {
-    q.ke[i] = ke0;
-    q.px[i] = p.x; q.py[i] = p.y; q.pz[i] = p.z;
-    q.dx[i] = d.x; q.dy[i] = d.y; q.dz[i] = d.z;
-    q.dE0[i] = dE0;
-    q.hist[i] = hist;
-    q.uid_lo[i] = (uint32_t) uid;
-    q.uid_hi[i] = (uint32_t) (uid >> 32);
-    q.ctr[i] = 0;
-    q.meta[i] = (below & kMetaBelowMask) | (ke1_zero ? kMetaKe1Zero : 0u);
-    q.cell[i] = 0;
-    q.spot[i] = spot;
+/// A place in a queue for one more track, and its publication once written: at the end of the queue
+/// the running wave reads while a draining wave (see wave_body) has room there, else in the next
+/// wave's.  `joins`: the track is not yet counted among the live ones.
+struct Slot {
+    Queue    q;
+    uint32_t i;
+    bool     marked;   // in the running wave's queue
+    bool     ok;       // false: neither queue had room (the error flag is set)
+};
+
+__device__ __forceinline__ Slot
+append_slot(const WaveParams& P, bool joins) {
+    if (P.ready) {
+        const uint32_t i = (uint32_t) (atomicAdd(&P.drain->live, kLiveEntry + (joins ? 1ull : 0ull)) >> 32);
+        if (i < P.in.capacity) return Slot{ P.in, i, true, true };
+        atomicAdd(&P.drain->live, ~0ull);   // it waits for the next wave, and this one no longer for it
+    }
+    const uint32_t i  = atomicAdd(P.n_out, 1u);
+    const bool     ok = i < P.out.capacity;
+    if (!ok) atomicOr(P.error_flag, 2u);
+    return Slot{ P.out, i, false, ok };
+}
+
+__device__ __forceinline__ void
+publish_slot(const WaveParams& P, const Slot& s) {
+    if (s.marked) {
+        __threadfence();   // the entry before its mark
+        *reinterpret_cast<volatile uint32_t*>(P.ready + s.i) = P.epoch;
+    }
 }
 
 /// Emit one daughter that survived the stack-limit check: move it to the world frame, score it
@@ -533,22 +550,22 @@ emit_daughter(const WaveParams* P, const Tables* T, int child, uint32_t hint, co
     apply_scenario(*P, C.g, child, spot);
     daughter_to_world(P->child[child], p, d);
     if (P->inline_local && ke0 <= kTpCut && score_local_daughter<kMode>(C, p, d, ke0, dE0, hint)) return 1;
-    if (P->ready) {
-        const uint32_t i = (uint32_t) (atomicAdd(P->live, kLiveEntry + 1ull) >> 32);
-        if (i < P->in.capacity) {
-            write_daughter(P->in, i, below, uid, hist, spot, ke0, ke1_zero, p, d, dE0);
-            __threadfence();   // the entry before its mark
-            *reinterpret_cast<volatile uint32_t*>(P->ready + i) = P->epoch;
-            return 0;
-        }
-        atomicAdd(P->live, ~0ull);   // no room: it waits for the next wave
-    }
-    const uint32_t i = atomicAdd(P->n_out, 1u);
-    if (i >= P->out.capacity) {
-        atomicOr(P->error_flag, 2u);
-        return 2;
-    }
-    write_daughter(P->out, i, below, uid, hist, spot, ke0, ke1_zero, p, d, dE0);
+    const Slot s = append_slot(*P, true);
+    if (!s.ok) return 2;
+    const Queue&   q = s.q;
+    const uint32_t i = s.i;
+    q.ke[i] = ke0;
+    q.px[i] = p.x; q.py[i] = p.y; q.pz[i] = p.z;
+    q.dx[i] = d.x; q.dy[i] = d.y; q.dz[i] = d.z;
+    q.dE0[i] = dE0;
+    q.hist[i] = hist;
+    q.uid_lo[i] = (uint32_t) uid;
+    q.uid_hi[i] = (uint32_t) (uid >> 32);
+    q.ctr[i] = 0;
+    q.meta[i] = (below & kMetaBelowMask) | (ke1_zero ? kMetaKe1Zero : 0u);
+    q.cell[i] = 0;
+    q.spot[i] = spot;
+    publish_slot(*P, s);
     return 0;
 }
 
@@ -755,31 +772,10 @@ post_poi(Ctx& C, Trk& t, Rng& rng) {
     t.stopped = true;
 }
 
-/// The post-step of a nuclear interaction run inside the step loop (kernel instances that do not
-/// hand them to the post-step kernel): the track and its stream go in and out by value, which
-/// keeps the rarely-taken processes from pinning registers across the loop.
-struct PostState {
-    Trk t;
-    Rng rng;
-};
-
-template<int kMode>
-__device__ __forceinline__ PostState
-post_nuclear(const WaveParams* P, const Tables* T, Grid g, int child, bool dbg, float tcut, int proc, PostState s) {
-    Ctx C;
-    C.P = P; C.T = T; C.g = g; C.child = child; C.dbg = dbg; C.tcut = tcut;
-    C.spot = s.t.spot;
-    if (proc == 1) post_pp<kMode>(C, s.t, s.rng);
-    else if (proc == 2) post_poe<kMode>(C, s.t, s.rng);
-    else post_poi<kMode>(C, s.t, s.rng);
-    return s;
-}
-
 /// fippel_physics::stepping (mqi_fippel_physics.hpp:67-216).  A delta ray is produced here.  A
-/// nuclear interaction (1 p-p elastic, 2 p-O elastic, 3 p-O inelastic) either runs here too
-/// (kSplit false) or ends the step early: stepping returns the process and the post-step kernel
-/// (k_post) finishes the step after the wave (kSplit true).
-template<int kMode, bool kSplit>
+/// nuclear interaction (1 p-p elastic, 2 p-O elastic, 3 p-O inelastic) ends the step early: stepping
+/// returns the process, and post_record finishes the step elsewhere.
+template<int kMode>
 __device__ inline int
 stepping(Ctx& C, Trk& t, Rng& rng, float rho, float d2b) {
     t.spr0 = -1.0f;
@@ -844,17 +840,8 @@ stepping(Ctx& C, Trk& t, Rng& rng, float rho, float d2b) {
         const int proc = (u < c0) ? 0 : (u < c0 + c1) ? 1 : (u < c0 + c1 + c2) ? 2 : (u < c0 + c1 + c2 + c3) ? 3 : -1;
         if (proc == 0) {
             post_delta<kMode>(C, t, rng);   // ~15% of the steps
-        } else if (proc > 0) {       // ~0.2% of the steps
-            if constexpr (kSplit) {
-                return proc;
-            } else {
-                PostState ps;
-                ps.t   = t;
-                ps.rng = rng;
-                ps     = post_nuclear<kMode>(C.P, C.T, C.g, C.child, C.dbg, C.tcut, proc, ps);
-                t      = ps.t;
-                rng    = ps.rng;
-            }
+        } else if (proc > 0) {
+            return proc;                    // ~0.2% of the steps
         }
     }
     return 0;
@@ -903,16 +890,17 @@ track_meta(const Trk& t) {
            ((uint32_t) t.child << kMetaChildShift) | ((t.npush & 1023u) << kMetaNpushShift);
 }
 
-/// Queue a track that left a child grid for the entry into child t.child (world frame).
-__device__ inline void
-requeue_entry(Ctx& C, const Trk& t, const Rng& rng) {
-    const Queue& q   = C.P->out;
-    const uint32_t i = atomicAdd(C.P->n_out, 1u);
-    if (i >= q.capacity) {
-        atomicOr(C.P->error_flag, 2u);
+/// Queue a track again: for the entry into child t.child (world frame), or with kMetaPhaseStep as
+/// `phase` mid-grid, in voxel `cnb`.  False when no queue had room.
+__device__ inline bool
+requeue_track(Ctx& C, const Trk& t, const Rng& rng, uint32_t phase, uint32_t cnb) {
+    const Slot s = append_slot(*C.P, false);
+    if (!s.ok) {
         count_event(kCntErr);
-        return;
+        return false;
     }
+    const Queue&   q = s.q;
+    const uint32_t i = s.i;
     q.ke[i] = t.ke0;
     q.px[i] = t.p0.x; q.py[i] = t.p0.y; q.pz[i] = t.p0.z;
     q.dx[i] = t.d0.x; q.dy[i] = t.d0.y; q.dz[i] = t.d0.z;
@@ -921,23 +909,16 @@ requeue_entry(Ctx& C, const Trk& t, const Rng& rng) {
     q.uid_lo[i] = (uint32_t) t.uid;
     q.uid_hi[i] = (uint32_t) (t.uid >> 32);
     q.ctr[i] = rng.ctr;
-    q.meta[i] = track_meta(t);
-    q.cell[i] = 0;
+    q.meta[i] = track_meta(t) | phase;
+    q.cell[i] = cnb;
     q.spot[i] = t.spot;
+    publish_slot(*C.P, s);
+    return true;
 }
 
-/// Hand a track whose step ended in nuclear process `proc` to the post-step kernel.  A track is
-/// handed over at most once per wave and every handed-over track was fetched from the wave's
-/// input, so the record array (sized like the input queue) cannot run out.
+/// What the post-step of nuclear process `proc` needs of a track whose step ended in it.
 __device__ inline void
-defer_track(Ctx& C, const Trk& t, const Rng& rng, uint32_t cnb, int proc) {
-    const uint32_t i = atomicAdd(C.P->n_def, 1u);
-    if (i >= C.P->in.capacity) {
-        atomicOr(C.P->error_flag, 2u);
-        count_event(kCntErr);
-        return;
-    }
-    Deferred& d = C.P->def[i];
+fill_record(Deferred& d, const Trk& t, const Rng& rng, uint32_t cnb) {
     d.ke0 = t.ke0;
     d.ke1 = t.ke1;
     d.p0[0] = t.p0.x; d.p0[1] = t.p0.y; d.p0[2] = t.p0.z;
@@ -952,31 +933,165 @@ defer_track(Ctx& C, const Trk& t, const Rng& rng, uint32_t cnb, int proc) {
     d.spot   = t.spot;
     d.meta   = (t.below & kMetaBelowMask) | (t.primary ? kMetaPrimary : 0u) | ((uint32_t) t.child << kMetaChildShift) |
              ((t.npush & 1023u) << kMetaNpushShift);
-    d.ctr  = rng.ctr;
-    d.proc = (uint32_t) proc;
+    d.ctr = rng.ctr;
 }
 
-/// Write a track that used up its step budget back to the next queue, mid-grid.
-__device__ inline void
-requeue_track(Ctx& C, const Trk& t, const Rng& rng) {
-    const Queue& q   = C.P->out;
-    const uint32_t i = atomicAdd(C.P->n_out, 1u);
-    if (i >= q.capacity) {
-        atomicOr(C.P->error_flag, 2u);
-        count_event(kCntErr);
+/// The rest of a step that ended in a nuclear interaction: the process's post_step
+/// (mqi_pp_elastic.hpp:119-219, mqi_po_elastic.hpp:96-217, mqi_po_inelastic.hpp:158-288), the step's
+/// scoring, the cell update and move() (mqi_transport.hpp:204-233); then the track is queued again
+/// -- mid-grid, at the entry of the next child, or not at all when it stopped or left the world.
+/// The random stream resumes where the step left it (the process draw was the first word of the
+/// block at counter ctr - 1).  Out of line: the step loop calls it only when the record array is
+/// full.
+/// `rec` is the calling thread's own copy.
+template<int kMode>
+static __device__ __noinline__ void
+post_record(const WaveParams* Pp, const Deferred* rec) {
+    const WaveParams& P = *Pp;
+    const Deferred&   d = *rec;
+    Ctx C;
+    C.P     = &P;
+    C.T     = reinterpret_cast<const Tables*>(P.tables);
+    C.dbg   = P.physics_debug != 0;
+    C.tcut  = P.t_cut;
+    Trk t;
+    t.ke0 = d.ke0;
+    t.ke1 = d.ke1;
+    t.p0  = make_float3(d.p0[0], d.p0[1], d.p0[2]);
+    t.d0  = make_float3(d.d0[0], d.d0[1], d.d0[2]);
+    t.p1  = make_float3(d.p1[0], d.p1[1], d.p1[2]);
+    t.d1  = t.d0;
+    t.dE  = d.dE;
+    t.ldE = 0.0f;
+    t.spr0 = d.spr0;
+    t.uid  = (uint64_t) d.uid_lo | ((uint64_t) d.uid_hi << 32);
+    t.hist = d.hist;
+    t.spot = d.spot;
+    t.below   = d.meta & kMetaBelowMask;
+    t.primary = (d.meta & kMetaPrimary) != 0;
+    t.child   = (int) ((d.meta >> kMetaChildShift) & 7u);
+    t.npush   = (d.meta >> kMetaNpushShift) & 1023u;
+    t.stopped = false;
+    Rng rng;
+    rng.k0     = P.k0;
+    rng.k1     = P.k1;
+    rng.hist   = d.hist;
+    rng.uid_lo = d.uid_lo;
+    rng.uid_hi = d.uid_hi;
+    rng.ctr    = d.ctr;
+    rng.blk    = philox_block(d.ctr - 1u, d.hist, d.uid_lo, d.uid_hi, P.k0, P.k1);
+    rng.pos    = 1;
+    rng.has2   = false;
+    C.child = t.child;
+    C.spot  = t.spot;
+    C.g     = make_grid(P.child[t.child], nullptr, nullptr, nullptr);
+    apply_scenario(P, C.g, t.child, t.spot);
+    const uint32_t nxy = (uint32_t) C.g.nx * (uint32_t) C.g.ny;
+    const uint32_t rem = d.cnb % nxy;
+    t.cell = make_int3((int) (rem % (uint32_t) C.g.nx), (int) (rem / (uint32_t) C.g.nx), (int) (d.cnb / nxy));
+    const uint32_t proc = d.mark & 3u;
+    if (proc == 1) post_pp<kMode>(C, t, rng);
+    else if (proc == 2) post_poe<kMode>(C, t, rng);
+    else post_poi<kMode>(C, t, rng);
+    score_step<kMode>(C, t, d.cnb, voxel_rho(C.g, d.cnb), grid_volume(C.g, t.cell));
+    if (!t.stopped) {
+        grid_step_index(C.g, t.p1, t.d1, t.cell);
+        t.p0  = t.p1;
+        t.d0  = t.d1;
+        t.ke0 = t.ke1;
+        t.dE = t.ldE = 0.0f;
+    }
+    if (!t.stopped && grid_valid(C.g, t.cell)) {
+        requeue_track(C, t, rng, kMetaPhaseStep, grid_cnb(C.g, t.cell));
         return;
     }
-    q.ke[i] = t.ke0;
-    q.px[i] = t.p0.x; q.py[i] = t.p0.y; q.pz[i] = t.p0.z;
-    q.dx[i] = t.d0.x; q.dy[i] = t.d0.y; q.dz[i] = t.d0.z;
-    q.dE0[i] = 0.0f;
-    q.hist[i] = t.hist;
-    q.uid_lo[i] = (uint32_t) t.uid;
-    q.uid_hi[i] = (uint32_t) (t.uid >> 32);
-    q.ctr[i] = rng.ctr;
-    q.meta[i] = track_meta(t) | kMetaPhaseStep;
-    q.cell[i] = grid_cnb(C.g, t.cell);
-    q.spot[i] = t.spot;
+    to_world(P.child[C.child], t.p0, t.d0);
+    ++t.child;
+    if (!t.stopped && t.child < P.n_children) {
+        requeue_track(C, t, rng, 0u, 0u);
+        return;
+    }
+    if (t.primary) count_event(kCntHist);
+    if (P.ready) atomicAdd(&P.drain->live, ~0ull);   // one live track fewer
+}
+
+/// A record in the array, into a copy of the thread's own: through L2, as L1 may hold a sector read
+/// before the record was written.
+__device__ inline void
+read_record(const Deferred* rec, Deferred& d) {
+    static_assert(sizeof(Deferred) % 4 == 0, "records are copied by words");
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(rec);
+    uint32_t*       dst = reinterpret_cast<uint32_t*>(&d);
+#pragma unroll
+    for (int k = 0; k < (int) (sizeof(Deferred) / 4); ++k) dst[k] = __ldcg(src + k);
+}
+
+/// Hand a track whose step ended in nuclear process `proc` to the post-step kernel, or in a draining
+/// wave to the warps that run the post-steps.  Returns false when a draining wave's record array is
+/// full: the record is then in `own`, for the lane to finish once its warp has no tracks.  (An
+/// ordinary wave hands over a track at most once, and its array is as long as its queue.)
+template<bool kDrain>
+__device__ inline bool
+defer_track(Ctx& C, const Trk& t, const Rng& rng, uint32_t cnb, int proc, Deferred& own) {
+    const WaveParams& P = *C.P;
+    const uint32_t    i = atomicAdd(&P.drain->tail, 1u);
+    if (i < P.def_cap) {
+        Deferred& d = P.def[i];
+        fill_record(d, t, rng, cnb);
+        if constexpr (kDrain) __threadfence();   // the record before its mark
+        *reinterpret_cast<volatile uint32_t*>(&d.mark) = (P.epoch << 2) | (uint32_t) proc;
+        return true;
+    }
+    if constexpr (kDrain) {
+        fill_record(own, t, rng, cnb);
+        own.mark = (uint32_t) proc;
+        return false;
+    }
+    atomicOr(P.error_flag, 2u);
+    count_event(kCntErr);
+    return true;
+}
+
+/// A draining wave's waiting post-steps: a warp takes up to 32 records that no other has taken and
+/// finishes them.  Returns the number of tracks still live before, and in `did` whether it found any.
+template<int kMode>
+static __device__ __noinline__ uint32_t
+post_waiting(const WaveParams* Pp, bool* did) {
+    const WaveParams& P    = *Pp;
+    const int         lane = threadIdx.x & 31;
+    uint32_t          base = 0, n = 0, left = 0;
+    if (lane == 0) {
+        const uint4    w    = __ldcv(reinterpret_cast<const uint4*>(P.drain));
+        const uint32_t tail = min(w.z, P.def_cap);
+        left                = w.x;
+        base                = w.w;
+        if (base < tail) {
+            n = min(tail - base, 32u);
+            if (atomicCAS(&P.drain->head, base, base + n) != base) n = 0;
+        }
+    }
+    left = __shfl_sync(0xFFFFFFFFu, left, 0);
+    n    = __shfl_sync(0xFFFFFFFFu, n, 0);
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    if ((uint32_t) lane < n) {
+        const Deferred* rec   = P.def + base + lane;
+        uint32_t        polls = 0;
+        // its writer has taken the place and is about to fill it
+        while (*reinterpret_cast<const volatile uint32_t*>(&rec->mark) >> 2 != P.epoch && ++polls < kDrainPolls) {
+        }
+        if (polls < kDrainPolls) {
+            __threadfence();   // the mark before the record
+            Deferred d;
+            read_record(rec, d);
+            post_record<kMode>(&P, &d);
+        } else {
+            count_event(kCntErr);
+            atomicAdd(&P.drain->live, ~0ull);
+        }
+    }
+    __syncwarp();
+    *did = n != 0;
+    return left;
 }
 
 /// A wave: persistent warps, a lane to a track, until the queue is used up.  A lane claims a queue
@@ -986,14 +1101,17 @@ requeue_track(Ctx& C, const Trk& t, const Rng& rng) {
 ///
 /// A wave drains (P.ready given) when its daughters go to the end of the queue it is reading: a lane
 /// whose index lies past the end keeps it and looks for the track each time round, and the warps
-/// leave when the count of live tracks -- queued or held, the low word of P.live -- is 0.  So a run of
-/// any number of generations is one launch and lasts as long as its longest chain of tracks, instead
-/// of the sum of each generation's longest.  No warp that holds a track waits for another, so the
-/// wave ends whichever blocks are resident.  Each entry is published by its own mark (P.ready[i] =
-/// P.epoch, a number of this launch's own) after a fence.  P.lanes < 32 spreads few tracks over more
-/// warps: a warp's step takes the sum of its lanes' different branches, so the fewer tracks share a
-/// warp, the sooner each ends.
-template<int kMode, bool kSplit>
+/// leave when the count of live tracks (the low word of DrainState::live: queued, held, or waiting
+/// for a post-step) is 0.  So a run of any number of generations is one launch and lasts as long as
+/// its longest chain of tracks, instead of the sum of each generation's longest.  A track stopped at a
+/// nuclear interaction becomes a record (defer_track) that one of a few warps without tracks
+/// finishes, or any warp that has run out of tracks; the step loop carries none of that code.  A warp
+/// that holds a track waits for no other, and one that holds none runs what waits, so the wave ends
+/// whichever blocks are resident.  Entries and records are published by marks of their own (the
+/// launch's epoch) after a fence.  P.lanes < 32 spreads few tracks over more warps: a warp's step
+/// takes the sum of its lanes' different branches, so the fewer tracks share a warp, the sooner each
+/// ends.
+template<int kMode, bool kDrain>
 __device__ __forceinline__ void
 wave_body(const WaveParams& P) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1037,26 +1155,31 @@ wave_body(const WaveParams& P) {
     C.tcut   = P.t_cut;
     uint32_t n_steps = 0;
 
-    Rng rng;
-    rng.k0 = P.k0;
-    rng.k1 = P.k1;
-    Trk  t;
-    bool     have    = false;   // the lane holds a track
-    bool     waits   = false;   // the lane holds queue index `ticket` and waits for a track there
-    bool     in_grid = false;
-    uint32_t ticket  = 0;
-    uint32_t slice = 0;
-    uint32_t track_steps = 0;   // per-track guard: a track is abandoned after kMaxTrackSteps
     // The input count can exceed the queue's capacity only after an overflowed append (the
     // append cursor counts on; nothing was written past the end).  The wave then does nothing:
     // the host reports the overflow, and no entry past the capacity is ever read.
     const uint32_t n_raw  = *P.n_in;
     const uint32_t n_in   = (n_raw > P.in.capacity || (*P.error_flag & 2u)) ? 0u : n_raw;
-    const bool     drains = !kSplit && P.ready != nullptr && n_in > 0;
     const int      lane   = threadIdx.x & 31;
-    bool           open   = lane < P.lanes;
-    uint32_t       polls  = 0;
+    // one warp in kPostEvery blocks takes no tracks and runs the waiting post-steps
+    const bool     posts  = kDrain && blockIdx.x % kPostEvery == kPostEvery - 1 && threadIdx.x >= blockDim.x - 32;
+    bool           open   = lane < P.lanes && !posts;   // the lane takes tracks
+    bool           waits  = false;                      // it holds queue index `ticket` and waits for a track there
+    bool           parked = false;                      // it holds a record, `own`, that the array had no room for
+    uint32_t       ticket = 0, polls = 0;
+    Deferred       own;
 
+    while (n_in > 0) {
+    // ---- the step loop, while the warp holds a track.  What follows it calls the post-steps: no track
+    // lives there, so the step's registers are not saved across those calls.
+    Rng rng;
+    rng.k0 = P.k0;
+    rng.k1 = P.k1;
+    Trk  t;
+    bool     have    = false;   // the lane holds a track
+    bool     in_grid = false;
+    uint32_t slice = 0;
+    uint32_t track_steps = 0;   // per-track guard: a track is abandoned after kMaxTrackSteps
     for (;;) {
         // ---- a queue index for every lane without one (one atomic per warp) ----
         const bool     want  = open && !have && !waits;
@@ -1074,7 +1197,7 @@ wave_body(const WaveParams& P) {
         // ---- the track at that index, once there is one ----
         if (waits) {
             bool there = ticket < n_in;
-            if (!there && drains) {
+            if (kDrain && !there) {
                 there = ticket < P.in.capacity && *reinterpret_cast<volatile uint32_t*>(P.ready + ticket) == P.epoch;
                 if (there) __threadfence();   // the mark before the entry
             } else if (!there) {
@@ -1090,7 +1213,7 @@ wave_body(const WaveParams& P) {
                 in_grid = step_phase;
                 slice   = 0;
                 track_steps = 0;
-                count_event(kCntTracks);
+                if (!kDrain || rng.ctr == 0u) count_event(kCntTracks);   // not one resumed after a post-step
                 if (step_phase) {
                     C.child = t.child;
                     C.g     = make_grid(P.child[t.child], s_edges[t.child][0], s_edges[t.child][1], s_edges[t.child][2]);
@@ -1102,23 +1225,9 @@ wave_body(const WaveParams& P) {
             }
         }
         const unsigned held = __ballot_sync(0xFFFFFFFFu, have);
-        if (!held) {
-            if (!drains) break;
-            // no track is left anywhere when the count of live ones is 0: nothing can follow.  The warps
-            // look for their own entry more often than at that one word.
-            if ((polls & 3u) == 0u) {
-                uint32_t left = 0;
-                if (lane == 0) left = (uint32_t) *reinterpret_cast<volatile unsigned long long*>(P.live);
-                if (__shfl_sync(0xFFFFFFFFu, left, 0) == 0u) break;
-            }
-            if (++polls > kDrainPolls) {   // never: a live track ends within kMaxTrackSteps steps
-                if (lane == 0) count_event(kCntErr);
-                break;
-            }
-            __nanosleep(500);
-            continue;
-        }
-        polls = 0;
+        if (!held) break;
+        polls       = 0;
+        bool handed = false;   // to a post-step: the track is still live
         if (have && !in_grid) {
             // ---- child entry (mqi_transport.hpp:161-190) ----
             C.child = t.child;
@@ -1159,11 +1268,13 @@ wave_body(const WaveParams& P) {
             const uint32_t cnb = grid_cnb(C.g, t.cell);
             const float    rho = voxel_rho(C.g, cnb);
             const float    d2b = grid_exit(C.g, t.p0, t.d0, t.cell);
-            const int      nuclear = stepping<kMode, kSplit>(C, t, rng, rho, d2b);
+            const int      nuclear = stepping<kMode>(C, t, rng, rho, d2b);
             ++n_steps;
-            if (kSplit && nuclear) {   // the post-step kernel finishes this step and queues the track
-                defer_track(C, t, rng, cnb, nuclear);
-                have = false;
+            if (nuclear) {   // the step is finished, and the track queued, elsewhere
+                parked = !defer_track<kDrain>(C, t, rng, cnb, nuclear, own);
+                open   = open && !parked;
+                have   = false;
+                handed = true;
             } else {
                 if (++track_steps > kMaxTrackSteps) {   // no physical track comes near this; never hang
                     t.stopped = true;
@@ -1191,16 +1302,38 @@ wave_body(const WaveParams& P) {
                         have = false;
                     }
                 } else if (P.max_slice_steps && ++slice >= P.max_slice_steps) {
-                    requeue_track(C, t, rng);
+                    requeue_track(C, t, rng, kMetaPhaseStep, grid_cnb(C.g, t.cell));
                     have = false;
                 }
             }
         }
-        if (drains) {
+        if constexpr (kDrain) {
             // tracks that ended leave the count of live ones after their daughters have joined it
-            const unsigned ended = held & ~__ballot_sync(0xFFFFFFFFu, have);
-            if (ended && lane == 0) atomicAdd(P.live, 0ull - (unsigned long long) __popc(ended));
+            const unsigned ended = held & ~__ballot_sync(0xFFFFFFFFu, have || handed);
+            if (ended && lane == 0) atomicAdd(&P.drain->live, 0ull - (unsigned long long) __popc(ended));
         }
+    }
+    if constexpr (!kDrain) break;
+    // ---- the warp holds no track
+    if (__any_sync(0xFFFFFFFFu, parked)) {
+        if (parked) post_record<kMode>(&P, &own);
+        __syncwarp();
+        open   = open || parked;
+        parked = false;
+        continue;
+    }
+    // It runs waiting post-steps, and leaves when no track is live: nothing can follow.
+    bool did;
+    if (post_waiting<kMode>(&P, &did) == 0u) break;
+    if (did) {
+        polls = 0;
+        continue;
+    }
+    if (++polls > kDrainPolls) {   // never: a live track ends within kMaxTrackSteps steps
+        if (lane == 0) count_event(kCntErr);
+        break;
+    }
+    __nanosleep(100);
     }
 
     // ---- counters: one global atomic per block and field ----
@@ -1210,84 +1343,17 @@ wave_body(const WaveParams& P) {
     if (threadIdx.x == 0 && s_cnt[kCntErr]) atomicOr(P.error_flag, 1u);
 }
 
-/// The post-step kernel's body: for each track the wave stopped at a nuclear interaction, the rest
-/// of its step as the wave would have run it -- the process's post_step (mqi_pp_elastic.hpp:119-219,
-/// mqi_po_elastic.hpp:96-217, mqi_po_inelastic.hpp:158-288), the step's scoring, the cell update
-/// and move() (mqi_transport.hpp:204-233) -- then the track goes to the next wave's queue: mid-grid,
-/// at the entry of the next child, or nowhere when it stopped or left the world.  The random
-/// stream resumes where the step left it (the process draw was the first word of the block at
-/// counter ctr - 1), so the track draws the same numbers as if the wave had run the process.
+/// The post-step kernel's body: every record that an ordinary wave left.
 template<int kMode>
 __device__ __forceinline__ void
 post_body(const WaveParams& P) {
-    Ctx C;
-    C.P     = &P;
-    C.T     = reinterpret_cast<const Tables*>(P.tables);
-    C.dbg   = P.physics_debug != 0;
-    C.tcut  = P.t_cut;
     if (threadIdx.x < 8) s_cnt[threadIdx.x] = 0u;
     __syncthreads();
-    const uint32_t n_raw  = *P.n_def;
-    const uint32_t n      = n_raw > P.in.capacity ? P.in.capacity : n_raw;   // past it: flagged, not written
+    const uint32_t n = min(P.drain->tail, P.def_cap);   // the wave finished those past the array itself
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const Deferred& d = P.def[i];
-        Trk t;
-        t.ke0 = d.ke0;
-        t.ke1 = d.ke1;
-        t.p0  = make_float3(d.p0[0], d.p0[1], d.p0[2]);
-        t.d0  = make_float3(d.d0[0], d.d0[1], d.d0[2]);
-        t.p1  = make_float3(d.p1[0], d.p1[1], d.p1[2]);
-        t.d1  = t.d0;
-        t.dE  = d.dE;
-        t.ldE = 0.0f;
-        t.spr0 = d.spr0;
-        t.uid  = (uint64_t) d.uid_lo | ((uint64_t) d.uid_hi << 32);
-        t.hist = d.hist;
-        t.spot = d.spot;
-        t.below   = d.meta & kMetaBelowMask;
-        t.primary = (d.meta & kMetaPrimary) != 0;
-        t.child   = (int) ((d.meta >> kMetaChildShift) & 7u);
-        t.npush   = (d.meta >> kMetaNpushShift) & 1023u;
-        t.stopped = false;
-        Rng rng;
-        rng.k0     = P.k0;
-        rng.k1     = P.k1;
-        rng.hist   = d.hist;
-        rng.uid_lo = d.uid_lo;
-        rng.uid_hi = d.uid_hi;
-        rng.ctr    = d.ctr;
-        rng.blk    = philox_block(d.ctr - 1u, d.hist, d.uid_lo, d.uid_hi, P.k0, P.k1);
-        rng.pos    = 1;
-        rng.has2   = false;
-        C.child = t.child;
-        C.spot  = t.spot;
-        C.g     = make_grid(P.child[t.child], nullptr, nullptr, nullptr);
-        apply_scenario(P, C.g, t.child, t.spot);
-        const uint32_t nxy = (uint32_t) C.g.nx * (uint32_t) C.g.ny;
-        const uint32_t rem = d.cnb % nxy;
-        t.cell = make_int3((int) (rem % (uint32_t) C.g.nx), (int) (rem / (uint32_t) C.g.nx), (int) (d.cnb / nxy));
-        if (d.proc == 1) post_pp<kMode>(C, t, rng);
-        else if (d.proc == 2) post_poe<kMode>(C, t, rng);
-        else post_poi<kMode>(C, t, rng);
-        score_step<kMode>(C, t, d.cnb, voxel_rho(C.g, d.cnb), grid_volume(C.g, t.cell));
-        if (!t.stopped) {
-            grid_step_index(C.g, t.p1, t.d1, t.cell);
-            t.p0  = t.p1;
-            t.d0  = t.d1;
-            t.ke0 = t.ke1;
-            t.dE = t.ldE = 0.0f;
-        }
-        if (!t.stopped && grid_valid(C.g, t.cell)) {
-            requeue_track(C, t, rng);
-            continue;
-        }
-        to_world(P.child[C.child], t.p0, t.d0);
-        ++t.child;
-        if (t.stopped || t.child >= P.n_children) {
-            if (t.primary) count_event(kCntHist);
-            continue;
-        }
-        requeue_entry(C, t, rng);
+        Deferred d;
+        read_record(P.def + i, d);
+        post_record<kMode>(&P, &d);
     }
     __syncthreads();
     if (threadIdx.x < 8 && s_cnt[threadIdx.x]) atomicAdd(&P.stats[threadIdx.x], (unsigned long long) s_cnt[threadIdx.x]);
@@ -1324,59 +1390,37 @@ write_vertex_entry(const Queue& q, uint32_t i, const mqi_vertex* __restrict__ v,
 }
 
 __global__ void
-k_load_primaries(Queue q, const mqi_vertex* __restrict__ v, const uint32_t* __restrict__ spot_ids, uint64_t h0,
+k_load_primaries(Queue q, uint32_t dst, const mqi_vertex* __restrict__ v, const uint32_t* __restrict__ spot_ids, uint64_t h0,
                  uint32_t n, uint32_t n_scen) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n * n_scen) return;
-    write_vertex_entry(q, i, v, spot_ids, h0 + i / n_scen, i % n_scen);
-}
-
-/// One thread: size the top-up of the queue holding *n_in entries (what the previous wave left).
-/// After a queue overflow (error bit 2) nothing more is loaded and the remaining waves of the
-/// graph find an empty queue.
-__global__ void
-k_topup(TopUp* tu, uint32_t* n_in, const uint32_t* error_flag) {
-    if (*error_flag & 2u) {
-        tu->count = 0;
-        *n_in     = 0;
-        return;
-    }
-    const uint32_t have = *n_in;
-    uint64_t       want = have < tu->target ? (tu->target - have) / tu->n_scen : 0ull;
-    const uint64_t left = tu->end - tu->next;
-    if (want > left) want = left;
-    tu->base  = tu->next;
-    tu->dst   = have;
-    tu->count = (uint32_t) (want * tu->n_scen);
-    tu->next += want;
-    *n_in = have + tu->count;
-}
-
-__global__ void
-k_load_topup(Queue q, const TopUp* __restrict__ tu, const mqi_vertex* __restrict__ v,
-             const uint32_t* __restrict__ spot_ids) {
-    const uint32_t n = tu->count, S = tu->n_scen, dst = tu->dst;
-    const uint64_t base = tu->base;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        write_vertex_entry(q, dst + i, v, spot_ids, base + i / S, i % S);
+    write_vertex_entry(q, dst + i, v, spot_ids, h0 + i / n_scen, i % n_scen);
 }
 
 cudaError_t
-launch_load_primaries(const Queue& q, const mqi_vertex* v, const uint32_t* spot_ids, uint64_t h0, uint32_t n,
+launch_load_primaries(const Queue& q, uint32_t dst, const mqi_vertex* v, const uint32_t* spot_ids, uint64_t h0, uint32_t n,
                       uint32_t n_scen, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     const uint32_t m = n * n_scen;
-    k_load_primaries<<<(m + 255) / 256, 256, 0, s>>>(q, v, spot_ids, h0, n, n_scen);
+    k_load_primaries<<<(m + 255) / 256, 256, 0, s>>>(q, dst, v, spot_ids, h0, n, n_scen);
     return cudaGetLastError();
 }
 
 /// The wave kernel in the launch shapes the tuner chooses from: (threads per block, minimum
-/// resident blocks per SM).  The register budget each shape implies is what differs.  Mode 0
-/// (DIRECT ROIs, simple scorer callbacks) comes in every shape; the other modes in 128 x 5.
-template<int kBlock, int kMinBlocks, int kMode, bool kSplit>
+/// resident blocks per SM).  The register budget each shape implies is what differs.  The common modes
+/// (DIRECT ROIs, simple scorer callbacks) come in every shape; the other modes in 128 x 5.
+template<int kBlock, int kMinBlocks, int kMode>
 __global__ void __launch_bounds__(kBlock, kMinBlocks)
 k_wave(const __grid_constant__ WaveParams P) {
-    wave_body<kMode, kSplit>(P);
+    wave_body<kMode, false>(P);
+}
+
+/// The draining wave, in every mode in two shapes.  A kernel apart from the ordinary wave, whose step
+/// loop is 15% faster for not sharing its registers and its image with the post-steps.
+template<int kMinBlocks, int kMode>
+__global__ void __launch_bounds__(kDrainBlock, kMinBlocks)
+k_drain(const __grid_constant__ WaveParams P) {
+    wave_body<kMode, true>(P);
 }
 
 constexpr int kPostBlock = 128;
@@ -1403,25 +1447,39 @@ wave_edge_floats(const ChildDev* c, int n) {
     return (f + 3) & ~3;
 }
 
-/// One wave.  With kSplit: the record count of the post-step kernel cleared, the wave kernel, then
-/// the post-step kernel over the tracks the wave stopped at nuclear interactions (a grid-stride
-/// loop over a count it reads on the device).  Without: the wave kernel alone.
-template<int B, int M, int K, bool S>
+/// An ordinary wave and the post-step kernel over the records it left (a grid-stride loop over a
+/// count it reads on the device).
+template<int B, int M, int K>
 static cudaError_t
 launch_variant(const WaveParams& p, int grid, cudaStream_t s) {
     const int   smem = wave_smem_bytes(p);
-    cudaError_t e    = cudaFuncSetAttribute(k_wave<B, M, K, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if constexpr (S) {
-        if (e == cudaSuccess) e = cudaMemsetAsync(p.n_def, 0, sizeof(uint32_t), s);
-    }
+    cudaError_t e    = cudaFuncSetAttribute(k_wave<B, M, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) {
         (void) cudaGetLastError();   // the failed call's error is returned here, not left for the next launch
         return e;
     }
-    if (p.max_blocks) grid = std::min(grid, p.max_blocks);
-    k_wave<B, M, K, S><<<grid, B, smem, s>>>(p);
-    if constexpr (S) k_post<K><<<grid, kPostBlock, 0, s>>>(p);
+    k_wave<B, M, K><<<grid, B, smem, s>>>(p);
+    k_post<K><<<grid, kPostBlock, 0, s>>>(p);
     return cudaGetLastError();
+}
+
+template<int M, int K>
+static cudaError_t
+launch_drain_shape(const WaveParams& p, int sms, cudaStream_t s) {
+    const int   smem = wave_smem_bytes(p);
+    cudaError_t e    = cudaFuncSetAttribute(k_drain<M, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) {
+        (void) cudaGetLastError();
+        return e;
+    }
+    k_drain<M, K><<<std::min(sms * M, p.max_blocks), kDrainBlock, smem, s>>>(p);
+    return cudaGetLastError();
+}
+
+template<int K>
+static cudaError_t
+launch_drain(const WaveParams& p, int sms, cudaStream_t s) {
+    return p.drain_shape == 4 ? launch_drain_shape<4, K>(p, sms, s) : launch_drain_shape<5, K>(p, sms, s);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1430,9 +1488,7 @@ launch_variant(const WaveParams& p, int grid, cudaStream_t s) {
 // taken a step yet form a class of their own, placed after the sorted tracks: they arrive grouped
 // (one spot's histories, one energy, neighbouring voxels) and keep that grouping, which
 // interleaving them with other spots of the same energy would break.  Protons are the only
-// transported particle type (moqui stacks only protons), so the type key is constant.  Each
-// kernel reads the entry count on the device and returns at once below sort_min, so the sort can
-// sit in a captured graph.  A warp claims one range per distinct class (one atomic each), so
+// transported particle type (moqui stacks only protons), so the type key is constant.  A warp claims one range per distinct class (one atomic each), so
 // entries of one class keep their order within a warp.
 // ------------------------------------------------------------------------------------------
 constexpr int kFreshPrimaryClass = kSortBins - 1;
@@ -1522,55 +1578,46 @@ launch_sort(const WaveParams& p, int grid, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-/// Instances: the split form in every launch shape of the common modes (one dose-like scorer, DIRECT
-/// ROIs) and in 128 x 5 for the others; the inline form in two shapes of the common modes and in
-/// 128 x 5 for the others: small runs, among them tps_env's per-spot runs with any scorers.
+/// Sort the wave's input when asked to, then run the instance of the run's scoring mode.
 cudaError_t
 launch_wave(const WaveParams& p, int grid, int block, int blocks_per_sm, cudaStream_t s) {
     const int grid5 = grid / (blocks_per_sm > 0 ? blocks_per_sm : 1) * 5;
+    if (!p.def || !p.drain) return cudaErrorInvalidValue;   // the post-steps need their records
     if (p.sort_bins) {
         const cudaError_t e = launch_sort(p, grid5, s);
         if (e != cudaSuccess) return e;
     }
-    if (!p.split) {
-        const bool wide = block != 128;
+    if (p.ready) {
+        const int sms = grid5 / 5;
         switch (p.kernel_mode) {
-        case 0:
-            return wide ? launch_variant<256, 2, 0, false>(p, grid, s) : launch_variant<128, 5, 0, false>(p, grid5, s);
-        case kModeSingle:
-            return wide ? launch_variant<256, 2, kModeSingle, false>(p, grid, s)
-                        : launch_variant<128, 5, kModeSingle, false>(p, grid5, s);
-        case kModeStat: return launch_variant<128, 5, kModeStat, false>(p, grid5, s);
-        case kModeDij: return launch_variant<128, 5, kModeDij, false>(p, grid5, s);
-        case kModeFull: return launch_variant<128, 5, kModeFull, false>(p, grid5, s);
+        case 0: return launch_drain<0>(p, sms, s);
+        case kModeSingle: return launch_drain<kModeSingle>(p, sms, s);
+        case kModeStat: return launch_drain<kModeStat>(p, sms, s);
+        case kModeDij: return launch_drain<kModeDij>(p, sms, s);
+        case kModeFull: return launch_drain<kModeFull>(p, sms, s);
         case kModeRoi:
-        case kModeFull | kModeRoi: return launch_variant<128, 5, kModeFull | kModeRoi, false>(p, grid5, s);
-        default: return launch_variant<128, 5, kModeAll, false>(p, grid5, s);
+        case kModeFull | kModeRoi: return launch_drain<kModeFull | kModeRoi>(p, sms, s);
+        default: return launch_drain<kModeAll>(p, sms, s);
         }
     }
-    if (!p.def || !p.n_def) return cudaErrorInvalidValue;   // the split form needs its record array
     switch (p.kernel_mode) {
-    case 0: break;
-    case kModeStat: return launch_variant<128, 5, kModeStat, true>(p, grid5, s);
+    case 0:
+        if (block != 128) return launch_variant<256, 2, 0>(p, grid, s);
+        if (blocks_per_sm >= 6) return launch_variant<128, 6, 0>(p, grid, s);
+        if (blocks_per_sm == 5) return launch_variant<128, 5, 0>(p, grid, s);
+        return launch_variant<128, 4, 0>(p, grid, s);
     case kModeSingle:
-        if (block == 128) {
-            if (blocks_per_sm >= 6) return launch_variant<128, 6, kModeSingle, true>(p, grid, s);
-            if (blocks_per_sm == 5) return launch_variant<128, 5, kModeSingle, true>(p, grid, s);
-            return launch_variant<128, 4, kModeSingle, true>(p, grid, s);
-        }
-        return launch_variant<256, 2, kModeSingle, true>(p, grid, s);
-    case kModeFull: return launch_variant<128, 5, kModeFull, true>(p, grid5, s);
-    case kModeRoi: return launch_variant<128, 5, kModeRoi, true>(p, grid5, s);
-    case kModeDij: return launch_variant<128, 5, kModeDij, true>(p, grid5, s);   // Dij (+ dose-like), DIRECT ROIs
-    case kModeFull | kModeRoi: return launch_variant<128, 5, kModeFull | kModeRoi, true>(p, grid5, s);
-    default: return launch_variant<128, 5, kModeAll, true>(p, grid5, s);   // any mode with Dij
+        if (block != 128) return launch_variant<256, 2, kModeSingle>(p, grid, s);
+        if (blocks_per_sm >= 6) return launch_variant<128, 6, kModeSingle>(p, grid, s);
+        if (blocks_per_sm == 5) return launch_variant<128, 5, kModeSingle>(p, grid, s);
+        return launch_variant<128, 4, kModeSingle>(p, grid, s);
+    case kModeStat: return launch_variant<128, 5, kModeStat>(p, grid5, s);
+    case kModeFull: return launch_variant<128, 5, kModeFull>(p, grid5, s);
+    case kModeRoi: return launch_variant<128, 5, kModeRoi>(p, grid5, s);
+    case kModeDij: return launch_variant<128, 5, kModeDij>(p, grid5, s);   // Dij (+ dose-like), DIRECT ROIs
+    case kModeFull | kModeRoi: return launch_variant<128, 5, kModeFull | kModeRoi>(p, grid5, s);
+    default: return launch_variant<128, 5, kModeAll>(p, grid5, s);   // any mode with Dij
     }
-    if (block == 128) {
-        if (blocks_per_sm >= 6) return launch_variant<128, 6, 0, true>(p, grid, s);
-        if (blocks_per_sm == 5) return launch_variant<128, 5, 0, true>(p, grid, s);
-        return launch_variant<128, 4, 0, true>(p, grid, s);
-    }
-    return launch_variant<256, 2, 0, true>(p, grid, s);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1855,20 +1902,11 @@ write_sampled_entry(const Queue& q, uint32_t i, const mqi_spot* __restrict__ spo
 }
 
 __global__ void
-k_sample_primaries(Queue q, const mqi_spot* __restrict__ spots, const uint64_t* __restrict__ cum, uint32_t n_spots,
+k_sample_primaries(Queue q, uint32_t dst, const mqi_spot* __restrict__ spots, const uint64_t* __restrict__ cum, uint32_t n_spots,
                    uint64_t h0, uint32_t n, uint32_t n_scen, uint32_t k0, uint32_t k1) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n * n_scen) return;
-    write_sampled_entry(q, i, spots, cum, n_spots, h0 + i / n_scen, i % n_scen, k0, k1);
-}
-
-__global__ void
-k_sample_topup(Queue q, const TopUp* __restrict__ tu, const mqi_spot* __restrict__ spots,
-               const uint64_t* __restrict__ cum, uint32_t n_spots, uint32_t k0, uint32_t k1) {
-    const uint32_t n = tu->count, S = tu->n_scen, dst = tu->dst;
-    const uint64_t base = tu->base;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        write_sampled_entry(q, dst + i, spots, cum, n_spots, base + i / S, i % S, k0, k1);
+    write_sampled_entry(q, dst + i, spots, cum, n_spots, h0 + i / n_scen, i % n_scen, k0, k1);
 }
 
 __global__ void
@@ -1888,11 +1926,11 @@ k_sample_vertices(mqi_vertex* __restrict__ out, uint32_t* __restrict__ spot_out,
 }
 
 cudaError_t
-launch_sample_primaries(const Queue& q, const mqi_spot* spots, const uint64_t* cum, uint32_t n_spots, uint64_t h0,
+launch_sample_primaries(const Queue& q, uint32_t dst, const mqi_spot* spots, const uint64_t* cum, uint32_t n_spots, uint64_t h0,
                         uint32_t n, uint32_t n_scen, uint32_t k0, uint32_t k1, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     const uint32_t m = n * n_scen;
-    k_sample_primaries<<<(m + 127) / 128, 128, 0, s>>>(q, spots, cum, n_spots, h0, n, n_scen, k0, k1);
+    k_sample_primaries<<<(m + 127) / 128, 128, 0, s>>>(q, dst, spots, cum, n_spots, h0, n, n_scen, k0, k1);
     return cudaGetLastError();
 }
 
@@ -1901,26 +1939,6 @@ launch_sample_vertices(mqi_vertex* out, uint32_t* spot_out, const mqi_spot* spot
                        uint64_t h0, uint32_t n, uint32_t k0, uint32_t k1, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     k_sample_vertices<<<(n + 127) / 128, 128, 0, s>>>(out, spot_out, spots, cum, n_spots, h0, n, k0, k1);
-    return cudaGetLastError();
-}
-
-cudaError_t
-launch_topup(TopUp* tu, uint32_t* n_in, const uint32_t* error_flag, cudaStream_t s) {
-    k_topup<<<1, 1, 0, s>>>(tu, n_in, error_flag);
-    return cudaGetLastError();
-}
-
-cudaError_t
-launch_load_topup(const Queue& q, const TopUp* tu, const mqi_vertex* v, const uint32_t* spot_ids, int sms,
-                  cudaStream_t s) {
-    k_load_topup<<<sms * 8, 256, 0, s>>>(q, tu, v, spot_ids);
-    return cudaGetLastError();
-}
-
-cudaError_t
-launch_sample_topup(const Queue& q, const TopUp* tu, const mqi_spot* spots, const uint64_t* cum, uint32_t n_spots,
-                    uint32_t k0, uint32_t k1, int sms, cudaStream_t s) {
-    k_sample_topup<<<sms * 8, 128, 0, s>>>(q, tu, spots, cum, n_spots, k0, k1);
     return cudaGetLastError();
 }
 

@@ -26,12 +26,13 @@
 //     caller before a retry.
 // Errors are reported as status codes; mqi_last_error(NULL) returns the message.
 #include <string>
+#include <utility>
 
 #include <cuda_runtime.h>
 
 #include "mqi_device.cuh"
 #include "mqi_gpu.h"
-#include "mqi_internal.h"
+#include "mqi_ctx.h"
 
 using namespace mqi_gpu;
 
@@ -43,15 +44,18 @@ constexpr uint32_t kNoallocQueueCap     = 3u * kNoallocChunk;  // entries per qu
 constexpr size_t   kNoallocCol          = (size_t) kNoallocQueueCap * 4;   // bytes per queue column
 constexpr int      kNoallocCols         = 15;
 constexpr size_t   kNoallocQueueBytes   = kNoallocCol * kNoallocCols;
-constexpr size_t   kNoallocCounterBytes = 256;                 // 8 x u32 counters, 8 x u64 stats
+constexpr size_t   kNoallocCounterBytes = 256;                 // 12 x u32 counters, 8 x u64 stats
+constexpr uint32_t kNoallocRecords      = 8192;                // post-step records; a wave finishes those past them itself
+constexpr size_t   kNoallocMarkBytes    = kNoallocCol + kNoallocRecords * sizeof(Deferred);   // ready marks, records
 constexpr size_t   kNoallocScratchBytes = 24u << 20;
 constexpr uint64_t kNoallocMaxHistories = 1ull << 24;
 constexpr int      kNoallocTableFloats  = 6 * MQI_TABLE_N + MQI_DENSITY_CORRECTION_N;
 
-static_assert(2 * kNoallocQueueBytes + kNoallocCounterBytes <= kNoallocScratchBytes, "scratch too small");
+static_assert(2 * kNoallocQueueBytes + kNoallocCounterBytes + kNoallocMarkBytes <= kNoallocScratchBytes, "scratch too small");
 static_assert(kNoallocCol % 256 == 0, "queue columns must stay 256-byte aligned");
 
-// The scratch: two SoA particle queues followed by the wave counters and run statistics.
+// The scratch: two SoA particle queues followed by the wave counters, the run statistics and the
+// marks and post-step records of draining waves.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocScratchBytes];
 // The physics tables the wave kernel stages into shared memory, in its order (the six 600-node
 // tables, then the HU density-correction factors), initialised at compile time.
@@ -178,8 +182,14 @@ mqi_transport_noalloc(int nx, int ny, int nz, const float* d_xe, const float* d_
     P.inline_local     = 1;
     P.head             = counters + 2;
     P.error_flag       = counters + 3;
-    P.lanes            = 32;
-    P.split            = 0;   // nuclear post-steps inside the wave: no post-step records to hold
+    P.n_in             = counters;
+    P.n_out            = counters + 1;
+    P.drain            = reinterpret_cast<DrainState*>(counters + 8);
+    unsigned char* marks = base + 2 * kNoallocQueueBytes + kNoallocCounterBytes;
+    P.ready            = reinterpret_cast<uint32_t*>(marks);
+    P.def              = reinterpret_cast<Deferred*>(marks + kNoallocCol);
+    P.def_cap          = kNoallocRecords;
+    P.epoch            = 1;   // the marks are cleared before every wave
     P.stats            = stats;
     P.spot_ids         = nullptr;
     P.tables           = tables;
@@ -193,32 +203,26 @@ mqi_transport_noalloc(int nx, int ny, int nz, const float* d_xe, const float* d_
     Queue*    B = &qb;
     for (uint64_t h = 0; h < n_histories; h += kNoallocChunk) {
         const uint32_t n = (uint32_t) ((n_histories - h) < kNoallocChunk ? (n_histories - h) : kNoallocChunk);
-        e = launch_load_primaries(*A, d_vertices, nullptr, h, n, 1, stream);
-        // a copy from pageable host memory returns once its source has been staged, so `n` may
-        // change before the copy reaches the device
-        if (e == cudaSuccess) e = cudaMemcpyAsync(counters, &n, sizeof(uint32_t), cudaMemcpyHostToDevice, stream);
-        if (e != cudaSuccess) return noalloc_fail(MQI_ERR_CUDA, std::string("mqi_transport_noalloc: ") + cudaGetErrorString(e));
-        int cur = 0;
-        for (int wave = 0;; ++wave) {
+        e = launch_load_primaries(*A, 0, d_vertices, nullptr, h, n, 1, stream);
+        uint32_t count = n;   // entries of the wave's queue: the load, then what found no room in it
+        for (int wave = 0; count > 0; ++wave) {
             if (wave > 100000) return noalloc_fail(MQI_ERR_DEVICE, "mqi_transport_noalloc: wave limit reached");
-            P.in    = *A;
-            P.out   = *B;
-            P.n_in  = counters + cur;
-            P.n_out = counters + (1 - cur);
-            uint32_t host_counts[4] = { 0, 0, 0, 0 };
-            e = cudaMemsetAsync(counters + (1 - cur), 0, sizeof(uint32_t), stream);
-            if (e == cudaSuccess) e = cudaMemsetAsync(counters + 2, 0, sizeof(uint32_t), stream);
+            P.in  = *A;
+            P.out = *B;
+            plan_drain(P, count, sms);
+            // a copy from pageable host memory returns once its source has been staged, so it may go
+            // out of scope before the copy reaches the device
+            uint32_t host_counts[12] = { count, 0, 0, 0, 0, 0, 0, 0, count, count, 0, 0 };
+            if (e == cudaSuccess) e = cudaMemcpyAsync(counters, host_counts, sizeof(host_counts), cudaMemcpyHostToDevice, stream);
+            if (e == cudaSuccess) e = cudaMemsetAsync(marks, 0, kNoallocMarkBytes, stream);
             if (e == cudaSuccess) e = launch_wave(P, grid, block, grid / sms, stream);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(host_counts, counters, sizeof(host_counts), cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(host_counts, counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
             if (e != cudaSuccess) return noalloc_fail(MQI_ERR_CUDA, std::string("mqi_transport_noalloc: ") + cudaGetErrorString(e));
             if (host_counts[3] & 2u) return noalloc_fail(MQI_ERR_OVERFLOW, "mqi_transport_noalloc: particle queue overflow (static scratch)");
             if (host_counts[3] & 1u) return noalloc_fail(MQI_ERR_DEVICE, "mqi_transport_noalloc: a bounded device loop gave up");
-            if (host_counts[1 - cur] == 0) break;
-            Queue* t = A;
-            A        = B;
-            B        = t;
-            cur      = 1 - cur;
+            count = host_counts[1];
+            std::swap(A, B);
         }
     }
     return MQI_OK;
