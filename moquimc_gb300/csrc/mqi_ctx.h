@@ -20,6 +20,12 @@
 namespace mqi_gpu
 {
 
+/// A child's material table at one density scale.
+struct Material {
+    float   scale = 1.0f;
+    float4* mat = nullptr;
+};
+
 struct ChildHost {
     int    nx = 0, ny = 0, nz = 0;
     float* xe = nullptr;
@@ -27,6 +33,7 @@ struct ChildHost {
     float* ze = nullptr;
     float* rho = nullptr;
     bool   has_rho = false;
+    std::vector<Material> mats;   // built by the first transport after the density or the curves changed
     float  rf[9], ri[9], tr[3];
     int    identity = 1;
 };

@@ -76,6 +76,7 @@ struct ChildDev {
     const float* ye;
     const float* ze;
     const float* rho;
+    const float4* mat;   // {density, spr_default's density factor, radiation length, -} per voxel, or null
     float        rf[9], ri[9], tr[3];
     int          identity;
     int          scorer_begin, n_scorers;
@@ -153,6 +154,7 @@ struct WaveParams {
     int       scen_stride;      // floats per scenario in scen_edges: nx+1 + ny+1 + nz+1
     const float* scen_edges;    // device: per-scenario x, y, z edges of scen_child
     float     scen_scale[kMaxScenarios];   // per-scenario density scale
+    const float4* scen_mat[kMaxScenarios]; // and the materials at that scale
     Queue     in;
     Queue     out;
     const uint32_t* n_in;       // device: number of entries in `in`
@@ -241,6 +243,9 @@ cudaError_t launch_sample_primaries(const Queue& q, uint32_t dst, const mqi_spot
                                     cudaStream_t s);
 cudaError_t launch_sample_vertices(mqi_vertex* out, uint32_t* spot_out, const mqi_spot* spots, const uint64_t* cum,
                                    uint32_t n_spots, uint64_t h0, uint32_t n, uint32_t k0, uint32_t k1, cudaStream_t s);
+// {density * scale, spr_default's density factor, radiation length, -} of n voxels.
+cudaError_t launch_materials(const float* rho, uint64_t n, float scale, int dbg, const CalibDev& calib, float4* mat, int sms,
+                             cudaStream_t s);
 cudaError_t launch_wave(const WaveParams& p, int grid, int block, int blocks_per_sm, cudaStream_t s);
 int         wave_smem_bytes(const WaveParams& p);
 int         wave_edge_floats(const ChildDev* c, int n);

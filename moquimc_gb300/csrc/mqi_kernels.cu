@@ -122,14 +122,28 @@ x0_table(const CalibDev& c, float rho) {
 /// The run's stopping-power ratio (compute_rsp_): the tables are out of line, so the default
 /// curve's step loop carries one uniform branch and a call.
 __device__ __forceinline__ float
-spr_of(const CalibDev& c, float rho, float Ek, bool dbg) {
-    return c.mode ? spr_table(c, rho, Ek) : spr_default(rho, Ek, dbg);
+spr_of(const CalibDev& c, const float4& m, float Ek, bool dbg) {
+    return c.mode ? spr_table(c, m.x, Ek) : spr_from_factor(m.x, Ek, dbg, m.y);
 }
 
-/// The run's radiation length (compute_rl_).
-__device__ __forceinline__ float
-x0_of(const CalibDev& c, float rho, bool dbg) {
-    return c.mode ? x0_table(c, rho) : radiation_length_default(rho, dbg);
+/// The same where it runs rarely.
+__device__ __noinline__ float
+spr_rare(const CalibDev* c, float rho, float factor, float Ek, bool dbg) {
+    return spr_of(*c, make_float4(rho, factor, 0.0f, 0.0f), Ek, dbg);
+}
+
+/// A voxel's material from its density: the density (g/mm^3), spr_default's density factor, and the
+/// run's radiation length (compute_rl_), both functions of the density alone.
+__device__ __forceinline__ float4
+material_from(const CalibDev& c, float rho, bool dbg) {
+    return make_float4(rho, spr_density_factor(rho), c.mode ? x0_table(c, rho) : radiation_length_default(rho, dbg), 0.0f);
+}
+
+/// Voxel cnb's material where no table holds it.
+__device__ __noinline__ float4
+material_rare(const WaveParams* P, int child, uint32_t sw, uint32_t cnb) {
+    const float scale = P->n_scen > 1 && child == P->scen_child ? P->scen_scale[sw >> kScenShift] : 1.0f;
+    return material_from(P->calib, __fmul_rn(P->child[child].rho[cnb], scale), P->physics_debug != 0);
 }
 
 __device__ inline Grid
@@ -139,8 +153,7 @@ make_grid(const ChildDev& c, const float* sxe, const float* sye, const float* sz
     g.xe = sxe ? sxe : c.xe;
     g.ye = sye ? sye : c.ye;
     g.ze = sze ? sze : c.ze;
-    g.rho = c.rho;
-    g.rho_scale = 1.0f;
+    g.mat = c.mat;
     return g;
 }
 
@@ -154,15 +167,34 @@ apply_scenario(const WaveParams& P, Grid& g, int child, uint32_t sw) {
         g.xe        = e;
         g.ye        = e + g.nx + 1;
         g.ze        = e + g.nx + g.ny + 2;
-        g.rho_scale = P.scen_scale[s];
+        g.mat       = P.scen_mat[s];
     }
 }
 
-/// Density of voxel cnb in the track's scenario: hu_to_density(hu) * DensityScaling as one FP32
-/// product (mqi_tps_env.hpp:766-769); the scale is 1 outside robust runs.
-__device__ inline float
-voxel_rho(const Grid& g, uint32_t cnb) {
-    return __fmul_rn(g.rho[cnb], g.rho_scale);
+/// The material of voxel cnb in the track's scenario: hu_to_density(hu) * DensityScaling as one FP32
+/// product (mqi_tps_env.hpp:766-769; the scale is 1 outside robust runs) and what follows from it.  The
+/// power and the logarithm in it took 8% of a step's instructions, so a context tabulates them per
+/// voxel (k_materials); a step reads them with its density, one 16-byte load from the same sector.
+__device__ __forceinline__ float4
+voxel_material(const Ctx& C, uint32_t cnb) {
+    if (C.g.mat) return C.g.mat[cnb];
+    return material_rare(C.P, C.child, C.spot, cnb);
+}
+
+__global__ void
+k_materials(const float* __restrict__ rho, uint64_t n, float scale, int dbg, const __grid_constant__ CalibDev calib,
+            float4* __restrict__ mat) {
+    for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < n; i += (uint64_t) gridDim.x * blockDim.x)
+        mat[i] = material_from(calib, __fmul_rn(rho[i], scale), dbg != 0);
+}
+
+cudaError_t
+launch_materials(const float* rho, uint64_t n, float scale, int dbg, const CalibDev& calib, float4* mat, int sms,
+                 cudaStream_t s) {
+    if (n == 0) return cudaSuccess;
+    k_materials<<<(unsigned) std::min<uint64_t>((n + 255) / 256, (uint64_t) sms * 8), 256, 0, s>>>(rho, n, scale, dbg, calib,
+                                                                                                 mat);
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------------------------------
@@ -332,7 +364,8 @@ compute_hit(int type, const Trk& t, float rho, float vol, float dose_w) {
 /// the slab-phantom throughput, the ROI mappings alone another 11%.
 template<int kMode = kModeAll>
 __device__ inline void
-score_step(Ctx& C, const Trk& t, uint32_t cnb, float rho, float vol) {
+score_step(Ctx& C, const Trk& t, uint32_t cnb, const float4& m, float vol) {
+    const float rho = m.x;
     constexpr bool kDij  = (kMode & kModeDij) != 0;
     constexpr bool kFull = (kMode & kModeFull) != 0;
     constexpr bool kRoi  = (kMode & kModeRoi) != 0;
@@ -342,7 +375,7 @@ score_step(Ctx& C, const Trk& t, uint32_t cnb, float rho, float vol) {
         const ScorerDev& s  = C.P->scorer[0];
         float            vf = t.dE + t.ldE;
         if (s.type == MQI_SCORER_DOSE_W) {
-            const float spr = t.spr0 >= 0.0f ? t.spr0 : spr_of(C.P->calib, rho, t.ke0, C.dbg);
+            const float spr = t.spr0 >= 0.0f ? t.spr0 : spr_rare(&C.P->calib, rho, m.y, t.ke0, C.dbg);
             vf              = (rho < 1.0e-7f) ? 0.0f : div_guarded(vf * 1.60218e-10f, vol * rho * spr);
         }
         tally_add(s.tally, cnb, (double) vf, cnb > 0 && vf > 0.0f);
@@ -355,7 +388,7 @@ score_step(Ctx& C, const Trk& t, uint32_t cnb, float rho, float vol) {
         if (ch.n_scorers == 0) return;
         const ScorerDev& sd  = C.P->scorer[ch.scorer_begin];
         const ScorerDev& sp  = C.P->scorer[ch.scorer_begin + 1];
-        const float      spr = t.spr0 >= 0.0f ? t.spr0 : spr_of(C.P->calib, rho, t.ke0, C.dbg);
+        const float      spr = t.spr0 >= 0.0f ? t.spr0 : spr_rare(&C.P->calib, rho, m.y, t.ke0, C.dbg);
         const float dose_w = (rho < 1.0e-7f) ? 0.0f : div_guarded((t.dE + t.ldE) * 1.60218e-10f, vol * rho * spr);
         if (!(dose_w > 0.0f)) return;
         const double   v  = (double) dose_w;
@@ -368,7 +401,7 @@ score_step(Ctx& C, const Trk& t, uint32_t cnb, float rho, float vol) {
     }
     const WaveParams& P   = *C.P;
     const ChildDev&   ch  = P.child[C.child];
-    const float       spr = t.spr0 >= 0.0f ? t.spr0 : spr_of(P.calib, rho, t.ke0, C.dbg);
+    const float       spr = t.spr0 >= 0.0f ? t.spr0 : spr_rare(&P.calib, rho, m.y, t.ke0, C.dbg);
     // dose_to_water of the step, shared by the dose, dose^2 and Dij scorers (Dw_pointer,
     // mqi_scorer_energy_deposit.hpp:23-40): 0 in vacuum voxels
     const float dose_w = (rho < 1.0e-7f) ? 0.0f : div_guarded((t.dE + t.ldE) * 1.60218e-10f, vol * rho * spr);
@@ -458,11 +491,10 @@ last_step_pos_spr(const Tables* T, float3 p0, float3 d0, float ke0, float dE, fl
     return make_float3(p0.x + d0.x * sl, p0.y + d0.y * sl, p0.z + d0.z * sl);
 }
 
-/// The same, out of line and with the ratio computed here (the step loop's cut branch, which ends
-/// each track once).
+/// The same, out of line (the step loop's cut branch, which ends each track once).
 __device__ __noinline__ float3
-last_step_pos(const Tables* T, const CalibDev* cal, bool dbg, float3 p0, float3 d0, float ke0, float dE, float rho) {
-    return last_step_pos_spr(T, p0, d0, ke0, dE, rho, spr_of(*cal, rho, ke0, dbg));
+last_step_pos(const Tables* T, float3 p0, float3 d0, float ke0, float dE, float rho, float spr) {
+    return last_step_pos_spr(T, p0, d0, ke0, dE, rho, spr);
 }
 
 /// What the reference does when it pops a deposit-only daughter (kinetic energy at or below
@@ -484,7 +516,8 @@ score_local_daughter(Ctx& C, float3 pw, float3 dw, float ke0, float dE0, uint32_
                        index_axis_hint(C.g.ze, C.g.nz, p.z, d.z, hint.z));
     if (!grid_valid(C.g, t.cell)) return false;
     const uint32_t cnb = grid_cnb(C.g, t.cell);
-    const float    rho = voxel_rho(C.g, cnb);
+    const float4   m   = voxel_material(C, cnb);
+    const float    rho = m.x;
     if (rho < 1.0e-7f) return false;
     const float d2b = grid_exit(C.g, p, d, t.cell);
     if (d2b < 0.0f) return true;   // the voxel loop breaks before scoring
@@ -495,10 +528,10 @@ score_local_daughter(Ctx& C, float3 pw, float3 dw, float ke0, float dE0, uint32_
     t.primary = false;
     if (rho <= 99.9f) {
         t.dE += t.ke0;
-        t.spr0 = spr_of(C.P->calib, rho, t.ke0, C.dbg);   // computed once for the position and the score
+        t.spr0 = spr_of(C.P->calib, m, t.ke0, C.dbg);   // computed once for the position and the score
         t.p1   = last_step_pos_spr(C.T, p, d, t.ke0, t.dE, rho, t.spr0);
     }
-    score_step<kMode>(C, t, cnb, rho, grid_volume(C.g, t.cell));
+    score_step<kMode>(C, t, cnb, m, grid_volume(C.g, t.cell));
     return true;
 }
 
@@ -625,16 +658,16 @@ energy_loss(const Tables& T, const Rel& rel, float rho, float len, float spr, fl
 /// block of random words is laid out as: [0] free path, [1,2] Box-Muller pair (straggling,
 /// scattering angle), [3] azimuth.
 __device__ inline void
-along_step(Ctx& C, Trk& t, const Rel& rel, float len, float rho, float spr, float z_strag, float z_mcs,
+along_step(Ctx& C, Trk& t, const Rel& rel, float len, const float4& m, float spr, float z_strag, float z_mcs,
            float u_phi) {
-    const float dE = energy_loss(*C.T, rel, rho, len, spr, z_strag);
+    const float dE = energy_loss(*C.T, rel, m.x, len, spr, z_strag);
     float       r  = 1.0f;
     if (dE >= t.ke0) {
         r         = t.ke0 / dE;
         t.stopped = true;
     }
     const float P     = rel.momentum();
-    const float X0    = x0_of(C.P->calib, rho, C.dbg);
+    const float X0    = m.z;
     const float s     = div_rn(kEs, P);
     const float th_n  = div_rn(s * s, rel.beta_sq) * len;
     const float th_sq = C.P->calib.mode ? th_n / X0 : div_rn(th_n, X0);   // a user's X0 may lie anywhere
@@ -777,7 +810,8 @@ post_poi(Ctx& C, Trk& t, Rng& rng) {
 /// returns the process, and post_record finishes the step elsewhere.
 template<int kMode>
 __device__ inline int
-stepping(Ctx& C, Trk& t, Rng& rng, float rho, float d2b) {
+stepping(Ctx& C, Trk& t, Rng& rng, const float4& m, float d2b) {
+    const float rho = m.x;
     t.spr0 = -1.0f;
     if (rho < 1.0e-7f) {
         t.p1 = advance(t.p0, t.d0, d2b);
@@ -791,14 +825,15 @@ stepping(Ctx& C, Trk& t, Rng& rng, float rho, float d2b) {
         if (t.ke0 < 0.0f) t.ke0 = 0.0f;
         t.dE += t.ke0;
         t.ke1 -= t.ke0;
-        t.p1      = last_step_pos(C.T, &C.P->calib, C.dbg, t.p0, t.d0, t.ke0, t.dE, rho);
+        t.spr0    = spr_rare(&C.P->calib, rho, m.y, t.ke0, C.dbg);   // for the position and the score
+        t.p1      = last_step_pos(C.T, t.p0, t.d0, t.ke0, t.dE, rho, t.spr0);
         t.stopped = true;
         return 0;
     }
     const Tables& T = *C.T;
     rng.begin_step();
     const Rel   rel(t.ke0);
-    const float spr      = spr_of(C.P->calib, rho, t.ke0, C.dbg);
+    const float spr      = spr_of(C.P->calib, m, t.ke0, C.dbg);
     const float dedx     = dedx_lookup(T, rel.Ek);
     const float cur_min  = div_by(kMaxStep * spr * rho, kWaterDensity, kPerWaterDensity);
     const float max_loss = -1.0f * cur_min * dedx;
@@ -832,7 +867,7 @@ stepping(Ctx& C, Trk& t, Rng& rng, float rho, float d2b) {
     const bool interaction = !to_boundary && (mfp < d2b || fabsf(mfp - d2b) < kGeoTol) &&
                              (mfp < step_limit || fabsf(mfp - step_limit) < kGeoTol);
     const float len = to_boundary ? d2b : (interaction ? mfp : step_limit);
-    along_step(C, t, rel, len, rho, spr, z1, z2, u_phi);
+    along_step(C, t, rel, len, m, spr, z1, z2, u_phi);
     t.spr0 = spr;
     if (interaction && t.ke1 > kTpCut) {
         const float u = cs_sum * rng.uniform();
@@ -993,7 +1028,7 @@ post_record(const WaveParams* Pp, const Deferred* rec) {
     if (proc == 1) post_pp<kMode>(C, t, rng);
     else if (proc == 2) post_poe<kMode>(C, t, rng);
     else post_poi<kMode>(C, t, rng);
-    score_step<kMode>(C, t, d.cnb, voxel_rho(C.g, d.cnb), grid_volume(C.g, t.cell));
+    score_step<kMode>(C, t, d.cnb, voxel_material(C, d.cnb), grid_volume(C.g, t.cell));
     if (!t.stopped) {
         grid_step_index(C.g, t.p1, t.d1, t.cell);
         t.p0  = t.p1;
@@ -1266,9 +1301,9 @@ wave_body(const WaveParams& P) {
             // ---- one voxel step (mqi_transport.hpp:192-233) ----
             C.spot = t.spot;
             const uint32_t cnb = grid_cnb(C.g, t.cell);
-            const float    rho = voxel_rho(C.g, cnb);
+            const float4   mat = voxel_material(C, cnb);
             const float    d2b = grid_exit(C.g, t.p0, t.d0, t.cell);
-            const int      nuclear = stepping<kMode>(C, t, rng, rho, d2b);
+            const int      nuclear = stepping<kMode>(C, t, rng, mat, d2b);
             ++n_steps;
             if (nuclear) {   // the step is finished, and the track queued, elsewhere
                 parked = !defer_track<kDrain>(C, t, rng, cnb, nuclear, own);
@@ -1282,7 +1317,7 @@ wave_body(const WaveParams& P) {
                 }
                 bool leave = true;
                 if (!(d2b < 0.0f)) {
-                    score_step<kMode>(C, t, cnb, rho, grid_volume(C.g, t.cell));
+                    score_step<kMode>(C, t, cnb, mat, grid_volume(C.g, t.cell));
                     if (!t.stopped) {
                         grid_step_index(C.g, t.p1, t.d1, t.cell);
                         t.p0  = t.p1;
@@ -1787,10 +1822,10 @@ k_eval_hits(const __grid_constant__ ChildDev c, const __grid_constant__ CalibDev
         const uint32_t v   = cnb[i];
         const uint32_t nxy = (uint32_t) g.nx * (uint32_t) g.ny;
         const int3     cell = make_int3((int) (v % nxy % (uint32_t) g.nx), (int) (v % nxy / (uint32_t) g.nx), (int) (v / nxy));
-        const float rho = g.rho[v];
+        const float rho = c.rho[v];
         const float vol = grid_volume(g, cell);
         // dose_to_water of the step exactly as score_step forms it
-        const float spr    = spr_of(cal, rho, t.ke0, dbg != 0);
+        const float spr    = spr_of(cal, material_from(cal, rho, dbg != 0), t.ke0, dbg != 0);
         const float dose_w = (rho < 1.0e-7f) ? 0.0f : (t.dE + t.ldE) * 1.60218e-10f / (vol * rho * spr);
         out[i]             = compute_hit(type, t, rho, vol, dose_w);
     }
