@@ -584,6 +584,7 @@ make_wave_params(mqi_ctx* c, uint64_t seed, WaveParams& P) {
         if (!s0.stat_mode && s0.tstride == 1 && (s0.type == MQI_SCORER_EDEP || s0.type == MQI_SCORER_DOSE_W))
             P.kernel_mode = kModeSingle;
     }
+    if (P.kernel_mode == kModeDij && c->scorers.size() == 1) P.kernel_mode = kModeDijAlone;
     if (P.kernel_mode == 0 && c->scorers.size() == 3) {
         // a dose scorer followed by the statistics pair, all DIRECT, on one child
         const ScorerHost& a = c->scorers[0];

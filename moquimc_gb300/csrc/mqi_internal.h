@@ -48,6 +48,8 @@ constexpr int kModeStat = 16;  // one dose-to-water scorer and the statistics pa
                                // child (any number of children and scenarios): tps_env's Dose with
                                // StoppingStatistics
 
+constexpr int kModeDijAlone = 32;   // one Dij scorer, DIRECT ROI, nothing else: tps_env's Dij runs
+
 /// Flat device description of one scorer (scorer<R> + roi_t, mqi_scorer.hpp:39-79,
 /// mqi_roi.hpp:18-194).
 struct ScorerDev {

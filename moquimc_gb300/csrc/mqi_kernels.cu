@@ -213,59 +213,47 @@ tally_add(double* tally, uint64_t slot, double v, bool valid) {
     if (valid) atomicAdd(&tally[slot], v);
 }
 
-/// Hash of a Dij key: the splitmix64 finalizer (Steele, Lea & Flood, "Fast splittable
-/// pseudorandom number generators", OOPSLA 2014).
-__device__ inline uint64_t
-dij_hash(uint64_t k) {
-    k ^= k >> 30;
-    k *= 0xBF58476D1CE4E5B9ull;
-    k ^= k >> 27;
-    k *= 0x94D049BB133111EBull;
-    k ^= k >> 31;
-    return k;
+/// Hash of a Dij key (tables have at most 2^32 slots): odd multiples of the voxel and the spot, mixed by
+/// the "lowbias32" finaliser (Wellons, "Prospecting for Hash Functions", 2018).  A spot's voxels
+/// never collide in the 32 bits.  In 32-bit arithmetic, as a 64-bit product takes several instructions.
+__device__ inline uint32_t
+dij_hash(uint32_t spot, uint32_t voxel) {
+    uint32_t h = voxel * 0x9E3779B1u ^ spot * 0x85EBCA77u;
+    h ^= h >> 16;
+    h *= 0x7FEB352Du;
+    h ^= h >> 15;
+    h *= 0x846CA68Bu;
+    h ^= h >> 16;
+    return h;
 }
 
-/// Add v to the Dij entry (spot, voxel).  Lanes of the warp with the same table and key are
-/// combined first (two match rounds: the key, then the table), so one insertion is issued per
-/// distinct entry.  The leader probes linearly from the hashed slot: a slot holding the key takes
-/// the add; an empty slot is claimed with one 64-bit CAS.  After kDijMaxProbes probes the table
-/// counts as full and the error flag's bit 4 is set.  Claims are not counted here (a counter
+/// Add v to the Dij entry (spot, voxel): a linear probe from the hashed slot.  A slot holding the key
+/// takes the add; an empty slot is claimed with one 64-bit CAS.  After kDijMaxProbes probes the table
+/// counts as full and the error flag's bit 4 is set.  Each lane inserts for itself: lanes of a warp
+/// stand at different depths and rarely share an entry, and combining those that do
+/// (__match_any_sync on the key and the table, shuffles) cost 5% of the transport of a 75-spot Dij
+/// (28.5 -> 27.1 ms without, 26.9 with the 32-bit hash, 25.3 in an instance of its own).  Claims are not counted here (a counter
 /// bumped on every claim, one address for every SM, cost 8% of the Dij transport): the occupied
 /// slots are counted by one pass over the table when the count is needed (k_dij_count).
 __device__ inline void
 dij_add(const ScorerDev& s, uint32_t* error_flag, uint32_t spot, uint32_t voxel, double v, bool valid) {
-    DijSlot* const           table      = s.dij;
-    const uint64_t           table_mask = s.dij_mask;
-    if (s.hit_log && valid) {   // recorded insertions, for checking the table against a replay
+    if (!valid) return;
+    if (s.hit_log) {   // recorded insertions, for checking the table against a replay
         const unsigned long long i = atomicAdd(s.hit_count, 1ull);
         if (i < s.hit_cap) s.hit_log[i] = DijHit{ voxel, spot, v };
     }
-    const unsigned           mask  = __activemask();
-    const unsigned long long key   = ((((unsigned long long) spot) << 32) | voxel) + 1ull;
-    const unsigned           peers = __match_any_sync(mask, valid ? key : 0ull) &
-                           __match_any_sync(mask, (unsigned long long) table);
-    if (!valid) return;
-    double   sum = v;
-    if (__popc(peers) > 1) {
-        sum = 0.0;
-        unsigned m = peers;
-        while (m) {
-            const int src = __ffs(m) - 1;
-            sum += __shfl_sync(peers, v, src);
-            m &= m - 1;
-        }
-        if ((int) (threadIdx.x & 31) != __ffs(peers) - 1) return;
-    }
-    uint64_t slot = dij_hash(key) & table_mask;
+    const unsigned long long key  = ((((unsigned long long) spot) << 32) | voxel) + 1ull;
+    const uint32_t           mask = (uint32_t) s.dij_mask;
+    uint32_t                 slot = dij_hash(spot, voxel) & mask;
     for (uint32_t probe = 0; probe < kDijMaxProbes; ++probe) {
-        DijSlot* e = table + slot;
+        DijSlot*           e = s.dij + slot;
         unsigned long long k = *reinterpret_cast<volatile unsigned long long*>(&e->key);
         if (k == 0ull) k = atomicCAS(&e->key, 0ull, key);
         if (k == 0ull || k == key) {
-            atomicAdd(&e->value, sum);
+            atomicAdd(&e->value, v);
             return;
         }
-        slot = (slot + 1) & table_mask;
+        slot = (slot + 1u) & mask;
     }
     atomicOr(error_flag, 4u);
 }
@@ -397,6 +385,16 @@ score_step(Ctx& C, const Trk& t, uint32_t cnb, const float4& m, float vol) {
         double* pair = sp.tally + (sc * sp.tally_len + cnb) * 2;    // DIRECT: get_mask_idx(cnb) = cnb
         atomicAdd(pair, v);
         atomicAdd(pair + 1, v * v);
+        return;
+    }
+    if constexpr (kMode == kModeDijAlone) {
+        // dose_to_water into the one table: no per-scorer loop (as for the single dense scorer)
+        const ChildDev& ch = C.P->child[C.child];
+        if (ch.n_scorers == 0) return;
+        const float    spr    = t.spr0 >= 0.0f ? t.spr0 : spr_rare(&C.P->calib, rho, m.y, t.ke0, C.dbg);
+        const float    dose_w = (rho < 1.0e-7f) ? 0.0f : div_guarded((t.dE + t.ldE) * 1.60218e-10f, vol * rho * spr);
+        const uint32_t col    = (C.spot & kSpotMask) == kNoSpot ? 0u : (C.spot & kSpotMask);
+        dij_add(C.P->scorer[0], C.P->error_flag, col, cnb, (double) dose_w, cnb > 0 && dose_w > 0.0f);
         return;
     }
     const WaveParams& P   = *C.P;
@@ -1629,6 +1627,7 @@ launch_wave(const WaveParams& p, int grid, int block, int blocks_per_sm, cudaStr
         case kModeSingle: return launch_drain<kModeSingle>(p, sms, s);
         case kModeStat: return launch_drain<kModeStat>(p, sms, s);
         case kModeDij: return launch_drain<kModeDij>(p, sms, s);
+        case kModeDijAlone: return launch_drain<kModeDijAlone>(p, sms, s);
         case kModeFull: return launch_drain<kModeFull>(p, sms, s);
         case kModeRoi:
         case kModeFull | kModeRoi: return launch_drain<kModeFull | kModeRoi>(p, sms, s);
@@ -1649,7 +1648,8 @@ launch_wave(const WaveParams& p, int grid, int block, int blocks_per_sm, cudaStr
     case kModeStat: return launch_variant<128, 5, kModeStat>(p, grid5, s);
     case kModeFull: return launch_variant<128, 5, kModeFull>(p, grid5, s);
     case kModeRoi: return launch_variant<128, 5, kModeRoi>(p, grid5, s);
-    case kModeDij: return launch_variant<128, 5, kModeDij>(p, grid5, s);   // Dij (+ dose-like), DIRECT ROIs
+    case kModeDij: return launch_variant<128, 5, kModeDij>(p, grid5, s);   // Dij + dose-like, DIRECT ROIs
+    case kModeDijAlone: return launch_variant<128, 5, kModeDijAlone>(p, grid5, s);
     case kModeFull | kModeRoi: return launch_variant<128, 5, kModeFull | kModeRoi>(p, grid5, s);
     default: return launch_variant<128, 5, kModeAll>(p, grid5, s);   // any mode with Dij
     }

@@ -115,3 +115,25 @@ def test_dij_and_scenarios(gpu_ctx_factory):
         res[-1] += (d.tally(ids[0]), d.stats()["steps"])
     for x, y in zip(*res):
         np.testing.assert_allclose(x, y, rtol=2.0 ** -23, atol=1e-300)
+
+
+@pytest.mark.parametrize("mode", [-1, 1])
+@pytest.mark.parametrize("capacity", [1 << 21, 1 << 13])
+def test_dij_alone_instance(gpu_ctx_factory, mode, capacity):
+    """A Dij scorer by itself runs an instance of its own; beside a dense scorer it takes the generic
+    scoring loop.  The same matrix from a sparse table and from one that is mostly full."""
+    sp = workloads.spot_plan(2, 2, 6.0, 0.5, 3.0, (60.0, 90.0), (300.0, 700.0))
+    csr = []
+    for extra in (False, True):
+        c, cid = _box(gpu_ctx_factory, False)
+        c.set_post_step_mode(mode)
+        dij = c.add_dij_scorer(cid, capacity=capacity)
+        if extra:
+            c.add_scorer(cid, capi.EDEP)
+        n = c.set_spot_plan(sp)
+        c.transport_plan(0, n, 23)
+        csr.append(c.dij_build(dij).csr())
+    np.testing.assert_array_equal(csr[0][0], csr[1][0])
+    np.testing.assert_array_equal(csr[0][1], csr[1][1])
+    np.testing.assert_allclose(csr[0][2], csr[1][2], rtol=2.0 ** -23, atol=0)
+    assert csr[0][0][-1] > capacity // 2 or capacity > 1 << 13
