@@ -189,6 +189,7 @@ mqi_destroy(mqi_ctx* c) {
         dij_release(s);
     }
     cudaFree(c->stat_scratch);
+    cudaFree(c->build_scratch);
     cudaFree(c->plan_spots);
     cudaFree(c->plan_cum);
     cudaFree(c->scen_edges);

@@ -25,14 +25,38 @@ bit_length(uint64_t v) {
 
 void
 free_csr(DijCsr& m) {
-    cudaFree(m.s_indptr); cudaFree(m.s_voxel); cudaFree(m.s_value);
-    cudaFree(m.v_row); cudaFree(m.v_indptr); cudaFree(m.v_spot); cudaFree(m.v_value);
-    cudaFree(m.seg_start); cudaFree(m.row_seg); cudaFree(m.seg_order); cudaFree(m.bwd_cursor);
-    cudaFree(m.partial); cudaFree(m.fwd_row_first); cudaFree(m.fwd_run_k);
+    cudaFree(m.slab);
     m = DijCsr{};
 }
 
-/// Device buffers freed on scope exit unless released.
+/// Arrays cut from one allocation, each on a 256-byte boundary.  Laid out first with no memory, for
+/// its size.
+struct Carve {
+    char*  base = nullptr;
+    size_t used = 0;
+    template<typename T>
+    void
+    take(T*& p, uint64_t n) {
+        p = base ? reinterpret_cast<T*>(base + used) : nullptr;
+        used += (std::max<uint64_t>(n, 1) * sizeof(T) + 255) & ~(size_t) 255;
+    }
+};
+
+/// At least `bytes` in p, whose contents are not kept: what is there when that is enough and not far
+/// more, else an allocation of its own.  (A build's two dozen allocations took 1.5 ms of a 4 ms build.)
+cudaError_t
+ensure_bytes(void*& p, size_t& have, size_t bytes) {
+    if (p && have >= bytes && have / 4 <= bytes) return cudaSuccess;
+    cudaFree(p);
+    p             = nullptr;
+    have          = 0;
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaSuccess) have = bytes;
+    else p = nullptr;
+    return e;
+}
+
+/// Device buffers freed on scope exit.
 struct Scratch {
     std::vector<void*> ptrs;
     template<typename T>
@@ -42,10 +66,6 @@ struct Scratch {
         cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), std::max<uint64_t>(n, 1) * sizeof(T));
         if (e == cudaSuccess) ptrs.push_back(p);
         return e;
-    }
-    void
-    release(void* p) {
-        ptrs.erase(std::remove(ptrs.begin(), ptrs.end(), p), ptrs.end());
     }
     ~Scratch() {
         for (void* p : ptrs) cudaFree(p);
@@ -87,7 +107,7 @@ dij_release(ScorerHost& s) {
 
 cudaError_t
 dij_reset(ScorerHost& s, int sms, cudaStream_t st) {
-    free_csr(s.csr);
+    s.csr.built   = false;
     cudaError_t e = dij_clear(s.dij, s.dij_cap, sms, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(s.dij_count, 0, sizeof(unsigned long long), st);
     return e;
@@ -202,61 +222,114 @@ mqi_dij_build(mqi_ctx* c, int id, uint32_t n_spots, double scale, uint64_t* nnz_
     const uint64_t nvox = (uint64_t) ch.nx * ch.ny * ch.nz;
     DeviceGuard g(c->device);
     cudaStream_t st = c->stream;
-    free_csr(s.csr);
+    s.csr.built = false;
     unsigned long long count = 0;
     MQI_CUDA(c, dij_count(s.dij, s.dij_cap, s.dij_count, c->num_sms, st), "mqi_dij_build: count");
     MQI_CUDA(c, cudaMemcpyAsync(&count, s.dij_count, sizeof(count), cudaMemcpyDeviceToHost, st), "mqi_dij_build");
     MQI_CUDA(c, cudaStreamSynchronize(st), "mqi_dij_build");
     const uint64_t n = count;
+    const int      vbits = bit_length(nvox - 1), sbits = bit_length((uint64_t) n_spots - 1);
 
-    Scratch sc;
-    unsigned long long *ka, *kb, *kc, *cursor;
-    uint32_t *ia, *ib, *ic, *hist, *offs, *scan, *flags, *rowid;
-    const uint64_t hw = radix_hist_words(n);
-    MQI_CUDA(c, sc.alloc(ka, n), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(kb, n), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(kc, n), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(ia, n), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(ib, n), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(ic, n), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(hist, hw), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(offs, hw), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(scan, std::max(scan_scratch_words(hw), scan_scratch_words(n))), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(flags, n), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(rowid, n), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(cursor, 1), "mqi_dij_build: allocation");
+    // the sort's buffers
+    unsigned long long *keys, *keys_alt, *cursor;
+    uint32_t *vals, *vals_alt, *hist, *offs, *scan, *bad;
+    auto lay_out_scratch = [&](Carve cv) {
+        const uint64_t hw = radix_hist_words(n);
+        cv.take(keys, n);
+        cv.take(keys_alt, n);
+        cv.take(vals, n);
+        cv.take(vals_alt, n);
+        cv.take(hist, hw);
+        cv.take(offs, hw);
+        cv.take(scan, scan_scratch_words(hw));
+        cv.take(cursor, 1);
+        cv.take(bad, 1);
+        return cv.used;
+    };
+    const size_t scratch_bytes = lay_out_scratch(Carve{});
+    struct GiveBack {   // at the end, when it is large
+        mqi_ctx* c;
+        ~GiveBack() {
+            if (c->build_scratch_bytes <= kKeepScratch) return;
+            cudaFree(c->build_scratch);
+            c->build_scratch       = nullptr;
+            c->build_scratch_bytes = 0;
+        }
+    } give_back{ c };
 
+    // the matrix: segments of the backward are bounded by whole ones and one more per row, voxel rows by
+    // the entries and by the voxels
     DijCsr m;
-    m.n_spots  = n_spots;
-    m.n_voxels = nvox;
-    m.nnz      = n;
-    MQI_CUDA(c, sc.alloc(m.s_indptr, (uint64_t) n_spots + 1), "mqi_dij_build: allocation");
-    // entry arrays padded to whole groups of four: the products read them with 16-byte loads
-    MQI_CUDA(c, sc.alloc(m.s_voxel, n + 4), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(m.s_value, n + 4), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(m.v_spot, n + 4), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(m.v_value, n + 4), "mqi_dij_build: allocation");
+    const uint64_t max_seg = n / kDijSegment + std::min<uint64_t>(n_spots, n), max_vrows = std::min(n, nvox);
+    const uint64_t n_runs  = (n + kFwdEntries - 1) / kFwdEntries;
+    auto lay_out = [&](Carve cv) {
+        cv.take(m.s_indptr, (uint64_t) n_spots + 1);
+        // entry arrays padded to whole groups of four: the products read them with 16-byte loads
+        cv.take(m.s_voxel, n + 4);
+        cv.take(m.s_value, n + 4);
+        cv.take(m.v_spot, n + 4);
+        cv.take(m.v_value, n + 4);
+        cv.take(m.v_row, max_vrows);
+        cv.take(m.v_indptr, max_vrows + 1);
+        cv.take(m.seg_start, max_seg + 1);
+        cv.take(m.row_seg, (uint64_t) n_spots + 1);
+        cv.take(m.seg_order, max_seg);
+        cv.take(m.partial, max_seg);
+        cv.take(m.bwd_cursor, 1);
+        cv.take(m.fwd_row_first, n_runs + 1);
+        cv.take(m.fwd_run_k, n_runs + 1);
+        return cv.used;
+    };
+    const size_t csr_bytes = lay_out(Carve{});
+    // products queued on any stream may still read the last matrix
+    if (s.csr.slab) MQI_CUDA(c, cudaDeviceSynchronize(), "mqi_dij_build");
+    MQI_CUDA(c, ensure_bytes(c->build_scratch, c->build_scratch_bytes, scratch_bytes), "mqi_dij_build: allocation");
+    MQI_CUDA(c, ensure_bytes(s.csr.slab, s.csr.slab_bytes, csr_bytes), "mqi_dij_build: allocation");
+    lay_out_scratch(Carve{ static_cast<char*>(c->build_scratch) });
+    lay_out(Carve{ static_cast<char*>(s.csr.slab) });
+    m.slab       = s.csr.slab;
+    m.slab_bytes = s.csr.slab_bytes;
+    m.n_spots    = n_spots;
+    m.n_voxels   = nvox;
+    m.nnz        = n;
 
-    // 1. compact the table to (spot * n_voxels + voxel, slot) pairs
-    MQI_CUDA(c, dij_compact(s.dij, s.dij_cap, nvox, ka, ia, n, cursor, c->num_sms, st), "mqi_dij_build: compact");
+    // 1. the table's entries, in any order
+    MQI_CUDA(c, dij_compact(s.dij, s.dij_cap, vbits, n_spots, scale, keys, vals, n, cursor, bad, c->num_sms, st),
+             "mqi_dij_build: compact");
     unsigned long long got = 0;
+    uint32_t           is_bad = 0;
     MQI_CUDA(c, cudaMemcpyAsync(&got, cursor, sizeof(got), cudaMemcpyDeviceToHost, st), "mqi_dij_build");
+    MQI_CUDA(c, cudaMemcpyAsync(&is_bad, bad, sizeof(is_bad), cudaMemcpyDeviceToHost, st), "mqi_dij_build");
     MQI_CUDA(c, cudaStreamSynchronize(st), "mqi_dij_build");
     if (got != n) return fail(c, MQI_ERR_DEVICE, "mqi_dij_build: occupied slots disagree with the insertion count");
+    if (is_bad) return fail(c, MQI_ERR_INVALID, "mqi_dij_build: the table holds a spot index >= n_spots");
 
-    // 2. sort by (spot, voxel): spot rows, voxels ascending
-    unsigned long long* skeys = ka;
-    uint32_t*           sslot = ia;
-    MQI_CUDA(c, radix_sort_pairs(skeys, sslot, kb, ib, n, bit_length((uint64_t) n_spots * nvox - 1), hist, offs, scan, st),
-             "mqi_dij_build: sort");
-    MQI_CUDA(c, dij_row_bounds(skeys, n, nvox, n_spots, m.s_indptr, st), "mqi_dij_build");
+    // 2. voxel rows, spots ascending: by spot, then (stable) by voxel
+    MQI_CUDA(c, radix_sort_pairs(keys, vals, keys_alt, vals_alt, n, vbits, sbits, hist, offs, scan, st), "mqi_dij_build: sort");
+    MQI_CUDA(c, radix_sort_pairs(keys, vals, keys_alt, vals_alt, n, 0, vbits, hist, offs, scan, st), "mqi_dij_build: sort");
+    MQI_CUDA(c, dij_count_rows(keys, n, vbits, offs, hist, scan, st), "mqi_dij_build");
+    uint32_t tail[2] = { 0, 0 };
+    if (n) {
+        const uint64_t last = (n - 1) / kRowTile;
+        MQI_CUDA(c, cudaMemcpyAsync(&tail[0], offs + last, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "mqi_dij_build");
+        MQI_CUDA(c, cudaMemcpyAsync(&tail[1], hist + last, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "mqi_dij_build");
+        MQI_CUDA(c, cudaStreamSynchronize(st), "mqi_dij_build");
+    }
+    m.n_vrows = (uint64_t) tail[0] + tail[1];
+    if (n == 0) MQI_CUDA(c, cudaMemsetAsync(m.v_indptr, 0, sizeof(uint64_t), st), "mqi_dij_build");
+    MQI_CUDA(c, dij_voxel_rows(keys, vals, n, vbits, offs, m.v_row, m.v_indptr, m.v_spot, m.v_value, st), "mqi_dij_build");
+
+    // 3. spot rows, voxels ascending: those sorted (stable) by spot
+    MQI_CUDA(c, radix_sort_pairs(keys, vals, keys_alt, vals_alt, n, vbits, sbits, hist, offs, scan, st), "mqi_dij_build: sort");
+    MQI_CUDA(c, dij_row_bounds(keys, n, vbits, n_spots, m.s_indptr, st), "mqi_dij_build");
+    MQI_CUDA(c, dij_spot_rows(keys, vals, n, vbits, m.s_voxel, m.s_value, st), "mqi_dij_build");
     std::vector<uint64_t> indptr(n_spots + 1);
     MQI_CUDA(c, cudaMemcpyAsync(indptr.data(), m.s_indptr, indptr.size() * sizeof(uint64_t), cudaMemcpyDeviceToHost, st),
              "mqi_dij_build");
     MQI_CUDA(c, cudaStreamSynchronize(st), "mqi_dij_build");
-    if (indptr[n_spots] != n) return fail(c, MQI_ERR_INVALID, "mqi_dij_build: the table holds a spot index >= n_spots");
+    if (indptr[n_spots] != n) return fail(c, MQI_ERR_DEVICE, "mqi_dij_build: the sorted rows do not hold every entry");
     // backward segments: each row cut into runs of at most kDijSegment entries, and their work
-    // order: by the voxel of their first entry (the free sort buffers are reused below)
+    // order: by the voxel of their first entry (the sort buffers are free now)
     {
         std::vector<uint64_t> seg;
         std::vector<uint32_t> row_seg(n_spots + 1);
@@ -267,65 +340,25 @@ mqi_dij_build(mqi_ctx* c, int id, uint32_t n_spots, double scale, uint64_t* nnz_
         row_seg[n_spots] = (uint32_t) seg.size();
         m.n_seg = seg.size();
         seg.push_back(n);
-        MQI_CUDA(c, sc.alloc(m.seg_start, seg.size()), "mqi_dij_build: allocation");
-        MQI_CUDA(c, sc.alloc(m.row_seg, row_seg.size()), "mqi_dij_build: allocation");
-        MQI_CUDA(c, sc.alloc(m.seg_order, m.n_seg), "mqi_dij_build: allocation");
-        MQI_CUDA(c, sc.alloc(m.partial, m.n_seg), "mqi_dij_build: allocation");
-        MQI_CUDA(c, sc.alloc(m.bwd_cursor, 1), "mqi_dij_build: allocation");
         MQI_CUDA(c, cudaMemsetAsync(m.bwd_cursor, 0, sizeof(uint32_t), st), "mqi_dij_build");
         MQI_CUDA(c, cudaMemcpyAsync(m.seg_start, seg.data(), seg.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, st),
                  "mqi_dij_build");
         MQI_CUDA(c, cudaMemcpyAsync(m.row_seg, row_seg.data(), row_seg.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
                                     st), "mqi_dij_build");
         if (m.n_seg) {
-            unsigned long long* okeys = (skeys == ka) ? kb : ka;
-            unsigned long long* okalt = kc;
-            uint32_t*           oval  = (sslot == ia) ? ib : ia;
-            uint32_t*           ovalt = ic;
-            MQI_CUDA(c, dij_seg_order_keys(m.seg_start, (uint32_t) m.n_seg, skeys, nvox, okeys, oval, st), "mqi_dij_build");
-            MQI_CUDA(c, radix_sort_pairs(okeys, oval, okalt, ovalt, m.n_seg, bit_length(nvox - 1), hist, offs, scan, st),
+            MQI_CUDA(c, dij_seg_order_keys(m.seg_start, (uint32_t) m.n_seg, m.s_voxel, keys, vals, st), "mqi_dij_build");
+            MQI_CUDA(c, radix_sort_pairs(keys, vals, keys_alt, vals_alt, m.n_seg, 0, vbits, hist, offs, scan, st),
                      "mqi_dij_build: sort");
-            MQI_CUDA(c, cudaMemcpyAsync(m.seg_order, oval, m.n_seg * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st),
+            MQI_CUDA(c, cudaMemcpyAsync(m.seg_order, vals, m.n_seg * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st),
                      "mqi_dij_build");
         }
         MQI_CUDA(c, cudaStreamSynchronize(st), "mqi_dij_build");   // the host vectors are copied from
     }
 
-    // 3. spot-row entries, and (voxel, position) pairs for the voxel-row layout
-    unsigned long long* vkeys = (skeys == ka) ? kb : ka;
-    uint32_t*           vpos  = (sslot == ia) ? ib : ia;
-    MQI_CUDA(c, dij_spot_rows(skeys, sslot, n, nvox, s.dij, scale, m.s_voxel, m.s_value, vkeys, vpos, st),
-             "mqi_dij_build");
-    unsigned long long* kalt = kc;
-    uint32_t*           ialt = ic;
-    MQI_CUDA(c, radix_sort_pairs(vkeys, vpos, kalt, ialt, n, bit_length(nvox - 1), hist, offs, scan, st),
-             "mqi_dij_build: sort");
-
-    // 4. voxel rows: row starts by flag + scan
-    MQI_CUDA(c, dij_row_flags(vkeys, n, flags, st), "mqi_dij_build");
-    MQI_CUDA(c, scan_exclusive_u32(flags, rowid, n, scan, st), "mqi_dij_build");
-    uint32_t tail[2] = { 0, 0 };
-    if (n) {
-        MQI_CUDA(c, cudaMemcpyAsync(&tail[0], rowid + n - 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "mqi_dij_build");
-        MQI_CUDA(c, cudaMemcpyAsync(&tail[1], flags + n - 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "mqi_dij_build");
-        MQI_CUDA(c, cudaStreamSynchronize(st), "mqi_dij_build");
-    }
-    m.n_vrows = n ? (uint64_t) tail[0] + tail[1] : 0;
-    MQI_CUDA(c, sc.alloc(m.v_row, m.n_vrows), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(m.v_indptr, m.n_vrows + 1), "mqi_dij_build: allocation");
-    if (n == 0) MQI_CUDA(c, cudaMemsetAsync(m.v_indptr, 0, sizeof(uint64_t), st), "mqi_dij_build");
-    MQI_CUDA(c, dij_voxel_rows(vkeys, vpos, n, skeys, nvox, m.s_value, flags, rowid, m.v_row, m.v_indptr, m.v_spot,
-                               m.v_value, st), "mqi_dij_build");
-    // 5. the forward blocks' first rows
-    MQI_CUDA(c, sc.alloc(m.fwd_row_first, (n + kFwdEntries - 1) / kFwdEntries + 1), "mqi_dij_build: allocation");
-    MQI_CUDA(c, sc.alloc(m.fwd_run_k, (n + kFwdEntries - 1) / kFwdEntries + 1), "mqi_dij_build: allocation");
+    // 4. the forward blocks' first rows
     MQI_CUDA(c, dij_forward_blocks(m.v_indptr, m.n_vrows, n, m.fwd_row_first, m.fwd_run_k, &m.n_fwd_blocks, st),
              "mqi_dij_build");
     MQI_CUDA(c, cudaStreamSynchronize(st), "mqi_dij_build");
-    for (void* p : { (void*) m.s_indptr, (void*) m.s_voxel, (void*) m.s_value, (void*) m.v_row, (void*) m.v_indptr,
-                     (void*) m.v_spot, (void*) m.v_value, (void*) m.seg_start, (void*) m.row_seg, (void*) m.seg_order,
-                     (void*) m.bwd_cursor, (void*) m.partial, (void*) m.fwd_row_first, (void*) m.fwd_run_k })
-        sc.release(p);
     m.built = true;
     s.csr   = m;
     if (nnz_out) *nnz_out = n;

@@ -42,6 +42,8 @@ struct ChildHost {
 /// and voxel rows (only voxels with an entry).
 struct DijCsr {
     bool      built = false;
+    void*     slab = nullptr;       // one allocation that holds all arrays; kept for the next build
+    size_t    slab_bytes = 0;
     uint32_t  n_spots = 0;
     uint64_t  n_voxels = 0;
     uint64_t  nnz = 0;
@@ -63,6 +65,8 @@ struct DijCsr {
     uint32_t* fwd_row_first = nullptr;   // n_fwd_blocks + 1: first voxel row of each forward block
     uint64_t* fwd_run_k = nullptr;       // n_fwd_blocks + 1: first entry of each forward block's rows
 };
+
+constexpr size_t kKeepScratch = (size_t) 512 << 20;   // largest Dij build scratch a context keeps
 
 struct ScorerHost {
     int       child = 0;
@@ -103,7 +107,7 @@ std::string& thread_error_slot();
 
 /// Free a Dij scorer's table and matrix (mqi_capi_dij.cu).
 void dij_release(ScorerHost& s);
-/// Empty a Dij scorer's table and drop its matrix.
+/// Empty a Dij scorer's table; its matrix is no longer built.
 cudaError_t dij_reset(ScorerHost& s, int sms, cudaStream_t st);
 
 /// The shape of a draining wave over n queue entries.  While every track has a lane of its own, the
@@ -174,6 +178,8 @@ struct mqi_ctx {
     uint64_t                wave_launches = 0;
     double                  wave_ms = 0.0;
     cudaEvent_t             ev0 = nullptr, ev1 = nullptr;
+    void*                   build_scratch = nullptr;  // the last Dij build's sort buffers, when at most kKeepScratch
+    size_t                  build_scratch_bytes = 0;
     unsigned long long*     stat_scratch = nullptr;   // 3 x u64 for the statistics reductions
     mqi_spot*               plan_spots = nullptr;     // spot plan (device)
     uint64_t*               plan_cum = nullptr;       // cumulative histories, n_plan_spots + 1 (device)

@@ -12,6 +12,8 @@
 // Both products are gathers with a fixed reduction order: no atomics, reproducible results.
 #include <algorithm>
 #include <cstdint>
+#include <utility>
+
 #include <cuda_runtime.h>
 
 #include "mqi_internal.h"
@@ -22,10 +24,12 @@ namespace mqi_gpu
 namespace
 {
 
-constexpr int kThreads = 256;   // radix sort block
-constexpr int kItems   = 8;     // keys per thread per pass
+constexpr int kThreads = 256;   // radix sort and compaction block
+constexpr int kItems   = 16;    // keys per thread per radix pass
 constexpr int kTile    = kThreads * kItems;
+constexpr int kCompactItems = 8;    // table slots per thread and round of the compaction
 constexpr int kScanTile = 2048;
+static_assert(kScanTile == kRowTile, "the host finds the last tile");
 
 __device__ inline unsigned
 lanemask_lt() {
@@ -34,32 +38,63 @@ lanemask_lt() {
 
 // ---- compaction -----------------------------------------------------------------------------
 
-/// Append every occupied slot as (spot * n_voxels + voxel, slot index); warp-aggregated cursor.
-__global__ void
-k_dij_compact(const DijSlot* __restrict__ tab, uint64_t cap, uint64_t n_voxels, unsigned long long* __restrict__ keys,
-              uint32_t* __restrict__ idx, uint64_t n_max, unsigned long long* __restrict__ cursor) {
-    const uint64_t stride = (uint64_t) gridDim.x * blockDim.x;
-    const uint64_t span   = (cap + stride - 1) / stride * stride;   // every lane runs the same trip count
-    for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < span; i += stride) {
-        unsigned long long k = 0;
-        if (i < cap) k = tab[i].key;
-        const bool     valid = k != 0ull;
-        const unsigned b     = __ballot_sync(0xFFFFFFFFu, valid);
-        if (!b) continue;
-        unsigned long long base = 0;
-        const int          lead = __ffs(b) - 1;
-        if ((int) (threadIdx.x & 31) == lead) base = atomicAdd(cursor, (unsigned long long) __popc(b));
-        base = __shfl_sync(0xFFFFFFFFu, base, lead);
-        if (valid) {
-            const unsigned long long raw   = k - 1ull;
-            const uint64_t           spot  = raw >> 32;
-            const uint64_t           voxel = raw & 0xFFFFFFFFull;
-            const uint64_t           pos   = base + __popc(b & lanemask_lt());
-            if (pos < n_max) {   // the host compares the cursor with n_max afterwards
-                keys[pos] = spot * n_voxels + voxel;
-                idx[pos]  = (uint32_t) i;
-            }
+/// Append every occupied slot as ((spot << vbits) | voxel, FP32 value = FP64 tally x scale, rounded
+/// once), in no particular order.  Bound by HBM: 16 B read per slot, 12 B written per entry.  A block
+/// gathers its 2048 slots' entries in shared memory, so one atomic on the cursor serves them all
+/// (one a warp took 3.3 ms for 2^27 slots, now 0.42: 4 M atomics on one address), the
+/// narrow FP64 pipe sees whole warps of entries, and the writes are dense.  `bad` is set where a spot
+/// is not below n_spots.
+__global__ void __launch_bounds__(kThreads)
+k_dij_compact(const DijSlot* __restrict__ tab, uint64_t cap, int vbits, uint32_t n_spots, double scale,
+              unsigned long long* __restrict__ keys, uint32_t* __restrict__ vals, uint64_t n_max,
+              unsigned long long* __restrict__ cursor, uint32_t* __restrict__ bad) {
+    constexpr int kRound = kThreads * kCompactItems;
+    __shared__ unsigned long long s_key[kRound];
+    __shared__ double             s_val[kRound];
+    __shared__ uint32_t           s_n;
+    __shared__ unsigned long long s_base;
+    const int lane = threadIdx.x & 31;
+    for (uint64_t r0 = (uint64_t) blockIdx.x * kRound; r0 < cap; r0 += (uint64_t) gridDim.x * kRound) {
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
+        ulonglong2 e[kCompactItems];   // DijSlot: key, value
+#pragma unroll
+        for (int k = 0; k < kCompactItems; ++k) {
+            const uint64_t i = r0 + (uint64_t) k * kThreads + threadIdx.x;
+            e[k] = i < cap ? reinterpret_cast<const ulonglong2*>(tab)[i] : make_ulonglong2(0ull, 0ull);
         }
+        uint32_t mine = 0;
+#pragma unroll
+        for (int k = 0; k < kCompactItems; ++k) mine += e[k].x != 0ull;
+        uint32_t before = mine;   // inclusive, then exclusive, over the warp
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, before, o);
+            if (lane >= o) before += y;
+        }
+        uint32_t warp_base = 0;
+        if (lane == 31) warp_base = atomicAdd(&s_n, before);
+        uint32_t at = __shfl_sync(0xFFFFFFFFu, warp_base, 31) + before - mine;
+#pragma unroll
+        for (int k = 0; k < kCompactItems; ++k)
+            if (e[k].x != 0ull) {
+                s_key[at] = e[k].x - 1ull;
+                s_val[at] = __longlong_as_double((long long) e[k].y);
+                ++at;
+            }
+        __syncthreads();
+        const uint32_t n = s_n;
+        if (threadIdx.x == 0) s_base = n ? atomicAdd(cursor, (unsigned long long) n) : 0ull;
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < n; j += kThreads) {
+            const uint64_t pos  = s_base + j;
+            const uint64_t spot = s_key[j] >> 32;
+            if (pos < n_max) {   // the host compares the cursor with n_max afterwards
+                keys[pos] = (spot << vbits) | (s_key[j] & 0xFFFFFFFFull);
+                vals[pos] = __float_as_uint((float) (s_val[j] * scale));
+            }
+            if (spot >= n_spots) *bad = 1u;
+        }
+        __syncthreads();
     }
 }
 
@@ -147,8 +182,8 @@ k_scan_add(uint32_t* __restrict__ out, uint64_t n, const uint32_t* __restrict__ 
 
 // ---- radix sort -----------------------------------------------------------------------------
 
-__global__ void
-k_radix_hist(const unsigned long long* __restrict__ keys, uint64_t n, int shift, uint32_t* __restrict__ hist,
+__global__ void __launch_bounds__(kThreads)
+k_radix_hist(const unsigned long long* __restrict__ keys, uint64_t n, int shift, uint32_t mask, uint32_t* __restrict__ hist,
              uint32_t n_tiles) {
     __shared__ uint32_t cnt[256];
     cnt[threadIdx.x] = 0;
@@ -157,75 +192,108 @@ k_radix_hist(const unsigned long long* __restrict__ keys, uint64_t n, int shift,
 #pragma unroll
     for (int r = 0; r < kItems; ++r) {
         const uint64_t i = t0 + (uint64_t) r * kThreads + threadIdx.x;
-        if (i < n) atomicAdd(&cnt[(keys[i] >> shift) & 255u], 1u);
+        if (i < n) atomicAdd(&cnt[(uint32_t) (keys[i] >> shift) & mask], 1u);
     }
     __syncthreads();
-    hist[(uint64_t) threadIdx.x * n_tiles + blockIdx.x] = cnt[threadIdx.x];
+    if (threadIdx.x <= mask) hist[(uint64_t) threadIdx.x * n_tiles + blockIdx.x] = cnt[threadIdx.x];
 }
 
-/// Stable scatter of one 8-bit digit.  The tile is visited in input order (round, warp, lane);
-/// an element's destination is its tile's digit offset + the count of equal digits before it in
-/// earlier rounds, earlier warps of its round, and lower lanes of its warp.
-__global__ void
+/// Shared memory of k_radix_scatter.
+struct RadixSmem {
+    unsigned long long key[kTile];
+    uint32_t           val[kTile];
+    uint32_t           cnt[kThreads / 32][256];   // per warp and digit: a count, then a place in the tile
+    uint32_t           first[256];                // the digit's first place in the tile
+    uint32_t           offs[256];                 // and its first place in the output
+    uint32_t           ws[32];
+};
+
+/// Stable scatter of one digit of at most 8 bits.  A warp takes 512 consecutive elements of the tile,
+/// 32 at a time in input order, and ranks each among its equals by warp votes alone; the block then
+/// turns the warps' counts into places, puts the tile in order in shared memory and writes it out, a
+/// run of each digit's elements at a time.  Bound by HBM (12 B read and written per element).  With
+/// the ranking across the block (three barriers per 256 elements) and each element stored from
+/// registers, 11.7 M elements took 180 us a pass (now 70).
+__global__ void __launch_bounds__(kThreads, 3)
 k_radix_scatter(const unsigned long long* __restrict__ kin, const uint32_t* __restrict__ vin,
-                unsigned long long* __restrict__ kout, uint32_t* __restrict__ vout, uint64_t n, int shift,
+                unsigned long long* __restrict__ kout, uint32_t* __restrict__ vout, uint64_t n, int shift, uint32_t mask,
                 const uint32_t* __restrict__ offs, uint32_t n_tiles) {
+    extern __shared__ __align__(16) unsigned char radix_smem[];
+    RadixSmem& S    = *reinterpret_cast<RadixSmem*>(radix_smem);
+    const int  warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int kWarps = kThreads / 32;
-    __shared__ uint32_t base[256];
-    __shared__ uint32_t wcnt[kWarps][256];
-    __shared__ uint32_t wpre[kWarps][256];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    base[threadIdx.x] = offs[(uint64_t) threadIdx.x * n_tiles + blockIdx.x];
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) wcnt[w][threadIdx.x] = 0;
+    for (int w = 0; w < kWarps; ++w) S.cnt[w][threadIdx.x] = 0;
+    if (threadIdx.x <= mask) S.offs[threadIdx.x] = offs[(uint64_t) threadIdx.x * n_tiles + blockIdx.x];
     __syncthreads();
-    const uint64_t t0 = (uint64_t) blockIdx.x * kTile;
-    for (int r = 0; r < kItems; ++r) {
-        const uint64_t i     = t0 + (uint64_t) r * kThreads + threadIdx.x;
-        const bool     valid = i < n;
-        unsigned long long k = 0;
-        uint32_t           v = 0;
-        uint32_t           d = 0x100u;   // matches no digit
-        if (valid) {
-            k = kin[i];
-            v = vin[i];
-            d = (uint32_t) ((k >> shift) & 255u);
-        }
-        const unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
-        const uint32_t rank  = __popc(peers & lanemask_lt());
-        if (valid && lane == __ffs(peers) - 1) wcnt[warp][d] = __popc(peers);
-        __syncthreads();
-        {
-            const int dd  = threadIdx.x;
-            uint32_t  run = base[dd];
+    const uint64_t t0   = (uint64_t) blockIdx.x * kTile;
+    const uint32_t size = (uint32_t) (n - t0 < (uint64_t) kTile ? n - t0 : (uint64_t) kTile);
+    const uint32_t w0   = (uint32_t) warp * 32 * kItems;
+    unsigned long long k[kItems];
+    uint32_t           v[kItems], rank[kItems];
 #pragma unroll
-            for (int w = 0; w < kWarps; ++w) {
-                const uint32_t c = wcnt[w][dd];
-                wpre[w][dd]      = run;
-                run += c;
-                wcnt[w][dd] = 0;
-            }
-            base[dd] = run;
+    for (int r = 0; r < kItems; ++r) {
+        const uint32_t i = w0 + (uint32_t) r * 32 + lane;
+        k[r] = 0ull;
+        v[r] = 0u;
+        if (i < size) {
+            k[r] = kin[t0 + i];
+            v[r] = vin[t0 + i];
         }
-        __syncthreads();
-        if (valid) {
-            const uint32_t pos = wpre[warp][d] + rank;
-            kout[pos] = k;
-            vout[pos] = v;
+    }
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+        const bool     valid = w0 + (uint32_t) r * 32 + lane < size;
+        const uint32_t d     = valid ? (uint32_t) (k[r] >> shift) & mask : 0x100u;   // 0x100 matches no digit
+        const unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
+        uint32_t       seen  = 0;
+        if (valid) seen = S.cnt[warp][d];
+        __syncwarp();
+        if (valid && lane == __ffs(peers) - 1) S.cnt[warp][d] = seen + __popc(peers);
+        __syncwarp();
+        rank[r] = seen + __popc(peers & lanemask_lt());
+    }
+    __syncthreads();
+    {   // a thread a digit: places of the warps' shares
+        uint32_t total = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const uint32_t c     = S.cnt[w][threadIdx.x];
+            S.cnt[w][threadIdx.x] = total;
+            total += c;
         }
-        __syncthreads();
+        uint32_t       all;
+        const uint32_t first = block_exclusive_scan(total, S.ws, all);
+        S.first[threadIdx.x] = first;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kItems; ++r)
+        if (w0 + (uint32_t) r * 32 + lane < size) {
+            const uint32_t d   = (uint32_t) (k[r] >> shift) & mask;
+            const uint32_t pos = S.first[d] + S.cnt[warp][d] + rank[r];
+            S.key[pos] = k[r];
+            S.val[pos] = v[r];
+        }
+    __syncthreads();
+    for (uint32_t j = threadIdx.x; j < size; j += kThreads) {
+        const unsigned long long x = S.key[j];
+        const uint32_t           d = (uint32_t) (x >> shift) & mask;
+        const uint32_t           o = S.offs[d] + (j - S.first[d]);
+        kout[o] = x;
+        vout[o] = S.val[j];
     }
 }
 
 // ---- CSR assembly ---------------------------------------------------------------------------
 
-/// indptr[r] = lower_bound(keys, r * row_span) for r in [0, n_rows].
+/// indptr[r] = lower_bound(keys, r << vbits) for r in [0, n_rows].
 __global__ void
-k_row_bounds(const unsigned long long* __restrict__ keys, uint64_t n, uint64_t row_span, uint64_t n_rows,
+k_row_bounds(const unsigned long long* __restrict__ keys, uint64_t n, int vbits, uint64_t n_rows,
              uint64_t* __restrict__ indptr) {
     const uint64_t r = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (r > n_rows) return;
-    const unsigned long long target = r * row_span;
+    const unsigned long long target = r << vbits;
     uint64_t lo = 0, hi = n;
     while (lo < hi) {
         const uint64_t mid = (lo + hi) >> 1;
@@ -234,54 +302,79 @@ k_row_bounds(const unsigned long long* __restrict__ keys, uint64_t n, uint64_t r
     indptr[r] = lo;
 }
 
-/// Spot-row CSR entries: voxel column and FP32 value (FP64 tally x scale, rounded once).
+/// Spot-row entries: the voxel column and the value of each sorted key.
 __global__ void
-k_spot_rows(const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ slot, uint64_t n,
-            uint64_t n_voxels, const DijSlot* __restrict__ tab, double scale, uint32_t* __restrict__ vox,
-            float* __restrict__ val, unsigned long long* __restrict__ vkeys, uint32_t* __restrict__ vpos) {
-    const uint64_t k = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const uint32_t v = (uint32_t) (keys[k] % n_voxels);
-    vox[k]   = v;
-    val[k]   = (float) (tab[slot[k]].value * scale);
-    vkeys[k] = v;
-    vpos[k]  = (uint32_t) k;
+k_spot_rows(const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ vals, uint64_t n, uint32_t vmask,
+            uint32_t* __restrict__ vox, uint32_t* __restrict__ val) {
+    const uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    vox[i] = (uint32_t) keys[i] & vmask;
+    val[i] = vals[i];
 }
 
-__global__ void
-k_row_flags(const unsigned long long* __restrict__ vkeys, uint64_t n, uint32_t* __restrict__ flags) {
-    const uint64_t j = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < n) flags[j] = (j == 0 || vkeys[j] != vkeys[j - 1]) ? 1u : 0u;
+/// Whether entry j of the voxel-sorted keys starts a row.
+__device__ inline bool
+starts_row(const unsigned long long* __restrict__ keys, uint64_t j, uint32_t vmask) {
+    return j == 0 || (((uint32_t) keys[j] ^ (uint32_t) keys[j - 1]) & vmask) != 0u;
 }
 
-/// Voxel-row entries: spot column and value from the spot-row entry they came from; row starts.
-__global__ void
-k_voxel_rows(const unsigned long long* __restrict__ vkeys, const uint32_t* __restrict__ vpos, uint64_t n,
-             const unsigned long long* __restrict__ skeys, uint64_t n_voxels, const float* __restrict__ sval,
-             const uint32_t* __restrict__ flags, const uint32_t* __restrict__ rowid, uint32_t* __restrict__ row_voxel,
-             uint64_t* __restrict__ indptr, uint32_t* __restrict__ spot, float* __restrict__ val) {
-    const uint64_t j = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const uint32_t p = vpos[j];
-    spot[j] = (uint32_t) (skeys[p] / n_voxels);
-    val[j]  = sval[p];
-    if (flags[j]) {
-        row_voxel[rowid[j]] = (uint32_t) vkeys[j];
-        indptr[rowid[j]]    = j;
+/// Rows that start in each tile of kScanTile entries.
+__global__ void __launch_bounds__(kThreads)
+k_count_rows(const unsigned long long* __restrict__ keys, uint64_t n, uint32_t vmask, uint32_t* __restrict__ tiles) {
+    __shared__ uint32_t sum;
+    if (threadIdx.x == 0) sum = 0;
+    __syncthreads();
+    const uint64_t t0 = (uint64_t) blockIdx.x * kScanTile;
+    uint32_t       c  = 0;
+#pragma unroll
+    for (int r = 0; r < kScanTile / kThreads; ++r) {
+        const uint64_t j = t0 + (uint64_t) r * kThreads + threadIdx.x;
+        c += j < n && starts_row(keys, j, vmask);
     }
-    if (j == n - 1) indptr[rowid[j] + flags[j]] = n;
+    c = __reduce_add_sync(0xFFFFFFFFu, c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&sum, c);
+    __syncthreads();
+    if (threadIdx.x == 0) tiles[blockIdx.x] = sum;
+}
+
+/// Voxel-row entries -- the spot column and the value of each sorted key -- and the rows' voxels and
+/// first entries; tiles[b] = the rows that start before tile b.
+__global__ void __launch_bounds__(kThreads)
+k_voxel_rows(const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ vals, uint64_t n, int vbits,
+             const uint32_t* __restrict__ tiles, uint32_t* __restrict__ row_voxel, uint64_t* __restrict__ indptr,
+             uint32_t* __restrict__ spot, uint32_t* __restrict__ val) {
+    __shared__ uint32_t ws[32];
+    const uint32_t vmask = (uint32_t) ((1ull << vbits) - 1ull);
+    const uint64_t t0    = (uint64_t) blockIdx.x * kScanTile;
+    uint32_t       row   = tiles[blockIdx.x];
+    for (int r = 0; r < kScanTile / kThreads; ++r) {
+        const uint64_t j     = t0 + (uint64_t) r * kThreads + threadIdx.x;
+        const bool     start = j < n && starts_row(keys, j, vmask);
+        uint32_t       total;
+        const uint32_t at = row + block_exclusive_scan(start ? 1u : 0u, ws, total);
+        if (j < n) {
+            const unsigned long long k = keys[j];
+            spot[j] = (uint32_t) (k >> vbits);
+            val[j]  = vals[j];
+            if (start) {
+                row_voxel[at] = (uint32_t) k & vmask;
+                indptr[at]    = j;
+            }
+            if (j == n - 1) indptr[at + (start ? 1u : 0u)] = n;
+        }
+        row += total;
+    }
 }
 
 // ---- backward segments: their work order ---------------------------------------------------
 
-/// Sort keys of the backward's work order: the voxel of each segment's first entry (the keys are
-/// the sorted spot * n_voxels + voxel pairs).
+/// Sort keys of the backward's work order: the voxel of each segment's first entry.
 __global__ void
-k_seg_keys(const uint64_t* __restrict__ seg_start, uint32_t n_seg, const unsigned long long* __restrict__ keys,
-           uint64_t n_voxels, unsigned long long* __restrict__ okeys, uint32_t* __restrict__ oval) {
+k_seg_keys(const uint64_t* __restrict__ seg_start, uint32_t n_seg, const uint32_t* __restrict__ vox,
+           unsigned long long* __restrict__ okeys, uint32_t* __restrict__ oval) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_seg) return;
-    okeys[i] = keys[seg_start[i]] % n_voxels;
+    okeys[i] = vox[seg_start[i]];
     oval[i]  = i;
 }
 
@@ -696,11 +789,14 @@ dij_count(const DijSlot* tab, uint64_t cap, unsigned long long* out, int sms, cu
 }
 
 cudaError_t
-dij_compact(const DijSlot* tab, uint64_t cap, uint64_t n_voxels, unsigned long long* keys, uint32_t* idx,
-            uint64_t n_max, unsigned long long* cursor, int sms, cudaStream_t s) {
+dij_compact(const DijSlot* tab, uint64_t cap, int vbits, uint32_t n_spots, double scale, unsigned long long* keys,
+            uint32_t* vals, uint64_t n_max, unsigned long long* cursor, uint32_t* bad, int sms, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    k_dij_compact<<<sms * 8, 256, 0, s>>>(tab, cap, n_voxels, keys, idx, n_max, cursor);
+    const uint64_t rounds = (cap + kThreads * kCompactItems - 1) / (kThreads * kCompactItems);
+    k_dij_compact<<<(unsigned) std::min<uint64_t>(rounds, (uint64_t) sms * 6), kThreads, 0, s>>>(tab, cap, vbits, n_spots, scale,
+                                                                                              keys, vals, n_max, cursor, bad);
     return cudaGetLastError();
 }
 
@@ -726,55 +822,58 @@ radix_hist_words(uint64_t n) {
 
 cudaError_t
 radix_sort_pairs(unsigned long long*& keys, uint32_t*& vals, unsigned long long*& keys_alt, uint32_t*& vals_alt,
-                 uint64_t n, int bits, uint32_t* hist, uint32_t* offs, uint32_t* scan_scratch, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
+                 uint64_t n, int first_bit, int bits, uint32_t* hist, uint32_t* offs, uint32_t* scan_scratch,
+                 cudaStream_t s) {
+    if (n == 0 || bits <= 0) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(RadixSmem));
+    if (e != cudaSuccess) return e;
     const uint32_t n_tiles = (uint32_t) ((n + kTile - 1) / kTile);
-    const uint64_t words   = 256ull * n_tiles;
-    for (int shift = 0; shift < bits; shift += 8) {
-        k_radix_hist<<<n_tiles, kThreads, 0, s>>>(keys, n, shift, hist, n_tiles);
-        cudaError_t e = scan_exclusive_u32(hist, offs, words, scan_scratch, s);
-        if (e != cudaSuccess) return e;
-        k_radix_scatter<<<n_tiles, kThreads, 0, s>>>(keys, vals, keys_alt, vals_alt, n, shift, offs, n_tiles);
+    // the fewest passes of at most 8 bits, of nearly equal width: fewer digits make longer runs
+    const int passes = (bits + 7) / 8;
+    for (int p = 0, bit = first_bit; p < passes; ++p) {
+        const int      width = (first_bit + bits - bit + passes - p - 1) / (passes - p);
+        const uint32_t mask  = (1u << width) - 1u;
+        k_radix_hist<<<n_tiles, kThreads, 0, s>>>(keys, n, bit, mask, hist, n_tiles);
+        if ((e = scan_exclusive_u32(hist, offs, (uint64_t) (mask + 1u) * n_tiles, scan_scratch, s)) != cudaSuccess) return e;
+        k_radix_scatter<<<n_tiles, kThreads, sizeof(RadixSmem), s>>>(keys, vals, keys_alt, vals_alt, n, bit, mask, offs, n_tiles);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        unsigned long long* tk = keys;
-        keys                   = keys_alt;
-        keys_alt               = tk;
-        uint32_t* tv           = vals;
-        vals                   = vals_alt;
-        vals_alt               = tv;
+        std::swap(keys, keys_alt);
+        std::swap(vals, vals_alt);
+        bit += width;
     }
+    return cudaSuccess;
+}
+
+cudaError_t
+dij_row_bounds(const unsigned long long* keys, uint64_t n, int vbits, uint64_t n_rows, uint64_t* indptr, cudaStream_t s) {
+    k_row_bounds<<<blocks_for(n_rows + 1, 256), 256, 0, s>>>(keys, n, vbits, n_rows, indptr);
     return cudaGetLastError();
 }
 
 cudaError_t
-dij_row_bounds(const unsigned long long* keys, uint64_t n, uint64_t row_span, uint64_t n_rows, uint64_t* indptr,
+dij_spot_rows(const unsigned long long* keys, const uint32_t* vals, uint64_t n, int vbits, uint32_t* vox, float* val,
+              cudaStream_t s) {
+    if (n == 0) return cudaSuccess;
+    k_spot_rows<<<blocks_for(n, 256), 256, 0, s>>>(keys, vals, n, (uint32_t) ((1ull << vbits) - 1ull), vox,
+                                                  reinterpret_cast<uint32_t*>(val));
+    return cudaGetLastError();
+}
+
+cudaError_t
+dij_count_rows(const unsigned long long* keys, uint64_t n, int vbits, uint32_t* tiles, uint32_t* tile_rows, uint32_t* scratch,
                cudaStream_t s) {
-    k_row_bounds<<<blocks_for(n_rows + 1, 256), 256, 0, s>>>(keys, n, row_span, n_rows, indptr);
-    return cudaGetLastError();
+    if (n == 0) return cudaSuccess;
+    const uint64_t nt = (n + kScanTile - 1) / kScanTile;
+    k_count_rows<<<(unsigned) nt, kThreads, 0, s>>>(keys, n, (uint32_t) ((1ull << vbits) - 1ull), tile_rows);
+    return scan_exclusive_u32(tile_rows, tiles, nt, scratch, s);
 }
 
 cudaError_t
-dij_spot_rows(const unsigned long long* keys, const uint32_t* slot, uint64_t n, uint64_t n_voxels, const DijSlot* tab,
-              double scale, uint32_t* vox, float* val, unsigned long long* vkeys, uint32_t* vpos, cudaStream_t s) {
+dij_voxel_rows(const unsigned long long* keys, const uint32_t* vals, uint64_t n, int vbits, const uint32_t* tiles,
+               uint32_t* row_voxel, uint64_t* indptr, uint32_t* spot, float* val, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    k_spot_rows<<<blocks_for(n, 256), 256, 0, s>>>(keys, slot, n, n_voxels, tab, scale, vox, val, vkeys, vpos);
-    return cudaGetLastError();
-}
-
-cudaError_t
-dij_row_flags(const unsigned long long* vkeys, uint64_t n, uint32_t* flags, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    k_row_flags<<<blocks_for(n, 256), 256, 0, s>>>(vkeys, n, flags);
-    return cudaGetLastError();
-}
-
-cudaError_t
-dij_voxel_rows(const unsigned long long* vkeys, const uint32_t* vpos, uint64_t n, const unsigned long long* skeys,
-               uint64_t n_voxels, const float* sval, const uint32_t* flags, const uint32_t* rowid, uint32_t* row_voxel,
-               uint64_t* indptr, uint32_t* spot, float* val, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    k_voxel_rows<<<blocks_for(n, 256), 256, 0, s>>>(vkeys, vpos, n, skeys, n_voxels, sval, flags, rowid, row_voxel,
-                                                   indptr, spot, val);
+    k_voxel_rows<<<(unsigned) ((n + kScanTile - 1) / kScanTile), kThreads, 0, s>>>(
+        keys, vals, n, vbits, tiles, row_voxel, indptr, spot, reinterpret_cast<uint32_t*>(val));
     return cudaGetLastError();
 }
 
@@ -788,10 +887,10 @@ dij_forward_blocks(const uint64_t* indptr, uint64_t n_rows, uint64_t nnz, uint32
 }
 
 cudaError_t
-dij_seg_order_keys(const uint64_t* seg_start, uint32_t n_seg, const unsigned long long* keys, uint64_t n_voxels,
-                   unsigned long long* okeys, uint32_t* oval, cudaStream_t s) {
+dij_seg_order_keys(const uint64_t* seg_start, uint32_t n_seg, const uint32_t* vox, unsigned long long* okeys, uint32_t* oval,
+                   cudaStream_t s) {
     if (n_seg == 0) return cudaSuccess;
-    k_seg_keys<<<blocks_for(n_seg, 256), 256, 0, s>>>(seg_start, n_seg, keys, n_voxels, okeys, oval);
+    k_seg_keys<<<blocks_for(n_seg, 256), 256, 0, s>>>(seg_start, n_seg, vox, okeys, oval);
     return cudaGetLastError();
 }
 

@@ -198,23 +198,26 @@ void set_thread_error(const char* msg);
 cudaError_t dij_clear(DijSlot* tab, uint64_t cap, int sms, cudaStream_t s);
 // Occupied slots of a Dij table into *out (cleared first).
 cudaError_t dij_count(const DijSlot* tab, uint64_t cap, unsigned long long* out, int sms, cudaStream_t s);
-cudaError_t dij_compact(const DijSlot* tab, uint64_t cap, uint64_t n_voxels, unsigned long long* keys, uint32_t* idx,
-                        uint64_t n_max, unsigned long long* cursor, int sms, cudaStream_t s);
+// Entries of a table as keys (spot << vbits) | voxel and FP32 value bits; *bad where a spot >= n_spots.
+cudaError_t dij_compact(const DijSlot* tab, uint64_t cap, int vbits, uint32_t n_spots, double scale, unsigned long long* keys,
+                        uint32_t* vals, uint64_t n_max, unsigned long long* cursor, uint32_t* bad, int sms, cudaStream_t s);
 uint64_t    scan_scratch_words(uint64_t n);
 cudaError_t scan_exclusive_u32(const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* scratch, cudaStream_t s);
 uint64_t    radix_hist_words(uint64_t n);
+// Stable sort by key bits [first_bit, first_bit + bits); the sorted pairs end up in keys, vals.
 cudaError_t radix_sort_pairs(unsigned long long*& keys, uint32_t*& vals, unsigned long long*& keys_alt,
-                             uint32_t*& vals_alt, uint64_t n, int bits, uint32_t* hist, uint32_t* offs,
+                             uint32_t*& vals_alt, uint64_t n, int first_bit, int bits, uint32_t* hist, uint32_t* offs,
                              uint32_t* scan_scratch, cudaStream_t s);
-cudaError_t dij_row_bounds(const unsigned long long* keys, uint64_t n, uint64_t row_span, uint64_t n_rows,
-                           uint64_t* indptr, cudaStream_t s);
-cudaError_t dij_spot_rows(const unsigned long long* keys, const uint32_t* slot, uint64_t n, uint64_t n_voxels,
-                          const DijSlot* tab, double scale, uint32_t* vox, float* val, unsigned long long* vkeys,
-                          uint32_t* vpos, cudaStream_t s);
-cudaError_t dij_row_flags(const unsigned long long* vkeys, uint64_t n, uint32_t* flags, cudaStream_t s);
-cudaError_t dij_voxel_rows(const unsigned long long* vkeys, const uint32_t* vpos, uint64_t n,
-                           const unsigned long long* skeys, uint64_t n_voxels, const float* sval, const uint32_t* flags,
-                           const uint32_t* rowid, uint32_t* row_voxel, uint64_t* indptr, uint32_t* spot, float* val,
+cudaError_t dij_row_bounds(const unsigned long long* keys, uint64_t n, int vbits, uint64_t n_rows, uint64_t* indptr,
+                           cudaStream_t s);
+cudaError_t dij_spot_rows(const unsigned long long* keys, const uint32_t* vals, uint64_t n, int vbits, uint32_t* vox,
+                          float* val, cudaStream_t s);
+constexpr uint64_t kRowTile = 2048;   // entries of a tile of dij_count_rows
+// tiles[b] = voxel rows that start before tile b of the voxel-sorted keys; tile_rows: those in it.
+cudaError_t dij_count_rows(const unsigned long long* keys, uint64_t n, int vbits, uint32_t* tiles, uint32_t* tile_rows,
+                           uint32_t* scratch, cudaStream_t s);
+cudaError_t dij_voxel_rows(const unsigned long long* keys, const uint32_t* vals, uint64_t n, int vbits,
+                           const uint32_t* tiles, uint32_t* row_voxel, uint64_t* indptr, uint32_t* spot, float* val,
                            cudaStream_t s);
 constexpr uint64_t kFwdEntries = 4096;    // entries whose rows one forward block owns
 constexpr uint64_t kFwdStage   = 8192;    // staged products per forward block (rows up to 4096 entries)
@@ -229,8 +232,8 @@ cudaError_t dij_forward(const uint32_t* row_voxel, const uint64_t* indptr, const
                         const uint64_t* run_k, uint64_t n_blocks, const uint32_t* spot, const float* val, const void* w,
                         void* dose, int fp64, uint32_t* err, int sms, cudaStream_t s);
 constexpr uint64_t kDijSegment = 16384;   // entries per backward segment (segments never cross a row)
-cudaError_t dij_seg_order_keys(const uint64_t* seg_start, uint32_t n_seg, const unsigned long long* keys,
-                               uint64_t n_voxels, unsigned long long* okeys, uint32_t* oval, cudaStream_t s);
+cudaError_t dij_seg_order_keys(const uint64_t* seg_start, uint32_t n_seg, const uint32_t* vox, unsigned long long* okeys,
+                               uint32_t* oval, cudaStream_t s);
 cudaError_t dij_backward(const uint32_t* order, const uint64_t* seg_start, uint32_t n_seg, const uint32_t* row_seg,
                          uint32_t n_rows, const uint32_t* vox, const float* val, double* partial, uint32_t* cursor,
                          const void* g, void* grad, int fp64, int sms, cudaStream_t s);
