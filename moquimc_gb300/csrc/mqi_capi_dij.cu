@@ -235,8 +235,8 @@ mqi_dij_build(mqi_ctx* c, int id, uint32_t n_spots, double scale, uint64_t* nnz_
     uint32_t *vals, *vals_alt, *hist, *offs, *scan, *bad;
     auto lay_out_scratch = [&](Carve cv) {
         const uint64_t hw = radix_hist_words(n);
-        cv.take(keys, n);
-        cv.take(keys_alt, n);
+        cv.take(keys, n + 1);
+        cv.take(keys_alt, n + 1);
         cv.take(vals, n);
         cv.take(vals_alt, n);
         cv.take(hist, hw);
@@ -260,17 +260,21 @@ mqi_dij_build(mqi_ctx* c, int id, uint32_t n_spots, double scale, uint64_t* nnz_
     // the matrix: segments of the backward are bounded by whole ones and one more per row, voxel rows by
     // the entries and by the voxels
     DijCsr m;
-    const uint64_t max_seg = n / kDijSegment + std::min<uint64_t>(n_spots, n), max_vrows = std::min(n, nvox);
+    m.spot16 = n_spots <= 65536;
+    const uint64_t segment = dij_segment(n, c->num_sms);
+    const uint64_t max_seg = n / segment + std::min<uint64_t>(n_spots, n), max_vrows = std::min(n, nvox);
     const uint64_t n_runs  = (n + kFwdEntries - 1) / kFwdEntries;
     auto lay_out = [&](Carve cv) {
         cv.take(m.s_indptr, (uint64_t) n_spots + 1);
-        // entry arrays padded to whole groups of four: the products read them with 16-byte loads
-        cv.take(m.s_voxel, n + 4);
-        cv.take(m.s_value, n + 4);
-        cv.take(m.v_spot, n + 4);
-        cv.take(m.v_value, n + 4);
+        // entry arrays padded to whole groups of eight: the products read them in 16-byte pieces
+        unsigned char* v_spot = nullptr;
+        cv.take(m.s_voxel, n + 8);
+        cv.take(m.s_value, n + 8);
+        cv.take(v_spot, (n + 8) * (m.spot16 ? sizeof(uint16_t) : sizeof(uint32_t)));
+        cv.take(m.v_value, n + 8);
         cv.take(m.v_row, max_vrows);
-        cv.take(m.v_indptr, max_vrows + 1);
+        cv.take(m.v_off, max_vrows);
+        m.v_spot = v_spot;
         cv.take(m.seg_start, max_seg + 1);
         cv.take(m.row_seg, (uint64_t) n_spots + 1);
         cv.take(m.seg_order, max_seg);
@@ -316,8 +320,17 @@ mqi_dij_build(mqi_ctx* c, int id, uint32_t n_spots, double scale, uint64_t* nnz_
         MQI_CUDA(c, cudaStreamSynchronize(st), "mqi_dij_build");
     }
     m.n_vrows = (uint64_t) tail[0] + tail[1];
-    if (n == 0) MQI_CUDA(c, cudaMemsetAsync(m.v_indptr, 0, sizeof(uint64_t), st), "mqi_dij_build");
-    MQI_CUDA(c, dij_voxel_rows(keys, vals, n, vbits, offs, m.v_row, m.v_indptr, m.v_spot, m.v_value, st), "mqi_dij_build");
+    // the forward runs' first rows are found from the rows' first entries, in the sort's spare buffer
+    uint64_t* indptr_v = reinterpret_cast<uint64_t*>(keys_alt);
+    if (n == 0) MQI_CUDA(c, cudaMemsetAsync(indptr_v, 0, sizeof(uint64_t), st), "mqi_dij_build");
+    // the forward multiplies whole groups: spot 0 past the end
+    MQI_CUDA(c, cudaMemsetAsync(static_cast<char*>(m.v_spot) + n * (m.spot16 ? 2 : 4), 0, 8 * (m.spot16 ? 2 : 4), st),
+             "mqi_dij_build");
+    MQI_CUDA(c, cudaMemsetAsync(m.v_value + n, 0, 8 * sizeof(float), st), "mqi_dij_build");
+    MQI_CUDA(c, dij_voxel_rows(keys, vals, n, vbits, offs, m.v_row, m.v_off, indptr_v, m.v_spot, m.spot16, m.v_value, st),
+             "mqi_dij_build");
+    MQI_CUDA(c, dij_forward_blocks(indptr_v, m.n_vrows, n, m.fwd_row_first, m.fwd_run_k, &m.n_fwd_blocks, st),
+             "mqi_dij_build");
 
     // 3. spot rows, voxels ascending: those sorted (stable) by spot
     MQI_CUDA(c, radix_sort_pairs(keys, vals, keys_alt, vals_alt, n, vbits, sbits, hist, offs, scan, st), "mqi_dij_build: sort");
@@ -328,14 +341,14 @@ mqi_dij_build(mqi_ctx* c, int id, uint32_t n_spots, double scale, uint64_t* nnz_
              "mqi_dij_build");
     MQI_CUDA(c, cudaStreamSynchronize(st), "mqi_dij_build");
     if (indptr[n_spots] != n) return fail(c, MQI_ERR_DEVICE, "mqi_dij_build: the sorted rows do not hold every entry");
-    // backward segments: each row cut into runs of at most kDijSegment entries, and their work
+    // backward segments: each row cut into runs of at most `segment` entries, and their work
     // order: by the voxel of their first entry (the sort buffers are free now)
     {
         std::vector<uint64_t> seg;
         std::vector<uint32_t> row_seg(n_spots + 1);
         for (uint32_t r = 0; r < n_spots; ++r) {
             row_seg[r] = (uint32_t) seg.size();
-            for (uint64_t b = indptr[r]; b < indptr[r + 1]; b += kDijSegment) seg.push_back(b);
+            for (uint64_t b = indptr[r]; b < indptr[r + 1]; b += segment) seg.push_back(b);
         }
         row_seg[n_spots] = (uint32_t) seg.size();
         m.n_seg = seg.size();
@@ -355,10 +368,6 @@ mqi_dij_build(mqi_ctx* c, int id, uint32_t n_spots, double scale, uint64_t* nnz_
         MQI_CUDA(c, cudaStreamSynchronize(st), "mqi_dij_build");   // the host vectors are copied from
     }
 
-    // 4. the forward blocks' first rows
-    MQI_CUDA(c, dij_forward_blocks(m.v_indptr, m.n_vrows, n, m.fwd_row_first, m.fwd_run_k, &m.n_fwd_blocks, st),
-             "mqi_dij_build");
-    MQI_CUDA(c, cudaStreamSynchronize(st), "mqi_dij_build");
     m.built = true;
     s.csr   = m;
     if (nnz_out) *nnz_out = n;
@@ -417,8 +426,8 @@ mqi_dij_matvec(mqi_ctx* c, int id, const void* w, void* dose, int fp64, int on_d
         dd = td;
     }
     MQI_CUDA(c, cudaMemsetAsync(dd, 0, m.n_voxels * es, c->stream), "mqi_dij_matvec");
-    MQI_CUDA(c, dij_forward(m.v_row, m.v_indptr, m.fwd_row_first, m.fwd_run_k, m.n_fwd_blocks, m.v_spot, m.v_value,
-                            dw, dd, fp64, c->counters + 3, c->num_sms, c->stream), "mqi_dij_matvec");
+    MQI_CUDA(c, dij_forward(m.v_row, m.v_off, m.fwd_row_first, m.fwd_run_k, m.n_fwd_blocks, m.v_spot, m.spot16,
+                            m.v_value, dw, dd, fp64, c->counters + 3, c->num_sms, c->stream), "mqi_dij_matvec");
     if (!on_device) {
         uint32_t flag = 0;
         MQI_CUDA(c, cudaMemcpyAsync(dose, dd, m.n_voxels * es, cudaMemcpyDeviceToHost, c->stream), "mqi_dij_matvec");

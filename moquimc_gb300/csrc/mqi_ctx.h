@@ -52,8 +52,9 @@ struct DijCsr {
     uint32_t* s_voxel = nullptr;    // nnz
     float*    s_value = nullptr;    // nnz
     uint32_t* v_row = nullptr;      // n_vrows: voxel of each voxel row
-    uint64_t* v_indptr = nullptr;   // n_vrows + 1
-    uint32_t* v_spot = nullptr;     // nnz
+    uint16_t* v_off = nullptr;      // n_vrows: the row's first entry, modulo kFwdEntries
+    void*     v_spot = nullptr;     // nnz: uint16_t with spot16, else uint32_t
+    bool      spot16 = false;       // n_spots <= 65536
     float*    v_value = nullptr;    // nnz
     uint64_t  n_seg = 0;            // backward segments: contiguous runs of one row's entries
     uint64_t* seg_start = nullptr;  // n_seg + 1

@@ -12,6 +12,7 @@
 // Both products are gathers with a fixed reduction order: no atomics, reproducible results.
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 #include <utility>
 
 #include <cuda_runtime.h>
@@ -337,12 +338,14 @@ k_count_rows(const unsigned long long* __restrict__ keys, uint64_t n, uint32_t v
     if (threadIdx.x == 0) tiles[blockIdx.x] = sum;
 }
 
-/// Voxel-row entries -- the spot column and the value of each sorted key -- and the rows' voxels and
-/// first entries; tiles[b] = the rows that start before tile b.
+/// Voxel-row entries -- the spot column (Spot: 16 bits where the columns allow) and the value of each
+/// sorted key -- and the rows' voxels, first entries (indptr) and those within their stretch of
+/// kFwdEntries (off); tiles[b] = the rows that start before tile b.
+template<typename Spot>
 __global__ void __launch_bounds__(kThreads)
 k_voxel_rows(const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ vals, uint64_t n, int vbits,
-             const uint32_t* __restrict__ tiles, uint32_t* __restrict__ row_voxel, uint64_t* __restrict__ indptr,
-             uint32_t* __restrict__ spot, uint32_t* __restrict__ val) {
+             const uint32_t* __restrict__ tiles, uint32_t* __restrict__ row_voxel, uint16_t* __restrict__ off,
+             uint64_t* __restrict__ indptr, Spot* __restrict__ spot, uint32_t* __restrict__ val) {
     __shared__ uint32_t ws[32];
     const uint32_t vmask = (uint32_t) ((1ull << vbits) - 1ull);
     const uint64_t t0    = (uint64_t) blockIdx.x * kScanTile;
@@ -354,11 +357,12 @@ k_voxel_rows(const unsigned long long* __restrict__ keys, const uint32_t* __rest
         const uint32_t at = row + block_exclusive_scan(start ? 1u : 0u, ws, total);
         if (j < n) {
             const unsigned long long k = keys[j];
-            spot[j] = (uint32_t) (k >> vbits);
+            spot[j] = (Spot) (k >> vbits);
             val[j]  = vals[j];
             if (start) {
                 row_voxel[at] = (uint32_t) k & vmask;
                 indptr[at]    = j;
+                off[at]       = (uint16_t) (j % kFwdEntries);
             }
             if (j == n - 1) indptr[at + (start ? 1u : 0u)] = n;
         }
@@ -400,61 +404,68 @@ k_fwd_blocks(const uint64_t* __restrict__ indptr, uint64_t n_rows, uint64_t n_bl
     run_k[b]         = indptr[r];
 }
 
-/// dose[row_voxel[r]] = sum_k val[k] * w[spot[k]] over voxel rows (D.w).  A block stages the
-/// products of its rows' entries -- a contiguous run of at most kFwdEntries + the longest row,
-/// read with coalesced loads -- in shared memory, then each thread sums whole rows from there in
-/// entry order (a fixed order: the result does not depend on the launch).  A run longer than the
-/// staging buffer (a row of more than kFwdStage - kFwdEntries entries) is summed from global
-/// memory instead, in the same order.  Accumulates in T.
-template<typename T>
+/// Where a voxel row lies: the rows of run b start in entries [b * kFwdEntries, (b + 1) * kFwdEntries),
+/// so two bytes a row say where (an 8-byte row pointer was a fifth of what the product read on a
+/// plan's matrix, which has about four entries to a row).
+__device__ __forceinline__ void
+row_span(const uint16_t* __restrict__ off, uint32_t r, uint32_t r1, uint64_t base, uint64_t k1, uint64_t& rb, uint64_t& re) {
+    rb = base + off[r];
+    re = r + 1 < r1 ? base + off[r + 1] : k1;
+}
+
+/// dose[row_voxel[r]] = sum_k val[k] * w[spot[k]] over voxel rows (D.w), in FP64.  Block b stages
+/// the products of run b's entries -- at most kFwdEntries + the longest row, read with coalesced
+/// loads -- in shared memory, then each thread sums whole rows from there in entry order (a fixed
+/// order: the result does not depend on the launch).  A run longer than the staging buffer (a row of
+/// more than kFwdStage - kFwdEntries entries) is summed from global memory instead, in the same order.
+template<typename Spot>
 __global__ void __launch_bounds__(256)
-k_dij_forward(const uint32_t* __restrict__ row_voxel, const uint64_t* __restrict__ indptr,
-              const uint32_t* __restrict__ row_first, const uint32_t* __restrict__ spot, const float* __restrict__ val,
-              const T* __restrict__ w, T* __restrict__ dose) {
+k_dij_forward(const uint32_t* __restrict__ row_voxel, const uint16_t* __restrict__ off,
+              const uint32_t* __restrict__ row_first, const uint64_t* __restrict__ run_k, const Spot* __restrict__ spot,
+              const float* __restrict__ val, const double* __restrict__ w, double* __restrict__ dose) {
+    using Spot4 = typename std::conditional<sizeof(Spot) == 2, ushort4, uint4>::type;
     extern __shared__ __align__(16) unsigned char fwd_smem[];
-    T* prod = reinterpret_cast<T*>(fwd_smem);
+    double* prod = reinterpret_cast<double*>(fwd_smem);
     const uint32_t r0 = row_first[blockIdx.x], r1 = row_first[blockIdx.x + 1];
     if (r0 >= r1) return;
-    const uint64_t k0 = indptr[r0], k1 = indptr[r1];
+    const uint64_t base = blockIdx.x * kFwdEntries, k0 = run_k[blockIdx.x], k1 = run_k[blockIdx.x + 1];
     const bool     staged = k1 - k0 <= kFwdStage;
     // the thread's first row is read before the staging, so that its latency overlaps it
     uint32_t r  = r0 + threadIdx.x;
     uint64_t rb = 0, re = 0;
     uint32_t rv = 0;
     if (r < r1) {
-        rb = indptr[r];
-        re = indptr[r + 1];
+        row_span(off, r, r1, base, k1, rb, re);
         rv = row_voxel[r];
     }
     if (staged) {
-        // 16-byte loads of whole groups of four entries (the arrays are padded to whole groups);
+        // loads of whole groups of four entries (the arrays are padded to whole groups);
         // entries of the group outside [k0, k1) are skipped
-        const uint4*   s4 = reinterpret_cast<const uint4*>(spot);
+        const Spot4*   s4 = reinterpret_cast<const Spot4*>(spot);
         const float4*  v4 = reinterpret_cast<const float4*>(val);
         const uint64_t q1 = (k1 + 3) >> 2;
 #pragma unroll 2
         for (uint64_t q = (k0 >> 2) + threadIdx.x; q < q1; q += blockDim.x) {
-            const uint4    ss = s4[q];
+            const Spot4    ss = s4[q];
             const float4   vv = v4[q];
             const uint64_t k  = q << 2;
-            if (k >= k0 && k < k1) prod[k - k0] = (T) vv.x * w[ss.x];
-            if (k + 1 >= k0 && k + 1 < k1) prod[k + 1 - k0] = (T) vv.y * w[ss.y];
-            if (k + 2 >= k0 && k + 2 < k1) prod[k + 2 - k0] = (T) vv.z * w[ss.z];
-            if (k + 3 >= k0 && k + 3 < k1) prod[k + 3 - k0] = (T) vv.w * w[ss.w];
+            if (k >= k0 && k < k1) prod[k - k0] = (double) vv.x * w[ss.x];
+            if (k + 1 >= k0 && k + 1 < k1) prod[k + 1 - k0] = (double) vv.y * w[ss.y];
+            if (k + 2 >= k0 && k + 2 < k1) prod[k + 2 - k0] = (double) vv.z * w[ss.z];
+            if (k + 3 >= k0 && k + 3 < k1) prod[k + 3 - k0] = (double) vv.w * w[ss.w];
         }
         __syncthreads();
     }
     while (r < r1) {
-        T acc = T(0);
+        double acc = 0.0;
         if (staged)
             for (uint64_t k = rb; k < re; ++k) acc += prod[k - k0];
         else
-            for (uint64_t k = rb; k < re; ++k) acc += (T) val[k] * w[spot[k]];
+            for (uint64_t k = rb; k < re; ++k) acc += (double) val[k] * w[spot[k]];
         dose[rv] = acc;
         r += blockDim.x;
         if (r < r1) {
-            rb = indptr[r];
-            re = indptr[r + 1];
+            row_span(off, r, r1, base, k1, rb, re);
             rv = row_voxel[r];
         }
     }
@@ -500,14 +511,15 @@ mbar_try_wait(uint64_t* bar, uint32_t parity) {
 
 /// The rows and entries of one run of the persistent forward, as thread 0 found them.
 struct FwdRun {
-    unsigned long long k0, k1, a0;   // entries [k0, k1); staged from a0 (k0 rounded down to a group of four)
+    unsigned long long k0, k1, a0;   // entries [k0, k1); staged from a0 (k0 rounded down to a group of eight)
     uint32_t           r0, r1;       // voxel rows [r0, r1)
     uint32_t           staged, pad;
 };
 static_assert(sizeof(FwdRun) == 40, "FwdRun layout");
 
-constexpr uint32_t kFwdPipeHeader     = 256;                                  // kFwdStages mbarriers + FwdRuns
-constexpr uint32_t kFwdPipeStageBytes = (uint32_t) kFwdPipeStageEntries * 8;  // spots then values
+constexpr int      kFwdRowsAhead  = 2;     // rows a thread reads ahead
+constexpr int      kFwdBatch      = 4;     // products a thread forms at a time
+constexpr uint32_t kFwdPipeHeader = 256;   // kFwdStages mbarriers + FwdRuns
 static_assert(kFwdStages * (8 + sizeof(FwdRun)) <= kFwdPipeHeader, "forward header");
 
 /// D.w in FP32, persistent, through a ring of kFwdStages shared-memory stages.  Each CTA walks the
@@ -515,18 +527,27 @@ static_assert(kFwdStages * (8 + sizeof(FwdRun)) <= kFwdPipeHeader, "forward head
 /// [b * kFwdEntries, (b + 1) * kFwdEntries), row_first[b] to row_first[b + 1], first entry
 /// run_k[b]).  While the block forms and sums run i from one stage, the copy engine fills the
 /// others with runs i + 1 .. i + kFwdStages - 1: thread 0 issues two untiled bulk copies per run
-/// (its spots and values, rounded out to whole 16-byte groups; the arrays are padded) completing
-/// on that stage's mbarrier, so each CTA keeps kFwdStages - 1 runs' bytes in flight while it
-/// computes.  In a run the block multiplies each value by w[spot] in place, then each thread sums
+/// (its spots and values, rounded out to whole groups of eight entries; the arrays are padded)
+/// completing on that stage's mbarrier, so each CTA keeps kFwdStages - 1 runs' bytes in flight while
+/// it computes.  In a run the block multiplies each value by w[spot] in place, then each thread sums
 /// whole rows from there in entry order (as k_dij_forward does): the result does not depend on
 /// the grid.  Waits are bounded: a block whose copies have not landed after ~1 s of polling sets
 /// bit 8 of `err`, waits (bounded) for its other stages' copies and returns.  A run longer than a
 /// stage (kFwdPipeStageEntries entries: a row of more than ~2000 spots) is summed from global memory.
+///
+/// It reads an entry's spot (2 or 4 bytes) and value and 6 bytes a row, and writes the dose: on a
+/// 500-spot CT matrix (9.1e7 entries, 1.5e7 rows) 235 us before the 2-byte spots and row offsets, 195
+/// now, 0.55 of the measured copy rate.  What is left is latency between the barriers of a run:
+/// neither the product pass, the row sums nor the stores cost more than 25 us by themselves, and
+/// weights in shared memory, shorter runs and deeper rings gave nothing.
+template<typename Spot>
 __global__ void __launch_bounds__(kFwdPipeThreads)
-k_dij_forward_pipe(const uint32_t* __restrict__ row_voxel, const uint64_t* __restrict__ indptr,
+k_dij_forward_pipe(const uint32_t* __restrict__ row_voxel, const uint16_t* __restrict__ off,
                    const uint32_t* __restrict__ row_first, const uint64_t* __restrict__ run_k, uint64_t n_blocks,
-                   const uint32_t* __restrict__ spot, const float* __restrict__ val, const float* __restrict__ w,
+                   const Spot* __restrict__ spot, const float* __restrict__ val, const float* __restrict__ w,
                    float* __restrict__ dose, uint32_t* __restrict__ err) {
+    constexpr uint32_t kSpotBytes  = (uint32_t) kFwdPipeStageEntries * sizeof(Spot);
+    constexpr uint32_t kStageBytes = kSpotBytes + (uint32_t) kFwdPipeStageEntries * sizeof(float);
     extern __shared__ __align__(16) unsigned char fwd_smem[];
     uint64_t*      bar  = reinterpret_cast<uint64_t*>(fwd_smem);
     FwdRun*        runs = reinterpret_cast<FwdRun*>(fwd_smem + 8 * kFwdStages);
@@ -551,16 +572,16 @@ k_dij_forward_pipe(const uint32_t* __restrict__ row_voxel, const uint64_t* __res
         R.r1  = pf_r1;
         R.k0  = pf_k0;
         R.k1  = pf_k1;
-        R.a0  = R.k0 & ~3ull;
+        R.a0  = R.k0 & ~7ull;
         R.pad = 0;
-        const unsigned long long a1 = (R.k1 + 3ull) & ~3ull;
+        const unsigned long long a1 = (R.k1 + 7ull) & ~7ull;
         R.staged = (R.r0 < R.r1 && a1 - R.a0 <= kFwdPipeStageEntries) ? 1u : 0u;
         if (R.staged) {
-            const uint32_t bytes = (uint32_t) ((a1 - R.a0) * sizeof(uint32_t));
-            unsigned char* st    = data + (size_t) s * kFwdPipeStageBytes;
-            mbar_expect_tx(&bar[s], 2 * bytes);
-            bulk_load(st, spot + R.a0, bytes, &bar[s]);
-            bulk_load(st + kFwdPipeStageEntries * sizeof(uint32_t), val + R.a0, bytes, &bar[s]);
+            const uint32_t m  = (uint32_t) (a1 - R.a0);
+            unsigned char* st = data + (size_t) s * kStageBytes;
+            mbar_expect_tx(&bar[s], m * (uint32_t) (sizeof(Spot) + sizeof(float)));
+            bulk_load(st, spot + R.a0, m * (uint32_t) sizeof(Spot), &bar[s]);
+            bulk_load(st + kSpotBytes, val + R.a0, m * (uint32_t) sizeof(float), &bar[s]);
         }
         runs[s] = R;
     };
@@ -589,17 +610,19 @@ k_dij_forward_pipe(const uint32_t* __restrict__ row_voxel, const uint64_t* __res
         }
         const FwdRun R = runs[s];
         if (R.r0 < R.r1) {
-            uint32_t r  = R.r0 + tid;
-            uint64_t rb = 0, re = 0;
-            uint32_t rv = 0;
-            if (r < R.r1) {
-                rb = indptr[r];
-                re = indptr[r + 1];
-                rv = row_voxel[r];
+            const uint64_t base = b * kFwdEntries;
+            // the thread's first rows, all read before the wait: one latency, and that behind the copies
+            uint32_t rv[kFwdRowsAhead], ob[kFwdRowsAhead], oe[kFwdRowsAhead];
+#pragma unroll
+            for (int i = 0; i < kFwdRowsAhead; ++i) {
+                const uint32_t r = R.r0 + tid + i * kFwdPipeThreads;
+                if (r < R.r1) {
+                    rv[i] = row_voxel[r];
+                    ob[i] = off[r];
+                    oe[i] = r + 1 < R.r1 ? off[r + 1] : (uint32_t) (R.k1 - base);
+                }
             }
-            uint32_t* s_spot = reinterpret_cast<uint32_t*>(data + (size_t) s * kFwdPipeStageBytes);
-            float*    s_val  = reinterpret_cast<float*>(data + (size_t) s * kFwdPipeStageBytes +
-                                                       kFwdPipeStageEntries * sizeof(uint32_t));
+            float* s_val = reinterpret_cast<float*>(data + (size_t) s * kStageBytes + kSpotBytes);
             if (R.staged) {
                 bool     done  = false;
                 uint32_t spins = 0;
@@ -610,23 +633,34 @@ k_dij_forward_pipe(const uint32_t* __restrict__ row_voxel, const uint64_t* __res
                     failed = true;
                     break;
                 }
-                for (uint64_t k = R.k0 + tid; k < R.k1; k += blockDim.x) s_val[k - R.a0] *= w[s_spot[k - R.a0]];
+                const Spot*    s_spot = reinterpret_cast<const Spot*>(data + (size_t) s * kStageBytes);
+                const uint32_t m0 = (uint32_t) (R.k0 - R.a0), m1 = (uint32_t) (R.k1 - R.a0);
+                for (uint32_t k = m0 + tid; k < m1; k += kFwdBatch * kFwdPipeThreads) {
+                    float x[kFwdBatch];
+#pragma unroll
+                    for (int i = 0; i < kFwdBatch; ++i)
+                        x[i] = k + i * kFwdPipeThreads < m1 ? w[s_spot[k + i * kFwdPipeThreads]] : 0.0f;
+#pragma unroll
+                    for (int i = 0; i < kFwdBatch; ++i)
+                        if (k + i * kFwdPipeThreads < m1) s_val[k + i * kFwdPipeThreads] *= x[i];
+                }
                 __syncthreads();
             }
-            while (r < R.r1) {
+            auto row_sum = [&](uint32_t o0, uint32_t o1) {
                 float acc = 0.0f;
-                if (R.staged)
-                    for (uint64_t k = rb; k < re; ++k) acc += s_val[k - R.a0];
-                else
-                    for (uint64_t k = rb; k < re; ++k) acc += val[k] * w[spot[k]];
-                dose[rv] = acc;
-                r += blockDim.x;
-                if (r < R.r1) {
-                    rb = indptr[r];
-                    re = indptr[r + 1];
-                    rv = row_voxel[r];
+                if (R.staged) {
+                    const uint32_t e = (uint32_t) (base + o1 - R.a0);
+                    for (uint32_t k = (uint32_t) (base + o0 - R.a0); k < e; ++k) acc += s_val[k];
+                } else {
+                    for (uint64_t k = base + o0; k < base + o1; ++k) acc += val[k] * w[spot[k]];
                 }
-            }
+                return acc;
+            };
+#pragma unroll
+            for (int i = 0; i < kFwdRowsAhead; ++i)
+                if (R.r0 + tid + i * kFwdPipeThreads < R.r1) dose[rv[i]] = row_sum(ob[i], oe[i]);
+            for (uint32_t r = R.r0 + tid + kFwdRowsAhead * kFwdPipeThreads; r < R.r1; r += kFwdPipeThreads)
+                dose[row_voxel[r]] = row_sum(off[r], r + 1 < R.r1 ? off[r + 1] : (uint32_t) (R.k1 - base));
         }
         __syncthreads();   // stage s is free: the next iteration refills it
         s = s + 1 == kFwdStages ? 0 : s + 1;
@@ -647,7 +681,7 @@ k_dij_forward_pipe(const uint32_t* __restrict__ row_voxel, const uint64_t* __res
 
 /// grad[s] = sum_k val[k] * g[voxel[k]] over spot rows (the transposed operator), in two passes
 /// with a fixed order.  Pass 1 (k_dij_backward_segments): the entries are cut into segments of at
-/// most kDijSegment entries that never cross a row; one block sums a segment's products (signed
+/// most dij_segment(nnz) entries that never cross a row; one block sums a segment's products (signed
 /// terms of a gradient cancel, so plain FP32 sums lose digits: a double-float accumulator per
 /// thread for FP32 g, FP64 for FP64 g; FP64 across the block) into one FP64 partial.  Pass 2
 /// (k_dij_backward_rows): one thread per row adds its segments' partials in order.  Rows of very
@@ -701,10 +735,10 @@ segment_sum(uint64_t b, uint64_t e, const uint32_t* __restrict__ vox, const floa
             const uint4    vv = v4[q];
             const float4   aa = a4[q];
             const uint64_t k  = q << 2;
-            if (k >= b && k < e) d += (double) aa.x * g[vv.x];
-            if (k + 1 >= b && k + 1 < e) d += (double) aa.y * g[vv.y];
-            if (k + 2 >= b && k + 2 < e) d += (double) aa.z * g[vv.z];
-            if (k + 3 >= b && k + 3 < e) d += (double) aa.w * g[vv.w];
+            if (k >= b && k < e) d = __fma_rn((double) aa.x, g[vv.x], d);
+            if (k + 1 >= b && k + 1 < e) d = __fma_rn((double) aa.y, g[vv.y], d);
+            if (k + 2 >= b && k + 2 < e) d = __fma_rn((double) aa.z, g[vv.z], d);
+            if (k + 3 >= b && k + 3 < e) d = __fma_rn((double) aa.w, g[vv.w], d);
         }
         return d;
     }
@@ -746,16 +780,20 @@ k_dij_backward_segments(const uint32_t* __restrict__ order, uint32_t n_seg, cons
     }
 }
 
+/// A warp a row: its lanes add every 32nd segment's partial, then each other in a fixed tree.  (A
+/// thread a row read its partials one after the other: 13.5 us for 500 rows of 14.)
 template<typename T>
 __global__ void
 k_dij_backward_rows(const uint32_t* __restrict__ row_seg, uint32_t n_rows, const double* __restrict__ partial,
                     T* __restrict__ grad, uint32_t* __restrict__ cursor) {
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r == 0 && cursor) *cursor = 0u;
+    const uint32_t r    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    if (r == 0 && lane == 0 && cursor) *cursor = 0u;
     if (r >= n_rows) return;
     double d = 0.0;
-    for (uint32_t k = row_seg[r]; k < row_seg[r + 1]; ++k) d += partial[k];
-    grad[r] = (T) d;
+    for (uint32_t k = row_seg[r] + lane, e = row_seg[r + 1]; k < e; k += 32) d += partial[k];
+    for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xFFFFFFFFu, d, o);
+    if (lane == 0) grad[r] = (T) d;
 }
 
 __global__ void
@@ -870,10 +908,14 @@ dij_count_rows(const unsigned long long* keys, uint64_t n, int vbits, uint32_t* 
 
 cudaError_t
 dij_voxel_rows(const unsigned long long* keys, const uint32_t* vals, uint64_t n, int vbits, const uint32_t* tiles,
-               uint32_t* row_voxel, uint64_t* indptr, uint32_t* spot, float* val, cudaStream_t s) {
+               uint32_t* row_voxel, uint16_t* off, uint64_t* indptr, void* spot, bool spot16, float* val, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    k_voxel_rows<<<(unsigned) ((n + kScanTile - 1) / kScanTile), kThreads, 0, s>>>(
-        keys, vals, n, vbits, tiles, row_voxel, indptr, spot, reinterpret_cast<uint32_t*>(val));
+    const unsigned nt = (unsigned) ((n + kScanTile - 1) / kScanTile);
+    uint32_t*      v  = reinterpret_cast<uint32_t*>(val);
+    if (spot16)
+        k_voxel_rows<<<nt, kThreads, 0, s>>>(keys, vals, n, vbits, tiles, row_voxel, off, indptr, (uint16_t*) spot, v);
+    else
+        k_voxel_rows<<<nt, kThreads, 0, s>>>(keys, vals, n, vbits, tiles, row_voxel, off, indptr, (uint32_t*) spot, v);
     return cudaGetLastError();
 }
 
@@ -894,29 +936,38 @@ dij_seg_order_keys(const uint64_t* seg_start, uint32_t n_seg, const uint32_t* vo
     return cudaGetLastError();
 }
 
-cudaError_t
-dij_forward(const uint32_t* row_voxel, const uint64_t* indptr, const uint32_t* row_first, const uint64_t* run_k,
-            uint64_t n_blocks, const uint32_t* spot, const float* val, const void* w, void* dose, int fp64, uint32_t* err,
-            int sms, cudaStream_t s) {
-    if (n_blocks == 0) return cudaSuccess;
+template<typename Spot>
+static cudaError_t
+forward(const uint32_t* row_voxel, const uint16_t* off, const uint32_t* row_first, const uint64_t* run_k, uint64_t n_blocks,
+        const Spot* spot, const float* val, const void* w, void* dose, int fp64, uint32_t* err, int sms, cudaStream_t s) {
     static_assert(kFwdStage * sizeof(double) <= 227 * 1024, "staging buffer exceeds shared memory");
     if (fp64) {
         const size_t sm = kFwdStage * sizeof(double);
-        cudaError_t  e  = cudaFuncSetAttribute(k_dij_forward<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
+        cudaError_t  e  = cudaFuncSetAttribute(k_dij_forward<Spot>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
         if (e != cudaSuccess) return e;
-        k_dij_forward<double><<<(unsigned) n_blocks, 256, sm, s>>>(row_voxel, indptr, row_first, spot, val,
-                                                                  (const double*) w, (double*) dose);
+        k_dij_forward<Spot><<<(unsigned) n_blocks, 256, sm, s>>>(row_voxel, off, row_first, run_k, spot, val,
+                                                                (const double*) w, (double*) dose);
     } else {
-        constexpr size_t sm = kFwdPipeHeader + kFwdStages * (size_t) kFwdPipeStageBytes;
-        static_assert(kFwdPipeBlocksPerSm * (sm + 1024) <= 228 * 1024, "the persistent forward blocks must fit one SM");
-        cudaError_t e = cudaFuncSetAttribute(k_dij_forward_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
+        constexpr size_t sm = kFwdPipeHeader + kFwdStages * kFwdPipeStageEntries * (sizeof(Spot) + sizeof(float));
+        constexpr int    per_sm = sizeof(Spot) == 2 ? 3 : 2;
+        static_assert(per_sm * (sm + 1024) <= 228 * 1024, "the persistent forward blocks must fit one SM");
+        cudaError_t e = cudaFuncSetAttribute(k_dij_forward_pipe<Spot>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
         if (e != cudaSuccess) return e;
-        const uint64_t cap  = (uint64_t) sms * kFwdPipeBlocksPerSm;
+        const uint64_t cap  = (uint64_t) sms * per_sm;
         const unsigned grid = (unsigned) (n_blocks < cap ? n_blocks : cap);
-        k_dij_forward_pipe<<<grid, kFwdPipeThreads, sm, s>>>(row_voxel, indptr, row_first, run_k, n_blocks, spot, val,
-                                                            (const float*) w, (float*) dose, err);
+        k_dij_forward_pipe<Spot><<<grid, kFwdPipeThreads, sm, s>>>(row_voxel, off, row_first, run_k, n_blocks, spot, val,
+                                                                  (const float*) w, (float*) dose, err);
     }
     return cudaGetLastError();
+}
+
+cudaError_t
+dij_forward(const uint32_t* row_voxel, const uint16_t* off, const uint32_t* row_first, const uint64_t* run_k,
+            uint64_t n_blocks, const void* spot, bool spot16, const float* val, const void* w, void* dose, int fp64,
+            uint32_t* err, int sms, cudaStream_t s) {
+    if (n_blocks == 0) return cudaSuccess;
+    return spot16 ? forward(row_voxel, off, row_first, run_k, n_blocks, (const uint16_t*) spot, val, w, dose, fp64, err, sms, s)
+                  : forward(row_voxel, off, row_first, run_k, n_blocks, (const uint32_t*) spot, val, w, dose, fp64, err, sms, s);
 }
 
 cudaError_t
@@ -934,7 +985,7 @@ dij_backward(const uint32_t* order, const uint64_t* seg_start, uint32_t n_seg, c
             k_dij_backward_segments<float><<<grid, 256, 0, s>>>(order, n_seg, seg_start, vox, val, (const float*) g,
                                                                 partial, cursor);
     }
-    const unsigned rb = (n_rows + 255) / 256;
+    const unsigned rb = (n_rows + 7) / 8;   // a warp a row
     if (fp64) k_dij_backward_rows<double><<<rb, 256, 0, s>>>(row_seg, n_rows, partial, (double*) grad, cursor);
     else k_dij_backward_rows<float><<<rb, 256, 0, s>>>(row_seg, n_rows, partial, (float*) grad, cursor);
     return cudaGetLastError();

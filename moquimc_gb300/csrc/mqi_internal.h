@@ -217,8 +217,8 @@ constexpr uint64_t kRowTile = 2048;   // entries of a tile of dij_count_rows
 cudaError_t dij_count_rows(const unsigned long long* keys, uint64_t n, int vbits, uint32_t* tiles, uint32_t* tile_rows,
                            uint32_t* scratch, cudaStream_t s);
 cudaError_t dij_voxel_rows(const unsigned long long* keys, const uint32_t* vals, uint64_t n, int vbits,
-                           const uint32_t* tiles, uint32_t* row_voxel, uint64_t* indptr, uint32_t* spot, float* val,
-                           cudaStream_t s);
+                           const uint32_t* tiles, uint32_t* row_voxel, uint16_t* off, uint64_t* indptr, void* spot,
+                           bool spot16, float* val, cudaStream_t s);
 constexpr uint64_t kFwdEntries = 4096;    // entries whose rows one forward block owns
 constexpr uint64_t kFwdStage   = 8192;    // staged products per forward block (rows up to 4096 entries)
 cudaError_t dij_forward_blocks(const uint64_t* indptr, uint64_t n_rows, uint64_t nnz, uint32_t* row_first,
@@ -226,12 +226,19 @@ cudaError_t dij_forward_blocks(const uint64_t* indptr, uint64_t n_rows, uint64_t
 constexpr uint64_t kFwdPipeStageEntries = 6144;   // entries one stage of the persistent forward holds
 constexpr int      kFwdStages           = 2;      // its ring of stages (one run in flight while one is summed)
 constexpr int      kFwdPipeThreads      = 512;    // persistent forward block
-constexpr int      kFwdPipeBlocksPerSm  = 2;      // two 96 KB blocks per SM
 constexpr uint32_t kBulkSpinLimit = 1u << 20;   // bounded polls of a bulk-copy mbarrier
-cudaError_t dij_forward(const uint32_t* row_voxel, const uint64_t* indptr, const uint32_t* row_first,
-                        const uint64_t* run_k, uint64_t n_blocks, const uint32_t* spot, const float* val, const void* w,
-                        void* dose, int fp64, uint32_t* err, int sms, cudaStream_t s);
-constexpr uint64_t kDijSegment = 16384;   // entries per backward segment (segments never cross a row)
+cudaError_t dij_forward(const uint32_t* row_voxel, const uint16_t* off, const uint32_t* row_first,
+                        const uint64_t* run_k, uint64_t n_blocks, const void* spot, bool spot16, const float* val,
+                        const void* w, void* dose, int fp64, uint32_t* err, int sms, cudaStream_t s);
+// Entries per backward segment (segments never cross a row): about one segment to a resident block
+// (8 per SM), within limits: a smaller matrix is cut finer, or most SMs would have nothing to sum.
+constexpr uint64_t kDijSegmentMin = 1024, kDijSegmentMax = 16384;
+inline uint64_t
+dij_segment(uint64_t nnz, int sms) {
+    uint64_t seg = kDijSegmentMin;
+    while (seg < kDijSegmentMax && seg * (uint64_t) sms * 8 < nnz) seg *= 2;
+    return seg;
+}
 cudaError_t dij_seg_order_keys(const uint64_t* seg_start, uint32_t n_seg, const uint32_t* vox, unsigned long long* okeys,
                                uint32_t* oval, cudaStream_t s);
 cudaError_t dij_backward(const uint32_t* order, const uint64_t* seg_start, uint32_t n_seg, const uint32_t* row_seg,

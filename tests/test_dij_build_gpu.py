@@ -32,16 +32,27 @@ def _check(c, dij, n_spots, nxyz):
     np.testing.assert_allclose(data, want, rtol=2.0 ** -23, atol=0)
     dose = np.zeros(nv)
     np.add.at(dose, key % nv, data.astype(np.float64))
-    np.testing.assert_allclose(c.dij_matvec(dij, np.ones(n_spots), nv), dose, rtol=1e-13, atol=0)
+    np.testing.assert_allclose(c.dij_matvec(dij, np.ones(n_spots), nv), dose, rtol=1e-13 * max(1, n_spots // 100), atol=0)
+    # FP32: a sum of m positive terms in order is off by at most m roundings
+    longest = np.bincount(key % nv).max() if len(key) else 1
+    np.testing.assert_allclose(c.dij_matvec(dij, np.ones(n_spots, np.float32), nv), dose, rtol=longest * 2.0 ** -24, atol=0)
+    g = np.random.default_rng(1).standard_normal(nv)
+    want = np.zeros(n_spots)
+    np.add.at(want, key // nv, data.astype(np.float64) * g[key % nv])
+    size = np.zeros(n_spots)
+    np.add.at(size, key // nv, np.abs(data.astype(np.float64) * g[key % nv]))
+    assert (np.abs(c.dij_rmatvec(dij, g, n_spots) - want) <= 1e-12 * size).all()
     return op
 
 
 @pytest.mark.parametrize("nxyz, spots, per_spot", [((1, 1, 2), 1, 3), ((3, 2, 5), 2, 40), ((16, 16, 65), 5, 200),
-                                                   ((64, 64, 130), 9, 300), ((64, 64, 130), 260, 12)])
+                                                   ((64, 64, 130), 9, 300), ((64, 64, 130), 260, 12),
+                                                   ((1, 1, 2), 7000, 2), ((2, 2, 5), 66_000, 1)])
 def test_build_against_the_recorded_insertions(gpu_ctx_factory, nxyz, spots, per_spot):
+    """The last two: rows longer than a stage of the forward, and columns past 16 bits."""
     c, cid = _context(gpu_ctx_factory, nxyz)
     dij = c.add_dij_scorer(cid, capacity=1 << 20)
-    c.dij_record_hits(dij, 1 << 22)
+    c.dij_record_hits(dij, 1 << 23)
     sp = workloads.spot_plan(spots, 1, 40.0 / spots, 0.5, 3.0, (60.0, 110.0), (per_spot, per_spot + 1))
     n = c.set_spot_plan(sp)
     c.transport_plan(0, n, 3)
