@@ -610,8 +610,6 @@ make_wave_params(mqi_ctx* c, uint64_t seed, WaveParams& P) {
     P.error_flag      = c->counters + 3;
     P.n_in            = c->counters + 0;
     P.n_out           = c->counters + 1;
-    P.def             = c->def;
-    P.def_cap         = c->queue_cap;
     P.drain           = reinterpret_cast<DrainState*>(c->counters + 8);
     P.stats           = c->stats;
     P.spot_ids        = c->has_spots ? c->spot_ids : nullptr;
@@ -642,6 +640,36 @@ load_histories(mqi_ctx* c, const WaveParams& P, const Queue& q, uint32_t have, u
     return MQI_OK;
 }
 
+/// Post-step records for a wave over n entries: as many, as an ordinary wave hands over each track at most
+/// once; half as many more in a draining one, which seldom needs them (wave_body finishes those past
+/// the end itself, slower).
+int
+ensure_records(mqi_ctx* c, WaveParams& P, uint32_t n, bool drains) {
+    const uint64_t want = drains ? (uint64_t) n + n / 2 + 4096 : n;
+    if (c->def_cap < want) {
+        cudaFree(c->def);
+        c->def     = nullptr;
+        c->def_cap = 0;
+        const uint64_t cap = std::max<uint64_t>(want, 1u << 16);
+        MQI_CUDA(c, cudaMalloc(&c->def, cap * sizeof(Deferred)), "mqi_transport: record allocation");
+        MQI_CUDA(c, cudaMemsetAsync(c->def, 0, cap * sizeof(Deferred), c->stream), "mqi_transport");
+        c->def_cap = (uint32_t) cap;
+    }
+    P.def     = c->def;
+    P.def_cap = c->def_cap;
+    return MQI_OK;
+}
+
+/// The queue sort's scratch, on its first use.
+int
+ensure_sort(mqi_ctx* c) {
+    if (c->qsort.q.capacity >= c->queue_cap && c->sort_bins) return MQI_OK;
+    MQI_CUDA(c, alloc_queue(c->qsort, c->queue_cap), "mqi_transport: sort allocation");
+    if (!c->sort_bins) MQI_CUDA(c, cudaMalloc(&c->sort_bins, 2 * kSortBins * sizeof(uint32_t)), "mqi_transport: sort allocation");
+    MQI_CUDA(c, cudaMemsetAsync(c->sort_bins, 0, 2 * kSortBins * sizeof(uint32_t), c->stream), "mqi_transport");
+    return MQI_OK;
+}
+
 /// One wave over the n entries of queue A, of which the first `old` are no fresh primaries; what it
 /// leaves for the next is in B, and its count and the error flag in host_counts[1] and [3].
 int
@@ -651,10 +679,12 @@ run_wave(mqi_ctx* c, WaveParams& P, const QueueBuf& A, const QueueBuf& B, uint32
     P.ready = nullptr;
     P.epoch = 0;
     P.lanes = 32;
+    int rc  = ensure_records(c, P, n, drains);
+    if (rc != MQI_OK) return rc;
     if (drains) {
         if (++c->epoch >> 30) {   // the marks of 2^30 waves ago
             MQI_CUDA(c, cudaMemsetAsync(c->ready, 0, (size_t) c->queue_cap * sizeof(uint32_t), c->stream), "mqi_transport");
-            MQI_CUDA(c, cudaMemsetAsync(c->def, 0, (size_t) c->queue_cap * sizeof(Deferred), c->stream), "mqi_transport");
+            MQI_CUDA(c, cudaMemsetAsync(c->def, 0, (size_t) c->def_cap * sizeof(Deferred), c->stream), "mqi_transport");
             c->epoch = 1;
         }
         P.ready = c->ready;
@@ -663,7 +693,9 @@ run_wave(mqi_ctx* c, WaveParams& P, const QueueBuf& A, const QueueBuf& B, uint32
     }
     // fresh primaries keep their order: a queue that holds nothing else is not sorted
     const bool sort = c->sort_min > 0 && old > 0 && n >= c->sort_min;
-    P.sort_bins     = sort ? c->sort_bins : nullptr;
+    if (sort && (rc = ensure_sort(c)) != MQI_OK) return rc;
+    P.sort_tmp  = c->qsort.q;
+    P.sort_bins = sort ? c->sort_bins : nullptr;
     const uint32_t counts[12] = { n, 0, 0, 0, 0, 0, 0, 0, n, n, 0, 0 };
     std::memcpy(c->host_counts, counts, sizeof(counts));
     MQI_CUDA(c, cudaMemcpyAsync(c->counters, c->host_counts, sizeof(counts), cudaMemcpyHostToDevice, c->stream),
@@ -722,20 +754,12 @@ run_transport(mqi_ctx* c, uint64_t h0, uint64_t h1, uint64_t seed, bool plan) {
     DeviceGuard g(c->device);
     const uint32_t need = c->primary_chunk * 3u;
     if (c->queue_cap < need) {
-        cudaFree(c->def);
         cudaFree(c->ready);
-        c->def        = nullptr;
         c->ready      = nullptr;
         cudaError_t e = alloc_queue(c->qa, need);
+        if (e == cudaSuccess) e = alloc_queue(c->qb, need);
         if (e == cudaSuccess) e = cudaMalloc(&c->ready, (size_t) need * sizeof(uint32_t));
         if (e == cudaSuccess) e = cudaMemsetAsync(c->ready, 0, (size_t) need * sizeof(uint32_t), c->stream);
-        c->epoch = 0;
-        if (e == cudaSuccess) e = alloc_queue(c->qb, need);
-        if (e == cudaSuccess) e = cudaMalloc(&c->def, (size_t) need * sizeof(Deferred));
-        if (e == cudaSuccess) e = cudaMemsetAsync(c->def, 0, (size_t) need * sizeof(Deferred), c->stream);
-        if (e == cudaSuccess) e = alloc_queue(c->qsort, need);
-        if (e == cudaSuccess && !c->sort_bins) e = cudaMalloc(&c->sort_bins, 2 * kSortBins * sizeof(uint32_t));
-        if (e == cudaSuccess) e = cudaMemsetAsync(c->sort_bins, 0, 2 * kSortBins * sizeof(uint32_t), c->stream);
         if (e != cudaSuccess) {
             c->queue_cap = 0;
             return cuda_fail(c, e, "mqi_transport: queue allocation");
@@ -744,7 +768,6 @@ run_transport(mqi_ctx* c, uint64_t h0, uint64_t h1, uint64_t seed, bool plan) {
     }
     WaveParams P;
     make_wave_params(c, seed, P);
-    P.sort_tmp = c->qsort.q;
     P.sort_min = c->sort_min;
     uint32_t  flags = 0;
     const int rc    = run_waves(c, P, h0, h1, plan, flags);

@@ -156,8 +156,9 @@ struct mqi_ctx {
     bool                    has_spots = false;
     mqi_gpu::QueueBuf       qa, qb;
     uint32_t                queue_cap = 0;
-    mqi_gpu::Deferred*      def = nullptr;          // tracks a wave stopped at nuclear interactions (queue_cap)
-    mqi_gpu::QueueBuf       qsort;                  // scratch of the energy-bin queue sort (queue_cap)
+    mqi_gpu::Deferred*      def = nullptr;          // tracks a wave stopped at nuclear interactions
+    uint32_t                def_cap = 0;
+    mqi_gpu::QueueBuf       qsort;                  // scratch of the energy-bin queue sort (queue_cap, on first use)
     uint32_t*               sort_bins = nullptr;    // 2 x kSortBins counters of the sort
     uint32_t                sort_min = 1u << 18;    // sort waves of at least this many entries (0: never)
     uint32_t*               ready = nullptr;        // marks of the entries a draining wave appended (queue_cap)
