@@ -724,7 +724,13 @@ run_wave(mqi_ctx* c, WaveParams& P, const QueueBuf& A, const QueueBuf& B, uint32
 int
 run_waves(mqi_ctx* c, WaveParams& P, uint64_t h0, uint64_t h1, bool plan, uint32_t& flags) {
     const uint32_t S      = c->n_scen;
-    const uint32_t target = std::max<uint32_t>(c->primary_chunk / S, 1u) * S;
+    // A run of at most two queue loads goes in one where a primary leaves well under one track behind
+    // (every run but those that queue debug physics' deposit-only daughters): the queue holds three
+    // loads, and a second, partial load would pay for a drain of its own (3 M histories on the CT: 60.0
+    // -> 55.5 ms; longer runs gain nothing from larger loads).
+    const uint64_t all    = (h1 - h0) * (uint64_t) S;
+    const bool     in_one = c->streamed && all <= 2ull * c->primary_chunk && (P.inline_local || !P.physics_debug);
+    const uint32_t target = in_one ? (uint32_t) all : std::max<uint32_t>(c->primary_chunk / S, 1u) * S;
     const bool     may_drain = c->post_step_mode != 1 && P.max_slice_steps == 0;
     const QueueBuf *A = &c->qa, *B = &c->qb;
     uint64_t        h = h0;

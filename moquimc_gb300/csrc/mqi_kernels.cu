@@ -1213,6 +1213,8 @@ wave_body(const WaveParams& P) {
     bool     in_grid = false;
     uint32_t slice = 0;
     uint32_t track_steps = 0;   // per-track guard: a track is abandoned after kMaxTrackSteps
+    unsigned held = 0u;         // the lanes that hold one
+    uint32_t turn = 0;
     for (;;) {
         // ---- a queue index for every lane without one (one atomic per warp) ----
         const bool     want  = open && !have && !waits;
@@ -1227,8 +1229,11 @@ wave_body(const WaveParams& P) {
                 waits  = true;
             }
         }
-        // ---- the track at that index, once there is one ----
-        if (waits) {
+        // ---- the track at that index, once there is one.  Beyond the wave's first entries that takes a
+        // read from L2, which the warp's other lanes wait for: a warp with tracks looks at once, and then
+        // every eighth time.
+        if constexpr (kDrain) ++turn;
+        if (waits && (!kDrain || ticket < n_in || want || held == 0u || (turn & 7u) == 0u)) {
             bool there = ticket < n_in;
             if (kDrain && !there) {
                 there = ticket < P.in.capacity && *reinterpret_cast<volatile uint32_t*>(P.ready + ticket) == P.epoch;
@@ -1257,7 +1262,7 @@ wave_body(const WaveParams& P) {
                 }
             }
         }
-        const unsigned held = __ballot_sync(0xFFFFFFFFu, have);
+        held = __ballot_sync(0xFFFFFFFFu, have);
         if (!held) break;
         polls       = 0;
         bool handed = false;   // to a post-step: the track is still live
