@@ -65,6 +65,31 @@ drop_materials(mqi_ctx* c) {
     for (ChildHost& ch : c->children) drop_materials(ch);
 }
 
+/// Tabulate a CONTOUR scorer's ROI by voxel (8 bytes per 32 voxels).  Without the memory, or where the
+/// runs are not ones that a table can hold, the search stays.
+void
+build_roi_words(mqi_ctx* c, ScorerHost& s, uint64_t n_vox) {
+    const uint64_t n = (n_vox + 31) / 32;
+    ScorerDev      d{};
+    d.roi_method = s.roi_method; d.roi_len = s.roi_len;
+    d.start = s.start; d.stride = s.stride; d.acc = s.acc;
+    uint32_t *counts = nullptr, *ranks = nullptr, *scratch = nullptr, *bad = nullptr;
+    uint32_t  is_bad = 1;
+    cudaError_t e = cudaMalloc(&s.roi_words, n * sizeof(uint2));
+    if (e == cudaSuccess) e = cudaMalloc(&counts, n * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&ranks, n * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&scratch, scan_scratch_words(n) * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&bad, sizeof(uint32_t));
+    if (e == cudaSuccess) e = launch_roi_words(d, n_vox, s.roi_words, counts, ranks, scratch, bad, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&is_bad, bad, sizeof(is_bad), cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    cudaFree(counts); cudaFree(ranks); cudaFree(scratch); cudaFree(bad);
+    if (e == cudaSuccess && !is_bad) return;
+    (void) cudaGetLastError();
+    cudaFree(s.roi_words);
+    s.roi_words = nullptr;
+}
+
 void
 identity3(float* m) {
     for (int i = 0; i < 9; ++i) m[i] = (i % 4 == 0) ? 1.0f : 0.0f;
@@ -183,7 +208,7 @@ mqi_destroy(mqi_ctx* c) {
         drop_materials(ch);
     }
     for (auto& s : c->scorers) {
-        cudaFree(s.start); cudaFree(s.stride); cudaFree(s.acc);
+        cudaFree(s.start); cudaFree(s.stride); cudaFree(s.acc); cudaFree(s.roi_words);
         if (s.owns) cudaFree(s.tally);
         cudaFree(s.batch_s1); cudaFree(s.batch_s2);
         dij_release(s);
@@ -460,6 +485,7 @@ mqi_add_scorer(mqi_ctx* c, int child_id, int type, int roi_method, uint32_t roi_
     } else {
         return fail(c, MQI_ERR_INVALID, "mqi_add_scorer: unknown roi method");
     }
+    if (roi_method == MQI_ROI_CONTOUR) build_roi_words(c, s, nvox);
     s.copies = c->n_scen;
     MQI_CUDA(c, cudaMalloc(&s.tally, s.total() * sizeof(double)), "mqi_add_scorer");
     MQI_CUDA(c, cudaMemset(s.tally, 0, s.total() * sizeof(double)), "mqi_add_scorer");
@@ -555,7 +581,7 @@ make_wave_params(mqi_ctx* c, uint64_t seed, WaveParams& P) {
         const ScorerHost& s = c->scorers[i];
         ScorerDev&        d = P.scorer[i];
         d.type = s.type; d.roi_method = s.roi_method; d.stat_mode = s.stat_mode;
-        d.roi_len = s.roi_len; d.start = s.start; d.stride = s.stride; d.acc = s.acc;
+        d.roi_len = s.roi_len; d.start = s.start; d.stride = s.stride; d.acc = s.acc; d.roi_words = s.roi_words;
         d.tally = s.tally; d.tally_len = s.tally_len; d.tstride = s.tstride;
         d.dij = s.dij; d.dij_mask = s.dij_cap ? s.dij_cap - 1 : 0;
         d.hit_log = s.hit_log; d.hit_count = s.hit_count; d.hit_cap = s.hit_cap;
@@ -1267,7 +1293,7 @@ mqi_eval_roi(mqi_ctx* c, int scorer_id, const uint32_t* voxels, uint64_t n, int3
         if (voxels[i] >= nvox) return fail(c, MQI_ERR_INVALID, "mqi_eval_roi: a voxel index is outside the grid");
     ScorerDev d{};
     d.type = s.type; d.roi_method = s.roi_method; d.stat_mode = s.stat_mode;
-    d.roi_len = s.roi_len; d.start = s.start; d.stride = s.stride; d.acc = s.acc;
+    d.roi_len = s.roi_len; d.start = s.start; d.stride = s.stride; d.acc = s.acc; d.roi_words = s.roi_words;
     DeviceGuard g(c->device);
     uint32_t* dv = nullptr;
     int32_t*  di = nullptr;
@@ -1373,6 +1399,7 @@ mqi_add_stat_scorers(mqi_ctx* c, int child_id, int roi_method, uint32_t roi_leng
             MQI_CUDA(c, cudaMalloc(&s.acc, roi_length * sizeof(uint32_t)), "mqi_add_stat_scorers");
             MQI_CUDA(c, cudaMemcpy(s.stride, roi_stride, roi_length * sizeof(uint32_t), cudaMemcpyHostToDevice), "mqi_add_stat_scorers");
             MQI_CUDA(c, cudaMemcpy(s.acc, roi_acc, roi_length * sizeof(uint32_t), cudaMemcpyHostToDevice), "mqi_add_stat_scorers");
+            build_roi_words(c, s, nvox);
         }
         s.copies = c->n_scen;
         s.tstride = 2;

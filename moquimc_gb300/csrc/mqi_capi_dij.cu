@@ -143,7 +143,7 @@ mqi_add_dij_scorer(mqi_ctx* c, int child_id, int roi_method, uint32_t roi_length
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         dij_release(s);
-        cudaFree(s.start); cudaFree(s.stride); cudaFree(s.acc);
+        cudaFree(s.start); cudaFree(s.stride); cudaFree(s.acc); cudaFree(s.roi_words);
         c->scorers.pop_back();
         return cuda_fail(c, e, "mqi_add_dij_scorer");
     }

@@ -78,6 +78,7 @@ struct ScorerHost {
     uint32_t* start = nullptr;
     uint32_t* stride = nullptr;
     uint32_t* acc = nullptr;
+    uint2*    roi_words = nullptr; // a CONTOUR ROI by voxel (ScorerDev::roi_words)
     double*   tally = nullptr;
     uint64_t  tally_len = 0;       // per scenario; the tally holds copies * tally_len values
     uint32_t  copies = 1;          // robust scenarios: one tally per scenario, scenario-major

@@ -61,6 +61,7 @@ struct ScorerDev {
     const uint32_t* start;
     const uint32_t* stride;
     const uint32_t* acc;
+    const uint2*    roi_words;     // CONTOUR: {members of 32 voxels, members before them}, or null (searched)
     double*         tally;         // dense: value of key k in scenario c at tally[(c * tally_len + k) * tstride]
     uint64_t        tally_len;
     uint32_t        tstride;       // 1, or 2 for the interleaved statistics pair (dose, dose^2)
@@ -255,6 +256,9 @@ cudaError_t launch_sample_primaries(const Queue& q, uint32_t dst, const mqi_spot
                                     cudaStream_t s);
 cudaError_t launch_sample_vertices(mqi_vertex* out, uint32_t* spot_out, const mqi_spot* spots, const uint64_t* cum,
                                    uint32_t n_spots, uint64_t h0, uint32_t n, uint32_t k0, uint32_t k1, cudaStream_t s);
+// The words of a CONTOUR ROI (n_vox / 32 each of words, counts and ranks); *bad: they do not hold its mapping.
+cudaError_t launch_roi_words(const ScorerDev& s, uint64_t n_vox, uint2* words, uint32_t* counts, uint32_t* ranks,
+                             uint32_t* scratch, uint32_t* bad, cudaStream_t st);
 // {density * scale, spr_default's density factor, radiation length, -} of n voxels.
 cudaError_t launch_materials(const float* rho, uint64_t n, float scale, int dbg, const CalibDev& calib, float4* mat, int sms,
                              cudaStream_t s);

@@ -271,13 +271,40 @@ roi_lower_bound(const ScorerDev& s, uint32_t v) {
     return first;
 }
 
+/// The CONTOUR mappings by the run that holds v.
+__device__ inline int32_t
+contour_idx(const ScorerDev& s, uint32_t v) {
+    const int32_t c = roi_lower_bound(s, v) - 1;
+    if (c < 0) return -1;
+    return (v - s.start[c] < s.stride[c]) ? 1 : -1;
+}
+
+__device__ inline int32_t
+contour_mask_idx(const ScorerDev& s, uint32_t v) {
+    const int32_t c = roi_lower_bound(s, v) - 1;
+    if (c < 0) return -1;
+    uint32_t d = v - s.start[c];
+    if (d < s.stride[c]) {
+        if (c > 0) d += s.acc[c - 1];
+        return (int32_t) d;
+    }
+    return -1;
+}
+
+/// The same by table (k_roi_words): {which of 32 voxels are inside, how many before them}.  A step's
+/// search took a dozen dependent loads for each scorer.
+__device__ inline int32_t
+word_mask_idx(const uint2& w, uint32_t v) {
+    const uint32_t bit = 1u << (v & 31u);
+    return (w.x & bit) ? (int32_t) (w.y + (uint32_t) __popc(w.x & (bit - 1u))) : -1;
+}
+
 __device__ inline int32_t
 roi_idx(const ScorerDev& s, uint32_t v) {
     if (s.roi_method == MQI_ROI_INDIRECT) return (int32_t) s.start[v];
     if (s.roi_method == MQI_ROI_CONTOUR) {
-        const int32_t c = roi_lower_bound(s, v) - 1;
-        if (c < 0) return -1;
-        return (v - s.start[c] < s.stride[c]) ? 1 : -1;
+        if (s.roi_words) return (s.roi_words[v >> 5].x >> (v & 31u)) & 1u ? 1 : -1;
+        return contour_idx(s, v);
     }
     return (int32_t) v;
 }
@@ -286,16 +313,46 @@ __device__ inline int32_t
 roi_mask_idx(const ScorerDev& s, uint32_t v) {
     if (s.roi_method == MQI_ROI_INDIRECT) return (int32_t) s.start[v];
     if (s.roi_method == MQI_ROI_CONTOUR) {
-        const int32_t c = roi_lower_bound(s, v) - 1;
-        if (c < 0) return -1;
-        uint32_t d = v - s.start[c];
-        if (d < s.stride[c]) {
-            if (c > 0) d += s.acc[c - 1];
-            return (int32_t) d;
-        }
-        return -1;
+        if (s.roi_words) return word_mask_idx(s.roi_words[v >> 5], v);
+        return contour_mask_idx(s, v);
     }
     return (int32_t) v;
+}
+
+/// A CONTOUR ROI's words: a warp a word of 32 voxels, its members and their number.
+__global__ void
+k_roi_words(const __grid_constant__ ScorerDev s, uint64_t n_vox, uint2* __restrict__ words, uint32_t* __restrict__ counts) {
+    const uint64_t v = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x;
+    const unsigned b = __ballot_sync(0xFFFFFFFFu, v < n_vox && contour_idx(s, (uint32_t) v) > 0);
+    if ((threadIdx.x & 31) == 0 && v < n_vox) {
+        words[v >> 5].x = b;
+        counts[v >> 5]  = (uint32_t) __popc(b);
+    }
+}
+
+/// The ranks into the words, and *bad where the words do not give the search's answers: runs that are not
+/// in order, or whose accumulated lengths are not theirs, keep the search.
+__global__ void
+k_roi_check(const __grid_constant__ ScorerDev s, uint64_t n_vox, uint2* __restrict__ words, const uint32_t* __restrict__ ranks,
+            uint32_t* __restrict__ bad) {
+    const uint64_t v = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x;
+    if (v >= n_vox) return;
+    const uint2 w = make_uint2(words[v >> 5].x, ranks[v >> 5]);
+    if (word_mask_idx(w, (uint32_t) v) != contour_mask_idx(s, (uint32_t) v)) *bad = 1u;
+    if ((threadIdx.x & 31) == 0) words[v >> 5].y = w.y;
+}
+
+cudaError_t
+launch_roi_words(const ScorerDev& s, uint64_t n_vox, uint2* words, uint32_t* counts, uint32_t* ranks, uint32_t* scratch,
+                 uint32_t* bad, cudaStream_t st) {
+    const unsigned grid = (unsigned) ((n_vox + 255) / 256);
+    cudaError_t    e    = cudaMemsetAsync(bad, 0, sizeof(uint32_t), st);
+    if (e != cudaSuccess) return e;
+    k_roi_words<<<grid, 256, 0, st>>>(s, n_vox, words, counts);
+    e = scan_exclusive_u32(counts, ranks, (n_vox + 31) / 32, scratch, st);
+    if (e != cudaSuccess) return e;
+    k_roi_check<<<grid, 256, 0, st>>>(s, n_vox, words, ranks, bad);
+    return cudaGetLastError();
 }
 
 /// fp_compute_hit of the scorers that need nothing beyond the step's deposit and its
@@ -318,30 +375,50 @@ compute_hit_simple(int type, const Trk& t, float dose_w) {
     }
 }
 
-/// fp_compute_hit for every enum'd scorer: the simple ones plus dose_to_medium and the LET weights
-/// (FP64 square root and divisions), compiled only into the kernel instance of runs that use them.
+/// The scorers whose value is formed in FP64: dose_to_medium and the LET weights.
+__device__ inline bool
+in_fp64(int type) {
+    return type == MQI_SCORER_DOSE_M || (type >= MQI_SCORER_LETD_NUM && type <= MQI_SCORER_LETT_DEN);
+}
+
+/// A step's length and its deposit per length and density, which every LET weight is made of
+/// (mqi_scorer_energy_deposit.hpp:91-177).  GB300's FP64 pipe is narrow: the square root and the two
+/// divisions bound the LET runs, so they are formed once for all of a step's scorers.
+struct LetStep {
+    double length, let;
+    __device__ inline explicit LetStep(int) : length(0.0), let(0.0) {}
+    __device__ inline LetStep(const Trk& t, float rho) {
+        // the step length as the reference forms it: float differences squared in float, summed in double
+        const float  density = rho * 1000.0f;
+        const float  lx = t.p1.x - t.p0.x, ly = t.p1.y - t.p0.y, lz = t.p1.z - t.p0.z;
+        length = sqrt((double) (lx * lx) + (double) (ly * ly) + (double) (lz * lz));
+        let    = (double) t.dE / length / (double) density;
+    }
+};
+
+__device__ inline double
+let_weight(int type, const Trk& t, const LetStep& l) {
+    if (!(l.length > 0.0)) return 0.0;
+    switch (type) {
+    case MQI_SCORER_LETD_NUM: return (l.let >= 25.0) ? 0.0 : (double) t.dE * l.let;
+    case MQI_SCORER_LETD_DEN: return (l.let >= 25.0) ? 0.0 : (double) t.dE;
+    case MQI_SCORER_LETT_NUM: return l.length * l.let;
+    default: return l.length;   // MQI_SCORER_LETT_DEN
+    }
+}
+
+__device__ inline double
+dose_to_medium(const Trk& t, float rho, float vol) {
+    return t.primary ? (double) t.dE * 1.60218e-13 * 1000.0 / (double) (vol * rho) : 0.0;
+}
+
+/// fp_compute_hit for every enum'd scorer.
 __device__ inline double
 compute_hit(int type, const Trk& t, float rho, float vol, float dose_w) {
-    if (type == MQI_SCORER_DOSE_M)
-        return t.primary ? (double) t.dE * 1.60218e-13 * 1000.0 / (double) (vol * rho) : 0.0;
-    if (type < MQI_SCORER_LETD_NUM || type > MQI_SCORER_LETT_DEN) {
-        const double v = (double) compute_hit_simple(type, t, dose_w);
-        return type == MQI_SCORER_DOSE_W2 ? v * v : v;
-    }
-    // LET scorers (mqi_scorer_energy_deposit.hpp:91-177)
-    // the step length as the reference forms it: float differences squared in float, summed in double
-    const float  density = rho * 1000.0f;
-    const float  lx = t.p1.x - t.p0.x, ly = t.p1.y - t.p0.y, lz = t.p1.z - t.p0.z;
-    const double length = sqrt((double) (lx * lx) + (double) (ly * ly) + (double) (lz * lz));
-    if (!(length > 0.0)) return 0.0;
-    const double let = (double) t.dE / length / (double) density;
-    switch (type) {
-    case MQI_SCORER_LETD_NUM: return (let >= 25.0) ? 0.0 : (double) t.dE * let;
-    case MQI_SCORER_LETD_DEN: return (let >= 25.0) ? 0.0 : (double) t.dE;
-    case MQI_SCORER_LETT_NUM: return length * let;
-    case MQI_SCORER_LETT_DEN: return length;
-    default: return 0.0;
-    }
+    if (type == MQI_SCORER_DOSE_M) return dose_to_medium(t, rho, vol);
+    if (in_fp64(type)) return let_weight(type, t, LetStep(t, rho));
+    const double v = (double) compute_hit_simple(type, t, dose_w);
+    return type == MQI_SCORER_DOSE_W2 ? v * v : v;
 }
 
 /// Score one step of track t in voxel cnb with every scorer of the current child.  The kernel
@@ -403,6 +480,8 @@ score_step(Ctx& C, const Trk& t, uint32_t cnb, const float4& m, float vol) {
     // dose_to_water of the step, shared by the dose, dose^2 and Dij scorers (Dw_pointer,
     // mqi_scorer_energy_deposit.hpp:23-40): 0 in vacuum voxels
     const float dose_w = (rho < 1.0e-7f) ? 0.0f : div_guarded((t.dE + t.ldE) * 1.60218e-10f, vol * rho * spr);
+    [[maybe_unused]] LetStep let(0);
+    [[maybe_unused]] bool    has_let = false;
     for (int si = 0; si < ch.n_scorers; ++si) {
         const ScorerDev& s = P.scorer[ch.scorer_begin + si];
         bool     ok;
@@ -418,17 +497,30 @@ score_step(Ctx& C, const Trk& t, uint32_t cnb, const float4& m, float vol) {
         }
         double v;
         bool   pos;
-        if (kFull) {
-            v   = ok ? compute_hit(s.type, t, rho, vol, dose_w) : 0.0;
+        if (kFull && in_fp64(s.type)) {
+            v = 0.0;
+            if (ok && s.type == MQI_SCORER_DOSE_M) {
+                v = dose_to_medium(t, rho, vol);
+            } else if (ok) {
+                if (!has_let) let = LetStep(t, rho);
+                has_let = true;
+                v       = let_weight(s.type, t, let);
+            }
             pos = v > 0.0;
+            if (s.double_score) v += v;
         } else {
-            // the FP64 pipe is narrow: filter in FP32, convert once, square only for dose^2
-            const float vf = ok ? compute_hit_simple(s.type, t, dose_w) : 0.0f;
-            pos            = vf > 0.0f;
-            v              = (double) vf;
-            if (s.type == MQI_SCORER_DOSE_W2) v *= v;
+            // the FP64 pipe is narrow: filter and double (exactly) in FP32, convert once, square only for
+            // dose^2
+            float vf = ok ? compute_hit_simple(s.type, t, dose_w) : 0.0f;
+            pos      = vf > 0.0f;
+            const bool square = s.type == MQI_SCORER_DOSE_W2;
+            if (s.double_score && !square) vf += vf;
+            v = (double) vf;
+            if (square) {
+                v *= v;
+                if (s.double_score) v += v;
+            }
         }
-        if (s.double_score) v += v;
         if (kDij && s.type == MQI_SCORER_DIJ) {
             // insert_hashtable(data_, cnb, spot_ind, ...) (mqi_transport.hpp:204-225); a history
             // without a spot index lands in column 0
