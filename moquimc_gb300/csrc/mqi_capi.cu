@@ -640,17 +640,18 @@ make_wave_params(mqi_ctx* c, uint64_t seed, WaveParams& P) {
     P.stats           = c->stats;
     P.spot_ids        = c->has_spots ? c->spot_ids : nullptr;
     P.tables          = c->tables;
-    P.smem_edge_floats = wave_edge_floats(P.child, P.n_children);
     if (c->n_scen > 1) {
         P.n_scen      = (int) c->n_scen;
         P.scen_child  = c->scen_child;
-        P.scen_stride = c->scen_stride;
+        P.scen_floats = c->scen_floats;
         P.scen_edges  = c->scen_edges;
         for (uint32_t k = 0; k < c->n_scen; ++k) {
             P.scen_scale[k] = c->scen_scale[k];
             P.scen_mat[k]   = materials(c, c->scen_child, c->scen_scale[k]);
+            for (int a = 0; a < 3; ++a) P.scen_off[k][a] = c->scen_off[k][a];
         }
     }
+    P.smem_edge_floats = wave_edge_floats(P);
 }
 
 /// Load or sample n histories from h, once per scenario, behind the `have` entries of a queue.
@@ -872,17 +873,24 @@ mqi_set_scenarios(mqi_ctx* c, int child_id, uint32_t n, const float* xe, const f
     DeviceGuard g(c->device);
     for (ChildHost& ch : c->children) drop_materials(ch);   // those of the scales before
     float* edges = nullptr;
-    int    stride = 0;
+    std::vector<float> host;
+    std::vector<std::array<uint32_t, 3>> off;
     if (n > 1) {
+        // scenarios that shift other axes, or only scale the density, share an axis's array: each
+        // different one is kept once (21 scenarios of three shifts an axis: 9 arrays, which then fit a
+        // block's shared memory)
         const ChildHost& ch = c->children[child_id];
-        stride = ch.nx + ch.ny + ch.nz + 3;
-        std::vector<float> host((size_t) n * stride);
-        for (uint32_t k = 0; k < n; ++k) {
-            float* e = host.data() + (size_t) k * stride;
-            std::memcpy(e, xe + (size_t) k * (ch.nx + 1), (ch.nx + 1) * sizeof(float));
-            std::memcpy(e + ch.nx + 1, ye + (size_t) k * (ch.ny + 1), (ch.ny + 1) * sizeof(float));
-            std::memcpy(e + ch.nx + ch.ny + 2, ze + (size_t) k * (ch.nz + 1), (ch.nz + 1) * sizeof(float));
-        }
+        const float*     in[3]  = { xe, ye, ze };
+        const size_t     len[3] = { (size_t) ch.nx + 1, (size_t) ch.ny + 1, (size_t) ch.nz + 1 };
+        off.resize(n);
+        for (int a = 0; a < 3; ++a)
+            for (uint32_t k = 0; k < n; ++k) {
+                const float* e = in[a] + k * len[a];
+                uint32_t     j = 0;
+                while (j < k && std::memcmp(host.data() + off[j][a], e, len[a] * sizeof(float)) != 0) ++j;
+                off[k][a] = j < k ? off[j][a] : (uint32_t) host.size();
+                if (j == k) host.insert(host.end(), e, e + len[a]);
+            }
         MQI_CUDA(c, cudaMalloc(&edges, host.size() * sizeof(float)), "mqi_set_scenarios");
         cudaError_t e = cudaMemcpy(edges, host.data(), host.size() * sizeof(float), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
@@ -909,7 +917,8 @@ mqi_set_scenarios(mqi_ctx* c, int child_id, uint32_t n, const float* xe, const f
     }
     cudaFree(c->scen_edges);
     c->scen_edges  = edges;
-    c->scen_stride = stride;
+    c->scen_floats = (int) host.size();
+    c->scen_off    = off;
     c->scen_child  = n > 1 ? child_id : -1;
     c->n_scen      = copies;
     c->scen_scale.assign(copies, 1.0f);

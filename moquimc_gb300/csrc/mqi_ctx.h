@@ -8,6 +8,7 @@
 #pragma once
 
 #include <algorithm>
+#include <array>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -194,8 +195,9 @@ struct mqi_ctx {
     int                     graph_waves = 8;          // kept for the tuner's records
     uint32_t                n_scen = 1;               // robust scenarios (1: none)
     int                     scen_child = -1;
-    int                     scen_stride = 0;
-    float*                  scen_edges = nullptr;     // device: n_scen x scen_stride
+    float*                  scen_edges = nullptr;     // device: the scenarios' different edge arrays
+    int                     scen_floats = 0;
+    std::vector<std::array<uint32_t, 3>> scen_off;    // each scenario's x, y and z arrays in it
     std::vector<float>      scen_scale;
 };
 

@@ -154,8 +154,9 @@ struct WaveParams {
     int       kernel_mode;      // kModeDij | kModeFull | kModeRoi: the scoring code the run needs
     int       n_scen;           // robust scenarios (0 or 1: none)
     int       scen_child;       // the child the scenarios vary
-    int       scen_stride;      // floats per scenario in scen_edges: nx+1 + ny+1 + nz+1
-    const float* scen_edges;    // device: per-scenario x, y, z edges of scen_child
+    int       scen_floats;      // length of scen_edges
+    const float* scen_edges;    // device: the different x, y and z edge arrays of scen_child's scenarios
+    uint32_t  scen_off[kMaxScenarios][3];   // where each scenario's three arrays start in it
     float     scen_scale[kMaxScenarios];   // per-scenario density scale
     const float4* scen_mat[kMaxScenarios]; // and the materials at that scale
     Queue     in;
@@ -264,7 +265,7 @@ cudaError_t launch_materials(const float* rho, uint64_t n, float scale, int dbg,
                              cudaStream_t s);
 cudaError_t launch_wave(const WaveParams& p, int grid, int block, int blocks_per_sm, cudaStream_t s);
 int         wave_smem_bytes(const WaveParams& p);
-int         wave_edge_floats(const ChildDev* c, int n);
+int         wave_edge_floats(const WaveParams& p);
 constexpr int kHuNodes = 3996;   // HU -1000 .. 2995, what hu_to_density's clamp leaves
 constexpr int kHuBlock = 512;
 // The correction factors at `table` become densities (once per context); the conversion looks them up.

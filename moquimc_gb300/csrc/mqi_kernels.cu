@@ -157,16 +157,19 @@ make_grid(const ChildDev& c, const float* sxe, const float* sye, const float* sz
     return g;
 }
 
+/// The scenarios' edge arrays as a block reads them: staged in shared memory when they fit (the arrays
+/// that scenarios have in common are kept once), else P.scen_edges.
+static __shared__ const float* s_scen_edges;
+
 /// The grid of `child` as the track with spot word `sw` sees it: a robust scenario of the
-/// scenario child has its own edges (setup shift) and density scale.
+/// scenario child has its own edges (setup shift) and materials (density scale).
 __device__ inline void
 apply_scenario(const WaveParams& P, Grid& g, int child, uint32_t sw) {
     if (P.n_scen > 1 && child == P.scen_child) {
-        const int    s = (int) (sw >> kScenShift);
-        const float* e = P.scen_edges + (size_t) s * P.scen_stride;
-        g.xe        = e;
-        g.ye        = e + g.nx + 1;
-        g.ze        = e + g.nx + g.ny + 2;
+        const int s = (int) (sw >> kScenShift);
+        g.xe        = s_scen_edges + P.scen_off[s][0];
+        g.ye        = s_scen_edges + P.scen_off[s][1];
+        g.ze        = s_scen_edges + P.scen_off[s][2];
         g.mat       = P.scen_mat[s];
     }
 }
@@ -1257,7 +1260,7 @@ wave_body(const WaveParams& P) {
         for (int c = 0; c < P.n_children; ++c) {
             const ChildDev& ch = P.child[c];
             const int need     = ch.nx + ch.ny + ch.nz + 3;
-            if (P.n_scen > 1 && c == P.scen_child) continue;   // scenario edges are read from global memory
+            if (P.n_scen > 1 && c == P.scen_child) continue;   // its scenarios' edges instead, below
             if (off + need > P.smem_edge_floats) break;
             float* e = sedges + off;
             for (int i = threadIdx.x; i <= ch.nx; i += blockDim.x) e[i] = ch.xe[i];
@@ -1270,6 +1273,10 @@ wave_body(const WaveParams& P) {
             }
             off += need;
         }
+        const bool fits = P.n_scen > 1 && off + P.scen_floats <= P.smem_edge_floats;
+        if (fits)
+            for (int i = threadIdx.x; i < P.scen_floats; i += blockDim.x) sedges[off + i] = P.scen_edges[i];
+        if (threadIdx.x == 0) s_scen_edges = fits ? sedges + off : P.scen_edges;
     }
     __syncthreads();
 
@@ -1478,6 +1485,7 @@ template<int kMode>
 __device__ __forceinline__ void
 post_body(const WaveParams& P) {
     if (threadIdx.x < 8) s_cnt[threadIdx.x] = 0u;
+    if (threadIdx.x == 0) s_scen_edges = P.scen_edges;
     __syncthreads();
     const uint32_t n = min(P.drain->tail, P.def_cap);   // the wave finished those past the array itself
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1567,13 +1575,16 @@ wave_smem_bytes(const WaveParams& p) {
 }
 
 int
-wave_edge_floats(const ChildDev* c, int n) {
+wave_edge_floats(const WaveParams& p) {
+    constexpr int kMost = 3 * 2048 + 12;
     int f = 0;
-    for (int i = 0; i < n; ++i) {
-        const int need = c[i].nx + c[i].ny + c[i].nz + 3;
-        if (f + need > 3 * 2048 + 12) break;
+    for (int i = 0; i < p.n_children; ++i) {
+        if (p.n_scen > 1 && i == p.scen_child) continue;
+        const int need = p.child[i].nx + p.child[i].ny + p.child[i].nz + 3;
+        if (f + need > kMost) break;
         f += need;
     }
+    if (p.n_scen > 1 && f + p.scen_floats <= kMost) f += p.scen_floats;
     return (f + 3) & ~3;
 }
 
@@ -1794,12 +1805,12 @@ k_hu_to_density(const float* __restrict__ table, const int16_t* __restrict__ hu,
     auto density = [&](int h) { return tab[min(max(h, -1000), 2995) + 1000]; };
     const uint64_t n8 = vec ? n / 8 : 0;
     for (uint64_t g = first; g < n8; g += stride) {
-        const int4 q = reinterpret_cast<const int4*>(hu)[g];
+        const int4 q = __ldcs(reinterpret_cast<const int4*>(hu) + g);
         auto lo = [&](int w) { return density((int) (int16_t) (w & 0xFFFF)); };
         auto hi = [&](int w) { return density(w >> 16); };
         float4* o = reinterpret_cast<float4*>(rho) + 2 * g;
-        o[0]      = make_float4(lo(q.x), hi(q.x), lo(q.y), hi(q.y));
-        o[1]      = make_float4(lo(q.z), hi(q.z), lo(q.w), hi(q.w));
+        __stcs(o, make_float4(lo(q.x), hi(q.x), lo(q.y), hi(q.y)));
+        __stcs(o + 1, make_float4(lo(q.z), hi(q.z), lo(q.w), hi(q.w)));
     }
     for (uint64_t i = n8 * 8 + first; i < n; i += stride) rho[i] = density(hu[i]);
 }

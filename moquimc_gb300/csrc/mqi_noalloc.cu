@@ -193,7 +193,7 @@ mqi_transport_noalloc(int nx, int ny, int nz, const float* d_xe, const float* d_
     P.stats            = stats;
     P.spot_ids         = nullptr;
     P.tables           = tables;
-    P.smem_edge_floats = wave_edge_floats(P.child, 1);
+    P.smem_edge_floats = wave_edge_floats(P);
 
     // counters and statistics start at zero for every call (the array keeps the last call's)
     e = cudaMemsetAsync(counters, 0, kNoallocCounterBytes, stream);
