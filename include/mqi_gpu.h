@@ -356,11 +356,12 @@ int mqi_run_until_stat(mqi_ctx* ctx, int dose_id, int dose2_id, uint64_t histori
                        uint64_t* histories_done, double* achieved);
 
 /* Launch shape of the transport (no counterpart in moqui, whose launch is fixed at 512 threads per
- * block).  block: threads per block (multiple of 32, <= 256); blocks_per_sm: resident blocks per
- * SM the wave kernel is launched with; slice_steps: voxel steps a track takes before it is
- * re-queued (0 = run each track to completion); primary_chunk: primaries loaded per queue
- * generation.  block, blocks_per_sm and primary_chunk keep their values when <= 0, slice_steps
- * when < 0.  Results do not depend on any of these. */
+ * block).  block: threads per block (multiple of 32, <= 256); blocks_per_sm: blocks per SM, at most 64.
+ * The wave kernel runs one block per SM of about their product: 768 threads from 768 up, 640 from 640
+ * (the default, 128 x 5), else 512; the less common scoring modes always run 640.  slice_steps: voxel
+ * steps a track takes before it is re-queued (0 = run each track to completion); primary_chunk:
+ * primaries loaded per queue generation.  block, blocks_per_sm and primary_chunk keep their values
+ * when <= 0, slice_steps when < 0.  Results do not depend on any of these. */
 int mqi_set_tuning(mqi_ctx* ctx, int block, int blocks_per_sm, int slice_steps, int primary_chunk);
 
 /* How the queue is driven (no counterpart in moqui, which runs one kernel over all histories).
@@ -390,8 +391,8 @@ int mqi_set_queue_sort(mqi_ctx* ctx, uint32_t min_entries);
 
 /* One candidate of mqi_autotune and its measured rate. */
 typedef struct {
-    int      block;            /* threads per block of the wave kernel */
-    int      blocks_per_sm;    /* resident blocks per SM it is launched with */
+    int      block;            /* launch shape (mqi_set_tuning) */
+    int      blocks_per_sm;
     int      streamed;         /* launch mode (mqi_set_launch_mode) */
     int      graph_waves;
     uint32_t primary_chunk;    /* queue entries a wave starts with / histories per generation */

@@ -193,7 +193,6 @@ mqi_create(int device, mqi_ctx** out) {
         mqi_destroy(c);
         return cuda_fail(nullptr, e, "mqi_create: allocation");
     }
-    c->wave_grid = c->num_sms * 5;   // 128-thread blocks, 5 per SM (96 registers): fastest measured shape
     *out = c;
     return MQI_OK;
 }
@@ -266,7 +265,7 @@ mqi_set_tuning(mqi_ctx* c, int block, int blocks_per_sm, int slice_steps, int pr
     }
     if (blocks_per_sm > 0) {
         if (blocks_per_sm > 64) return fail(c, MQI_ERR_INVALID, "mqi_set_tuning: blocks_per_sm must be <= 64");
-        c->wave_grid = c->num_sms * blocks_per_sm;
+        c->wave_bps = blocks_per_sm;
     }
     if (slice_steps >= 0) c->max_slice_steps = (uint32_t) slice_steps;
     if (primary_chunk > 0) {
@@ -728,7 +727,7 @@ run_wave(mqi_ctx* c, WaveParams& P, const QueueBuf& A, const QueueBuf& B, uint32
     MQI_CUDA(c, cudaMemcpyAsync(c->counters, c->host_counts, sizeof(counts), cudaMemcpyHostToDevice, c->stream),
              "mqi_transport");
     MQI_CUDA(c, cudaEventRecord(c->ev0, c->stream), "mqi_transport");
-    MQI_CUDA(c, launch_wave(P, c->wave_grid, c->wave_block, c->wave_grid / c->num_sms, c->stream), "mqi_transport: wave");
+    MQI_CUDA(c, launch_wave(P, c->num_sms, c->wave_block * c->wave_bps, c->stream), "mqi_transport: wave");
     MQI_CUDA(c, cudaEventRecord(c->ev1, c->stream), "mqi_transport");
     MQI_CUDA(c, cudaMemcpyAsync(c->host_counts, c->counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream),
              "mqi_transport");
@@ -986,7 +985,7 @@ mqi_autotune(mqi_ctx* c, int source_plan, uint64_t h0, uint64_t h1, uint64_t see
     MQI_CUDA(c, cudaMemcpy(stats_saved, c->stats, sizeof(stats_saved), cudaMemcpyDeviceToHost), "mqi_autotune");
     const uint64_t waves0 = c->waves, kl0 = c->kernel_launches, wl0 = c->wave_launches;
     const double   wms0   = c->wave_ms;
-    const int blk0 = c->wave_block, grid0 = c->wave_grid, str0 = c->streamed, gw0 = c->graph_waves;
+    const int blk0 = c->wave_block, bps0 = c->wave_bps, str0 = c->streamed, gw0 = c->graph_waves;
     const uint32_t chunk0 = c->primary_chunk;
     int rc = MQI_OK;
     for (size_t i = 0; i < c->scorers.size() && rc == MQI_OK; ++i) {
@@ -1034,7 +1033,7 @@ mqi_autotune(mqi_ctx* c, int source_plan, uint64_t h0, uint64_t h1, uint64_t see
         for (size_t k = 0; k < cands.size() && rc == MQI_OK; ++k) {
             const Cand& q = cands[k];
             c->wave_block = q.block;
-            c->wave_grid = c->num_sms * q.bps;
+            c->wave_bps = q.bps;
             c->streamed = q.streamed;
             c->graph_waves = q.graph_waves;
             c->primary_chunk = q.chunk;
@@ -1065,12 +1064,12 @@ mqi_autotune(mqi_ctx* c, int source_plan, uint64_t h0, uint64_t h1, uint64_t see
     cudaMemcpy(c->stats, stats_saved, sizeof(stats_saved), cudaMemcpyHostToDevice);
     c->waves = waves0; c->kernel_launches = kl0; c->wave_launches = wl0; c->wave_ms = wms0;
     if (rc != MQI_OK || best < 0) {
-        c->wave_block = blk0; c->wave_grid = grid0; c->streamed = str0; c->graph_waves = gw0; c->primary_chunk = chunk0;
+        c->wave_block = blk0; c->wave_bps = bps0; c->streamed = str0; c->graph_waves = gw0; c->primary_chunk = chunk0;
         return rc != MQI_OK ? rc : fail(c, MQI_ERR_DEVICE, "mqi_autotune: no candidate ran");
     }
     const Cand& q = cands[best];
     c->wave_block = q.block;
-    c->wave_grid = c->num_sms * q.bps;
+    c->wave_bps = q.bps;
     c->streamed = q.streamed;
     c->graph_waves = q.graph_waves;
     c->primary_chunk = q.chunk;

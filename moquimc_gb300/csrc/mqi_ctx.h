@@ -114,14 +114,14 @@ void dij_release(ScorerHost& s);
 cudaError_t dij_reset(ScorerHost& s, int sms, cudaStream_t st);
 
 /// The shape of a draining wave over n queue entries.  While every track has a lane of its own, the
-/// wave lasts as long as a chain of steps takes, and four blocks per SM (128 registers, no spills)
-/// take them sooner; beyond that throughput counts, and five blocks do.  Few tracks are spread over
-/// the resident warps, and blocks are launched for about twice the tracks, not for every warp: those
+/// wave lasts as long as a chain of steps takes, and 16 warps per SM (128 registers, no spills) take
+/// them sooner; beyond that throughput counts, and 20 warps do.  Few tracks are spread over the
+/// resident warps, and blocks are launched for about twice the tracks, not for every warp: those
 /// without a track only poll.
 inline void
 plan_drain(WaveParams& P, uint32_t n, int sms) {
-    P.drain_shape = n <= (uint32_t) (sms * 4 * kDrainBlock) ? 4 : 5;
-    const uint32_t warps = (uint32_t) (sms * P.drain_shape * (kDrainBlock / 32));
+    P.drain_warps        = n <= (uint32_t) (sms * 16 * 32) ? 16 : 20;
+    const uint32_t warps = (uint32_t) (sms * P.drain_warps);
     P.lanes      = (int) std::min<uint32_t>((n + warps - 1) / warps, 32u);
     P.max_blocks = std::max<int>(sms, 2 * (int) ((n + 4 * P.lanes - 1) / (4 * P.lanes)));
 }
@@ -173,8 +173,8 @@ struct mqi_ctx {
     mqi_gpu::CalibDev       calib{};                // SPR / X0 curves (mode 0: the defaults)
     float*                  calib_buf = nullptr;    // device: the tables of calib (SPR then X0)
     int                     num_sms = 0;
-    int                     wave_block = 128;
-    int                     wave_grid = 0;
+    int                     wave_block = 128;         // threads per block and blocks per SM asked for
+    int                     wave_bps = 5;             // (launch_wave runs their product, as one block)
     uint32_t                max_slice_steps = 0;
     uint32_t                primary_chunk = 1u << 21;
     uint64_t                waves = 0;

@@ -177,15 +177,14 @@ struct WaveParams {
                                 // (null: the wave does not drain; its daughters go to `out`)
     uint32_t        epoch;      // a draining wave's number, unlike any that `ready` or `def` hold (30 bits)
     int             lanes;      // lanes of a warp that take tracks (1 .. 32)
-    int             max_blocks;  // a draining wave's blocks, at most
-    int             drain_shape; // a draining wave's blocks per SM, 4 or 5 (its register budget)
+    int             max_blocks;  // a draining wave's blocks of four warps, at most
+    int             drain_warps; // a draining wave's warps per SM, 16 or 20 (its register budget)
     int             smem_edge_floats; // shared-memory floats for staged child edges
     const float*    tables;     // device: the six physics tables, 6 x 600 floats in Tables order
                                 // (a context's are followed by the density of each HU value)
     CalibDev        calib;      // SPR / X0 curves
 };
 
-constexpr int kDrainBlock = 128;   // threads of a draining wave's block
 
 std::string& thread_error_slot();
 
@@ -263,7 +262,7 @@ cudaError_t launch_roi_words(const ScorerDev& s, uint64_t n_vox, uint2* words, u
 // {density * scale, spr_default's density factor, radiation length, -} of n voxels.
 cudaError_t launch_materials(const float* rho, uint64_t n, float scale, int dbg, const CalibDev& calib, float4* mat, int sms,
                              cudaStream_t s);
-cudaError_t launch_wave(const WaveParams& p, int grid, int block, int blocks_per_sm, cudaStream_t s);
+cudaError_t launch_wave(const WaveParams& p, int sms, int threads_per_sm, cudaStream_t s);
 int         wave_smem_bytes(const WaveParams& p);
 int         wave_edge_floats(const WaveParams& p);
 constexpr int kHuNodes = 3996;   // HU -1000 .. 2995, what hu_to_density's clamp leaves

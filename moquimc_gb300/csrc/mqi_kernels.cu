@@ -37,8 +37,8 @@ constexpr unsigned long long kLiveEntry = 1ull << 32;
 /// Polls a warp without tracks makes before it gives up on the others: seconds.
 constexpr uint32_t kDrainPolls = 1u << 24;
 
-/// A draining wave's blocks to one warp that only runs post-steps.
-constexpr uint32_t kPostEvery = 20;
+/// A draining wave's warps to one that only runs post-steps.
+constexpr uint32_t kPostEvery = 80;
 
 /// A track in registers: track_t<float> (mqi_track.hpp:48-205) reduced to what transport reads.
 struct Trk {
@@ -1293,8 +1293,9 @@ wave_body(const WaveParams& P) {
     const uint32_t n_raw  = *P.n_in;
     const uint32_t n_in   = (n_raw > P.in.capacity || (*P.error_flag & 2u)) ? 0u : n_raw;
     const int      lane   = threadIdx.x & 31;
-    // one warp in kPostEvery blocks takes no tracks and runs the waiting post-steps
-    const bool     posts  = kDrain && blockIdx.x % kPostEvery == kPostEvery - 1 && threadIdx.x >= blockDim.x - 32;
+    // one warp in kPostEvery takes no tracks and runs the waiting post-steps
+    const uint32_t warp   = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    const bool     posts  = kDrain && warp % kPostEvery == kPostEvery - 1;
     bool           open   = lane < P.lanes && !posts;   // the lane takes tracks
     bool           waits  = false;                      // it holds queue index `ticket` and waits for a track there
     bool           parked = false;                      // it holds a record, `own`, that the array had no room for
@@ -1544,19 +1545,25 @@ launch_load_primaries(const Queue& q, uint32_t dst, const mqi_vertex* v, const u
     return cudaGetLastError();
 }
 
-/// The wave kernel in the launch shapes the tuner chooses from: (threads per block, minimum
-/// resident blocks per SM).  The register budget each shape implies is what differs.  The common modes
-/// (DIRECT ROIs, simple scorer callbacks) come in every shape; the other modes in 128 x 5.
-template<int kBlock, int kMinBlocks, int kMode>
-__global__ void __launch_bounds__(kBlock, kMinBlocks)
+/// The wave kernel: one block per SM, of as many threads as its registers allow (512 at up to 128
+/// registers, 640 at 96, 768 at 80; the common modes -- DIRECT ROIs, simple scorer callbacks -- come in
+/// all three for the tuner, the others in 640).  Its step loop is bound by its instruction stream and
+/// the latencies in it.  Against blocks of 128 threads, five to the SM, the tables and edges lie in
+/// shared memory once, and L1 holds more of the materials: 1 M histories on the slab phantom 17.84 ->
+/// 16.65 ms, a CT plan with its statistics 55.0 -> 51.2, 21 scenarios 56.5 -> 54.2 (with 64 KB of the SM
+/// set aside as shared memory instead of the 32 this takes: the CT +1%, the scenarios +2.5%).
+template<int kThreads, int kMode>
+__global__ void __launch_bounds__(kThreads, 1)
 k_wave(const __grid_constant__ WaveParams P) {
     wave_body<kMode, false>(P);
 }
 
-/// The draining wave, in every mode in two shapes.  A kernel apart from the ordinary wave, whose step
-/// loop is 15% faster for not sharing its registers and its image with the post-steps.
-template<int kMinBlocks, int kMode>
-__global__ void __launch_bounds__(kDrainBlock, kMinBlocks)
+/// The draining wave, in every mode in two shapes: one block of 640 threads per SM, as above (100 000
+/// histories in water 5.97 -> 5.59 ms), or four of 128 where not all may be needed (512 threads in one
+/// block: 600 tracks 0.71 -> 0.81 ms, as fewer SMs share them).  A kernel apart from the ordinary wave,
+/// whose step loop is 15% faster for not sharing its registers and its image with the post-steps.
+template<int kThreads, int kMinBlocks, int kMode>
+__global__ void __launch_bounds__(kThreads, kMinBlocks)
 k_drain(const __grid_constant__ WaveParams P) {
     wave_body<kMode, true>(P);
 }
@@ -1590,37 +1597,38 @@ wave_edge_floats(const WaveParams& p) {
 
 /// An ordinary wave and the post-step kernel over the records it left (a grid-stride loop over a
 /// count it reads on the device).
-template<int B, int M, int K>
+template<int T, int K>
 static cudaError_t
-launch_variant(const WaveParams& p, int grid, cudaStream_t s) {
+launch_variant(const WaveParams& p, int sms, cudaStream_t s) {
     const int   smem = wave_smem_bytes(p);
-    cudaError_t e    = cudaFuncSetAttribute(k_wave<B, M, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e    = cudaFuncSetAttribute(k_wave<T, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) {
         (void) cudaGetLastError();   // the failed call's error is returned here, not left for the next launch
         return e;
     }
-    k_wave<B, M, K><<<grid, B, smem, s>>>(p);
-    k_post<K><<<grid, kPostBlock, 0, s>>>(p);
+    k_wave<T, K><<<sms, T, smem, s>>>(p);
+    k_post<K><<<sms * 5, kPostBlock, 0, s>>>(p);
     return cudaGetLastError();
 }
 
-template<int M, int K>
+template<int T, int M, int K>
 static cudaError_t
-launch_drain_shape(const WaveParams& p, int sms, cudaStream_t s) {
+launch_drain_shape(const WaveParams& p, int blocks, cudaStream_t s) {
     const int   smem = wave_smem_bytes(p);
-    cudaError_t e    = cudaFuncSetAttribute(k_drain<M, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e    = cudaFuncSetAttribute(k_drain<T, M, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) {
         (void) cudaGetLastError();
         return e;
     }
-    k_drain<M, K><<<std::min(sms * M, p.max_blocks), kDrainBlock, smem, s>>>(p);
+    k_drain<T, M, K><<<blocks, T, smem, s>>>(p);
     return cudaGetLastError();
 }
 
 template<int K>
 static cudaError_t
 launch_drain(const WaveParams& p, int sms, cudaStream_t s) {
-    return p.drain_shape == 4 ? launch_drain_shape<4, K>(p, sms, s) : launch_drain_shape<5, K>(p, sms, s);
+    return p.drain_warps == 16 ? launch_drain_shape<128, 4, K>(p, std::min(sms * 4, p.max_blocks), s)
+                               : launch_drain_shape<640, 1, K>(p, sms, s);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1721,15 +1729,13 @@ launch_sort(const WaveParams& p, int grid, cudaStream_t s) {
 
 /// Sort the wave's input when asked to, then run the instance of the run's scoring mode.
 cudaError_t
-launch_wave(const WaveParams& p, int grid, int block, int blocks_per_sm, cudaStream_t s) {
-    const int grid5 = grid / (blocks_per_sm > 0 ? blocks_per_sm : 1) * 5;
+launch_wave(const WaveParams& p, int sms, int threads_per_sm, cudaStream_t s) {
     if (!p.def || !p.drain) return cudaErrorInvalidValue;   // the post-steps need their records
     if (p.sort_bins) {
-        const cudaError_t e = launch_sort(p, grid5, s);
+        const cudaError_t e = launch_sort(p, sms * 5, s);
         if (e != cudaSuccess) return e;
     }
     if (p.ready) {
-        const int sms = grid5 / 5;
         switch (p.kernel_mode) {
         case 0: return launch_drain<0>(p, sms, s);
         case kModeSingle: return launch_drain<kModeSingle>(p, sms, s);
@@ -1744,22 +1750,20 @@ launch_wave(const WaveParams& p, int grid, int block, int blocks_per_sm, cudaStr
     }
     switch (p.kernel_mode) {
     case 0:
-        if (block != 128) return launch_variant<256, 2, 0>(p, grid, s);
-        if (blocks_per_sm >= 6) return launch_variant<128, 6, 0>(p, grid, s);
-        if (blocks_per_sm == 5) return launch_variant<128, 5, 0>(p, grid, s);
-        return launch_variant<128, 4, 0>(p, grid, s);
+        if (threads_per_sm >= 768) return launch_variant<768, 0>(p, sms, s);
+        if (threads_per_sm >= 640) return launch_variant<640, 0>(p, sms, s);
+        return launch_variant<512, 0>(p, sms, s);
     case kModeSingle:
-        if (block != 128) return launch_variant<256, 2, kModeSingle>(p, grid, s);
-        if (blocks_per_sm >= 6) return launch_variant<128, 6, kModeSingle>(p, grid, s);
-        if (blocks_per_sm == 5) return launch_variant<128, 5, kModeSingle>(p, grid, s);
-        return launch_variant<128, 4, kModeSingle>(p, grid, s);
-    case kModeStat: return launch_variant<128, 5, kModeStat>(p, grid5, s);
-    case kModeFull: return launch_variant<128, 5, kModeFull>(p, grid5, s);
-    case kModeRoi: return launch_variant<128, 5, kModeRoi>(p, grid5, s);
-    case kModeDij: return launch_variant<128, 5, kModeDij>(p, grid5, s);   // Dij + dose-like, DIRECT ROIs
-    case kModeDijAlone: return launch_variant<128, 5, kModeDijAlone>(p, grid5, s);
-    case kModeFull | kModeRoi: return launch_variant<128, 5, kModeFull | kModeRoi>(p, grid5, s);
-    default: return launch_variant<128, 5, kModeAll>(p, grid5, s);   // any mode with Dij
+        if (threads_per_sm >= 768) return launch_variant<768, kModeSingle>(p, sms, s);
+        if (threads_per_sm >= 640) return launch_variant<640, kModeSingle>(p, sms, s);
+        return launch_variant<512, kModeSingle>(p, sms, s);
+    case kModeStat: return launch_variant<640, kModeStat>(p, sms, s);
+    case kModeFull: return launch_variant<640, kModeFull>(p, sms, s);
+    case kModeRoi: return launch_variant<640, kModeRoi>(p, sms, s);
+    case kModeDij: return launch_variant<640, kModeDij>(p, sms, s);   // Dij + dose-like, DIRECT ROIs
+    case kModeDijAlone: return launch_variant<640, kModeDijAlone>(p, sms, s);
+    case kModeFull | kModeRoi: return launch_variant<640, kModeFull | kModeRoi>(p, sms, s);
+    default: return launch_variant<640, kModeAll>(p, sms, s);   // any mode with Dij
     }
 }
 

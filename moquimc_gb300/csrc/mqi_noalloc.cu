@@ -198,7 +198,6 @@ mqi_transport_noalloc(int nx, int ny, int nz, const float* d_xe, const float* d_
     // counters and statistics start at zero for every call (the array keeps the last call's)
     e = cudaMemsetAsync(counters, 0, kNoallocCounterBytes, stream);
     if (e != cudaSuccess) return noalloc_fail(MQI_ERR_CUDA, std::string("mqi_transport_noalloc: ") + cudaGetErrorString(e));
-    const int block = 128, grid = sms * 5;
     Queue*    A = &qa;
     Queue*    B = &qb;
     for (uint64_t h = 0; h < n_histories; h += kNoallocChunk) {
@@ -215,7 +214,7 @@ mqi_transport_noalloc(int nx, int ny, int nz, const float* d_xe, const float* d_
             uint32_t host_counts[12] = { count, 0, 0, 0, 0, 0, 0, 0, count, count, 0, 0 };
             if (e == cudaSuccess) e = cudaMemcpyAsync(counters, host_counts, sizeof(host_counts), cudaMemcpyHostToDevice, stream);
             if (e == cudaSuccess) e = cudaMemsetAsync(marks, 0, kNoallocMarkBytes, stream);
-            if (e == cudaSuccess) e = launch_wave(P, grid, block, grid / sms, stream);
+            if (e == cudaSuccess) e = launch_wave(P, sms, 640, stream);
             if (e == cudaSuccess) e = cudaMemcpyAsync(host_counts, counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
             if (e != cudaSuccess) return noalloc_fail(MQI_ERR_CUDA, std::string("mqi_transport_noalloc: ") + cudaGetErrorString(e));

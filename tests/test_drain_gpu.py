@@ -69,6 +69,19 @@ def test_daughters_that_outgrow_the_queue_wait_for_the_next_wave(gpu_ctx_factory
     assert got[1]["waves"] == waves
 
 
+@pytest.mark.parametrize("block, per_sm", [(32, 1), (128, 4), (256, 2), (128, 6), (256, 64)])
+@pytest.mark.parametrize("n", [1, 1201])
+def test_ordinary_waves_in_every_shape(gpu_ctx_factory, n, block, per_sm):
+    c, cid = _box(gpu_ctx_factory, False)
+    ids = [c.add_scorer(cid, capi.DOSE_W)]
+    v = ph.uniform_spot_vertices(n, np.random.default_rng(n), 150.0, (0.0, 0.0, 0.5), (30.0, 30.0))
+    ref = _run(c, ids, v, 1)
+    c.set_tuning(block=block, blocks_per_sm=per_sm)
+    got = _run(c, ids, v, 1)
+    _same(got, ref)
+    assert got[1]["waves"] == ref[1]["waves"]
+
+
 def _contour(rng):
     m = rng.random(int(np.prod(NXYZ))) < 0.5
     edge = np.flatnonzero(np.diff(np.concatenate([[0], m.view(np.int8), [0]])))
@@ -77,8 +90,9 @@ def _contour(rng):
             "acc": np.cumsum(stride).astype(np.uint32)}
 
 
+@pytest.mark.parametrize("n", [4001, 80_003])
 @pytest.mark.parametrize("scorers", ["edep", "pair", "two", "let", "contour", "let_contour"])
-def test_scoring_instances(gpu_ctx_factory, scorers):
+def test_scoring_instances(gpu_ctx_factory, scorers, n):
     c, cid = _box(gpu_ctx_factory, False)
     roi = _contour(np.random.default_rng(8)) if "contour" in scorers else {}
     if scorers == "edep":
@@ -91,7 +105,7 @@ def test_scoring_instances(gpu_ctx_factory, scorers):
         ids.append(c.add_scorer(cid, capi.EDEP_PRIMARY))
     if scorers.startswith("let"):
         ids += [c.add_scorer(cid, t, **roi) for t in (capi.LETD_NUM, capi.LETD_DEN)]
-    v = ph.uniform_spot_vertices(4001, np.random.default_rng(9), 140.0, (0.0, 0.0, 0.5), (30.0, 30.0))
+    v = ph.uniform_spot_vertices(n, np.random.default_rng(9), 140.0, (0.0, 0.0, 0.5), (30.0, 30.0))
     _same(_run(c, ids, v, -1), _run(c, ids, v, 1))
 
 
