@@ -731,8 +731,12 @@ energy_loss(const Tables& T, const Rel& rel, float rho, float len, float spr, fl
     if (x0 > rel.Ek && n > 0) n -= 1;
     if (x1 < rel.Ek && n < MQI_TABLE_N - 2) n += 1;
     float r = intpl1d_grid(rel.Ek, x0, x1, T.range[n], T.range[n + 1]);
-    if (r < lw) return rel.Ek;
-    r -= lw;
+    const bool all = r < lw;   // the step takes all the energy
+    r -= all ? 0.0f : lw;
+    // down to the node below the range left: two nodes at once, as a step seldom loses more (a single
+    // spot's chain of steps 6% shorter for it and for no early return)
+    const int down = (r < T.range[n]) + (r < T.range[max(n - 1, 0)]);
+    n              = max(n - down, 0);
     while (n > 0 && r < T.range[n]) --n;
     x0 = 0.1f + (float) n * 0.5f;
     x1 = x0 + 0.5f;
@@ -742,8 +746,7 @@ energy_loss(const Tables& T, const Rel& rel, float rho, float len, float spr, fl
     float       var     = div_by(dedx_term0() * rho, kWaterDensity, kPerWaterDensity) * lw;
     var *= div_rn(Te, rel.beta_sq) * (1.0f - 0.5f * rel.beta_sq);
     float ret = z * sqrt_rn(var) + dE_mean;
-    if (ret < 0.0f) ret = -ret;
-    return ret;
+    return all ? rel.Ek : fabsf(ret);
 }
 
 /// p_ionization_tabulated::along_step (mqi_p_ionization.hpp:349-420): CSDA loss with Gaussian
@@ -756,7 +759,7 @@ along_step(Ctx& C, Trk& t, const Rel& rel, float len, const float4& m, float spr
     const float dE = energy_loss(*C.T, rel, m.x, len, spr, z_strag);
     float       r  = 1.0f;
     if (dE >= t.ke0) {
-        r         = t.ke0 / dE;
+        r         = div_rn(t.ke0, dE);
         t.stopped = true;
     }
     const float P     = rel.momentum();
@@ -906,21 +909,18 @@ __device__ inline int
 stepping(Ctx& C, Trk& t, Rng& rng, const float4& m, float d2b) {
     const float rho = m.x;
     t.spr0 = -1.0f;
-    if (rho < 1.0e-7f) {
-        t.p1 = advance(t.p0, t.d0, d2b);
-        return 0;
-    }
-    if (rho > 99.9f) {
+    if ((rho < 1.0e-7f) | (rho > 99.9f) | (t.ke0 <= kTpCut)) {
+        if (rho < 1.0e-7f) {
+            t.p1 = advance(t.p0, t.d0, d2b);
+            return 0;
+        }
         t.stopped = true;
-        return 0;
-    }
-    if (t.ke0 <= kTpCut) {
+        if (rho > 99.9f) return 0;
         if (t.ke0 < 0.0f) t.ke0 = 0.0f;
         t.dE += t.ke0;
         t.ke1 -= t.ke0;
-        t.spr0    = spr_rare(&C.P->calib, rho, m.y, t.ke0, C.dbg);   // for the position and the score
-        t.p1      = last_step_pos(C.T, t.p0, t.d0, t.ke0, t.dE, rho, t.spr0);
-        t.stopped = true;
+        t.spr0 = spr_rare(&C.P->calib, rho, m.y, t.ke0, C.dbg);   // for the position and the score
+        t.p1   = last_step_pos(C.T, t.p0, t.d0, t.ke0, t.dE, rho, t.spr0);
         return 0;
     }
     const Tables& T = *C.T;
@@ -1547,11 +1547,13 @@ launch_load_primaries(const Queue& q, uint32_t dst, const mqi_vertex* v, const u
 
 /// The wave kernel: one block per SM, of as many threads as its registers allow (512 at up to 128
 /// registers, 640 at 96, 768 at 80; the common modes -- DIRECT ROIs, simple scorer callbacks -- come in
-/// all three for the tuner, the others in 640).  Its step loop is bound by its instruction stream and
-/// the latencies in it.  Against blocks of 128 threads, five to the SM, the tables and edges lie in
-/// shared memory once, and L1 holds more of the materials: 1 M histories on the slab phantom 17.84 ->
-/// 16.65 ms, a CT plan with its statistics 55.0 -> 51.2, 21 scenarios 56.5 -> 54.2 (with 64 KB of the SM
-/// set aside as shared memory instead of the 32 this takes: the CT +1%, the scenarios +2.5%).
+/// all three for the tuner, the others in 640).  Its step loop is bound by its instruction stream: of
+/// five warps to a scheduler 1.9 wait for a fixed latency and 1.0 for instructions, at an issue rate of
+/// 0.68.  Against blocks of 128 threads, five to the SM (1.8 warps waiting for instructions, the same
+/// number of instructions), the tables and edges take 32 KB of the SM once instead of 132 KB: 1 M
+/// histories on the slab phantom 17.84 -> 16.65 ms, a CT plan with its statistics 55.0 -> 51.2, 21
+/// scenarios 56.5 -> 54.2.  Two blocks of 320 threads got 0.3 of the slab's 1.2 ms; setting 64 KB aside
+/// cost the CT 1% and the scenarios 2.5%; a barrier a step, to share what is fetched, cost 20%.
 template<int kThreads, int kMode>
 __global__ void __launch_bounds__(kThreads, 1)
 k_wave(const __grid_constant__ WaveParams P) {
