@@ -114,13 +114,15 @@ void dij_release(ScorerHost& s);
 cudaError_t dij_reset(ScorerHost& s, int sms, cudaStream_t st);
 
 /// The shape of a draining wave over n queue entries.  While every track has a lane of its own, the
-/// wave lasts as long as a chain of steps takes, and 16 warps per SM (128 registers, no spills) take
-/// them sooner; beyond that throughput counts, and 20 warps do.  Few tracks are spread over the
+/// wave lasts as long as a chain of steps takes, and 12 warps per SM (168 registers, hardly a spill) take
+/// them sooner than 16 with 128 registers (5000 histories on the slab phantom 1.40 -> 1.19 ms, 50 000 in
+/// water 4.55 -> 4.03, twelve CT spots of 2500, one call each, 15.8 -> 13.8); beyond that throughput
+/// counts, and 20 warps do (with 12, 100 000 in water 5.2 -> 6.7).  Few tracks are spread over the
 /// resident warps, and blocks are launched for about twice the tracks, not for every warp: those
 /// without a track only poll.
 inline void
 plan_drain(WaveParams& P, uint32_t n, int sms) {
-    P.drain_warps        = n <= (uint32_t) (sms * 16 * 32) ? 16 : 20;
+    P.drain_warps        = n <= (uint32_t) (sms * 12 * 32) ? 12 : 20;
     const uint32_t warps = (uint32_t) (sms * P.drain_warps);
     P.lanes      = (int) std::min<uint32_t>((n + warps - 1) / warps, 32u);
     P.max_blocks = std::max<int>(sms, 2 * (int) ((n + 4 * P.lanes - 1) / (4 * P.lanes)));

@@ -178,7 +178,7 @@ struct WaveParams {
     uint32_t        epoch;      // a draining wave's number, unlike any that `ready` or `def` hold (30 bits)
     int             lanes;      // lanes of a warp that take tracks (1 .. 32)
     int             max_blocks;  // a draining wave's blocks of four warps, at most
-    int             drain_warps; // a draining wave's warps per SM, 16 or 20 (its register budget)
+    int             drain_warps; // a draining wave's warps per SM, 12 or 20 (its register budget)
     int             smem_edge_floats; // shared-memory floats for staged child edges
     const float*    tables;     // device: the six physics tables, 6 x 600 floats in Tables order
                                 // (a context's are followed by the density of each HU value)

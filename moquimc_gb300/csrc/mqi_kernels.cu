@@ -1561,9 +1561,10 @@ k_wave(const __grid_constant__ WaveParams P) {
 }
 
 /// The draining wave, in every mode in two shapes: one block of 640 threads per SM, as above (100 000
-/// histories in water 5.97 -> 5.59 ms), or four of 128 where not all may be needed (512 threads in one
-/// block: 600 tracks 0.71 -> 0.81 ms, as fewer SMs share them).  A kernel apart from the ordinary wave,
-/// whose step loop is 15% faster for not sharing its registers and its image with the post-steps.
+/// histories in water 5.97 -> 5.59 ms), or up to three of 128 where tracks are few (plan_drain; in one
+/// large block 600 tracks took 0.81 instead of 0.71 ms, as fewer SMs share them).  A kernel apart from the
+/// ordinary wave, whose step loop is 15% faster for not sharing its registers and its image with the
+/// post-steps.
 template<int kThreads, int kMinBlocks, int kMode>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
 k_drain(const __grid_constant__ WaveParams P) {
@@ -1629,7 +1630,7 @@ launch_drain_shape(const WaveParams& p, int blocks, cudaStream_t s) {
 template<int K>
 static cudaError_t
 launch_drain(const WaveParams& p, int sms, cudaStream_t s) {
-    return p.drain_warps == 16 ? launch_drain_shape<128, 4, K>(p, std::min(sms * 4, p.max_blocks), s)
+    return p.drain_warps == 12 ? launch_drain_shape<128, 3, K>(p, std::min(sms * 3, p.max_blocks), s)
                                : launch_drain_shape<640, 1, K>(p, sms, s);
 }
 

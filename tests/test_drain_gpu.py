@@ -41,7 +41,7 @@ def _run(c, ids, v, mode):
 
 
 @pytest.mark.parametrize("debug", [False, True])
-@pytest.mark.parametrize("n", [1, 2, 33, 607, 3041, 60_001, 97_281])
+@pytest.mark.parametrize("n", [1, 2, 33, 607, 1825, 3041, 58_368, 58_369, 60_001, 97_281])
 def test_sizes(gpu_ctx_factory, n, debug):
     c, cid = _box(gpu_ctx_factory, debug)
     ids = [c.add_scorer(cid, capi.DOSE_W)]
