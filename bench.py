@@ -278,7 +278,7 @@ def plan_section(torch, capi, workloads, args) -> dict:
         "plain_per_spot": {"primaries_per_s": plain_rate, "seconds_per_pass": t_p, "spots_timed": len(wl.spots),
                            "histories_timed": N, "launch_mode": "queue generations",
                            "sample": "the whole plan, one mqi_transport_plan call per spot",
-                           "streamed_with_graph_per_call": {"primaries_per_s": h_sub / t_ps, "spots": len(sub),
+                           "streamed_per_call": {"primaries_per_s": h_sub / t_ps, "spots": len(sub),
                                                             "sample": f"every {args.plain_stride}th spot"}},
         "batched_over_plain": batched / plain_rate,
         "time_to_1pct_sigma": {"criterion": "reference estimator <= 1% over voxels > 50% of max dose",
@@ -349,10 +349,10 @@ def dij_section(torch, capi, workloads, optimize, stride: int = 1) -> dict:
         torch.cuda.synchronize()
         times[name] = ev0.elapsed_time(ev1) / 10
     vr = c.dij_info(sid)["voxel_rows"]
-    # algorithmic bytes: what each product must move at least.  D.w: spot + value per entry, row
-    # voxel + indptr per voxel row, the dose zeroed and written.  D^T.g: voxel + value per entry,
+    # algorithmic bytes: what each product must move at least.  D.w: spot (2 bytes up to 65536 spots) +
+    # value per entry, row voxel + row start (2 bytes) per voxel row, the dose zeroed and written.  D^T.g: voxel + value per entry,
     # g read once per voxel that has an entry, the gradient and its FP64 partials per spot.
-    fwd_bytes = op.nnz * 8 + vr * 12 + op.n_voxels * 8
+    fwd_bytes = op.nnz * (6 if op.n_spots <= 65536 else 8) + vr * 6 + op.n_voxels * 8
     bwd_bytes = op.nnz * 8 + vr * 4 + op.n_spots * 16
     hbm = measured_peaks()["hbm_gbs"]
     out = {
@@ -531,8 +531,8 @@ def run_gpu(args, wl):
         "bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
         "frac": achieved / peaks["hbm_gbs"], "peak_source": f"{peaks['source']} hbm_gbs",
         "traffic": (tps * steps / max(launches, 1)) if tps else None,
-        "kernel": "k_wave (timed with its post-step kernel k_post, which finishes the ~0.2% of steps that end "
-                  "in a nuclear interaction)",
+        "kernel": "k_wave and k_drain, the ordinary and the draining wave (an ordinary wave is timed with k_post, which "
+                  "finishes the ~0.2% of steps that end in a nuclear interaction)",
         "algorithmic_bytes_per_launch": bytes_per_launch,
         "avg_launch_ms": wave_ms / max(launches, 1), "transport_steps_per_s": steps / (wave_ms / 1e3) if wave_ms else 0,
         "wave_share_of_step": wave_ms / ms if ms > 0 else None,

@@ -1548,11 +1548,11 @@ launch_load_primaries(const Queue& q, uint32_t dst, const mqi_vertex* v, const u
 /// The wave kernel: one block per SM, of as many threads as its registers allow (512 at up to 128
 /// registers, 640 at 96, 768 at 80; the common modes -- DIRECT ROIs, simple scorer callbacks -- come in
 /// all three for the tuner, the others in 640).  Its step loop is bound by its instruction stream: of
-/// five warps to a scheduler 1.9 wait for a fixed latency and 1.0 for instructions, at an issue rate of
-/// 0.68.  Against blocks of 128 threads, five to the SM (1.8 warps waiting for instructions, the same
-/// number of instructions), the tables and edges take 32 KB of the SM once instead of 132 KB: 1 M
-/// histories on the slab phantom 17.84 -> 16.65 ms, a CT plan with its statistics 55.0 -> 51.2, 21
-/// scenarios 56.5 -> 54.2.  Two blocks of 320 threads got 0.3 of the slab's 1.2 ms; setting 64 KB aside
+/// five warps to a scheduler 1.5 wait for a fixed latency and 0.8 for instructions, at an issue rate of
+/// 0.72.  Against blocks of 128 threads, five to the SM (1.8 instead of 1.0 warps waiting for
+/// instructions then, the same number of instructions), the tables and edges take 32 KB of the SM once
+/// instead of 132 KB: 1 M histories on the slab phantom 17.84 -> 16.65 ms, a CT plan with its statistics
+/// 55.0 -> 51.2, 21 scenarios 56.5 -> 54.2 (15.1, 50.4 and 53.1 since).  Two blocks of 320 threads got 0.3 of the slab's 1.2 ms; setting 64 KB aside
 /// cost the CT 1% and the scenarios 2.5%; a barrier a step, to share what is fetched, cost 20%.
 template<int kThreads, int kMode>
 __global__ void __launch_bounds__(kThreads, 1)
