@@ -118,14 +118,17 @@ cudaError_t dij_reset(ScorerHost& s, int sms, cudaStream_t st);
 /// them sooner than 16 with 128 registers (5000 histories on the slab phantom 1.40 -> 1.19 ms, 50 000 in
 /// water 4.55 -> 4.03, twelve CT spots of 2500, one call each, 15.8 -> 13.8); beyond that throughput
 /// counts, and 20 warps do (with 12, 100 000 in water 5.2 -> 6.7).  Few tracks are spread over the
-/// resident warps, and blocks are launched for about twice the tracks, not for every warp: those
-/// without a track only poll.
+/// resident warps, and no more blocks are launched than hold a lane for each, the warps that only run
+/// post-steps (kPostEvery) and a few to spare: those without a track poll, and fetch other code than
+/// their neighbours (with twice the warps 600 tracks took 0.637 instead of 0.615 ms, twelve CT spots 13.7
+/// instead of 12.9, 30 000 histories in water 3.9 instead of 3.7).
 inline void
 plan_drain(WaveParams& P, uint32_t n, int sms) {
     P.drain_warps        = n <= (uint32_t) (sms * 12 * 32) ? 12 : 20;
-    const uint32_t warps = (uint32_t) (sms * P.drain_warps);
-    P.lanes      = (int) std::min<uint32_t>((n + warps - 1) / warps, 32u);
-    P.max_blocks = std::max<int>(sms, 2 * (int) ((n + 4 * P.lanes - 1) / (4 * P.lanes)));
+    const uint32_t warps = (uint32_t) (sms * P.drain_warps) / kPostEvery * (kPostEvery - 1);
+    P.lanes              = (int) std::min<uint32_t>((n + warps - 1) / warps, 32u);
+    const uint32_t need  = (n + P.lanes - 1) / P.lanes;
+    P.max_blocks         = std::max<int>(sms, (int) ((need + need / 64 + 7) / 4));
 }
 
 struct DeviceGuard {

@@ -123,6 +123,10 @@ struct Deferred {
     uint32_t mark;     // process (1 p-p elastic, 2 p-O elastic, 3 p-O inelastic) | wave's epoch << 2
 };
 
+/// A draining wave's warps to one that only runs post-steps (with 40, 100 000 histories in water took 6%
+/// longer; with 240, 18%).
+constexpr uint32_t kPostEvery = 80;
+
 /// What the warps of a draining wave share, read as one 16-byte word.
 struct alignas(16) DrainState {
     unsigned long long live;   // entries of the queue being read << 32 | tracks not yet ended

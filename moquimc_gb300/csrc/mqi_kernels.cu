@@ -37,9 +37,6 @@ constexpr unsigned long long kLiveEntry = 1ull << 32;
 /// Polls a warp without tracks makes before it gives up on the others: seconds.
 constexpr uint32_t kDrainPolls = 1u << 24;
 
-/// A draining wave's warps to one that only runs post-steps.
-constexpr uint32_t kPostEvery = 80;
-
 /// A track in registers: track_t<float> (mqi_track.hpp:48-205) reduced to what transport reads.
 struct Trk {
     float    ke0, ke1;
