@@ -181,15 +181,18 @@ mqi_create(int device, mqi_ctx** out) {
     std::memcpy(&host[4 * MQI_TABLE_N], mqi_tab_cs_po_e, sizeof(mqi_tab_cs_po_e));
     std::memcpy(&host[5 * MQI_TABLE_N], mqi_tab_cs_po_i, sizeof(mqi_tab_cs_po_i));
     std::memcpy(&host[6 * MQI_TABLE_N], mqi_tab_density_correction, sizeof(mqi_tab_density_correction));
+    // all in the order of the context's stream, which the legacy stream's copies are not ordered with (a
+    // pageable one returns once staged): k_hu_table rewrites a part of what the copy brings
     if ((e = cudaMalloc(&c->tables, tbytes)) != cudaSuccess ||
-        (e = cudaMemcpy(c->tables, host.data(), tbytes, cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(c->tables, host.data(), tbytes, cudaMemcpyHostToDevice, c->stream)) != cudaSuccess ||
         (e = launch_hu_table(c->tables + 6 * MQI_TABLE_N, c->stream)) != cudaSuccess ||
         (e = cudaMalloc(&c->counters, 12 * sizeof(uint32_t))) != cudaSuccess ||
-        (e = cudaMemset(c->counters, 0, 12 * sizeof(uint32_t))) != cudaSuccess ||
+        (e = cudaMemsetAsync(c->counters, 0, 12 * sizeof(uint32_t), c->stream)) != cudaSuccess ||
         (e = cudaMalloc(&c->stats, 8 * sizeof(unsigned long long))) != cudaSuccess ||
-        (e = cudaMemset(c->stats, 0, 8 * sizeof(unsigned long long))) != cudaSuccess ||
+        (e = cudaMemsetAsync(c->stats, 0, 8 * sizeof(unsigned long long), c->stream)) != cudaSuccess ||
         (e = cudaMallocHost(&c->host_counts, 12 * sizeof(uint32_t))) != cudaSuccess ||
-        (e = cudaEventCreate(&c->ev0)) != cudaSuccess || (e = cudaEventCreate(&c->ev1)) != cudaSuccess) {
+        (e = cudaEventCreate(&c->ev0)) != cudaSuccess || (e = cudaEventCreate(&c->ev1)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(c->stream)) != cudaSuccess) {
         mqi_destroy(c);
         return cuda_fail(nullptr, e, "mqi_create: allocation");
     }
