@@ -326,8 +326,8 @@ mqi_set_calibration(mqi_ctx* c, int calib, uint32_t n_rho, float rho0, float drh
     c->calib_buf = nullptr;
     c->calib     = CalibDev{};
     MQI_CUDA(c, cudaMalloc(&c->calib_buf, (n_spr + n_rho) * sizeof(float)), "mqi_set_calibration");
-    MQI_CUDA(c, cudaMemcpy(c->calib_buf, spr, n_spr * sizeof(float), cudaMemcpyHostToDevice), "mqi_set_calibration");
-    MQI_CUDA(c, cudaMemcpy(c->calib_buf + n_spr, x0, n_rho * sizeof(float), cudaMemcpyHostToDevice),
+    MQI_CUDA(c, upload(c, c->calib_buf, spr, n_spr * sizeof(float)), "mqi_set_calibration");
+    MQI_CUDA(c, upload(c, c->calib_buf + n_spr, x0, n_rho * sizeof(float)),
              "mqi_set_calibration");
     c->calib.mode  = MQI_CALIB_TABLE;
     c->calib.n_rho = n_rho;
@@ -360,9 +360,9 @@ mqi_add_child(mqi_ctx* c, int nx, int ny, int nz, const float* xe, const float* 
     MQI_CUDA(c, cudaMalloc(&ch.xe, (nx + 1) * sizeof(float)), "mqi_add_child");
     MQI_CUDA(c, cudaMalloc(&ch.ye, (ny + 1) * sizeof(float)), "mqi_add_child");
     MQI_CUDA(c, cudaMalloc(&ch.ze, (nz + 1) * sizeof(float)), "mqi_add_child");
-    MQI_CUDA(c, cudaMemcpy(ch.xe, xe, (nx + 1) * sizeof(float), cudaMemcpyHostToDevice), "mqi_add_child");
-    MQI_CUDA(c, cudaMemcpy(ch.ye, ye, (ny + 1) * sizeof(float), cudaMemcpyHostToDevice), "mqi_add_child");
-    MQI_CUDA(c, cudaMemcpy(ch.ze, ze, (nz + 1) * sizeof(float), cudaMemcpyHostToDevice), "mqi_add_child");
+    MQI_CUDA(c, upload(c, ch.xe, xe, (nx + 1) * sizeof(float)), "mqi_add_child");
+    MQI_CUDA(c, upload(c, ch.ye, ye, (ny + 1) * sizeof(float)), "mqi_add_child");
+    MQI_CUDA(c, upload(c, ch.ze, ze, (nz + 1) * sizeof(float)), "mqi_add_child");
     MQI_CUDA(c, cudaMalloc(&ch.rho, (size_t) nx * ny * nz * sizeof(float)), "mqi_add_child");
     identity3(ch.rf);
     ch.tr[0] = ch.tr[1] = ch.tr[2] = 0.0f;
@@ -472,7 +472,7 @@ mqi_add_scorer(mqi_ctx* c, int child_id, int type, int roi_method, uint32_t roi_
     } else if (roi_method == MQI_ROI_INDIRECT) {
         if (!roi_start) return fail(c, MQI_ERR_INVALID, "mqi_add_scorer: INDIRECT needs roi_start (one entry per voxel)");
         MQI_CUDA(c, cudaMalloc(&s.start, nvox * sizeof(uint32_t)), "mqi_add_scorer");
-        MQI_CUDA(c, cudaMemcpy(s.start, roi_start, nvox * sizeof(uint32_t), cudaMemcpyHostToDevice), "mqi_add_scorer");
+        MQI_CUDA(c, upload(c, s.start, roi_start, nvox * sizeof(uint32_t)), "mqi_add_scorer");
         s.tally_len = nvox;
     } else if (roi_method == MQI_ROI_CONTOUR) {
         if (!roi_start || !roi_stride || !roi_acc || roi_length == 0)
@@ -480,9 +480,9 @@ mqi_add_scorer(mqi_ctx* c, int child_id, int type, int roi_method, uint32_t roi_
         MQI_CUDA(c, cudaMalloc(&s.start, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
         MQI_CUDA(c, cudaMalloc(&s.stride, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
         MQI_CUDA(c, cudaMalloc(&s.acc, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
-        MQI_CUDA(c, cudaMemcpy(s.start, roi_start, roi_length * sizeof(uint32_t), cudaMemcpyHostToDevice), "mqi_add_scorer");
-        MQI_CUDA(c, cudaMemcpy(s.stride, roi_stride, roi_length * sizeof(uint32_t), cudaMemcpyHostToDevice), "mqi_add_scorer");
-        MQI_CUDA(c, cudaMemcpy(s.acc, roi_acc, roi_length * sizeof(uint32_t), cudaMemcpyHostToDevice), "mqi_add_scorer");
+        MQI_CUDA(c, upload(c, s.start, roi_start, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
+        MQI_CUDA(c, upload(c, s.stride, roi_stride, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
+        MQI_CUDA(c, upload(c, s.acc, roi_acc, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
         s.tally_len = nvox;
     } else {
         return fail(c, MQI_ERR_INVALID, "mqi_add_scorer: unknown roi method");
@@ -490,7 +490,7 @@ mqi_add_scorer(mqi_ctx* c, int child_id, int type, int roi_method, uint32_t roi_
     if (roi_method == MQI_ROI_CONTOUR) build_roi_words(c, s, nvox);
     s.copies = c->n_scen;
     MQI_CUDA(c, cudaMalloc(&s.tally, s.total() * sizeof(double)), "mqi_add_scorer");
-    MQI_CUDA(c, cudaMemset(s.tally, 0, s.total() * sizeof(double)), "mqi_add_scorer");
+    MQI_CUDA(c, zero_out(c, s.tally, s.total() * sizeof(double)), "mqi_add_scorer");
     c->scorers.push_back(s);
     if (scorer_id) *scorer_id = (int) c->scorers.size() - 1;
     return MQI_OK;
@@ -849,8 +849,8 @@ mqi_set_spot_plan(mqi_ctx* c, const mqi_spot* spots, uint32_t n_spots, uint64_t*
     c->plan_cum   = nullptr;
     MQI_CUDA(c, cudaMalloc(&c->plan_spots, std::max<size_t>(n_spots, 1) * sizeof(mqi_spot)), "mqi_set_spot_plan");
     MQI_CUDA(c, cudaMalloc(&c->plan_cum, (n_spots + 1) * sizeof(uint64_t)), "mqi_set_spot_plan");
-    if (n_spots) MQI_CUDA(c, cudaMemcpy(c->plan_spots, spots, n_spots * sizeof(mqi_spot), cudaMemcpyHostToDevice), "mqi_set_spot_plan");
-    MQI_CUDA(c, cudaMemcpy(c->plan_cum, cum.data(), (n_spots + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice), "mqi_set_spot_plan");
+    if (n_spots) MQI_CUDA(c, upload(c, c->plan_spots, spots, n_spots * sizeof(mqi_spot)), "mqi_set_spot_plan");
+    MQI_CUDA(c, upload(c, c->plan_cum, cum.data(), (n_spots + 1) * sizeof(uint64_t)), "mqi_set_spot_plan");
     c->n_plan_spots    = n_spots;
     c->plan_histories  = cum[n_spots];
     c->plan_cum_host   = cum;
@@ -894,7 +894,7 @@ mqi_set_scenarios(mqi_ctx* c, int child_id, uint32_t n, const float* xe, const f
                 if (j == k) host.insert(host.end(), e, e + len[a]);
             }
         MQI_CUDA(c, cudaMalloc(&edges, host.size() * sizeof(float)), "mqi_set_scenarios");
-        cudaError_t e = cudaMemcpy(edges, host.data(), host.size() * sizeof(float), cudaMemcpyHostToDevice);
+        cudaError_t e = upload(c, edges, host.data(), host.size() * sizeof(float));
         if (e != cudaSuccess) {
             cudaFree(edges);
             return cuda_fail(c, e, "mqi_set_scenarios");
@@ -911,7 +911,7 @@ mqi_set_scenarios(mqi_ctx* c, int child_id, uint32_t n, const float* xe, const f
         s.tally  = nullptr;
         s.copies = copies;
         MQI_CUDA(c, cudaMalloc(&s.tally, s.tstride * s.total() * sizeof(double)), "mqi_set_scenarios");
-        MQI_CUDA(c, cudaMemset(s.tally, 0, s.tstride * s.total() * sizeof(double)), "mqi_set_scenarios");
+        MQI_CUDA(c, zero_out(c, s.tally, s.tstride * s.total() * sizeof(double)), "mqi_set_scenarios");
         if (s.partner >= 0) {   // the stat pair's dose^2 half lives in the same buffer
             c->scorers[s.partner].tally  = s.tally + 1;
             c->scorers[s.partner].copies = copies;
@@ -985,7 +985,8 @@ mqi_autotune(mqi_ctx* c, int source_plan, uint64_t h0, uint64_t h1, uint64_t see
     std::vector<double*> saved(c->scorers.size(), nullptr);
     std::vector<double*> scratch(c->scorers.size(), nullptr);
     unsigned long long   stats_saved[8];
-    MQI_CUDA(c, cudaMemcpy(stats_saved, c->stats, sizeof(stats_saved), cudaMemcpyDeviceToHost), "mqi_autotune");
+    MQI_CUDA(c, cudaMemcpyAsync(stats_saved, c->stats, sizeof(stats_saved), cudaMemcpyDeviceToHost, c->stream), "mqi_autotune");
+    MQI_CUDA(c, cudaStreamSynchronize(c->stream), "mqi_autotune");
     const uint64_t waves0 = c->waves, kl0 = c->kernel_launches, wl0 = c->wave_launches;
     const double   wms0   = c->wave_ms;
     const int blk0 = c->wave_block, bps0 = c->wave_bps, str0 = c->streamed, gw0 = c->graph_waves;
@@ -996,7 +997,7 @@ mqi_autotune(mqi_ctx* c, int source_plan, uint64_t h0, uint64_t h1, uint64_t see
         if (!s.owns) continue;
         const size_t bytes = s.tstride * s.total() * sizeof(double);
         cudaError_t e = cudaMalloc(&scratch[i], bytes);
-        if (e == cudaSuccess) e = cudaMemset(scratch[i], 0, bytes);
+        if (e == cudaSuccess) e = zero_out(c, scratch[i], bytes);
         if (e != cudaSuccess) rc = cuda_fail(c, e, "mqi_autotune: scratch tallies");
     }
     auto swap_tallies = [&]() {
@@ -1064,7 +1065,7 @@ mqi_autotune(mqi_ctx* c, int source_plan, uint64_t h0, uint64_t h1, uint64_t see
         swap_tallies();
     }
     for (double* p : scratch) cudaFree(p);
-    cudaMemcpy(c->stats, stats_saved, sizeof(stats_saved), cudaMemcpyHostToDevice);
+    upload(c, c->stats, stats_saved, sizeof(stats_saved));
     c->waves = waves0; c->kernel_launches = kl0; c->wave_launches = wl0; c->wave_ms = wms0;
     if (rc != MQI_OK || best < 0) {
         c->wave_block = blk0; c->wave_bps = bps0; c->streamed = str0; c->graph_waves = gw0; c->primary_chunk = chunk0;
@@ -1403,13 +1404,13 @@ mqi_add_stat_scorers(mqi_ctx* c, int child_id, int roi_method, uint32_t roi_leng
         const uint64_t n_start = (roi_method == MQI_ROI_INDIRECT) ? nvox : roi_length;
         if (roi_method != MQI_ROI_DIRECT) {
             MQI_CUDA(c, cudaMalloc(&s.start, n_start * sizeof(uint32_t)), "mqi_add_stat_scorers");
-            MQI_CUDA(c, cudaMemcpy(s.start, roi_start, n_start * sizeof(uint32_t), cudaMemcpyHostToDevice), "mqi_add_stat_scorers");
+            MQI_CUDA(c, upload(c, s.start, roi_start, n_start * sizeof(uint32_t)), "mqi_add_stat_scorers");
         }
         if (roi_method == MQI_ROI_CONTOUR) {
             MQI_CUDA(c, cudaMalloc(&s.stride, roi_length * sizeof(uint32_t)), "mqi_add_stat_scorers");
             MQI_CUDA(c, cudaMalloc(&s.acc, roi_length * sizeof(uint32_t)), "mqi_add_stat_scorers");
-            MQI_CUDA(c, cudaMemcpy(s.stride, roi_stride, roi_length * sizeof(uint32_t), cudaMemcpyHostToDevice), "mqi_add_stat_scorers");
-            MQI_CUDA(c, cudaMemcpy(s.acc, roi_acc, roi_length * sizeof(uint32_t), cudaMemcpyHostToDevice), "mqi_add_stat_scorers");
+            MQI_CUDA(c, upload(c, s.stride, roi_stride, roi_length * sizeof(uint32_t)), "mqi_add_stat_scorers");
+            MQI_CUDA(c, upload(c, s.acc, roi_acc, roi_length * sizeof(uint32_t)), "mqi_add_stat_scorers");
             build_roi_words(c, s, nvox);
         }
         s.copies = c->n_scen;
@@ -1417,7 +1418,7 @@ mqi_add_stat_scorers(mqi_ctx* c, int child_id, int roi_method, uint32_t roi_leng
         if (k == 0) {
             // dose and dose^2 of a voxel side by side: the two per-step updates hit one 16-byte slot
             MQI_CUDA(c, cudaMalloc(&s.tally, 2 * s.total() * sizeof(double)), "mqi_add_stat_scorers");
-            MQI_CUDA(c, cudaMemset(s.tally, 0, 2 * s.total() * sizeof(double)), "mqi_add_stat_scorers");
+            MQI_CUDA(c, zero_out(c, s.tally, 2 * s.total() * sizeof(double)), "mqi_add_stat_scorers");
         } else {
             s.tally = c->scorers[ids[0]].tally + 1;
             s.owns  = false;

@@ -230,6 +230,21 @@ valid_ctx(const mqi_ctx* c) {
     return c != nullptr;
 }
 
+/// Host data to device memory, and zeroes there, in the order of the context's stream and done on return.
+/// (cudaMemcpy and cudaMemset run on the legacy stream, which a non-blocking stream does not wait
+/// for, and may return before the device has the data.)
+inline cudaError_t
+upload(mqi_ctx* c, void* dst, const void* src, size_t bytes) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
+}
+
+inline cudaError_t
+zero_out(mqi_ctx* c, void* dst, size_t bytes) {
+    const cudaError_t e = cudaMemsetAsync(dst, 0, bytes, c->stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
+}
+
 }   // namespace mqi_gpu
 
 #define MQI_CUDA(c, expr, what)                                        \
