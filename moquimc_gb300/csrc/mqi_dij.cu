@@ -509,6 +509,13 @@ mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
+/// The calling thread's accesses to shared memory so far come before copies that are issued after a
+/// barrier: a bulk copy writes through another proxy than the threads do, which barriers alone do not order.
+__device__ __forceinline__ void
+fence_before_bulk() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 /// The rows and entries of one run of the persistent forward, as thread 0 found them.
 struct FwdRun {
     unsigned long long k0, k1, a0;   // entries [k0, k1); staged from a0 (k0 rounded down to a group of eight)
@@ -662,6 +669,7 @@ k_dij_forward_pipe(const uint32_t* __restrict__ row_voxel, const uint16_t* __res
             for (uint32_t r = R.r0 + tid + kFwdRowsAhead * kFwdPipeThreads; r < R.r1; r += kFwdPipeThreads)
                 dose[row_voxel[r]] = row_sum(off[r], r + 1 < R.r1 ? off[r + 1] : (uint32_t) (R.k1 - base));
         }
+        fence_before_bulk();
         __syncthreads();   // stage s is free: the next iteration refills it
         s = s + 1 == kFwdStages ? 0 : s + 1;
     }
