@@ -769,6 +769,9 @@ run_waves(mqi_ctx* c, WaveParams& P, uint64_t h0, uint64_t h1, bool plan, uint32
         uint32_t load = 0;
         if (old == 0 || (c->streamed && old < target))
             load = (uint32_t) std::min<uint64_t>((target - old) / S, h1 - h);
+        // a wave over more entries than its queue holds would run none of them
+        if (old + (uint64_t) load * S > A->q.capacity)
+            return fail(c, MQI_ERR_OVERFLOW, "mqi_transport: a load does not fit the particle queue");
         int rc = MQI_OK;
         if (load > 0 && (rc = load_histories(c, P, A->q, old, h, load, plan)) != MQI_OK) return rc;
         h += load;
@@ -787,7 +790,7 @@ run_waves(mqi_ctx* c, WaveParams& P, uint64_t h0, uint64_t h1, bool plan, uint32
 int
 run_transport(mqi_ctx* c, uint64_t h0, uint64_t h1, uint64_t seed, bool plan) {
     DeviceGuard g(c->device);
-    const uint32_t need = c->primary_chunk * 3u;
+    const uint32_t need = std::max(c->primary_chunk, c->n_scen) * 3u;   // a load holds at least one history's scenarios
     if (c->queue_cap < need) {
         cudaFree(c->ready);
         c->ready      = nullptr;
