@@ -171,7 +171,13 @@ int mqi_set_vertices(mqi_ctx* ctx, const mqi_vertex* v, const uint32_t* spot_ids
 
 /* Transport histories [h0, h1) of the current vertices with run seed `seed`, adding into the
  * tallies.  Replaces transport_particles_patient<float><<<...>>> (mqi_transport.hpp:113-250).
- * Blocks until the work is done. */
+ * Blocks until the work is done.
+ * The first transport after a change of a density, the curves, the physics options or the scenarios
+ * tabulates what a step needs of each voxel's material, 16 bytes per voxel of each child and for the
+ * scenarios' child per different density scale, and keeps the tables until the next such change: where
+ * they leave half of the free memory and take at most an eighth of the device's.  Without them a step
+ * computes the same values.  They are freed, as are the kept buffers of mqi_dij_build, when a call of this
+ * context would otherwise fail for want of memory. */
 int mqi_transport(mqi_ctx* ctx, uint64_t h0, uint64_t h1, uint64_t seed);
 
 /* A plan of spots whose histories are sampled on the device: history h belongs to spot s when

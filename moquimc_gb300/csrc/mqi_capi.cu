@@ -33,11 +33,11 @@ free_queue(QueueBuf& b) {
 
 /// One allocation per queue, carved into the SoA columns (each 256-byte aligned).
 cudaError_t
-alloc_queue(QueueBuf& b, uint32_t cap) {
+alloc_queue(mqi_ctx* c, QueueBuf& b, uint32_t cap) {
     free_queue(b);
     const size_t col   = ((size_t) cap * 4 + 255) & ~(size_t) 255;
     const int    ncols = 15;
-    cudaError_t  e     = cudaMalloc(&b.base, col * ncols);
+    cudaError_t  e     = device_alloc(c, b.base, col * ncols);
     if (e != cudaSuccess) return e;
     char* p = static_cast<char*>(b.base);
     auto  f = [&](int k) { return reinterpret_cast<float*>(p + col * k); };
@@ -64,6 +64,35 @@ drop_materials(mqi_ctx* c) {
     DeviceGuard g(c->device);
     for (ChildHost& ch : c->children) drop_materials(ch);
 }
+
+}   // namespace
+
+bool
+mqi_gpu::give_back(mqi_ctx* c) {
+    DeviceGuard g(c->device);
+    bool        any = false;
+    for (ChildHost& ch : c->children) {
+        any = any || !ch.mats.empty();
+        drop_materials(ch);
+    }
+    if (c->build_scratch) {
+        cudaFree(c->build_scratch);
+        c->build_scratch       = nullptr;
+        c->build_scratch_bytes = 0;
+        any                    = true;
+    }
+    for (ScorerHost& s : c->scorers)
+        if (s.csr.slab && !s.csr.built) {
+            cudaDeviceSynchronize();   // products queued before it went stale, on any stream
+            dij_drop_matrix(s);
+            any = true;
+        }
+    if (any) ++c->give_backs;
+    return any;
+}
+
+namespace
+{
 
 /// Tabulate a CONTOUR scorer's ROI by voxel (8 bytes per 32 voxels).  Without the memory, or where the
 /// runs are not ones that a table can hold, the search stays.
@@ -325,7 +354,7 @@ mqi_set_calibration(mqi_ctx* c, int calib, uint32_t n_rho, float rho0, float drh
     cudaFree(c->calib_buf);
     c->calib_buf = nullptr;
     c->calib     = CalibDev{};
-    MQI_CUDA(c, cudaMalloc(&c->calib_buf, (n_spr + n_rho) * sizeof(float)), "mqi_set_calibration");
+    MQI_CUDA(c, device_alloc(c, c->calib_buf, (n_spr + n_rho) * sizeof(float)), "mqi_set_calibration");
     MQI_CUDA(c, upload(c, c->calib_buf, spr, n_spr * sizeof(float)), "mqi_set_calibration");
     MQI_CUDA(c, upload(c, c->calib_buf + n_spr, x0, n_rho * sizeof(float)),
              "mqi_set_calibration");
@@ -357,13 +386,13 @@ mqi_add_child(mqi_ctx* c, int nx, int ny, int nz, const float* xe, const float* 
     DeviceGuard g(c->device);
     ChildHost ch;
     ch.nx = nx; ch.ny = ny; ch.nz = nz;
-    MQI_CUDA(c, cudaMalloc(&ch.xe, (nx + 1) * sizeof(float)), "mqi_add_child");
-    MQI_CUDA(c, cudaMalloc(&ch.ye, (ny + 1) * sizeof(float)), "mqi_add_child");
-    MQI_CUDA(c, cudaMalloc(&ch.ze, (nz + 1) * sizeof(float)), "mqi_add_child");
+    MQI_CUDA(c, device_alloc(c, ch.xe, (nx + 1) * sizeof(float)), "mqi_add_child");
+    MQI_CUDA(c, device_alloc(c, ch.ye, (ny + 1) * sizeof(float)), "mqi_add_child");
+    MQI_CUDA(c, device_alloc(c, ch.ze, (nz + 1) * sizeof(float)), "mqi_add_child");
     MQI_CUDA(c, upload(c, ch.xe, xe, (nx + 1) * sizeof(float)), "mqi_add_child");
     MQI_CUDA(c, upload(c, ch.ye, ye, (ny + 1) * sizeof(float)), "mqi_add_child");
     MQI_CUDA(c, upload(c, ch.ze, ze, (nz + 1) * sizeof(float)), "mqi_add_child");
-    MQI_CUDA(c, cudaMalloc(&ch.rho, (size_t) nx * ny * nz * sizeof(float)), "mqi_add_child");
+    MQI_CUDA(c, device_alloc(c, ch.rho, (size_t) nx * ny * nz * sizeof(float)), "mqi_add_child");
     identity3(ch.rf);
     ch.tr[0] = ch.tr[1] = ch.tr[2] = 0.0f;
     if (rot_fwd) std::memcpy(ch.rf, rot_fwd, sizeof(ch.rf));
@@ -406,8 +435,8 @@ mqi_hu_to_density(mqi_ctx* c, const int16_t* hu, float* rho, uint64_t n, float s
     }
     int16_t* dh = nullptr;
     float*   dr = nullptr;
-    MQI_CUDA(c, cudaMalloc(&dh, n * sizeof(int16_t) + 16), "mqi_hu_to_density");
-    cudaError_t e = cudaMalloc(&dr, n * sizeof(float) + 16);
+    MQI_CUDA(c, device_alloc(c, dh, n * sizeof(int16_t) + 16), "mqi_hu_to_density");
+    cudaError_t e = device_alloc(c, dr, n * sizeof(float) + 16);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dh, hu, n * sizeof(int16_t), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = launch_hu_to_density(c->tables + 6 * MQI_TABLE_N, dh, dr, n, scale, c->num_sms, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(rho, dr, n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
@@ -429,7 +458,7 @@ mqi_set_hu(mqi_ctx* c, int id, const int16_t* hu, float scale, int on_device) {
     const int16_t* src = hu;
     int16_t*       tmp = nullptr;
     if (!on_device) {
-        MQI_CUDA(c, cudaMalloc(&tmp, n * sizeof(int16_t)), "mqi_set_hu");
+        MQI_CUDA(c, device_alloc(c, tmp, n * sizeof(int16_t)), "mqi_set_hu");
         cudaError_t e = cudaMemcpyAsync(tmp, hu, n * sizeof(int16_t), cudaMemcpyHostToDevice, c->stream);
         if (e != cudaSuccess) { cudaFree(tmp); return cuda_fail(c, e, "mqi_set_hu"); }
         src = tmp;
@@ -471,15 +500,15 @@ mqi_add_scorer(mqi_ctx* c, int child_id, int type, int roi_method, uint32_t roi_
         s.tally_len = nvox;
     } else if (roi_method == MQI_ROI_INDIRECT) {
         if (!roi_start) return fail(c, MQI_ERR_INVALID, "mqi_add_scorer: INDIRECT needs roi_start (one entry per voxel)");
-        MQI_CUDA(c, cudaMalloc(&s.start, nvox * sizeof(uint32_t)), "mqi_add_scorer");
+        MQI_CUDA(c, device_alloc(c, s.start, nvox * sizeof(uint32_t)), "mqi_add_scorer");
         MQI_CUDA(c, upload(c, s.start, roi_start, nvox * sizeof(uint32_t)), "mqi_add_scorer");
         s.tally_len = nvox;
     } else if (roi_method == MQI_ROI_CONTOUR) {
         if (!roi_start || !roi_stride || !roi_acc || roi_length == 0)
             return fail(c, MQI_ERR_INVALID, "mqi_add_scorer: CONTOUR needs start/stride/acc arrays");
-        MQI_CUDA(c, cudaMalloc(&s.start, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
-        MQI_CUDA(c, cudaMalloc(&s.stride, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
-        MQI_CUDA(c, cudaMalloc(&s.acc, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
+        MQI_CUDA(c, device_alloc(c, s.start, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
+        MQI_CUDA(c, device_alloc(c, s.stride, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
+        MQI_CUDA(c, device_alloc(c, s.acc, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
         MQI_CUDA(c, upload(c, s.start, roi_start, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
         MQI_CUDA(c, upload(c, s.stride, roi_stride, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
         MQI_CUDA(c, upload(c, s.acc, roi_acc, roi_length * sizeof(uint32_t)), "mqi_add_scorer");
@@ -489,7 +518,7 @@ mqi_add_scorer(mqi_ctx* c, int child_id, int type, int roi_method, uint32_t roi_
     }
     if (roi_method == MQI_ROI_CONTOUR) build_roi_words(c, s, nvox);
     s.copies = c->n_scen;
-    MQI_CUDA(c, cudaMalloc(&s.tally, s.total() * sizeof(double)), "mqi_add_scorer");
+    MQI_CUDA(c, device_alloc(c, s.tally, s.total() * sizeof(double)), "mqi_add_scorer");
     MQI_CUDA(c, zero_out(c, s.tally, s.total() * sizeof(double)), "mqi_add_scorer");
     c->scorers.push_back(s);
     if (scorer_id) *scorer_id = (int) c->scorers.size() - 1;
@@ -504,7 +533,7 @@ mqi_set_vertices(mqi_ctx* c, const mqi_vertex* v, const uint32_t* spot_ids, uint
     if (n > c->vertex_cap) {
         cudaFree(c->vertices);
         c->vertices = nullptr;
-        MQI_CUDA(c, cudaMalloc(&c->vertices, n * sizeof(mqi_vertex)), "mqi_set_vertices");
+        MQI_CUDA(c, device_alloc(c, c->vertices, n * sizeof(mqi_vertex)), "mqi_set_vertices");
         c->vertex_cap = n;
     }
     if (spot_ids && !on_device)
@@ -517,7 +546,7 @@ mqi_set_vertices(mqi_ctx* c, const mqi_vertex* v, const uint32_t* spot_ids, uint
         if (n > c->spot_cap) {
             cudaFree(c->spot_ids);
             c->spot_ids = nullptr;
-            MQI_CUDA(c, cudaMalloc(&c->spot_ids, n * sizeof(uint32_t)), "mqi_set_vertices");
+            MQI_CUDA(c, device_alloc(c, c->spot_ids, n * sizeof(uint32_t)), "mqi_set_vertices");
             c->spot_cap = n;
         }
         MQI_CUDA(c, cudaMemcpyAsync(c->spot_ids, spot_ids, n * sizeof(uint32_t), k, c->stream), "mqi_set_vertices");
@@ -539,21 +568,31 @@ constexpr uint32_t kDrainMaxFresh = 1u << 19;
 /// The source stream of a plan history is keyed apart from its transport streams.
 constexpr uint32_t kSourceKeyXor = 0xA5A5A5A5u;
 
-/// Child i's materials at a density scale, tabulated on first use (0.3 ms for 52 M voxels); null, and
-/// the step computes them, when the table does not fit the device.
+/// Child i's materials at a density scale, tabulated on first use (0.3 ms for 52 M voxels); null, and the
+/// step computes them, when there is no room for the table.  A table only makes steps faster, so it
+/// takes no more than half of the memory that is free, a context's tables take no more than an eighth of
+/// the device's, and they are given back when an allocation would fail (device_alloc).  A table refused
+/// now may fit the next transport.
 const float4*
 materials(mqi_ctx* c, int i, float scale) {
     ChildHost& ch = c->children[i];
     for (const Material& m : ch.mats)
         if (std::memcmp(&m.scale, &scale, sizeof(scale)) == 0) return m.mat;
-    Material       m;
-    const uint64_t n = (uint64_t) ch.nx * ch.ny * ch.nz;
-    m.scale          = scale;
-    if (cudaMalloc(&m.mat, n * sizeof(float4)) != cudaSuccess ||
+    const uint64_t n     = (uint64_t) ch.nx * ch.ny * ch.nz;
+    const size_t   bytes = n * sizeof(float4);
+    size_t         held = 0, free = 0, total = 0;
+    for (const ChildHost& h : c->children) held += h.mats.size() * ((size_t) h.nx * h.ny * h.nz * sizeof(float4));
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess || bytes > free / 2 || held + bytes > total / 8) {
+        (void) cudaGetLastError();
+        return nullptr;
+    }
+    Material m;
+    m.scale = scale;
+    if (cudaMalloc(&m.mat, bytes) != cudaSuccess ||
         launch_materials(ch.rho, n, scale, c->physics_debug, c->calib, m.mat, c->num_sms, c->stream) != cudaSuccess) {
         (void) cudaGetLastError();
         cudaFree(m.mat);
-        m.mat = nullptr;
+        return nullptr;
     }
     ch.mats.push_back(m);
     return m.mat;
@@ -680,7 +719,7 @@ ensure_records(mqi_ctx* c, WaveParams& P, uint32_t n, bool drains) {
         c->def     = nullptr;
         c->def_cap = 0;
         const uint64_t cap = std::max<uint64_t>(want, 1u << 16);
-        MQI_CUDA(c, cudaMalloc(&c->def, cap * sizeof(Deferred)), "mqi_transport: record allocation");
+        MQI_CUDA(c, device_alloc(c, c->def, cap * sizeof(Deferred)), "mqi_transport: record allocation");
         MQI_CUDA(c, cudaMemsetAsync(c->def, 0, cap * sizeof(Deferred), c->stream), "mqi_transport");
         c->def_cap = (uint32_t) cap;
     }
@@ -693,8 +732,8 @@ ensure_records(mqi_ctx* c, WaveParams& P, uint32_t n, bool drains) {
 int
 ensure_sort(mqi_ctx* c) {
     if (c->qsort.q.capacity >= c->queue_cap && c->sort_bins) return MQI_OK;
-    MQI_CUDA(c, alloc_queue(c->qsort, c->queue_cap), "mqi_transport: sort allocation");
-    if (!c->sort_bins) MQI_CUDA(c, cudaMalloc(&c->sort_bins, 2 * kSortBins * sizeof(uint32_t)), "mqi_transport: sort allocation");
+    MQI_CUDA(c, alloc_queue(c, c->qsort, c->queue_cap), "mqi_transport: sort allocation");
+    if (!c->sort_bins) MQI_CUDA(c, device_alloc(c, c->sort_bins, 2 * kSortBins * sizeof(uint32_t)), "mqi_transport: sort allocation");
     MQI_CUDA(c, cudaMemsetAsync(c->sort_bins, 0, 2 * kSortBins * sizeof(uint32_t), c->stream), "mqi_transport");
     return MQI_OK;
 }
@@ -708,7 +747,8 @@ run_wave(mqi_ctx* c, WaveParams& P, const QueueBuf& A, const QueueBuf& B, uint32
     P.ready = nullptr;
     P.epoch = 0;
     P.lanes = 32;
-    int rc  = ensure_records(c, P, n, drains);
+    const uint64_t given = c->give_backs;
+    int            rc    = ensure_records(c, P, n, drains);
     if (rc != MQI_OK) return rc;
     if (drains) {
         if (++c->epoch >> 30) {   // the marks of 2^30 waves ago
@@ -723,6 +763,10 @@ run_wave(mqi_ctx* c, WaveParams& P, const QueueBuf& A, const QueueBuf& B, uint32
     // fresh primaries keep their order: a queue that holds nothing else is not sorted
     const bool sort = c->sort_min > 0 && old > 0 && n >= c->sort_min;
     if (sort && (rc = ensure_sort(c)) != MQI_OK) return rc;
+    if (c->give_backs != given) {   // the material tables made room: the steps compute what was in them
+        for (ChildDev& d : P.child) d.mat = nullptr;
+        for (const float4*& m : P.scen_mat) m = nullptr;
+    }
     P.sort_tmp  = c->qsort.q;
     P.sort_bins = sort ? c->sort_bins : nullptr;
     const uint32_t counts[12] = { n, 0, 0, 0, 0, 0, 0, 0, n, n, 0, 0 };
@@ -794,9 +838,9 @@ run_transport(mqi_ctx* c, uint64_t h0, uint64_t h1, uint64_t seed, bool plan) {
     if (c->queue_cap < need) {
         cudaFree(c->ready);
         c->ready      = nullptr;
-        cudaError_t e = alloc_queue(c->qa, need);
-        if (e == cudaSuccess) e = alloc_queue(c->qb, need);
-        if (e == cudaSuccess) e = cudaMalloc(&c->ready, (size_t) need * sizeof(uint32_t));
+        cudaError_t e = alloc_queue(c, c->qa, need);
+        if (e == cudaSuccess) e = alloc_queue(c, c->qb, need);
+        if (e == cudaSuccess) e = device_alloc(c, c->ready, (size_t) need * sizeof(uint32_t));
         if (e == cudaSuccess) e = cudaMemsetAsync(c->ready, 0, (size_t) need * sizeof(uint32_t), c->stream);
         if (e != cudaSuccess) {
             c->queue_cap = 0;
@@ -850,8 +894,8 @@ mqi_set_spot_plan(mqi_ctx* c, const mqi_spot* spots, uint32_t n_spots, uint64_t*
     cudaFree(c->plan_cum);
     c->plan_spots = nullptr;
     c->plan_cum   = nullptr;
-    MQI_CUDA(c, cudaMalloc(&c->plan_spots, std::max<size_t>(n_spots, 1) * sizeof(mqi_spot)), "mqi_set_spot_plan");
-    MQI_CUDA(c, cudaMalloc(&c->plan_cum, (n_spots + 1) * sizeof(uint64_t)), "mqi_set_spot_plan");
+    MQI_CUDA(c, device_alloc(c, c->plan_spots, std::max<size_t>(n_spots, 1) * sizeof(mqi_spot)), "mqi_set_spot_plan");
+    MQI_CUDA(c, device_alloc(c, c->plan_cum, (n_spots + 1) * sizeof(uint64_t)), "mqi_set_spot_plan");
     if (n_spots) MQI_CUDA(c, upload(c, c->plan_spots, spots, n_spots * sizeof(mqi_spot)), "mqi_set_spot_plan");
     MQI_CUDA(c, upload(c, c->plan_cum, cum.data(), (n_spots + 1) * sizeof(uint64_t)), "mqi_set_spot_plan");
     c->n_plan_spots    = n_spots;
@@ -896,7 +940,7 @@ mqi_set_scenarios(mqi_ctx* c, int child_id, uint32_t n, const float* xe, const f
                 off[k][a] = j < k ? off[j][a] : (uint32_t) host.size();
                 if (j == k) host.insert(host.end(), e, e + len[a]);
             }
-        MQI_CUDA(c, cudaMalloc(&edges, host.size() * sizeof(float)), "mqi_set_scenarios");
+        MQI_CUDA(c, device_alloc(c, edges, host.size() * sizeof(float)), "mqi_set_scenarios");
         cudaError_t e = upload(c, edges, host.data(), host.size() * sizeof(float));
         if (e != cudaSuccess) {
             cudaFree(edges);
@@ -913,7 +957,7 @@ mqi_set_scenarios(mqi_ctx* c, int child_id, uint32_t n, const float* xe, const f
         cudaFree(s.tally);
         s.tally  = nullptr;
         s.copies = copies;
-        MQI_CUDA(c, cudaMalloc(&s.tally, s.tstride * s.total() * sizeof(double)), "mqi_set_scenarios");
+        MQI_CUDA(c, device_alloc(c, s.tally, s.tstride * s.total() * sizeof(double)), "mqi_set_scenarios");
         MQI_CUDA(c, zero_out(c, s.tally, s.tstride * s.total() * sizeof(double)), "mqi_set_scenarios");
         if (s.partner >= 0) {   // the stat pair's dose^2 half lives in the same buffer
             c->scorers[s.partner].tally  = s.tally + 1;
@@ -999,7 +1043,7 @@ mqi_autotune(mqi_ctx* c, int source_plan, uint64_t h0, uint64_t h1, uint64_t see
         ScorerHost& s = c->scorers[i];
         if (!s.owns) continue;
         const size_t bytes = s.tstride * s.total() * sizeof(double);
-        cudaError_t e = cudaMalloc(&scratch[i], bytes);
+        cudaError_t e = device_alloc(c, scratch[i], bytes);
         if (e == cudaSuccess) e = zero_out(c, scratch[i], bytes);
         if (e != cudaSuccess) rc = cuda_fail(c, e, "mqi_autotune: scratch tallies");
     }
@@ -1095,8 +1139,8 @@ mqi_sample_plan(mqi_ctx* c, uint64_t h0, uint64_t h1, uint64_t seed, mqi_vertex*
     const uint64_t n = h1 - h0;
     mqi_vertex* dv = nullptr;
     uint32_t*   ds = nullptr;
-    cudaError_t e  = cudaMalloc(&dv, n * sizeof(mqi_vertex));
-    if (e == cudaSuccess && spot_out) e = cudaMalloc(&ds, n * sizeof(uint32_t));
+    cudaError_t e  = device_alloc(c, dv, n * sizeof(mqi_vertex));
+    if (e == cudaSuccess && spot_out) e = device_alloc(c, ds, n * sizeof(uint32_t));
     for (uint64_t off = 0; e == cudaSuccess && off < n; off += 0x40000000ull) {
         const uint32_t m = (uint32_t) std::min<uint64_t>(0x40000000ull, n - off);
         e = launch_sample_vertices(dv + off, ds ? ds + off : nullptr, c->plan_spots, c->plan_cum, c->n_plan_spots,
@@ -1127,7 +1171,7 @@ mqi_get_tally(mqi_ctx* c, int id, double* out, uint64_t* n_out, int on_device) {
         MQI_CUDA(c, launch_copy_strided(s.tally, s.tstride, out, s.total(), c->num_sms, c->stream), "mqi_get_tally");
     } else {
         double* tmp = nullptr;
-        MQI_CUDA(c, cudaMalloc(&tmp, bytes), "mqi_get_tally");
+        MQI_CUDA(c, device_alloc(c, tmp, bytes), "mqi_get_tally");
         cudaError_t e = launch_copy_strided(s.tally, s.tstride, tmp, s.total(), c->num_sms, c->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(out, tmp, bytes, cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -1199,11 +1243,11 @@ mqi_trace_rays(mqi_ctx* c, int id, const float* rays, uint64_t n_rays, uint32_t 
     float*    d_dist = nullptr;
     int32_t*  d_cells = nullptr;
     uint32_t* d_counts = nullptr;
-    cudaError_t e = cudaMalloc(&d_rays, n_rays * 6 * sizeof(float) + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&d_cnb, slots * sizeof(uint64_t) + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&d_dist, slots * sizeof(float) + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&d_cells, slots * 3 * sizeof(int32_t) + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&d_counts, n_rays * sizeof(uint32_t) + 16);
+    cudaError_t e = device_alloc(c, d_rays, n_rays * 6 * sizeof(float) + 16);
+    if (e == cudaSuccess) e = device_alloc(c, d_cnb, slots * sizeof(uint64_t) + 16);
+    if (e == cudaSuccess) e = device_alloc(c, d_dist, slots * sizeof(float) + 16);
+    if (e == cudaSuccess) e = device_alloc(c, d_cells, slots * 3 * sizeof(int32_t) + 16);
+    if (e == cudaSuccess) e = device_alloc(c, d_counts, n_rays * sizeof(uint32_t) + 16);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_rays, rays, n_rays * 6 * sizeof(float), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = launch_trace_rays(d, d_rays, n_rays, max_steps, d_cnb, d_dist, d_cells, d_counts, c->stream);
     std::vector<uint32_t> counts(n_rays);
@@ -1242,8 +1286,8 @@ mqi_eval_physics(mqi_ctx* c, const float* energies, uint64_t n, float* out) {
     DeviceGuard g(c->device);
     float* de = nullptr;
     float* dout = nullptr;
-    cudaError_t e = cudaMalloc(&de, n * sizeof(float) + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&dout, n * 8 * sizeof(float) + 16);
+    cudaError_t e = device_alloc(c, de, n * sizeof(float) + 16);
+    if (e == cudaSuccess) e = device_alloc(c, dout, n * 8 * sizeof(float) + 16);
     if (e == cudaSuccess) e = cudaMemcpyAsync(de, energies, n * sizeof(float), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = launch_eval_physics(c->tables, de, n, dout, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, dout, n * 8 * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
@@ -1279,10 +1323,10 @@ mqi_eval_hits(mqi_ctx* c, int child_id, int scorer_type, const float* steps, con
     uint32_t* dc = nullptr;
     int32_t*  dp = nullptr;
     double*   dout = nullptr;
-    cudaError_t e = cudaMalloc(&ds, n * 9 * sizeof(float) + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&dc, n * sizeof(uint32_t) + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&dp, n * sizeof(int32_t) + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&dout, n * sizeof(double) + 16);
+    cudaError_t e = device_alloc(c, ds, n * 9 * sizeof(float) + 16);
+    if (e == cudaSuccess) e = device_alloc(c, dc, n * sizeof(uint32_t) + 16);
+    if (e == cudaSuccess) e = device_alloc(c, dp, n * sizeof(int32_t) + 16);
+    if (e == cudaSuccess) e = device_alloc(c, dout, n * sizeof(double) + 16);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ds, steps, n * 9 * sizeof(float), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dc, cnb, n * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dp, primary, n * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream);
@@ -1313,9 +1357,9 @@ mqi_eval_roi(mqi_ctx* c, int scorer_id, const uint32_t* voxels, uint64_t n, int3
     uint32_t* dv = nullptr;
     int32_t*  di = nullptr;
     int32_t*  dm = nullptr;
-    cudaError_t e = cudaMalloc(&dv, n * sizeof(uint32_t) + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&di, n * sizeof(int32_t) + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&dm, n * sizeof(int32_t) + 16);
+    cudaError_t e = device_alloc(c, dv, n * sizeof(uint32_t) + 16);
+    if (e == cudaSuccess) e = device_alloc(c, di, n * sizeof(int32_t) + 16);
+    if (e == cudaSuccess) e = device_alloc(c, dm, n * sizeof(int32_t) + 16);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dv, voxels, n * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = launch_eval_roi(d, dv, n, di, dm, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(idx, di, n * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream);
@@ -1339,7 +1383,7 @@ namespace
 int
 ensure_stat_scratch(mqi_ctx* c) {
     if (!c->stat_scratch)
-        MQI_CUDA(c, cudaMalloc(&c->stat_scratch, 3 * kMaxScenarios * sizeof(unsigned long long)), "statistics scratch");
+        MQI_CUDA(c, device_alloc(c, c->stat_scratch, 3 * kMaxScenarios * sizeof(unsigned long long)), "statistics scratch");
     return MQI_OK;
 }
 
@@ -1406,12 +1450,12 @@ mqi_add_stat_scorers(mqi_ctx* c, int child_id, int roi_method, uint32_t roi_leng
         s.type       = types[k];
         const uint64_t n_start = (roi_method == MQI_ROI_INDIRECT) ? nvox : roi_length;
         if (roi_method != MQI_ROI_DIRECT) {
-            MQI_CUDA(c, cudaMalloc(&s.start, n_start * sizeof(uint32_t)), "mqi_add_stat_scorers");
+            MQI_CUDA(c, device_alloc(c, s.start, n_start * sizeof(uint32_t)), "mqi_add_stat_scorers");
             MQI_CUDA(c, upload(c, s.start, roi_start, n_start * sizeof(uint32_t)), "mqi_add_stat_scorers");
         }
         if (roi_method == MQI_ROI_CONTOUR) {
-            MQI_CUDA(c, cudaMalloc(&s.stride, roi_length * sizeof(uint32_t)), "mqi_add_stat_scorers");
-            MQI_CUDA(c, cudaMalloc(&s.acc, roi_length * sizeof(uint32_t)), "mqi_add_stat_scorers");
+            MQI_CUDA(c, device_alloc(c, s.stride, roi_length * sizeof(uint32_t)), "mqi_add_stat_scorers");
+            MQI_CUDA(c, device_alloc(c, s.acc, roi_length * sizeof(uint32_t)), "mqi_add_stat_scorers");
             MQI_CUDA(c, upload(c, s.stride, roi_stride, roi_length * sizeof(uint32_t)), "mqi_add_stat_scorers");
             MQI_CUDA(c, upload(c, s.acc, roi_acc, roi_length * sizeof(uint32_t)), "mqi_add_stat_scorers");
             build_roi_words(c, s, nvox);
@@ -1420,7 +1464,7 @@ mqi_add_stat_scorers(mqi_ctx* c, int child_id, int roi_method, uint32_t roi_leng
         s.tstride = 2;
         if (k == 0) {
             // dose and dose^2 of a voxel side by side: the two per-step updates hit one 16-byte slot
-            MQI_CUDA(c, cudaMalloc(&s.tally, 2 * s.total() * sizeof(double)), "mqi_add_stat_scorers");
+            MQI_CUDA(c, device_alloc(c, s.tally, 2 * s.total() * sizeof(double)), "mqi_add_stat_scorers");
             MQI_CUDA(c, zero_out(c, s.tally, 2 * s.total() * sizeof(double)), "mqi_add_stat_scorers");
         } else {
             s.tally = c->scorers[ids[0]].tally + 1;
@@ -1462,8 +1506,8 @@ mqi_batch_accumulate(mqi_ctx* c, int scorer_id) {
     ScorerHost& s = c->scorers[scorer_id];
     DeviceGuard g(c->device);
     if (!s.batch_s1) {
-        MQI_CUDA(c, cudaMalloc(&s.batch_s1, s.total() * sizeof(double)), "mqi_batch_accumulate");
-        MQI_CUDA(c, cudaMalloc(&s.batch_s2, s.total() * sizeof(double)), "mqi_batch_accumulate");
+        MQI_CUDA(c, device_alloc(c, s.batch_s1, s.total() * sizeof(double)), "mqi_batch_accumulate");
+        MQI_CUDA(c, device_alloc(c, s.batch_s2, s.total() * sizeof(double)), "mqi_batch_accumulate");
         MQI_CUDA(c, cudaMemsetAsync(s.batch_s1, 0, s.total() * sizeof(double), c->stream), "mqi_batch_accumulate");
         MQI_CUDA(c, cudaMemsetAsync(s.batch_s2, 0, s.total() * sizeof(double), c->stream), "mqi_batch_accumulate");
         s.n_batches = 0;
@@ -1500,7 +1544,7 @@ mqi_get_batch_mean(mqi_ctx* c, int scorer_id, double* out, uint64_t* n_out, int 
     if (s.n_batches == 0) return fail(c, MQI_ERR_STATE, "mqi_get_batch_mean: no accumulated batch");
     DeviceGuard g(c->device);
     double* dst = out;
-    if (!on_device) MQI_CUDA(c, cudaMalloc(&dst, s.total() * sizeof(double)), "mqi_get_batch_mean");
+    if (!on_device) MQI_CUDA(c, device_alloc(c, dst, s.total() * sizeof(double)), "mqi_get_batch_mean");
     cudaError_t e = launch_copy_scaled(s.batch_s1, dst, s.total(), 1.0 / (double) s.n_batches, c->num_sms, c->stream);
     if (e == cudaSuccess && !on_device)
         e = cudaMemcpyAsync(out, dst, s.total() * sizeof(double), cudaMemcpyDeviceToHost, c->stream);

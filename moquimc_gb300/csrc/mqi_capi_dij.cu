@@ -61,9 +61,8 @@ struct Scratch {
     std::vector<void*> ptrs;
     template<typename T>
     cudaError_t
-    alloc(T*& p, uint64_t n) {
-        p = nullptr;
-        cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), std::max<uint64_t>(n, 1) * sizeof(T));
+    alloc(mqi_ctx* c, T*& p, uint64_t n) {
+        cudaError_t e = device_alloc(c, p, std::max<uint64_t>(n, 1) * sizeof(T));
         if (e == cudaSuccess) ptrs.push_back(p);
         return e;
     }
@@ -89,6 +88,11 @@ dij_scorer(mqi_ctx* c, int id, const char* who) {
 
 namespace mqi_gpu
 {
+
+void
+dij_drop_matrix(ScorerHost& s) {
+    free_csr(s.csr);
+}
 
 /// Called by mqi_destroy / mqi_reset_tallies.
 void
@@ -137,8 +141,8 @@ mqi_add_dij_scorer(mqi_ctx* c, int child_id, int roi_method, uint32_t roi_length
     s.tally_len = 0;
     s.type      = MQI_SCORER_DIJ;
     s.dij_cap   = cap;
-    cudaError_t e = cudaMalloc(&s.dij, cap * sizeof(DijSlot));
-    if (e == cudaSuccess) e = cudaMalloc(&s.dij_count, sizeof(unsigned long long));
+    cudaError_t e = device_alloc(c, s.dij, cap * sizeof(DijSlot));
+    if (e == cudaSuccess) e = device_alloc(c, s.dij_count, sizeof(unsigned long long));
     if (e == cudaSuccess) e = dij_reset(s, c->num_sms, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
@@ -164,8 +168,8 @@ mqi_dij_record_hits(mqi_ctx* c, int id, uint64_t capacity) {
     s.hit_count = nullptr;
     s.hit_cap   = 0;
     if (capacity == 0) return MQI_OK;
-    cudaError_t e = cudaMalloc(&s.hit_log, capacity * sizeof(DijHit));
-    if (e == cudaSuccess) e = cudaMalloc(&s.hit_count, sizeof(unsigned long long));
+    cudaError_t e = device_alloc(c, s.hit_log, capacity * sizeof(DijHit));
+    if (e == cudaSuccess) e = device_alloc(c, s.hit_count, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemsetAsync(s.hit_count, 0, sizeof(unsigned long long), c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
@@ -247,15 +251,15 @@ mqi_dij_build(mqi_ctx* c, int id, uint32_t n_spots, double scale, uint64_t* nnz_
         return cv.used;
     };
     const size_t scratch_bytes = lay_out_scratch(Carve{});
-    struct GiveBack {   // at the end, when it is large
+    struct Trim {   // gives it back at the end, when it is large
         mqi_ctx* c;
-        ~GiveBack() {
+        ~Trim() {
             if (c->build_scratch_bytes <= kKeepScratch) return;
             cudaFree(c->build_scratch);
             c->build_scratch       = nullptr;
             c->build_scratch_bytes = 0;
         }
-    } give_back{ c };
+    } trim{ c };
 
     // the matrix: segments of the backward are bounded by whole ones and one more per row, voxel rows by
     // the entries and by the voxels
@@ -287,8 +291,16 @@ mqi_dij_build(mqi_ctx* c, int id, uint32_t n_spots, double scale, uint64_t* nnz_
     const size_t csr_bytes = lay_out(Carve{});
     // products queued on any stream may still read the last matrix
     if (s.csr.slab) MQI_CUDA(c, cudaDeviceSynchronize(), "mqi_dij_build");
-    MQI_CUDA(c, ensure_bytes(c->build_scratch, c->build_scratch_bytes, scratch_bytes), "mqi_dij_build: allocation");
-    MQI_CUDA(c, ensure_bytes(s.csr.slab, s.csr.slab_bytes, csr_bytes), "mqi_dij_build: allocation");
+    auto allocate = [&] {
+        const cudaError_t e = ensure_bytes(c->build_scratch, c->build_scratch_bytes, scratch_bytes);
+        return e == cudaSuccess ? ensure_bytes(s.csr.slab, s.csr.slab_bytes, csr_bytes) : e;
+    };
+    cudaError_t e = allocate();
+    if (e == cudaErrorMemoryAllocation && give_back(c)) {   // which takes both of them too
+        (void) cudaGetLastError();
+        e = allocate();
+    }
+    MQI_CUDA(c, e, "mqi_dij_build: allocation");
     lay_out_scratch(Carve{ static_cast<char*>(c->build_scratch) });
     lay_out(Carve{ static_cast<char*>(s.csr.slab) });
     m.slab       = s.csr.slab;
@@ -419,8 +431,8 @@ mqi_dij_matvec(mqi_ctx* c, int id, const void* w, void* dose, int fp64, int on_d
     void*       dd = dose;
     if (!on_device) {
         char *tw, *td;
-        MQI_CUDA(c, sc.alloc(tw, m.n_spots * es), "mqi_dij_matvec");
-        MQI_CUDA(c, sc.alloc(td, m.n_voxels * es), "mqi_dij_matvec");
+        MQI_CUDA(c, sc.alloc(c, tw, m.n_spots * es), "mqi_dij_matvec");
+        MQI_CUDA(c, sc.alloc(c, td, m.n_voxels * es), "mqi_dij_matvec");
         MQI_CUDA(c, cudaMemcpyAsync(tw, w, m.n_spots * es, cudaMemcpyHostToDevice, c->stream), "mqi_dij_matvec");
         dw = tw;
         dd = td;
@@ -453,8 +465,8 @@ mqi_dij_rmatvec(mqi_ctx* c, int id, const void* gin, void* grad, int fp64, int o
     void*       dr = grad;
     if (!on_device) {
         char *tg, *tr;
-        MQI_CUDA(c, sc.alloc(tg, m.n_voxels * es), "mqi_dij_rmatvec");
-        MQI_CUDA(c, sc.alloc(tr, m.n_spots * es), "mqi_dij_rmatvec");
+        MQI_CUDA(c, sc.alloc(c, tg, m.n_voxels * es), "mqi_dij_rmatvec");
+        MQI_CUDA(c, sc.alloc(c, tr, m.n_spots * es), "mqi_dij_rmatvec");
         MQI_CUDA(c, cudaMemcpyAsync(tg, gin, m.n_voxels * es, cudaMemcpyHostToDevice, c->stream), "mqi_dij_rmatvec");
         dg = tg;
         dr = tr;

@@ -110,6 +110,8 @@ std::string& thread_error_slot();
 
 /// Free a Dij scorer's table and matrix (mqi_capi_dij.cu).
 void dij_release(ScorerHost& s);
+/// Free a Dij scorer's matrix.
+void dij_drop_matrix(ScorerHost& s);
 /// Empty a Dij scorer's table; its matrix is no longer built.
 cudaError_t dij_reset(ScorerHost& s, int sms, cudaStream_t st);
 
@@ -187,6 +189,7 @@ struct mqi_ctx {
     uint64_t                wave_launches = 0;
     double                  wave_ms = 0.0;
     cudaEvent_t             ev0 = nullptr, ev1 = nullptr;
+    uint64_t                give_backs = 0;           // times that give_back freed something
     void*                   build_scratch = nullptr;  // the last Dij build's sort buffers, when at most kKeepScratch
     size_t                  build_scratch_bytes = 0;
     unsigned long long*     stat_scratch = nullptr;   // 3 x u64 for the statistics reductions
@@ -228,6 +231,25 @@ cuda_fail(mqi_ctx* c, cudaError_t e, const char* what) {
 inline bool
 valid_ctx(const mqi_ctx* c) {
     return c != nullptr;
+}
+
+/// Free what the context can do without: the material tables, the kept sort buffers of a Dij build and the
+/// memory of matrices that are no longer built.  False when there was nothing.  Not while a wave runs.
+bool give_back(mqi_ctx* c);
+
+/// Device memory that a call cannot do without: before it fails for want of memory, the context gives
+/// back what it can.
+template<typename T>
+cudaError_t
+device_alloc(mqi_ctx* c, T*& p, size_t bytes) {
+    p             = nullptr;
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), bytes);
+    if (e == cudaErrorMemoryAllocation && give_back(c)) {
+        (void) cudaGetLastError();
+        e = cudaMalloc(reinterpret_cast<void**>(&p), bytes);
+    }
+    if (e != cudaSuccess) p = nullptr;
+    return e;
 }
 
 /// Host data to device memory, and zeroes there, in the order of the context's stream and done on return.
