@@ -234,7 +234,9 @@ int mqi_add_dij_scorer(mqi_ctx* ctx, int child_id, int roi_method, uint32_t roi_
 /* Build the Dij matrix from the table: n_spots columns (0: the spot plan's count), values = FP64
  * tally * scale rounded once to FP32 (save_sparse_file's scale: particles per history * RBE *
  * fractions, mqi_tps_env.hpp:1905-1930).  Builds the spot-row CSR and the voxel-row layout the
- * products read.  `nnz` receives the entry count.  Transporting again invalidates the matrix. */
+ * products read.  `nnz` receives the entry count.  Transporting again invalidates the matrix.  The
+ * context keeps up to 512 MB of the build's sort buffers for the next one, and an invalid matrix's
+ * memory until the next build or mqi_reset_tallies. */
 int mqi_dij_build(mqi_ctx* ctx, int scorer_id, uint32_t n_spots, double scale, uint64_t* nnz);
 
 /* The spot-row CSR, the layout of save_to_npz (moqui/base/mqi_io.hpp:251-320): shape
@@ -275,7 +277,8 @@ int mqi_dij_rmatvec(mqi_ctx* ctx, int scorer_id, const void* g, void* grad, int 
  * `out` may be NULL to query it. */
 int mqi_get_tally(mqi_ctx* ctx, int scorer_id, double* out, uint64_t* n_out, int on_device);
 
-/* Zero every tally and the run counters. */
+/* Zero every tally and the run counters; empty the Dij tables and drop their matrices, whose memory is
+ * kept for the next build up to 512 MB each. */
 int mqi_reset_tallies(mqi_ctx* ctx);
 
 int mqi_get_stats(mqi_ctx* ctx, mqi_stats* out);

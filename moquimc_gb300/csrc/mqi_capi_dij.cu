@@ -111,7 +111,8 @@ dij_release(ScorerHost& s) {
 
 cudaError_t
 dij_reset(ScorerHost& s, int sms, cudaStream_t st) {
-    s.csr.built   = false;
+    s.csr.built = false;
+    if (s.csr.slab_bytes > kKeepScratch) free_csr(s.csr);   // a smaller one is kept for the next build
     cudaError_t e = dij_clear(s.dij, s.dij_cap, sms, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(s.dij_count, 0, sizeof(unsigned long long), st);
     return e;

@@ -43,7 +43,7 @@ struct ChildHost {
 /// and voxel rows (only voxels with an entry).
 struct DijCsr {
     bool      built = false;
-    void*     slab = nullptr;       // one allocation that holds all arrays; kept for the next build
+    void*     slab = nullptr;       // one allocation that holds all arrays; kept for the next build (dij_reset)
     size_t    slab_bytes = 0;
     uint32_t  n_spots = 0;
     uint64_t  n_voxels = 0;
@@ -68,7 +68,9 @@ struct DijCsr {
     uint64_t* fwd_run_k = nullptr;       // n_fwd_blocks + 1: first entry of each forward block's rows
 };
 
-constexpr size_t kKeepScratch = (size_t) 512 << 20;   // largest Dij build scratch a context keeps
+// The largest build scratch that a context keeps, and the largest memory of a matrix that a reset leaves to
+// the next build: allocating takes a small part of the time of a larger build.
+constexpr size_t kKeepScratch = (size_t) 512 << 20;
 
 struct ScorerHost {
     int       child = 0;

@@ -7,6 +7,7 @@ import pytest
 
 from moquimc_gb300 import capi
 from moquimc_gb300 import phantom as ph
+from moquimc_gb300 import workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -128,3 +129,22 @@ def test_a_refused_table_is_tried_again(make, reference):
     c.transport(0, N, 9)
     _check(c, sid, reference)
     assert before - torch.cuda.mem_get_info()[0] > 0.9 * TABLE
+
+
+def test_a_reset_frees_a_large_matrix(make):
+    import torch
+
+    c = make()
+    c.set_physics(False)
+    nxyz = (200, 200, 200)
+    c.add_child(*ph.phantom_box_edges((200.0, 200.0, 200.0), (0.0, 0.0, -100.0), nxyz))
+    c.set_hu(0, np.zeros(nxyz[::-1], np.int16))
+    sid = c.add_dij_scorer(0, capacity=1 << 27)
+    total = c.set_spot_plan(workloads.spot_plan(20, 18, 8.0, 0.5, 4.0, (120.0, 150.0), (18_000.0, 22_000.0)))
+    c.transport_plan(0, total, 3)
+    assert c.dij_build(sid).nnz * 16 > 1.1 * 512 * MB      # at least 14 bytes an entry, and 6 a voxel row
+    before = torch.cuda.mem_get_info()[0]
+    c.reset()
+    assert torch.cuda.mem_get_info()[0] - before > 512 * MB
+    c.transport_plan(0, int(c.plan_cum[3]), 3)
+    assert c.dij_build(sid).csr()[0][-1] > 0
