@@ -808,8 +808,9 @@ run_waves(mqi_ctx* c, WaveParams& P, uint64_t h0, uint64_t h1, bool plan, uint32
     const QueueBuf *A = &c->qa, *B = &c->qb;
     uint64_t        h = h0;
     uint32_t        old = 0;
-    for (int wave = 0; h < h1 || old > 0; ++wave) {
-        if (wave > 200000) return fail(c, MQI_ERR_DEVICE, "mqi_transport: wave limit reached");
+    int             waves = 0;   // since histories were last loaded: a run may be of any number of loads
+    while (h < h1 || old > 0) {
+        if (++waves > 200000) return fail(c, MQI_ERR_DEVICE, "mqi_transport: wave limit reached");
         uint32_t load = 0;
         if (old == 0 || (c->streamed && old < target))
             load = (uint32_t) std::min<uint64_t>((target - old) / S, h1 - h);
@@ -818,6 +819,7 @@ run_waves(mqi_ctx* c, WaveParams& P, uint64_t h0, uint64_t h1, bool plan, uint32
             return fail(c, MQI_ERR_OVERFLOW, "mqi_transport: a load does not fit the particle queue");
         int rc = MQI_OK;
         if (load > 0 && (rc = load_histories(c, P, A->q, old, h, load, plan)) != MQI_OK) return rc;
+        if (load > 0) waves = 0;
         h += load;
         const bool drains = may_drain && (h == h1 || !c->streamed) &&
                             (c->post_step_mode == 0 || old > 0 || load * S < kDrainMaxFresh);
