@@ -84,7 +84,7 @@ typedef struct {
 /* ---- run counters ------------------------------------------------------------------------- */
 typedef struct {
     uint64_t histories;        /* primaries transported (moqui's tracked_particles)           */
-    uint64_t tracks;           /* tracks popped from the queue, primaries included             */
+    uint64_t tracks;           /* tracks started: primaries and queued daughters               */
     uint64_t steps;            /* voxel steps taken                                            */
     uint64_t secondaries;      /* daughters pushed to the queue                                */
     uint64_t local_daughters;  /* deposit-only daughters scored at creation (debug physics)    */

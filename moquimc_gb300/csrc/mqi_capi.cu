@@ -821,6 +821,7 @@ run_waves(mqi_ctx* c, WaveParams& P, uint64_t h0, uint64_t h1, bool plan, uint32
         if (load > 0 && (rc = load_histories(c, P, A->q, old, h, load, plan)) != MQI_OK) return rc;
         if (load > 0) waves = 0;
         h += load;
+        c->loaded += (uint64_t) load * S;
         const bool drains = may_drain && (h == h1 || !c->streamed) &&
                             (c->post_step_mode == 0 || old > 0 || load * S < kDrainMaxFresh);
         if ((rc = run_wave(c, P, *A, *B, old + load * S, old, drains)) != MQI_OK) return rc;
@@ -1036,7 +1037,7 @@ mqi_autotune(mqi_ctx* c, int source_plan, uint64_t h0, uint64_t h1, uint64_t see
     unsigned long long   stats_saved[8];
     MQI_CUDA(c, cudaMemcpyAsync(stats_saved, c->stats, sizeof(stats_saved), cudaMemcpyDeviceToHost, c->stream), "mqi_autotune");
     MQI_CUDA(c, cudaStreamSynchronize(c->stream), "mqi_autotune");
-    const uint64_t waves0 = c->waves, kl0 = c->kernel_launches, wl0 = c->wave_launches;
+    const uint64_t waves0 = c->waves, loaded0 = c->loaded, kl0 = c->kernel_launches, wl0 = c->wave_launches;
     const double   wms0   = c->wave_ms;
     const int blk0 = c->wave_block, bps0 = c->wave_bps, str0 = c->streamed, gw0 = c->graph_waves;
     const uint32_t chunk0 = c->primary_chunk;
@@ -1115,7 +1116,7 @@ mqi_autotune(mqi_ctx* c, int source_plan, uint64_t h0, uint64_t h1, uint64_t see
     }
     for (double* p : scratch) cudaFree(p);
     upload(c, c->stats, stats_saved, sizeof(stats_saved));
-    c->waves = waves0; c->kernel_launches = kl0; c->wave_launches = wl0; c->wave_ms = wms0;
+    c->waves = waves0; c->loaded = loaded0; c->kernel_launches = kl0; c->wave_launches = wl0; c->wave_ms = wms0;
     if (rc != MQI_OK || best < 0) {
         c->wave_block = blk0; c->wave_bps = bps0; c->streamed = str0; c->graph_waves = gw0; c->primary_chunk = chunk0;
         return rc != MQI_OK ? rc : fail(c, MQI_ERR_DEVICE, "mqi_autotune: no candidate ran");
@@ -1197,6 +1198,7 @@ mqi_reset_tallies(mqi_ctx* c) {
     MQI_CUDA(c, cudaMemsetAsync(c->counters + 3, 0, sizeof(uint32_t), c->stream), "mqi_reset_tallies");
     MQI_CUDA(c, cudaStreamSynchronize(c->stream), "mqi_reset_tallies");
     c->waves = 0;
+    c->loaded = 0;
     c->kernel_launches = 0;
     c->wave_launches = 0;
     c->wave_ms = 0.0;
@@ -1211,7 +1213,7 @@ mqi_get_stats(mqi_ctx* c, mqi_stats* out) {
     MQI_CUDA(c, cudaMemcpyAsync(v, c->stats, sizeof(v), cudaMemcpyDeviceToHost, c->stream), "mqi_get_stats");
     MQI_CUDA(c, cudaStreamSynchronize(c->stream), "mqi_get_stats");
     out->histories       = v[0];
-    out->tracks          = v[1];
+    out->tracks          = c->loaded + v[3];   // a resumed track is not another one, in whichever wave
     out->steps           = v[2];
     out->secondaries     = v[3];
     out->local_daughters = v[4];

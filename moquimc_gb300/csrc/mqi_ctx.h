@@ -187,6 +187,7 @@ struct mqi_ctx {
     uint32_t                max_slice_steps = 0;
     uint32_t                primary_chunk = 1u << 21;
     uint64_t                waves = 0;
+    uint64_t                loaded = 0;               // primaries put into the queue, once per scenario
     uint64_t                kernel_launches = 0;
     uint64_t                wave_launches = 0;
     double                  wave_ms = 0.0;

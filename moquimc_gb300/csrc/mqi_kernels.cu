@@ -27,8 +27,6 @@ constexpr uint32_t kMetaPhaseStep = 1u << 18;
 constexpr int      kMetaChildShift = 19;   // 3 bits
 constexpr int      kMetaNpushShift = 22;   // 10 bits
 
-enum StatIdx { ST_HIST = 0, ST_TRACKS, ST_STEPS, ST_SEC, ST_LOCAL, ST_DROP, ST_WAVES, ST_ERR };
-
 constexpr uint32_t kMaxTrackSteps = 1u << 20;
 
 /// WaveParams::live: queue entries in the high word, live tracks in the low one.
@@ -63,10 +61,10 @@ struct Ctx {
     float             tcut;
 };
 
-/// A block's event counters (indices of mqi_stats: histories, tracks, steps, secondaries queued,
+/// A block's event counters (indices of mqi_ctx::stats: histories, -, steps, secondaries queued,
 /// secondaries scored in place, secondaries dropped, -, errors), kept in shared memory so that the
 /// step loop does not carry them in registers; flushed once per block.
-enum { kCntHist = 0, kCntTracks = 1, kCntSteps = 2, kCntSec = 3, kCntLocal = 4, kCntDrop = 5, kCntErr = 7 };
+enum { kCntHist = 0, kCntSteps = 2, kCntSec = 3, kCntLocal = 4, kCntDrop = 5, kCntErr = 7 };
 static __shared__ unsigned int s_cnt[8];
 
 __device__ __forceinline__ void
@@ -1348,7 +1346,6 @@ wave_body(const WaveParams& P) {
                 in_grid = step_phase;
                 slice   = 0;
                 track_steps = 0;
-                if (!kDrain || rng.ctr == 0u) count_event(kCntTracks);   // not one resumed after a post-step
                 if (step_phase) {
                     C.child = t.child;
                     C.g     = make_grid(P.child[t.child], s_edges[t.child][0], s_edges[t.child][1], s_edges[t.child][2]);

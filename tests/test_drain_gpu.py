@@ -151,3 +151,20 @@ def test_dij_alone_instance(gpu_ctx_factory, mode, capacity):
     np.testing.assert_array_equal(csr[0][1], csr[1][1])
     np.testing.assert_allclose(csr[0][2], csr[1][2], rtol=2.0 ** -23, atol=0)
     assert csr[0][0][-1] > capacity // 2 or capacity > 1 << 13
+
+
+@pytest.mark.parametrize("shifter", [False, True])
+@pytest.mark.parametrize("debug", [False, True])
+def test_a_track_is_counted_once(gpu_ctx_factory, debug, shifter):
+    """Resumed after a nuclear interaction or a slice, a track is not another one: primaries and queued
+    daughters, whatever the waves."""
+    n = 3000
+    v = ph.uniform_spot_vertices(n, np.random.default_rng(3), 160.0, (0.0, 0.0, 60.0), (30.0, 30.0))
+    for mode, slices, streamed in ((-1, 0, 1), (0, 0, 0), (1, 0, 1), (1, 0, 0), (1, 7, 1), (-1, 7, 0)):
+        c, cid = _box(gpu_ctx_factory, debug, shifter)
+        c.add_scorer(cid, capi.EDEP)
+        c.set_tuning(slice_steps=slices)
+        c.set_launch_mode(streamed)
+        _, st = _run(c, [], v, mode)
+        assert st["tracks"] == n + st["secondaries"], (mode, slices, streamed)
+        assert st["secondaries"] > 0
