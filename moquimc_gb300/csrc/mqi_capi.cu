@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -1074,11 +1075,15 @@ mqi_autotune(mqi_ctx* c, int source_plan, uint64_t h0, uint64_t h1, uint64_t see
             chunks.back() = chunk;
         }
     }
+    // a scoring mode whose wave comes in one shape is timed in the setting's own
+    std::vector<std::pair<int, int>> shapes{ { blk0, bps0 } };
+    WaveParams P;
+    make_wave_params(c, seed, P);
+    if (wave_has_shapes(P.kernel_mode)) shapes = { { 128, 5 }, { 128, 4 }, { 128, 6 }, { 256, 2 } };
     std::vector<Cand> cands;
     for (int streamed : { 1, 0 })
         for (uint32_t chunk : chunks)
-            for (auto shape : { std::make_pair(128, 5), std::make_pair(128, 4), std::make_pair(128, 6), std::make_pair(256, 2) })
-                cands.push_back({ shape.first, shape.second, streamed, 8, chunk });
+            for (auto shape : shapes) cands.push_back({ shape.first, shape.second, streamed, gw0, chunk });
     uint32_t n = 0;
     int best = -1;
     double best_rate = 0.0;

@@ -267,6 +267,8 @@ cudaError_t launch_roi_words(const ScorerDev& s, uint64_t n_vox, uint2* words, u
 cudaError_t launch_materials(const float* rho, uint64_t n, float scale, int dbg, const CalibDev& calib, float4* mat, int sms,
                              cudaStream_t s);
 cudaError_t launch_wave(const WaveParams& p, int sms, int threads_per_sm, cudaStream_t s);
+// Whether that scoring mode's ordinary wave has an instance per launch shape.
+inline bool wave_has_shapes(int kernel_mode) { return kernel_mode == 0 || kernel_mode == kModeSingle; }
 int         wave_smem_bytes(const WaveParams& p);
 int         wave_edge_floats(const WaveParams& p);
 constexpr int kHuNodes = 3996;   // HU -1000 .. 2995, what hu_to_density's clamp leaves
