@@ -1,8 +1,9 @@
 """Build recipe for libmqigpu.so (the C ABI + sm_103a kernels) and the C++ host tools.
 
-Everything is compiled in-tree with nvcc/g++ directly (no CMake): two CUDA translation units
-compiled in parallel for ``sm_103a`` and linked into ``moquimc_gb300/_lib/libmqigpu.so``, plus the
-``phantom_env`` host executable that mirrors moqui's example driver on top of the C ABI.
+Everything is compiled in-tree with nvcc/g++ directly (no CMake): the CUDA translation units
+(``CUDA_SOURCES``) compiled in parallel for ``sm_103a`` and linked into
+``moquimc_gb300/_lib/libmqigpu.so``, plus the ``phantom_env`` and ``tps_env`` host executables that
+mirror moqui's drivers on top of the C ABI.
 """
 from __future__ import annotations
 

@@ -801,7 +801,8 @@ run_waves(mqi_ctx* c, WaveParams& P, uint64_t h0, uint64_t h1, bool plan, uint32
     // A run of at most two queue loads goes in one where a primary leaves well under one track behind
     // (every run but those that queue debug physics' deposit-only daughters): the queue holds three
     // loads, and a second, partial load would pay for a drain of its own (3 M histories on the CT: 60.0
-    // -> 55.5 ms; longer runs gain nothing from larger loads).
+    // -> 55.5 ms).  Longer runs keep their loads: 15 M histories on it took the same time with loads of
+    // 2^22, 2^23 and 2^24 entries.
     const uint64_t all    = (h1 - h0) * (uint64_t) S;
     const bool     in_one = c->streamed && all <= 2ull * c->primary_chunk && (P.inline_local || !P.physics_debug);
     const uint32_t target = in_one ? (uint32_t) all : std::max<uint32_t>(c->primary_chunk / S, 1u) * S;

@@ -7,8 +7,8 @@
 // table is compacted and sorted on the device, so both layouts come out in a fixed order:
 //   spot rows  (the reference's npz layout, shape [n_spots, n_voxels]): indptr / voxel / value,
 //              voxels ascending in a row -- the transposed operator, read by D^T.g;
-//   voxel rows (only voxels with an entry, "doubly compressed"): row voxel / indptr / spot /
-//              value, spots ascending in a row -- read by D.w.
+//   voxel rows (only voxels with an entry, "doubly compressed"): row voxel / row start in its run /
+//              spot / value, spots ascending in a row -- read by D.w.
 // Both products are gathers with a fixed reduction order: no atomics, reproducible results.
 #include <algorithm>
 #include <cstdint>
@@ -692,7 +692,7 @@ k_dij_forward_pipe(const uint32_t* __restrict__ row_voxel, const uint16_t* __res
 /// most dij_segment(nnz) entries that never cross a row; one block sums a segment's products (signed
 /// terms of a gradient cancel, so plain FP32 sums lose digits: a double-float accumulator per
 /// thread for FP32 g, FP64 for FP64 g; FP64 across the block) into one FP64 partial.  Pass 2
-/// (k_dij_backward_rows): one thread per row adds its segments' partials in order.  Rows of very
+/// (k_dij_backward_rows): a warp per row adds its segments' partials in a fixed tree.  Rows of very
 /// different lengths (1e4 to 3e6 entries at 2000 spots) thereby spread over every SM.
 /// s + c += a * b with no rounding error in the product (TwoProd: one FMA gives the product's
 /// rounding error) and Knuth's TwoSum for the addition: a double-float accumulator of about 48

@@ -205,7 +205,7 @@ launch_materials(const float* rho, uint64_t n, float scale, int dbg, const Calib
 /// distinct voxel) was measured slower on every workload -- 5.7% on the slab phantom, 6.6% on the
 /// synthetic-CT plan, 15% with the statistics pair -- because lanes of a warp run different
 /// histories and rarely share a voxel, while the match costs issue slots in an issue-bound kernel.
-/// The Dij insertion keeps the aggregation: there it saves hash probes.
+/// The Dij insertion does not combine lanes either (dij_add).
 __device__ inline void
 tally_add(double* tally, uint64_t slot, double v, bool valid) {
     if (valid) atomicAdd(&tally[slot], v);
@@ -1064,9 +1064,8 @@ fill_record(Deferred& d, const Trk& t, const Rng& rng, uint32_t cnb) {
 /// scoring, the cell update and move() (mqi_transport.hpp:204-233); then the track is queued again
 /// -- mid-grid, at the entry of the next child, or not at all when it stopped or left the world.
 /// The random stream resumes where the step left it (the process draw was the first word of the
-/// block at counter ctr - 1).  Out of line: the step loop calls it only when the record array is
-/// full.
-/// `rec` is the calling thread's own copy.
+/// block at counter ctr - 1).  Out of line: k_post runs it, and a draining wave's warps while they hold
+/// no track.  `rec` is the calling thread's own copy.
 template<int kMode>
 static __device__ __noinline__ void
 post_record(const WaveParams* Pp, const Deferred* rec) {
@@ -1482,7 +1481,7 @@ post_body(const WaveParams& P) {
     if (threadIdx.x < 8) s_cnt[threadIdx.x] = 0u;
     if (threadIdx.x == 0) s_scen_edges = P.scen_edges;
     __syncthreads();
-    const uint32_t n = min(P.drain->tail, P.def_cap);   // the wave finished those past the array itself
+    const uint32_t n = min(P.drain->tail, P.def_cap);   // none lie past it: a wave hands a track over at most once
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         Deferred d;
         read_record(P.def + i, d);
